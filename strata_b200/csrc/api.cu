@@ -398,7 +398,10 @@ bool use_prefill_down(const strata_moe_layer* L, uint32_t pairs, uint32_t n_grou
 // once), 128 with its deeper weight ring when they are small, 160 (three weight stages) for groups of about 128
 // rows, nearly all of which still fit one tile (c2, 128 rows per expert on average: 2.99 -> 2.96 ms per step).
 uint32_t prefill_ntile(const strata_moe_layer* L, uint64_t pairs, uint64_t n_groups) {
+    if (L->knobs.prefill_ntile == 64 || L->knobs.prefill_ntile == 32) return (uint32_t)L->knobs.prefill_ntile;
     if (L->knobs.prefill_ntile) return L->knobs.prefill_ntile == 128 ? 128u : (L->knobs.prefill_ntile == 160 ? 160u : 192u);
+    if (pairs <= 18u * n_groups) return 32u;
+    if (pairs <= 44u * n_groups) return 64u;
     if (pairs <= 96u * n_groups) return 128u;
     return pairs <= 140u * n_groups ? 160u : 192u;
 }
@@ -480,9 +483,10 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         if (!x_ready) {
             if (spread && !L->knobs.no_spread)
                 launch_rows_to_f16_spread(x_src, spread->dest, spread->k, spread->rows, spread->rows_dev, bound,
-                                          L->d.hidden, L->xg, L->x_rowscale, s);
+                                          L->d.hidden, L->xg, L->x_rowscale, s, L->d.format == STRATA_MOE_FMT_INT4G128);
             else
-                launch_rows_to_f16_bf16(x_src, perm, k_div, bound, L->d.hidden, L->xg, L->x_rowscale, s, pairs_dev);
+                launch_rows_to_f16_bf16(x_src, perm, k_div, bound, L->d.hidden, L->xg, L->x_rowscale, s, pairs_dev,
+                                        L->d.format == STRATA_MOE_FMT_INT4G128);
         }
         mark(ctx, 4);
         PrefillArgs p{};

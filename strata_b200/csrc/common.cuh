@@ -111,12 +111,13 @@ struct DecodeArgs {
 };
 void launch_decode_fp4_gate_up(const DecodeArgs& a, cudaStream_t s);
 void launch_decode_fp4_down(const DecodeArgs& a, cudaStream_t s);
+// int4_order: columns i and i + 4 of every eight are stored side by side (the order INT4 weight words decode in)
 void launch_rows_to_f16_bf16(const __nv_bfloat16* x, const uint32_t* perm, uint32_t k_div, uint32_t rows,
                              uint32_t C, void* hi, float* rowscale, cudaStream_t s,
-                             const uint32_t* rows_dev = nullptr);
+                             const uint32_t* rows_dev = nullptr, bool int4_order = false);
 void launch_rows_to_f16_spread(const __nv_bfloat16* x, const uint32_t* dest, uint32_t k, uint32_t rows,
                                const uint32_t* rows_dev, uint32_t dst_bound, uint32_t C, void* hi, float* rowscale,
-                               cudaStream_t s);
+                               cudaStream_t s, bool int4_order = false);
 void launch_rows_to_f16_f32(const float* x, uint32_t src_rows, uint32_t rows, uint32_t C, void* hi, void* lo,
                             float* rowscale, cudaStream_t s, const uint32_t* rows_dev = nullptr);
 void launch_mx_scale_range(const uint8_t* const* scales, uint32_t n, size_t bytes, uint32_t* emin,
@@ -143,9 +144,10 @@ struct PrefillArgs {
     uint32_t* tile_table;          // scratch of prefill_scratch_bytes()
     uint32_t* status;
     GluParams glu;                 // activation of the gate/up epilogue
-    uint32_t ntile;                // tokens per tile: 128, or anything else for 192 (large groups)
+    uint32_t ntile;                // tokens per tile (16 .. 192); the launch takes the next geometry that holds it
     uint32_t min_rows;             // only groups with at least this many rows get tiles (0 = all)
     uint32_t reuse_tiles;          // down-only launch: the tile list of the preceding gate/up launch is still valid
+    void* act_lo;                  // [pairs_cap, I] or nullptr: the activation travels as a 16-bit hi + lo pair (gate/up writes, down reads both)
     float* act_rowscale_out;       // gate/up: receives 1.0 for every row written (the activation is not pre-scaled), or nullptr
 };
 bool prefill_supported(int fmt, uint32_t H, uint32_t I);
@@ -163,6 +165,7 @@ int launch_prefill_gate_up(const PrefillArgs& a, const void* x16, const float* x
                            uint32_t pairs_cap, const void* wmaps, cudaStream_t s);
 int launch_prefill_down(const PrefillArgs& a, const void* act16, const float* act_rowscale, uint32_t pairs_cap,
                         const void* wmaps, cudaStream_t s);
+int prefill_encode_weight_map_bf16(void* out128, const void* w, uint32_t rows, uint32_t K);
 int prefill_encode_weight_map(void* out128, const void* packed, uint32_t rows, uint32_t K);
 int launch_prefill_bf16(const PrefillArgs& a, const void* x, uint32_t rows, const void* w_gate, const void* w_up,
                         const void* w_down, void* act, uint32_t rows_cap, cudaStream_t s);

@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(256) rows_to_f16_kernel(const void* __restrict
                                                           uint32_t C, __half* __restrict__ hi,
                                                           __half* __restrict__ lo,
                                                           float* __restrict__ rowscale,
-                                                          const uint32_t* __restrict__ rows_dev) {
+                                                          const uint32_t* __restrict__ rows_dev, bool int4_order) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t pos = blockIdx.x * 8u + (threadIdx.x >> 5);
     if (pos >= rows) return;
@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(256) rows_to_f16_kernel(const void* __restrict
     const uint32_t srow = perm ? perm[pos] / k_div : (src_rows ? pos % src_rows : pos);
     if (!SRC_F32) {
         warp_row_to_f16_bf16(static_cast<const __nv_bfloat16*>(src) + (size_t)srow * C, C, hi + (size_t)pos * C,
-                             rowscale + pos);
+                             rowscale + pos, int4_order);
         return;
     }
     float mx = 0.0f;
@@ -414,10 +414,10 @@ __global__ void __launch_bounds__(256) rows_to_f16_kernel(const void* __restrict
 }
 
 void launch_rows_to_f16_bf16(const __nv_bfloat16* x, const uint32_t* perm, uint32_t k_div, uint32_t rows,
-                             uint32_t C, void* hi, float* rowscale, cudaStream_t s, const uint32_t* rows_dev) {
+                             uint32_t C, void* hi, float* rowscale, cudaStream_t s, const uint32_t* rows_dev, bool int4_order) {
     if (rows == 0) return;
     rows_to_f16_kernel<false><<<(rows + 7) / 8, 256, 0, s>>>(x, perm, k_div, 0, rows, C,
-                                                            static_cast<__half*>(hi), nullptr, rowscale, rows_dev);
+                                                            static_cast<__half*>(hi), nullptr, rowscale, rows_dev, int4_order);
     ++g_kernel_launches;
 }
 
@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(256) rows_to_f16_spread_kernel(const __nv_bflo
                                                                  uint32_t rows, const uint32_t* __restrict__ rows_dev,
                                                                  uint32_t dst_bound, uint32_t C,
                                                                  __half* __restrict__ hi,
-                                                                 float* __restrict__ rowscale) {
+                                                                 float* __restrict__ rowscale, bool int4_order) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t t = blockIdx.x * 8u + (threadIdx.x >> 5);
     if (t >= rows) return;
@@ -436,15 +436,15 @@ __global__ void __launch_bounds__(256) rows_to_f16_spread_kernel(const __nv_bflo
     uint32_t mydst = lane < k ? dest[(size_t)t * k + lane] : 0xFFFFFFFFu;
     if (mydst >= dst_bound) mydst = 0xFFFFFFFFu;
     if (__ballot_sync(0xFFFFFFFFu, mydst != 0xFFFFFFFFu) == 0u) return;
-    warp_row_to_f16_bf16_spread(src + (size_t)t * C, C, hi, rowscale, mydst, k);
+    warp_row_to_f16_bf16_spread(src + (size_t)t * C, C, hi, rowscale, mydst, k, int4_order);
 }
 
 void launch_rows_to_f16_spread(const __nv_bfloat16* x, const uint32_t* dest, uint32_t k, uint32_t rows,
                                const uint32_t* rows_dev, uint32_t dst_bound, uint32_t C, void* hi, float* rowscale,
-                               cudaStream_t s) {
+                               cudaStream_t s, bool int4_order) {
     if (rows == 0) return;
     rows_to_f16_spread_kernel<<<(rows + 7) / 8, 256, 0, s>>>(x, dest, k, rows, rows_dev, dst_bound, C,
-                                                            static_cast<__half*>(hi), rowscale);
+                                                            static_cast<__half*>(hi), rowscale, int4_order);
     ++g_kernel_launches;
 }
 
@@ -453,7 +453,7 @@ void launch_rows_to_f16_f32(const float* x, uint32_t src_rows, uint32_t rows, ui
     if (rows == 0) return;
     rows_to_f16_kernel<true><<<(rows + 7) / 8, 256, 0, s>>>(x, nullptr, 1, src_rows, rows, C,
                                                            static_cast<__half*>(hi), static_cast<__half*>(lo),
-                                                           rowscale, rows_dev);
+                                                           rowscale, rows_dev, false);
     ++g_kernel_launches;
 }
 

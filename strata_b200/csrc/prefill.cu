@@ -41,26 +41,28 @@
 
 namespace smoe {
 
-// Tokens per tile: 192 (an expert with up to 192 rows is decoded once; two tensor-memory weight stages) when
-// groups are large, 128 (four weight stages: shorter handshakes for small tiles) when they are small, and 160
-// (three weight stages) for groups of about 128 rows, which a 128-token tile would split in two half the time.
+// Tokens per tile NT: 192 (an expert with up to 192 rows is decoded once) when groups are large, 160 for groups of
+// about 128 rows, 128 and below when they are small.  A stage is kKst columns of K: the roles hand a stage over through
+// barriers, and one hand-over (two waits, the MMAs, two commits) costs the issuing thread 400 to 700 clocks whatever
+// the stage holds, which set the pace of tiles of up to 128 tokens at 64 columns; with 192 or 160 tokens the MMAs of
+// 64 columns take longer than that and tensor memory has no room for more.
 template <int NT>
 struct Geo {
-    static_assert(NT == 128 || NT == 160 || NT == 192, "tile sizes");
+    static_assert(NT == 32 || NT == 64 || NT == 128 || NT == 160 || NT == 192, "tile sizes");
     static constexpr uint32_t kNTile = NT;
-    static constexpr uint32_t kAccCols = 2u * NT;                    // accumulator columns (2 tiles x NT)
-    static constexpr uint32_t kAStages = (512u - 2u * NT) / 64u;     // tensor-memory ring of decoded weight slices
-    static constexpr uint32_t kBStages = NT == 128 ? 8u : 6u;        // activation tiles in flight
-    static constexpr uint32_t kBTile = NT * 64u * 2u;                // bytes of one activation tile stage
+    static constexpr uint32_t kKst = NT <= 128 ? 128u : 64u;
+    static constexpr uint32_t kAccBufs = NT <= 64 ? 2u : 1u;                       // accumulator sets: the epilogue of a tile beside the next main loop
+    static constexpr uint32_t kAccCols = kAccBufs * 2u * NT;                       // accumulator columns (2 tiles x NT each)
+    static constexpr uint32_t kAStageCols = kKst;                                  // tensor-memory columns per A stage: 2 tiles x kKst / 2
+    static constexpr uint32_t kAStages = (512u - kAccCols) / kAStageCols;          // tensor-memory ring of decoded weight slices
+    static constexpr uint32_t kBTile = NT * kKst * 2u;                             // bytes of one activation stage
+    static constexpr uint32_t kBStages = NT <= 64 ? 4u : NT == 128 ? 3u : 6u;      // activation stages in flight
+    static constexpr uint32_t kPkBufs = NT == 32 ? 6u : NT == 64 ? 5u : NT == 128 ? 4u : NT == 160 ? 3u : 2u;
 };
-constexpr uint32_t kMaxAStages = 4;
+constexpr uint32_t kMaxStages = 8;   // barriers per ring
 constexpr uint32_t kMTile = 128;    // output features per tile
-constexpr uint32_t kBK = 64;        // K per pipeline stage (128 bytes of f16 per row)
-// Two rings: decoded weight tiles only have to bridge decode -> MMA (on-chip, short), while
-// the activation tiles arrive by TMA and need enough stages in flight to cover its latency.
-constexpr uint32_t kPkBufs = 2;      // packed-weight staging blocks (256 columns each) in flight
-constexpr uint32_t kAStageCols = 64;                    // tensor-memory columns per A stage: 2 tiles x (kBK / 2)
-constexpr uint32_t kATile = kMTile * kBK * 2;  // 16 KiB
+constexpr uint32_t kBK = 64;        // columns of one 128-byte swizzled row: the unit of TMA boxes and of a decode turn
+constexpr uint32_t kATile = kMTile * kBK * 2;  // 16 KiB: 128 weight rows x 64 columns of 16 bits
 constexpr uint32_t kDecodeWarps = 16;  // each lane decodes 32 columns of one row per stage
 constexpr uint32_t kEpilogueWarps = 8;   // two per tensor-memory lane quarter: even / odd 16-token chunks
 constexpr uint32_t kThreads = (4 + kDecodeWarps + kEpilogueWarps) * 32;
@@ -84,10 +86,10 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
 }
-// Bounded wait: false when the phase did not complete within the spin limit.  Each try_wait
-// carries a suspend-time hint: the hardware parks the thread until the phase completes or the
-// hint expires, so waiting warps (the epilogue during a main loop, producers on a full ring) do
-// not burn issue slots that the decode warps need.
+// Bounded waits: false when the phase did not complete within the limit (about two seconds) or another role raised
+// the abort flag.  Each try_wait carries a suspend-time hint: the hardware parks the thread until the phase completes
+// or the hint expires.  A polling warp takes issue slots from the decode warps of its scheduler, so tighter polling
+// is slower (measured on a 333-token INT4 step: gate/up 1.45 ms as here, 1.69 ms with a four-instruction poll loop).
 constexpr uint32_t kWaitHintNs = 4096;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const volatile uint32_t* abort_flag) {
     const uint32_t addr = smem_u32(bar);
@@ -135,48 +137,52 @@ __device__ __forceinline__ uint32_t umma_idesc_f16(uint32_t n, uint32_t ab_forma
     d |= (kMTile >> 4) << 24;   // M
     return d;
 }
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
+// The four K = 16 MMAs of one 64-column stage, A from tensor memory (lane = row, 32-bit column = two K values, 8
+// columns per MMA).  `never` is a value the compiler cannot see through that is never 0: the branches on it are not
+// taken and only end the basic blocks.  MMAs that follow one another in straight-line code run one after the
+// other without overlap (measured on 512 MMAs of 128 x N x 16, clocks per MMA: A in tensor memory 74 / 106 at
+// N = 128 / 192, A in shared memory 107 / 139); with a branch between them they pipeline (64 / 96 in both forms,
+// the tensor pipe's rate, and 21 at N = 16).
+__device__ __forceinline__ void umma4_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                             uint32_t accumulate, uint32_t never) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n .reg .pred p, t, q;\n .reg .b64 b1, b2, b3;\n .reg .b32 a1, a2, a3;\n"
+        " setp.ne.b32 p, %4, 0;\n setp.eq.b32 t, 0, 0;\n setp.eq.b32 q, %5, 0;\n"
+        " add.u64 b1, %2, 2;\n add.u64 b2, %2, 4;\n add.u64 b3, %2, 6;\n"
+        " add.u32 a1, %1, 8;\n add.u32 a2, %1, 16;\n add.u32 a3, %1, 24;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n @q bra DONE;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n @q bra DONE;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, t;\n @q bra DONE;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, t;\n DONE:\n}" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(never)
         : "memory");
 }
-// Same MMA with the A operand read from tensor memory (lane = row, 32-bit column = two K values).
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
+// The same four MMAs with both operands in shared memory (128-byte swizzled K-major tiles).
+__device__ __forceinline__ void umma4_f16_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                             uint32_t accumulate, uint32_t never) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n .reg .pred p, t, q;\n .reg .b64 a1, a2, a3, b1, b2, b3;\n"
+        " setp.ne.b32 p, %4, 0;\n setp.eq.b32 t, 0, 0;\n setp.eq.b32 q, %5, 0;\n"
+        " add.u64 b1, %2, 2;\n add.u64 b2, %2, 4;\n add.u64 b3, %2, 6;\n"
+        " add.u64 a1, %1, 2;\n add.u64 a2, %1, 4;\n add.u64 a3, %1, 6;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n @q bra DONE;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, t;\n @q bra DONE;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, t;\n @q bra DONE;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, t;\n DONE:\n}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(never)
         : "memory");
 }
-// This thread's 16 words -> 16 consecutive columns of its tensor-memory lane.
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t v[16]) {
+// This thread's 32 words -> 32 consecutive columns of its tensor-memory lane.
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t v[32]) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
-        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t v[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,"
-        "%28,%29,%30,%31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr)
-        : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t v[16]) {
     asm volatile(
@@ -189,13 +195,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t v[16]) {
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-__device__ __forceinline__ uint4 ldg_stream16_c(const void* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::128B.v4.u32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p));
-    return v;
-}
 
 // ------------------------------------------------------------------------------ decoders (f16)
 __device__ __forceinline__ void p_e2m1x8_f16(uint32_t w, uint32_t r[4]) {
@@ -210,44 +209,40 @@ __device__ __forceinline__ uint32_t p_mul_f16x2(uint32_t a, uint32_t b) {
     asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
+__device__ __forceinline__ uint32_t p_fma_f16x2(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
 __device__ __forceinline__ uint32_t p_sub_f16x2(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
-// 8 offset-binary INT4 nibbles -> 4 f16x2 of (q - 8) in natural column order.
-// Byte permutes gather adjacent nibbles and splice in the high byte 0x64: 0x6400 | q is the f16
-// number 1024 + q, and subtracting 1032 leaves q - 8 exactly.
-__device__ __forceinline__ uint32_t p_prmt(uint32_t a, uint32_t b, uint32_t sel) {
+// 8 offset-binary INT4 nibbles -> 4 f16x2 of (q - 8), register i = columns i and i + 4 (the activation rows are stored
+// in that order, see int4_slot).  Four nibbles of a word land in the low bits of 0x6400 halves with one logic
+// instruction each: 0x6400 | q is the f16 number 1024 + q, 0x6400 | 16 q is 1024 + 16 q, and one packed add or
+// multiply-add leaves q - 8 exactly.  9 instructions for 8 weights; the natural column order took 13.
+__device__ __forceinline__ uint32_t p_magic(uint32_t w, uint32_t mask) {
     uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(w), "r"(mask), "r"(0x64006400u));   // (w & mask) | 0x64006400
     return d;
 }
 __device__ __forceinline__ void p_int4x8_f16(uint32_t w, uint32_t r[4]) {
-    const uint32_t lo = w & 0x0F0F0F0Fu;          // nibbles 0,2,4,6
-    const uint32_t hi = (w >> 4) & 0x0F0F0F0Fu;   // nibbles 1,3,5,7
-    const uint32_t n03 = p_prmt(lo, hi, 0x5140u);  // bytes n0,n1,n2,n3
-    const uint32_t n47 = p_prmt(lo, hi, 0x7362u);  // bytes n4,n5,n6,n7
-    const uint32_t k64 = 0x00000064u, k1032 = 0x64086408u;
-    r[0] = p_sub_f16x2(p_prmt(n03, k64, 0x4140u), k1032);
-    r[1] = p_sub_f16x2(p_prmt(n03, k64, 0x4342u), k1032);
-    r[2] = p_sub_f16x2(p_prmt(n47, k64, 0x4140u), k1032);
-    r[3] = p_sub_f16x2(p_prmt(n47, k64, 0x4342u), k1032);
+    const uint32_t w8 = w >> 8;
+    const uint32_t k1032 = 0x64086408u, k16th = 0x2C002C00u, km72 = 0xD480D480u;   // 1032, 1 / 16, -72
+    r[0] = p_sub_f16x2(p_magic(w, 0x000F000Fu), k1032);
+    r[1] = p_fma_f16x2(p_magic(w, 0x00F000F0u), k16th, km72);
+    r[2] = p_sub_f16x2(p_magic(w8, 0x000F000Fu), k1032);
+    r[3] = p_fma_f16x2(p_magic(w8, 0x00F000F0u), k16th, km72);
 }
-
-// One row's 16 packed bytes (32 columns) -> 4 x 16-byte f16 chunks, scaled.
-// m[c] multiplies chunk c (8 columns).
-template <int FMT>
-__device__ __forceinline__ void decode16(const uint4& p, const uint32_t m[4], uint4 out[4]) {
-    const uint32_t w[4] = {p.x, p.y, p.z, p.w};
+// Pins 32 computed registers before whatever follows.
+__device__ __forceinline__ void keep32(const uint32_t v[32]) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        uint32_t r[4];
-        if (FMT == STRATA_MOE_FMT_INT4G128) p_int4x8_f16(w[c], r);
-        else p_e2m1x8_f16(w[c], r);
-        out[c] = make_uint4(p_mul_f16x2(r[0], m[c]), p_mul_f16x2(r[1], m[c]), p_mul_f16x2(r[2], m[c]),
-                            p_mul_f16x2(r[3], m[c]));
-    }
+    for (int i = 0; i < 32; i += 16)
+        asm volatile("" ::"r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3]), "r"(v[i + 4]), "r"(v[i + 5]), "r"(v[i + 6]),
+                     "r"(v[i + 7]), "r"(v[i + 8]), "r"(v[i + 9]), "r"(v[i + 10]), "r"(v[i + 11]), "r"(v[i + 12]), "r"(v[i + 13]),
+                     "r"(v[i + 14]), "r"(v[i + 15]));
 }
 
 // Activation tensor maps with boxes of 16, 32, 64 and 128 rows: a tile with few valid rows
@@ -264,20 +259,19 @@ struct TileInfo {
 template <int NT>
 struct __align__(1024) PrefillSmem {
     // 4-bit formats: packed staging [buffer][gate/down, up][kPkTile], then the activation ring.
-    // BF16 weights: w and b together are one arena that the kernel cuts into four stages of A tiles
-    // [stage][gate/down, up][kATile] followed by the activation stages that still fit.
-    uint8_t w[kPkBufs][2][kPkTile];
-    uint8_t b[Geo<NT>::kBStages][Geo<NT>::kBTile];   // activation tile
-    uint64_t full_a[kMaxAStages], empty_a[kMaxAStages], full_b[Geo<NT>::kBStages], empty_b[Geo<NT>::kBStages];
-    uint64_t pk_full[kPkBufs], pk_empty[kPkBufs];
-    uint64_t acc_full, acc_empty;
+    // BF16 weights: w and b together are one arena that the kernel cuts into stages of A tiles
+    // [stage][gate/down, up][64-column slab][kATile] followed by the activation stages that still fit.
+    uint8_t w[Geo<NT>::kPkBufs][2][kPkTile];
+    uint8_t b[Geo<NT>::kBStages][Geo<NT>::kBTile];   // activation stages: [slab of 64 columns][NT rows][128 B]
+    uint64_t full_a[kMaxStages], empty_a[kMaxStages], full_b[kMaxStages], empty_b[kMaxStages];
+    uint64_t pk_full[Geo<NT>::kPkBufs], pk_empty[Geo<NT>::kPkBufs];
+    uint64_t acc_full[2], acc_empty[2];
     uint32_t tmem_base;
     uint32_t abort_flag;
 };
 
-__device__ __forceinline__ bool tile_lookup(const uint32_t* table, uint32_t tile, uint32_t m_tiles, TileInfo& t,
-                                            uint32_t tile_feat = kMTile) {
-    const uint32_t total = table[0] * m_tiles;
+__device__ __forceinline__ bool tile_lookup(const uint32_t* table, uint32_t tile, uint32_t total, uint32_t m_tiles,
+                                            TileInfo& t, uint32_t tile_feat) {
     if (tile >= total) return false;
     const uint32_t j = tile / m_tiles;
     t.g = table[4 + 3 * j];
@@ -287,59 +281,102 @@ __device__ __forceinline__ bool tile_lookup(const uint32_t* table, uint32_t tile
     return true;
 }
 
+// Position of an activation column in the rows the INT4 tiles multiply: the decoder leaves the nibbles of a weight
+// word as the pairs (0,4) (1,5) (2,6) (3,7), so columns i and i + 4 of every eight lie side by side.
+__device__ __forceinline__ uint32_t int4_slot(uint32_t c) {
+    const uint32_t p = c & 7u;
+    return (c & ~7u) | ((p & 3u) << 1) | (p >> 2);
+}
+
+// After a wait on copies that an aborting producer issued but nobody may consume: give each a bounded chance to land.
+__device__ __forceinline__ void drain_copies(uint64_t* full, uint32_t issued, uint32_t stages) {
+    const uint32_t pending = issued < stages ? issued : stages;
+    for (uint32_t q = 0; q < pending; ++q) {
+        const uint32_t j = issued - 1u - q;
+        const uint32_t addr = smem_u32(&full[j % stages]);
+        for (uint32_t spin = 0; spin < (1u << 16); ++spin) {
+            uint32_t done;
+            asm volatile(
+                "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                " selp.u32 %0, 1, 0, p;\n}"
+                : "=r"(done)
+                : "r"(addr), "r"((j / stages) & 1u)
+                : "memory");
+            if (done) break;
+        }
+    }
+}
+
+// A position in a ring of N stages and the parity its barriers have there.
+template <uint32_t N>
+struct Ring {
+    uint32_t i = 0, ph = 0;
+    __device__ __forceinline__ void next(uint32_t step = 1u) {
+        i += step;
+        if (i >= N) { i -= N; ph ^= 1u; }
+    }
+};
+
 // MODE 0: gate + up tiles of the same 128 features, SwiGLU, act (16-bit) out.  K = H, features over I.
 // MODE 1: one down tile (128 features), y (fp32) out.                          K = I, features over H.
 // MODE 2: two adjacent down tiles (256 features) against the same activation tile -- halves the
 //         shared-memory traffic per MMA of MODE 1; needs H % 256 == 0.
 // DUAL (two weight tiles and two accumulators per activation tile) = MODE 0 or 2.
-template <int FMT, int MODE, int NT>
+// SPLIT: the activation is a 16-bit hi + lo pair; a stage holds the hi rows and behind them the lo rows, one MMA
+// multiplies both and the epilogue adds the two halves of the accumulator columns, so a tile holds NT / 2 tokens.
+template <int FMT, int MODE, int NT, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
-prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__ CUtensorMap map_a0,
-                   const __grid_constant__ CUtensorMap map_a1, PrefillArgs a, const float* __restrict__ rowscale,
-                   void* __restrict__ act_out_v, const CUtensorMap* __restrict__ wmaps /* [3][n_groups] */) {
+prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__ BMaps maps_lo,
+                   const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CUtensorMap map_a1, PrefillArgs a,
+                   const float* __restrict__ rowscale, void* __restrict__ act_out_v,
+                   const CUtensorMap* __restrict__ wmaps /* [3][n_groups] */) {
     extern __shared__ uint8_t smem_raw[];
+    using G = Geo<NT>;
     PrefillSmem<NT>& S =
         *reinterpret_cast<PrefillSmem<NT>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    constexpr uint32_t kNTile = Geo<NT>::kNTile, kAccCols = Geo<NT>::kAccCols, kAStages = Geo<NT>::kAStages;
-    // BF16 weights arrive as ready A tiles by TMA: the staging blocks and the activation ring are re-cut into four
-    // stages of weight tiles (two stages left a K-step waiting for a whole memory round trip: 112 K-steps of a
-    // router projection took 0.6 us each) and as many activation stages as the rest holds (4 at 128 tokens, 3 at 192)
-    constexpr bool BF = FMT == kFmtBf16W;
-    constexpr uint32_t kBfAStages = 4;
-    constexpr uint32_t kArena = kPkBufs * 2u * kPkTile + Geo<NT>::kBStages * Geo<NT>::kBTile;
-    constexpr uint32_t kBStages = BF ? (kArena - kBfAStages * 2u * kATile) / Geo<NT>::kBTile : Geo<NT>::kBStages;
-    static_assert(kBfAStages <= kMaxAStages && kBStages >= 2u && kBStages <= Geo<NT>::kBStages, "ring geometry");
-    static_assert(offsetof(PrefillSmem<NT>, b) == kPkBufs * 2u * kPkTile, "staging blocks and activation ring form one arena");
-    uint8_t* const arena = &S.w[0][0][0];
-    auto a_tile = [&](uint32_t stage, uint32_t which) -> uint8_t* { return arena + (stage * 2u + which) * kATile; };
-    auto b_tile = [&](uint32_t stage) -> uint8_t* {
-        return BF ? arena + kBfAStages * 2u * kATile + stage * Geo<NT>::kBTile : S.b[stage];
-    };
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     constexpr bool DUAL = MODE != 1;
     constexpr bool GU = MODE == 0;
+    constexpr bool BF = FMT == kFmtBf16W;
+    constexpr uint32_t kKst = G::kKst, kSlabs = kKst / kBK;
+    constexpr uint32_t kAccCols = G::kAccCols, kAccBufs = G::kAccBufs, kPkBufs = G::kPkBufs;
+    // BF16 weights arrive as ready A tiles by TMA: the staging blocks and the activation ring are re-cut into stages
+    // of weight tiles and as many activation stages as the rest holds
+    constexpr uint32_t kArena = kPkBufs * 2u * kPkTile + G::kBStages * G::kBTile;
+    constexpr uint32_t kBfATile = kSlabs * kATile;                       // one weight tile of a stage
+    constexpr uint32_t kBfAStage = (DUAL ? 2u : 1u) * kBfATile;
+    constexpr uint32_t kBfAWant = (NT <= 64 ? 192u : 128u) * 1024u / kBfAStage;
+    constexpr uint32_t kBfAStages = kBfAWant < kMaxStages ? kBfAWant : kMaxStages;
+    constexpr uint32_t kBfBFit = (kArena - kBfAStages * kBfAStage) / G::kBTile;
+    constexpr uint32_t kAStages = BF ? kBfAStages : G::kAStages;
+    constexpr uint32_t kBStages = BF ? (kBfBFit < kMaxStages ? kBfBFit : kMaxStages) : G::kBStages;
+    static_assert(kAStages >= 2u && kAStages <= kMaxStages && kBStages >= 2u && kBStages <= kMaxStages, "ring geometry");
+    static_assert(offsetof(PrefillSmem<NT>, b) == kPkBufs * 2u * kPkTile, "staging blocks and activation ring form one arena");
+    uint8_t* const arena = &S.w[0][0][0];
+    uint8_t* const b_base = BF ? arena + kBfAStages * kBfAStage : &S.b[0][0];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     constexpr uint32_t kTileFeat = MODE == 2 ? 2u * kMTile : kMTile;  // features per tile
     constexpr uint32_t kSecond = MODE == 2 ? kMTile : 0u;              // row offset of the second weight tile
     const uint32_t K = GU ? a.H : a.I;
     const uint32_t R = GU ? a.I : a.H;
     const uint32_t m_tiles = R / kTileFeat;
-    const uint32_t k_stages = K / kBK;
+    const uint32_t k_stages = K / kKst;
     volatile uint32_t* abort_flag = &S.abort_flag;
-    if (a.tile_table[0] == 0u) return;   // nothing listed (mixed dispatch with no large group): leave before any set-up
+    const uint32_t total = a.tile_table[0] * m_tiles;
+    if (total == 0u) return;   // nothing listed (mixed dispatch with no large group): leave before any set-up
 
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < kMaxAStages; ++s) {
-            // one arrival per producer warp, or one TMA transaction group for BF16 weights
-            // (a stage is decoded by half of the decode warps: the other half works on the next one)
-            mbar_init(&S.full_a[s], FMT == kFmtBf16W ? 1u : (DUAL ? kDecodeWarps / 2u : kDecodeWarps / 4u));
+        for (uint32_t s = 0; s < kMaxStages; ++s) {
+            // one arrival per decode warp that fills part of the stage (a 64-column stage is decoded by half of the
+            // decode warps, the other half works on the next one), or one TMA transaction group for BF16 weights
+            mbar_init(&S.full_a[s], BF ? 1u : kDecodeWarps / (kSlabs == 1u ? 2u : 1u) / (DUAL ? 1u : 2u));
             mbar_init(&S.empty_a[s], DUAL ? 2u : 1u);   // one commit per MMA issuer
-        }
-        for (uint32_t s = 0; s < Geo<NT>::kBStages; ++s) {
             mbar_init(&S.full_b[s], 1);
             mbar_init(&S.empty_b[s], DUAL ? 2u : 1u);
         }
-        mbar_init(&S.acc_full, DUAL ? 2u : 1u);
-        mbar_init(&S.acc_empty, kEpilogueWarps);  // one arrival per epilogue warp
+        for (uint32_t i = 0; i < 2u; ++i) {
+            mbar_init(&S.acc_full[i], DUAL ? 2u : 1u);
+            mbar_init(&S.acc_empty[i], kEpilogueWarps);  // one arrival per epilogue warp
+        }
         for (uint32_t i = 0; i < kPkBufs; ++i) {
             mbar_init(&S.pk_full[i], 1);
             mbar_init(&S.pk_empty[i], DUAL ? kDecodeWarps : kDecodeWarps / 2u);
@@ -357,314 +394,329 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = S.tmem_base;
+    // rows of the box that fetches n activation rows (boxes of 16, 32, 64 and 128 rows exist)
+    auto box_of = [](uint32_t n) { return n <= 16u ? 0u : (n <= 32u ? 1u : (n <= 64u ? 2u : 3u)); };
 
     if (warp == 0) {
-        // ---------------------------------------------------------------- TMA producer
+        // ---------------------------------------------------------------- TMA producer: activation rows
         if (lane == 0) {
-            uint32_t it = 0;
+            uint32_t issued = 0;
+            Ring<kBStages> rb;
             bool ok = true;
-            for (uint32_t tile = blockIdx.x; ok; tile += gridDim.x) {
-                TileInfo t;
-                if (!tile_lookup(a.tile_table, tile, m_tiles, t, kTileFeat)) break;
-                for (uint32_t ks = 0; ks < k_stages; ++ks, ++it) {
-                    const uint32_t s = it % kBStages, ph = (it / kBStages) & 1u;
-                    if (!mbar_wait(&S.empty_b[s], ph ^ 1u, abort_flag)) { ok = false; break; }
-                    const uint32_t bsel = t.n <= 16u ? 0u : (t.n <= 32u ? 1u : (t.n <= 64u ? 2u : 3u));
-                    const bool tail = t.n > 128u;   // rows from 128 on arrive as a second box: 64 rows (192-token tile) or 32
-                    constexpr uint32_t kTailSel = NT == 192 ? 2u : 1u, kTailRows = 16u << kTailSel;
-                    mbar_arrive_expect_tx(&S.full_b[s], ((16u << bsel) + (tail ? kTailRows : 0u)) * kBK * 2u);
-                    tma_load_2d(b_tile(s), &maps_b.m[bsel], ks * kBK, t.row0, &S.full_b[s]);
-                    if (tail) tma_load_2d(b_tile(s) + 128u * kBK * 2u, &maps_b.m[kTailSel], ks * kBK, t.row0 + 128u, &S.full_b[s]);
-                    if (FMT == kFmtBf16W) {
-                        const uint32_t sa = it % kBfAStages, pa = (it / kBfAStages) & 1u;
-                        if (!mbar_wait(&S.empty_a[sa], pa ^ 1u, abort_flag)) { ok = false; break; }
-                        mbar_arrive_expect_tx(&S.full_a[sa], DUAL ? 2u * kATile : kATile);
-                        tma_load_2d(a_tile(sa, 0), &map_a0, ks * kBK, t.m0, &S.full_a[sa]);
-                        if (DUAL) tma_load_2d(a_tile(sa, 1), &map_a1, ks * kBK, t.m0 + kSecond, &S.full_a[sa]);
+            TileInfo t, tn;
+            bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat);
+            for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
+                const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
+                const uint32_t bsel = box_of(t.n), rows = 16u << bsel;
+                const bool tail = NT > 128 && t.n > 128u;   // rows from 128 on arrive as a second box: 64 rows (192-token tile) or 32
+                constexpr uint32_t kTailSel = NT == 192 ? 2u : 1u, kTailRows = 16u << kTailSel;
+                const uint32_t bytes = (rows * (SPLIT ? 2u : 1u) + (tail ? kTailRows : 0u)) * kKst * 2u;
+                for (uint32_t ks = 0; ks < k_stages; ++ks) {
+                    if (!mbar_wait(&S.empty_b[rb.i], rb.ph ^ 1u, abort_flag)) { ok = false; break; }
+                    mbar_arrive_expect_tx(&S.full_b[rb.i], bytes);
+                    uint8_t* dst = b_base + rb.i * G::kBTile;
+#pragma unroll
+                    for (uint32_t h = 0; h < kSlabs; ++h) {
+                        const uint32_t x = ks * kKst + h * kBK;
+                        tma_load_2d(dst + h * (NT * 128u), &maps_b.m[bsel], x, t.row0, &S.full_b[rb.i]);
+                        if (SPLIT) tma_load_2d(dst + h * (NT * 128u) + rows * 128u, &maps_lo.m[bsel], x, t.row0, &S.full_b[rb.i]);
+                        if (tail) tma_load_2d(dst + h * (NT * 128u) + 128u * 128u, &maps_b.m[kTailSel], x, t.row0 + 128u, &S.full_b[rb.i]);
                     }
+                    ++issued;
+                    rb.next();
                 }
+                t = tn;
+                have = hn;
             }
             if (!ok) { *abort_flag = 1; atomicOr(a.status, kStatusWaitTimeout); }
-            if (*abort_flag) {
-                // copies issued but possibly not consumed: give each a bounded chance to land
-                // before the CTA's shared memory is released
-                const uint32_t pending = it < kBStages ? it : kBStages;
-                for (uint32_t q = 0; q < pending; ++q) {
-                    const uint32_t j = it - 1u - q;
-                    const uint32_t addr = smem_u32(&S.full_b[j % kBStages]);
-                    for (uint32_t spin = 0; spin < (1u << 16); ++spin) {
-                        uint32_t done;
-                        asm volatile(
-                            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                            " selp.u32 %0, 1, 0, p;\n}"
-                            : "=r"(done)
-                            : "r"(addr), "r"((j / kBStages) & 1u)
-                            : "memory");
-                        if (done) break;
-                    }
-                }
-            }
+            if (*abort_flag) drain_copies(S.full_b, issued, kBStages);
         }
     } else if (warp == 1 || warp == 3) {
         // ---------------------------------------------------------------- MMA issuers
         const uint32_t mi = warp == 3 ? 1u : 0u;   // which weight tile of the stage this thread feeds
         if (lane == 0 && (DUAL || mi == 0u)) {
-            uint32_t it = 0, tcount = 0;
+            Ring<kAStages> ra;
+            Ring<kBStages> rb;
+            Ring<kAccBufs> rc;
+            const uint64_t bdesc0 = umma_desc_sw128(smem_u32(b_base));
+            const uint64_t adesc0 = umma_desc_sw128(smem_u32(arena) + mi * kBfATile);
             bool ok = true;
-            for (uint32_t tile = blockIdx.x; ok; tile += gridDim.x, ++tcount) {
-                TileInfo t;
-                if (!tile_lookup(a.tile_table, tile, m_tiles, t, kTileFeat)) break;
-                if (!mbar_wait(&S.acc_empty, (tcount & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+            TileInfo t, tn;
+            bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat);
+            for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
+                const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
+                if (!mbar_wait(&S.acc_empty[rc.i], rc.ph ^ 1u, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t n = (t.n + 15u) & ~15u;
-                const uint32_t idesc = umma_idesc_f16(n, FMT == kFmtBf16W ? 1u : 0u);
-                const uint32_t d = tmem_base + mi * kNTile;
-                constexpr uint32_t kRing = BF ? kBfAStages : kAStages;
-                for (uint32_t ks = 0; ks < k_stages; ++ks, ++it) {
-                    const uint32_t sa = it % kRing, pa = (it / kRing) & 1u;
-                    const uint32_t sb = it % kBStages, pb = (it / kBStages) & 1u;
-                    if (!mbar_wait(&S.full_a[sa], pa, abort_flag) || !mbar_wait(&S.full_b[sb], pb, abort_flag)) {
+                const uint32_t n = SPLIT ? 32u << box_of(t.n) : (t.n + 15u) & ~15u;
+                const uint32_t idesc = umma_idesc_f16(n, BF ? 1u : 0u);
+                const uint32_t d = tmem_base + rc.i * (2u * NT) + mi * NT;
+                for (uint32_t ks = 0; ks < k_stages; ++ks) {
+                    if (!mbar_wait(&S.full_a[ra.i], ra.ph, abort_flag) || !mbar_wait(&S.full_b[rb.i], rb.ph, abort_flag)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t b = smem_u32(b_tile(sb));
-                    if (FMT == kFmtBf16W) {
-                        const uint32_t a0 = smem_u32(a_tile(sa, mi));
+                    const uint64_t bdesc = bdesc0 + rb.i * (G::kBTile >> 4);
+                    const uint64_t adesc = adesc0 + ra.i * (kBfAStage >> 4);
+                    const uint32_t ta = tmem_base + kAccCols + ra.i * G::kAStageCols + mi * (kKst / 2u);
 #pragma unroll
-                        for (uint32_t kk = 0; kk < kBK / 16u; ++kk) {
-                            umma_f16(d, umma_desc_sw128(a0 + kk * 32u), umma_desc_sw128(b + kk * 32u), idesc,
-                                     (ks | kk) ? 1u : 0u);
-                        }
-                    } else {
-                        // decoded weights of this stage: columns [ta, ta + 32) tile 0, [ta + 32, ta + 64) tile 1;
-                        // a K = 16 slice is 8 columns
-                        const uint32_t ta = tmem_base + kAccCols + sa * kAStageCols + mi * (kBK / 2u);
-#pragma unroll
-                        for (uint32_t kk = 0; kk < kBK / 16u; ++kk) {
-                            umma_f16_ts(d, ta + kk * 8u, umma_desc_sw128(b + kk * 32u), idesc, (ks | kk) ? 1u : 0u);
-                        }
+                    for (uint32_t h = 0; h < kSlabs; ++h) {
+                        if (BF) umma4_f16_ss(d, adesc + h * (kATile >> 4), bdesc + h * (NT * 128u >> 4), idesc, h ? 1u : ks, a.H);
+                        else umma4_f16_ts(d, ta + h * (kBK / 2u), bdesc + h * (NT * 128u >> 4), idesc, h ? 1u : ks, a.H);
                     }
-                    umma_commit(&S.empty_a[sa]);  // a stage is free once both issuers' MMAs have read it
-                    umma_commit(&S.empty_b[sb]);
+                    umma_commit(&S.empty_a[ra.i]);  // a stage is free once both issuers' MMAs have read it
+                    umma_commit(&S.empty_b[rb.i]);
+                    ra.next();
+                    rb.next();
                 }
-                if (ok) umma_commit(&S.acc_full);
+                if (ok) umma_commit(&S.acc_full[rc.i]);
+                rc.next();
+                t = tn;
+                have = hn;
             }
             if (!ok) { *abort_flag = 1; atomicOr(a.status, kStatusWaitTimeout); }
         }
     } else if (warp == 2) {
-        // ---------------------------------------------------------------- packed-weight TMA producer
-        if (lane == 0 && FMT != kFmtBf16W) {
-            const uint32_t blocks = (K + kPkCols - 1u) / kPkCols;
-            uint32_t bi = 0;
+        // ---------------------------------------------------------------- TMA producer: weights
+        if (lane == 0) {
+            uint32_t issued = 0;
             bool ok = true;
-            for (uint32_t tile = blockIdx.x; ok; tile += gridDim.x) {
-                TileInfo t;
-                if (!tile_lookup(a.tile_table, tile, m_tiles, t, kTileFeat)) break;
-                const CUtensorMap* m0 = wmaps + (GU ? 0u : 2u) * a.n_groups + t.g;
-                const CUtensorMap* m1 = wmaps + (GU ? 1u : 2u) * a.n_groups + t.g;
-                for (uint32_t q = 0; q < blocks; ++q, ++bi) {
-                    const uint32_t pb = bi % kPkBufs, ph = (bi / kPkBufs) & 1u;
-                    if (!mbar_wait(&S.pk_empty[pb], ph ^ 1u, abort_flag)) { ok = false; break; }
-                    mbar_arrive_expect_tx(&S.pk_full[pb], DUAL ? 2u * kPkTile : kPkTile);
-                    tma_load_2d(S.w[pb][0], m0, q * (kPkCols / 2u), t.m0, &S.pk_full[pb]);
-                    if (DUAL) tma_load_2d(S.w[pb][1], m1, q * (kPkCols / 2u), t.m0 + kSecond, &S.pk_full[pb]);
+            TileInfo t, tn;
+            Ring<BF ? kAStages : kPkBufs> rw;
+            const uint32_t blocks = BF ? k_stages : (K + kPkCols - 1u) / kPkCols;
+            bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat);
+            for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
+                const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
+                // BF16: a map per expert when there is a table, else the one matrix pair of the launch
+                const CUtensorMap* m0 = BF && !wmaps ? &map_a0 : wmaps + (GU ? 0u : 2u) * a.n_groups + t.g;
+                const CUtensorMap* m1 = BF && !wmaps ? &map_a1 : wmaps + (GU ? 1u : 2u) * a.n_groups + t.g;
+                for (uint32_t q = 0; q < blocks; ++q) {
+                    uint64_t* full = BF ? &S.full_a[rw.i] : &S.pk_full[rw.i % kPkBufs];
+                    uint64_t* empty = BF ? &S.empty_a[rw.i] : &S.pk_empty[rw.i % kPkBufs];
+                    if (!mbar_wait(empty, rw.ph ^ 1u, abort_flag)) { ok = false; break; }
+                    if (BF) {
+                        mbar_arrive_expect_tx(full, kBfAStage);
+                        uint8_t* dst = arena + rw.i * kBfAStage;
+#pragma unroll
+                        for (uint32_t h = 0; h < kSlabs; ++h) {
+                            tma_load_2d(dst + h * kATile, m0, q * kKst + h * kBK, t.m0, full);
+                            if (DUAL) tma_load_2d(dst + kBfATile + h * kATile, m1, q * kKst + h * kBK, t.m0 + kSecond, full);
+                        }
+                    } else {
+                        mbar_arrive_expect_tx(full, DUAL ? 2u * kPkTile : kPkTile);
+                        uint8_t* dst = arena + rw.i * (2u * kPkTile);
+                        tma_load_2d(dst, m0, q * (kPkCols / 2u), t.m0, full);
+                        if (DUAL) tma_load_2d(dst + kPkTile, m1, q * (kPkCols / 2u), t.m0 + kSecond, full);
+                    }
+                    ++issued;
+                    rw.next();
                 }
+                t = tn;
+                have = hn;
             }
             if (!ok) { *abort_flag = 1; atomicOr(a.status, kStatusWaitTimeout); }
             if (*abort_flag) {
-                for (uint32_t q = 0; q < (bi < kPkBufs ? bi : kPkBufs); ++q) {
-                    const uint32_t j = bi - 1u - q;
-                    const uint32_t addr = smem_u32(&S.pk_full[j % kPkBufs]);
-                    for (uint32_t spin = 0; spin < (1u << 16); ++spin) {
-                        uint32_t done;
-                        asm volatile(
-                            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                            " selp.u32 %0, 1, 0, p;\n}"
-                            : "=r"(done)
-                            : "r"(addr), "r"((j / kPkBufs) & 1u)
-                            : "memory");
-                        if (done) break;
-                    }
-                }
+                if (BF) drain_copies(S.full_a, issued, kAStages);
+                else drain_copies(S.pk_full, issued, kPkBufs);
             }
         }
-    } else if (warp < kFirstEpilogueWarp && FMT == kFmtBf16W) {
+    } else if (warp < kFirstEpilogueWarp && BF) {
         // BF16 weights need no decode: the TMA producer loads their tiles
     } else if (warp < kFirstEpilogueWarp) {
-        // ---------------------------------------------------------------- weight producers
-        // A warp can only write the tensor-memory lanes 32 * (warp % 4) .. + 31, and a lane holds one
-        // weight row: lane i of a decode warp owns row 32 * (warp % 4) + i of one weight tile and
-        // decodes all 64 of its columns in EVERY OTHER stage.  The four decode warps that share a lane
-        // quarter split into tile 0 / tile 1 and even / odd stages: a warp's chain for one stage (wait for
-        // the stage's columns, store, wait for the store, arrive) takes longer than the MMAs of a stage, and
-        // with every warp in every stage that chain set the pace of the whole pipeline; now two stages'
-        // chains overlap.  (32 consecutive rows reading the same swizzled 16-byte chunk index are free of
-        // bank conflicts.)  With one weight tile per stage (MODE 1) only the tile-0 warps work.
+        // ---------------------------------------------------------------- weight decoders
+        // A warp can only write the tensor-memory lanes 32 * (warp % 4) .. + 31, and a lane holds one weight row:
+        // lane i of a decode warp owns row 32 * (warp % 4) + i of one weight tile.  The four decode warps that share
+        // a lane quarter split into tile 0 / tile 1 and even / odd 64-column slabs: a warp takes every other slab,
+        // decodes it into 32 registers BEFORE it waits for the slab's place in tensor memory (the decode then
+        // overlaps the MMAs that still read that place), stores, and hands over.  (32 consecutive rows reading the
+        // same swizzled 16-byte chunk index are free of bank conflicts.)  With one weight tile per stage (MODE 1)
+        // only the tile-0 warps work.
         const uint32_t wd = warp - kFirstDecodeWarp;
         const uint32_t which = DUAL ? (wd >> 3) : 0u;
-        const uint32_t parity = (wd >> 2) & 1u;
+        const uint32_t sub = (wd >> 2) & 1u;
         const uint32_t arow = (warp & 3u) * 32u + lane;
-        constexpr uint32_t CH = 2u;  // 16-byte packed chunks per thread per stage
-        const bool active = DUAL || wd < kDecodeWarps / 2u;
-        // this thread's first column in an A stage: tile, then 16 columns (32 K values) per chunk
-        const uint32_t a_col = kAccCols + which * (kBK / 2u);
-        const uint32_t a_lane_addr = tmem_base + (((warp & 3u) * 32u) << 16) + a_col;
-        uint32_t it = 0, bi = 0;
-        bool ok = true;
-        for (uint32_t tile = blockIdx.x; ok && active; tile += gridDim.x) {
-            TileInfo t;
-            if (!tile_lookup(a.tile_table, tile, m_tiles, t, kTileFeat)) break;
-            const WeightTable& wt = GU ? (which ? a.up : a.gate) : a.down;
-            const uint32_t row = t.m0 + arow + which * kSecond;
-            const uint8_t* srow = wt.scales[t.g];
-            int32_t mx_off = 0;
-            if (FMT == STRATA_MOE_FMT_MXFP4) {
-                srow += (size_t)row * (K / 32u);
-                mx_off = 2 - (int32_t)wt.emin[t.g];
-            } else if (FMT == STRATA_MOE_FMT_NVFP4) {
-                srow += (size_t)row * (K / 16u);
-            } else {
-                srow += (size_t)row * (K / 128u) * 2u;
-            }
-            // Scale bytes of one 256-column block of this thread's row, fetched one block ahead:
-            // MXFP4 8 bytes, NVFP4 16 bytes, INT4 two BF16 values.
-            // Vector loads need the row's scale bytes aligned to the vector: true when K % 256 == 0
-            // (then every row holds a whole number of blocks); otherwise fall back to narrow loads.
-            const bool whole_blocks = (K % kPkCols) == 0u;
-            auto load_scales = [&](uint32_t q) -> uint4 {
-                const uint32_t nblk = (K + kPkCols - 1u) / kPkCols;
-                q = q < nblk ? q : nblk - 1u;
-                uint4 v = make_uint4(0, 0, 0, 0);
-                if (FMT == STRATA_MOE_FMT_MXFP4) {          // 8 bytes per block, rows 4-byte aligned
-                    if (whole_blocks) {
-                        const uint2 w = __ldg(reinterpret_cast<const uint2*>(srow + q * 8u));
-                        v.x = w.x; v.y = w.y;
-                    } else {
-                        v.x = __ldg(reinterpret_cast<const uint32_t*>(srow + q * 8u));
-                        if ((q + 1u) * 8u <= K / 32u) v.y = __ldg(reinterpret_cast<const uint32_t*>(srow + q * 8u + 4u));
-                    }
-                } else if (FMT == STRATA_MOE_FMT_NVFP4) {   // 16 bytes per block, rows 8-byte aligned
-                    if (whole_blocks) {
-                        v = __ldg(reinterpret_cast<const uint4*>(srow + q * 16u));
-                    } else {
-                        const uint2 w = __ldg(reinterpret_cast<const uint2*>(srow + q * 16u));
-                        v.x = w.x; v.y = w.y;
-                        if ((q + 1u) * 16u <= K / 16u) {
-                            const uint2 w2 = __ldg(reinterpret_cast<const uint2*>(srow + q * 16u + 8u));
-                            v.z = w2.x; v.w = w2.y;
-                        }
-                    }
-                } else {                                     // two BF16 per block, rows 2-byte aligned
-                    if (whole_blocks) {
-                        v.x = __ldg(reinterpret_cast<const uint32_t*>(srow + q * 4u));
-                    } else {
-                        v.x = __ldg(reinterpret_cast<const unsigned short*>(srow + q * 4u));
-                        if ((q + 1u) * 2u <= K / 128u)
-                            v.x |= (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(srow + q * 4u + 2u)) << 16;
+        const uint32_t a_lane = tmem_base + (((warp & 3u) * 32u) << 16) + kAccCols + which * (kKst / 2u) +
+                                (kSlabs == 2u ? sub * (kBK / 2u) : 0u);
+        const uint32_t off0 = ((2u * sub) ^ (arow & 7u)) << 4, off1 = off0 ^ 16u;   // this warp's first slab; the other is ^ 64
+        const WeightTable& wt = GU ? (which ? a.up : a.gate) : a.down;
+        const uint32_t blocks = (K + kPkCols - 1u) / kPkCols, k_slabs = K / kBK;
+        const size_t scale_row = FMT == STRATA_MOE_FMT_MXFP4 ? K / 32u : FMT == STRATA_MOE_FMT_NVFP4 ? K / 16u : K / 128u * 2u;
+        // Scale bytes of one 256-column block of a row: MXFP4 8 bytes, NVFP4 16 bytes, INT4 two BF16 values.  Vector
+        // loads need rows of whole blocks (K % 256 == 0); the last block of other rows takes narrow loads.
+        const bool whole_blocks = (K % kPkCols) == 0u;
+        auto load_scales = [&](const uint8_t* srow, uint32_t q) -> uint4 {
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (FMT == STRATA_MOE_FMT_MXFP4) {          // 8 bytes per block, rows 4-byte aligned
+                if (whole_blocks) {
+                    const uint2 w = __ldg(reinterpret_cast<const uint2*>(srow + q * 8u));
+                    v.x = w.x; v.y = w.y;
+                } else {
+                    v.x = __ldg(reinterpret_cast<const uint32_t*>(srow + q * 8u));
+                    if ((q + 1u) * 8u <= K / 32u) v.y = __ldg(reinterpret_cast<const uint32_t*>(srow + q * 8u + 4u));
+                }
+            } else if (FMT == STRATA_MOE_FMT_NVFP4) {   // 16 bytes per block, rows 8-byte aligned
+                if (whole_blocks) {
+                    v = __ldg(reinterpret_cast<const uint4*>(srow + q * 16u));
+                } else {
+                    const uint2 w = __ldg(reinterpret_cast<const uint2*>(srow + q * 16u));
+                    v.x = w.x; v.y = w.y;
+                    if ((q + 1u) * 16u <= K / 16u) {
+                        const uint2 w2 = __ldg(reinterpret_cast<const uint2*>(srow + q * 16u + 8u));
+                        v.z = w2.x; v.w = w2.y;
                     }
                 }
-                return v;
-            };
-            const uint32_t blocks = (K + kPkCols - 1u) / kPkCols;
-            uint4 sc_next = load_scales(0);
-            for (uint32_t q = 0; q < blocks && ok; ++q, ++bi) {
+            } else {                                     // two BF16 per block, rows 2-byte aligned
+                if (whole_blocks) {
+                    v.x = __ldg(reinterpret_cast<const uint32_t*>(srow + q * 4u));
+                } else {
+                    v.x = __ldg(reinterpret_cast<const unsigned short*>(srow + q * 4u));
+                    if ((q + 1u) * 2u <= K / 128u)
+                        v.x |= (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(srow + q * 4u + 2u)) << 16;
+                }
+            }
+            return v;
+        };
+        Ring<kAStages> ra;
+        if (kSlabs == 1u) ra.i = sub;      // 64-column stages: this warp fills every other one
+        Ring<kPkBufs> rp;
+        bool ok = true;
+        TileInfo t, tn;
+        bool have = (DUAL || wd < kDecodeWarps / 2u) && tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat);
+        const uint8_t *srow = nullptr, *sbase = nullptr;
+        uint32_t emin = 0;
+        uint4 sc_next = make_uint4(0, 0, 0, 0);
+        if (have) {
+            srow = wt.scales[t.g] + (t.m0 + arow + which * kSecond) * scale_row;
+            if (FMT == STRATA_MOE_FMT_MXFP4) emin = wt.emin[t.g];
+            sc_next = load_scales(srow, 0);
+        }
+        for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
+            // the next tile's entry, scale base and first scales are requested one step before they are needed: a chain of
+            // dependent loads at every tile start would stop the decoders for about a thousand clocks
+            const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
+            uint32_t emin_n = 0;
+            const uint32_t mx_add = (uint32_t)(2 - (int32_t)emin) * 0x04000400u;
+            for (uint32_t q = 0; q < blocks; ++q) {
                 const uint4 sc = sc_next;
-                sc_next = load_scales(q + 1u);
-                const uint32_t pb = bi % kPkBufs, pph = (bi / kPkBufs) & 1u;
-                if (!mbar_wait(&S.pk_full[pb], pph, abort_flag)) { ok = false; break; }
-                const uint8_t* pk_row = S.w[pb][which] + arow * 128u;
-                const uint32_t scw[4] = {sc.x, sc.y, sc.z, sc.w};
+                if (q + 1u < blocks) sc_next = load_scales(srow, q + 1u);
+                else if (hn && blocks > 1u) sc_next = load_scales(srow, 0);     // the next tile's row by now
+                if (!mbar_wait(&S.pk_full[rp.i], rp.ph, abort_flag)) { ok = false; break; }
+                const uint8_t* pk_row = arena + (rp.i * 2u + which) * kPkTile + arow * 128u;
+                const uint32_t sel[2] = {FMT == STRATA_MOE_FMT_NVFP4 ? (sub ? sc.y : sc.x) : sc.x,
+                                         FMT == STRATA_MOE_FMT_NVFP4 ? (sub ? sc.w : sc.z)
+                                                                     : (FMT == STRATA_MOE_FMT_MXFP4 ? sc.y : sc.x >> 16)};
 #pragma unroll
-                for (uint32_t j = 0; j < kPkCols / kBK; ++j) {
-                    const uint32_t ks = q * (kPkCols / kBK) + j;
-                    if (ks >= k_stages) break;
-                    const uint32_t s = it % kAStages, ph = (it / kAStages) & 1u;
-                    const bool mine = (it & 1u) == parity;
-                    ++it;
-                    if (!mine) continue;   // the other warp of this lane quarter and tile decodes this stage
-                    // this thread's packed bytes of the stage: 16-byte chunks 2j and 2j + 1, swizzled by row
-                    uint4 pkv[CH];
+                for (uint32_t jj = 0; jj < 2u; ++jj) {
+                    if (q * 4u + jj * 2u >= k_slabs) break;   // K % 256 == 128: the last block holds two slabs
+                    uint32_t v[32];
 #pragma unroll
-                    for (uint32_t c = 0; c < CH; ++c) {
-                        const uint32_t chunk = 2u * j + c;
-                        pkv[c] = *reinterpret_cast<const uint4*>(pk_row + ((chunk ^ (arow & 7u)) << 4));
-                    }
-                    // block multipliers of this thread's 32-column chunks
-                    uint32_t m[CH][4];
-#pragma unroll
-                    for (uint32_t c = 0; c < CH; ++c) {
-                        const uint32_t c32 = 2u * j + c;  // 32-column chunk inside the block
+                    for (uint32_t c = 0; c < 2u; ++c) {
+                        const uint4 p = *reinterpret_cast<const uint4*>(pk_row + ((c ? off1 : off0) ^ (jj * 64u)));
+                        uint32_t m[2];     // multipliers of the chunk's first and second 16 columns
                         if (FMT == STRATA_MOE_FMT_MXFP4) {
-                            const uint32_t e = (scw[c32 >> 2] >> (8u * (c32 & 3u))) & 0xFFu;
-                            const uint32_t h = (uint32_t)((int32_t)e + mx_off) << 10;
-                            m[c][0] = m[c][1] = m[c][2] = m[c][3] = h * 0x00010001u;
+                            // f16 exponent field e - emin + 2 in both halves (arithmetic modulo 2^32)
+                            m[0] = m[1] = __byte_perm(sel[jj], 0u, 0x4440u + 2u * sub + c) * 0x04000400u + mx_add;
                         } else if (FMT == STRATA_MOE_FMT_NVFP4) {
-                            const uint32_t sb = (scw[c32 >> 1] >> (16u * (c32 & 1u))) & 0xFFFFu;
                             uint32_t pair;
-                            asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(pair) : "h"((unsigned short)sb));
-                            m[c][0] = m[c][1] = __byte_perm(pair, pair, 0x1010);
-                            m[c][2] = m[c][3] = __byte_perm(pair, pair, 0x3232);
+                            asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(pair) : "h"((unsigned short)(sel[jj] >> (16u * c))));
+                            m[0] = __byte_perm(pair, pair, 0x1010);
+                            m[1] = __byte_perm(pair, pair, 0x3232);
                         } else {
-                            const uint32_t sb = (scw[0] >> (16u * (c32 >> 2))) & 0xFFFFu;
-                            const uint32_t h = __half_as_ushort(__float2half_rn(__uint_as_float(sb << 16)));
-                            m[c][0] = m[c][1] = m[c][2] = m[c][3] = h * 0x00010001u;
+                            const uint32_t h = __half_as_ushort(__float2half_rn(__uint_as_float(sel[jj] << 16)));
+                            m[0] = m[1] = h * 0x00010001u;
+                        }
+                        const uint32_t w[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+                        for (uint32_t i = 0; i < 4u; ++i) {
+                            uint32_t r[4];
+                            if (FMT == STRATA_MOE_FMT_INT4G128) p_int4x8_f16(w[i], r);
+                            else p_e2m1x8_f16(w[i], r);
+#pragma unroll
+                            for (uint32_t e = 0; e < 4u; ++e) v[c * 16u + i * 4u + e] = p_mul_f16x2(r[e], m[i >> 1]);
                         }
                     }
-                    if (!mbar_wait(&S.empty_a[s], ph ^ 1u, abort_flag)) { ok = false; break; }
-                    tc_fence_after();   // the MMAs that read this stage have completed
-#pragma unroll
-                    for (uint32_t c = 0; c < CH; ++c) {
-                        uint4 o[4];
-                        decode16<FMT>(pkv[c], m[c], o);
-                        const uint32_t v[16] = {o[0].x, o[0].y, o[0].z, o[0].w, o[1].x, o[1].y, o[1].z, o[1].w,
-                                                o[2].x, o[2].y, o[2].z, o[2].w, o[3].x, o[3].y, o[3].z, o[3].w};
-                        tmem_st16(a_lane_addr + s * kAStageCols + c * 16u, v);
+                    keep32(v);     // decoded before the wait below
+                    if (jj == 1u || q * 4u + 2u >= k_slabs) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&S.pk_empty[rp.i]);  // this warp is done reading the block
                     }
+                    if (!mbar_wait(&S.empty_a[ra.i], ra.ph ^ 1u, abort_flag)) { ok = false; break; }
+                    tc_fence_after();   // the MMAs that read this stage have completed
+                    tmem_st32(a_lane + ra.i * G::kAStageCols, v);
                     tmem_st_wait();
                     tc_fence_before();   // order the tensor-memory stores before the MMA issuer's reads
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&S.full_a[s]);
+                    if (lane == 0) mbar_arrive(&S.full_a[ra.i]);
+                    ra.next(kSlabs == 1u ? 2u : 1u);
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&S.pk_empty[pb]);  // this warp is done reading the block
+                if (!ok) break;
+                rp.next();
+                if (hn) {
+                    if (q == 0u) {
+                        sbase = wt.scales[tn.g];
+                        if (FMT == STRATA_MOE_FMT_MXFP4) emin_n = wt.emin[tn.g];
+                    }
+                    if (q + 2u == blocks || blocks == 1u) srow = sbase + (tn.m0 + arow + which * kSecond) * scale_row;
+                    if (blocks == 1u) sc_next = load_scales(srow, 0);
+                }
             }
+            t = tn;
+            have = hn;
+            emin = emin_n;
         }
         if (!ok) { *abort_flag = 1; atomicOr(a.status, kStatusWaitTimeout); }
     } else {
         // ---------------------------------------------------------------- epilogue
         const uint32_t ew = warp - kFirstEpilogueWarp;
         const uint32_t lane_base = (warp & 3u) * 32u;
-        uint32_t tcount = 0;
+        Ring<kAccBufs> rc;
         bool ok = true, bad = false;
-        (void)ew;
-        for (uint32_t tile = blockIdx.x; ok; tile += gridDim.x, ++tcount) {
-            TileInfo t;
-            if (!tile_lookup(a.tile_table, tile, m_tiles, t, kTileFeat)) break;
-            if (!mbar_wait(&S.acc_full, tcount & 1u, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            const uint32_t feat = t.m0 + lane_base + lane;
+        TileInfo t, tn;
+        bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat);
+        for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
+            const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
+            constexpr bool kNoPost = FMT == STRATA_MOE_FMT_INT4G128 || BF;
             float s0, s1 = 1.0f;
-            constexpr bool kNoPost = FMT == STRATA_MOE_FMT_INT4G128 || FMT == kFmtBf16W;
             if (GU) {
                 s0 = kNoPost ? 1.0f : a.gate.post_scale[t.g];
                 s1 = kNoPost ? 1.0f : a.up.post_scale[t.g];
             } else {
                 s0 = s1 = kNoPost ? 1.0f : a.down.post_scale[t.g];
             }
-            const uint32_t taddr = tmem_base + (lane_base << 16);
+            // one warp polls, the others sleep on a hardware barrier
+            if (ew == 0u && !mbar_wait(&S.acc_full[rc.i], rc.ph, abort_flag)) *abort_flag = 1;
+            asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueWarps * 32u) : "memory");
+            if (*abort_flag) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t feat = t.m0 + lane_base + lane;
+            const uint32_t act_col = FMT == STRATA_MOE_FMT_INT4G128 ? int4_slot(feat) : feat;   // the down tiles' column order
+            const uint32_t taddr = tmem_base + rc.i * (2u * NT) + (lane_base << 16);
+            const uint32_t lo_at = 16u << box_of(t.n);      // SPLIT: accumulator columns of the lo rows
             for (uint32_t c0 = (ew >> 2) * 16u; c0 < t.n; c0 += 16u * (kEpilogueWarps / 4u)) {
                 uint32_t g[16], u[16];
                 tmem_ld16(taddr + c0, g);
-                if (DUAL) tmem_ld16(taddr + kNTile + c0, u);
+                if (DUAL) tmem_ld16(taddr + NT + c0, u);
                 tmem_ld_wait();
+                if (SPLIT) {
+                    uint32_t l[16];
+                    tmem_ld16(taddr + lo_at + c0, l);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (uint32_t j = 0; j < 16u; ++j) g[j] = __float_as_uint(__uint_as_float(g[j]) + __uint_as_float(l[j]));
+                    if (DUAL) {
+                        tmem_ld16(taddr + NT + lo_at + c0, l);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (uint32_t j = 0; j < 16u; ++j) u[j] = __float_as_uint(__uint_as_float(u[j]) + __uint_as_float(l[j]));
+                    }
+                }
 #pragma unroll
                 for (uint32_t j = 0; j < 16u; ++j) {
                     if (c0 + j >= t.n) break;
                     const size_t pos = (size_t)t.row0 + c0 + j;
+                    const float rs = rowscale ? rowscale[pos] : 1.0f;   // undoes the pre-scale of the activation row
                     if (GU) {
                         if (a.act_rowscale_out != nullptr && feat == 0u) a.act_rowscale_out[pos] = 1.0f;
-                        const float rs = rowscale ? rowscale[pos] : 1.0f;
                         const float gv = __uint_as_float(g[j]) * s0 * rs, uv = __uint_as_float(u[j]) * s1 * rs;
                         float v;
                         if (a.glu.kind == STRATA_MOE_ACT_SWIGLU) {
@@ -674,13 +726,17 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
                         } else {
                             v = glu_other(gv, uv, a.glu);
                         }
-                        if (!(fabsf(v) <= 65504.0f)) bad = true;
-                        if (FMT == kFmtBf16W)
-                            static_cast<__nv_bfloat16*>(act_out_v)[pos * R + feat] = __float2bfloat16_rn(v);
-                        else
-                            static_cast<__half*>(act_out_v)[pos * R + feat] = __float2half_rn(v);
+                        if (!(fabsf(v) <= (BF ? 3.0e38f : 65504.0f))) bad = true;
+                        if (BF) {
+                            const __nv_bfloat16 h = __float2bfloat16_rn(v);
+                            static_cast<__nv_bfloat16*>(act_out_v)[pos * R + act_col] = h;
+                            if (a.act_lo) static_cast<__nv_bfloat16*>(a.act_lo)[pos * R + act_col] = __float2bfloat16_rn(v - __bfloat162float(h));
+                        } else {
+                            const __half h = __float2half_rn(v);
+                            static_cast<__half*>(act_out_v)[pos * R + act_col] = h;
+                            if (a.act_lo) static_cast<__half*>(a.act_lo)[pos * R + act_col] = __float2half_rn(v - __half2float(h));
+                        }
                     } else {
-                        const float rs = rowscale ? rowscale[pos] : 1.0f;   // pre-scaled activation rows
                         const float v = __uint_as_float(g[j]) * s0 * rs;
                         const float lim = a.y_half ? 65504.0f : 3.0e38f;
                         if (a.y_rowscale_out != nullptr && feat == 0u) a.y_rowscale_out[pos] = 1.0f;
@@ -698,7 +754,10 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&S.acc_empty);
+            if (lane == 0) mbar_arrive(&S.acc_empty[rc.i]);
+            rc.next();
+            t = tn;
+            have = hn;
         }
         if (!ok) { *abort_flag = 1; atomicOr(a.status, kStatusWaitTimeout); }
         if (bad) atomicOr(a.status, kStatusNonFiniteOutput);
@@ -778,31 +837,13 @@ bool prefill_supported(int fmt, uint32_t H, uint32_t I) {
 }
 
 size_t prefill_scratch_bytes(uint32_t n_groups, uint32_t pairs) {
-    return (4 + 3 * ((size_t)pairs / 128u + n_groups + 1)) * sizeof(uint32_t);   // the smaller tile size bounds it
+    return (4 + 3 * ((size_t)pairs / 16u + n_groups + 1)) * sizeof(uint32_t);   // the smallest tile size bounds it
 }
 
 static bool make_bmaps(BMaps* b, const void* base, uint64_t rows, uint64_t cols) {
     for (int i = 0; i < 4; ++i)
         if (!make_map(&b->m[i], base, rows, cols, 16u << i)) return false;
     return true;
-}
-
-template <int FMT, int NT>
-static int set_smem_attr(size_t smem) {
-    // the opt-in to more than 48 KB of dynamic shared memory is a per-device property of the function
-    static bool done[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
-    if (done[dev]) return 0;
-    if (cudaFuncSetAttribute(prefill_ffn_kernel<FMT, 0, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess ||
-        cudaFuncSetAttribute(prefill_ffn_kernel<FMT, 1, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess ||
-        cudaFuncSetAttribute(prefill_ffn_kernel<FMT, 2, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
-        return -2;
-    done[dev] = true;
-    return 0;
 }
 
 // Tensor map over one projection's packed 4-bit rows ([rows, K/2] bytes): 128-byte x 128-row
@@ -822,132 +863,146 @@ int prefill_encode_weight_map(void* out, const void* packed, uint32_t rows, uint
                : -1;
 }
 
-template <int FMT, int NT>
-static int launch_fmt(const PrefillArgs& a, const void* x16, const float* x_rowscale, void* act16,
-                      uint32_t pairs_cap, const void* wmaps, cudaStream_t s, cudaEvent_t mid) {
-    const CUtensorMap* wm = static_cast<const CUtensorMap*>(wmaps);
-    BMaps map_x, map_act;
-    if (!make_bmaps(&map_x, x16, pairs_cap, a.H) || !make_bmaps(&map_act, act16, pairs_cap, a.I)) return -1;
-    const CUtensorMap& dummy = map_x.m[0];
-    const size_t smem = sizeof(PrefillSmem<NT>) + 1024;
-    if (set_smem_attr<FMT, NT>(smem)) return -2;
-    prefill_tiles_kernel<<<1, 1024, 0, s>>>(a.offsets, a.n_groups, a.tile_table, a.min_rows, NT);
-    prefill_ffn_kernel<FMT, 0, NT><<<kNumSMs, kThreads, smem, s>>>(map_x, dummy, dummy, a, x_rowscale, act16, wm);
-    if (mid) cudaEventRecord(mid, s);
-    if (a.H % 256u == 0u)
-        prefill_ffn_kernel<FMT, 2, NT><<<kNumSMs, kThreads, smem, s>>>(map_act, dummy, dummy, a, nullptr, nullptr, wm);
-    else
-        prefill_ffn_kernel<FMT, 1, NT><<<kNumSMs, kThreads, smem, s>>>(map_act, dummy, dummy, a, nullptr, nullptr, wm);
-    g_kernel_launches += 3;
-    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+// Tensor map over one projection's BF16 rows ([rows, K]): boxes of 64 columns x 128 rows.
+int prefill_encode_weight_map_bf16(void* out, const void* w, uint32_t rows, uint32_t K) {
+    return make_map(static_cast<CUtensorMap*>(out), w, rows, K, kMTile) ? 0 : -1;
 }
 
-template <int FMT, int NT>
-static int launch_gate_up_fmt(const PrefillArgs& a, const void* x16, const float* x_rowscale, void* act16,
-                              uint32_t pairs_cap, const void* wmaps, cudaStream_t s) {
-    const CUtensorMap* wm = static_cast<const CUtensorMap*>(wmaps);
-    BMaps map_x;
-    if (!make_bmaps(&map_x, x16, pairs_cap, a.H)) return -1;
-    const CUtensorMap& dummy = map_x.m[0];
+// One kernel launch.  b_hi / b_lo: the 16-bit activation rows [rows_cap, K] (b_lo only when SPLIT); map_a0 / map_a1: the
+// weight matrices of a launch without a map table (wmaps == nullptr, BF16 only).
+template <int FMT, int MODE, int NT, bool SPLIT>
+static int launch_one(const PrefillArgs& a, const void* b_hi, const void* b_lo, uint32_t rows_cap,
+                      const CUtensorMap* map_a0, const CUtensorMap* map_a1, const float* rowscale, void* act_out,
+                      const void* wmaps, cudaStream_t s) {
+    // the opt-in to more than 48 KB of dynamic shared memory is a per-device property of the function
+    static bool done[64] = {};
     const size_t smem = sizeof(PrefillSmem<NT>) + 1024;
-    if (set_smem_attr<FMT, NT>(smem)) return -2;
-    prefill_tiles_kernel<<<1, 1024, 0, s>>>(a.offsets, a.n_groups, a.tile_table, a.min_rows, NT);
-    prefill_ffn_kernel<FMT, 0, NT><<<kNumSMs, kThreads, smem, s>>>(map_x, dummy, dummy, a, x_rowscale, act16, wm);
-    g_kernel_launches += 2;
-    return cudaGetLastError() == cudaSuccess ? 0 : -3;
-}
-
-int launch_prefill_gate_up(const PrefillArgs& a, const void* x16, const float* x_rowscale, void* act16,
-                           uint32_t pairs_cap, const void* wmaps, cudaStream_t s) {
-    const bool wide = a.ntile != 128u;
-    switch (a.fmt) {
-        case STRATA_MOE_FMT_MXFP4:
-            return wide ? launch_gate_up_fmt<STRATA_MOE_FMT_MXFP4, 192>(a, x16, x_rowscale, act16, pairs_cap, wmaps, s)
-                        : launch_gate_up_fmt<STRATA_MOE_FMT_MXFP4, 128>(a, x16, x_rowscale, act16, pairs_cap, wmaps, s);
-        case STRATA_MOE_FMT_NVFP4:
-            return wide ? launch_gate_up_fmt<STRATA_MOE_FMT_NVFP4, 192>(a, x16, x_rowscale, act16, pairs_cap, wmaps, s)
-                        : launch_gate_up_fmt<STRATA_MOE_FMT_NVFP4, 128>(a, x16, x_rowscale, act16, pairs_cap, wmaps, s);
-        default: return -1;
+    static_assert(sizeof(PrefillSmem<NT>) + 1024 <= 227u * 1024u, "shared memory");
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -2;
+    if (!done[dev]) {
+        if (cudaFuncSetAttribute(prefill_ffn_kernel<FMT, MODE, NT, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem) != cudaSuccess)
+            return -2;
+        done[dev] = true;
     }
-}
-
-// Down projection only, over f16 activation rows that carry a per-row factor (act_rowscale undoes it).
-template <int FMT, int NT>
-static int launch_down_fmt(const PrefillArgs& a, const void* act16, const float* act_rowscale, uint32_t pairs_cap,
-                           const void* wmaps, cudaStream_t s) {
-    const CUtensorMap* wm = static_cast<const CUtensorMap*>(wmaps);
-    BMaps map_act;
-    if (!make_bmaps(&map_act, act16, pairs_cap, a.I)) return -1;
-    const CUtensorMap& dummy = map_act.m[0];
-    const size_t smem = sizeof(PrefillSmem<NT>) + 1024;
-    if (set_smem_attr<FMT, NT>(smem)) return -2;
-    if (!a.reuse_tiles) {
-        prefill_tiles_kernel<<<1, 1024, 0, s>>>(a.offsets, a.n_groups, a.tile_table, a.min_rows, NT);
-        ++g_kernel_launches;
+    BMaps hi, lo;
+    const uint32_t K = MODE == 0 ? a.H : a.I;
+    if (!make_bmaps(&hi, b_hi, rows_cap, K)) return -1;
+    if (SPLIT) {
+        if (!make_bmaps(&lo, b_lo, rows_cap, K)) return -1;
+    } else {
+        lo = hi;
     }
-    if (a.H % 256u == 0u)
-        prefill_ffn_kernel<FMT, 2, NT><<<kNumSMs, kThreads, smem, s>>>(map_act, dummy, dummy, a, act_rowscale, nullptr, wm);
-    else
-        prefill_ffn_kernel<FMT, 1, NT><<<kNumSMs, kThreads, smem, s>>>(map_act, dummy, dummy, a, act_rowscale, nullptr, wm);
+    prefill_ffn_kernel<FMT, MODE, NT, SPLIT><<<kNumSMs, kThreads, smem, s>>>(
+        hi, lo, map_a0 ? *map_a0 : hi.m[0], map_a1 ? *map_a1 : hi.m[0], a, rowscale, act_out,
+        static_cast<const CUtensorMap*>(wmaps));
     ++g_kernel_launches;
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-int launch_prefill_down(const PrefillArgs& a, const void* act16, const float* act_rowscale, uint32_t pairs_cap,
-                        const void* wmaps, cudaStream_t s) {
-    const bool wide = a.ntile != 128u;
+static void launch_tiles(const PrefillArgs& a, cudaStream_t s) {
+    prefill_tiles_kernel<<<1, 1024, 0, s>>>(a.offsets, a.n_groups, a.tile_table, a.min_rows, a.ntile);
+    ++g_kernel_launches;
+}
+
+// Operands of the gate/up or the down launch beside PrefillArgs.
+struct Operands {
+    const void *hi, *lo;
+    uint32_t rows_cap;
+    const CUtensorMap *a0, *a1;
+    const float* rowscale;
+    void* act_out;
+    const void* wmaps;
+};
+
+template <int FMT>
+static int launch_gate_up_nt(const PrefillArgs& a, const Operands& o, cudaStream_t s) {
+    if (a.ntile <= 32u) return launch_one<FMT, 0, 32, false>(a, o.hi, nullptr, o.rows_cap, o.a0, o.a1, o.rowscale, o.act_out, o.wmaps, s);
+    if (a.ntile <= 64u) return launch_one<FMT, 0, 64, false>(a, o.hi, nullptr, o.rows_cap, o.a0, o.a1, o.rowscale, o.act_out, o.wmaps, s);
+    if (a.ntile <= 128u) return launch_one<FMT, 0, 128, false>(a, o.hi, nullptr, o.rows_cap, o.a0, o.a1, o.rowscale, o.act_out, o.wmaps, s);
+    if (a.ntile <= 160u) return launch_one<FMT, 0, 160, false>(a, o.hi, nullptr, o.rows_cap, o.a0, o.a1, o.rowscale, o.act_out, o.wmaps, s);
+    return launch_one<FMT, 0, 192, false>(a, o.hi, nullptr, o.rows_cap, o.a0, o.a1, o.rowscale, o.act_out, o.wmaps, s);
+}
+// o.lo set: the activation is a hi + lo pair and the tile holds twice the token rows.
+template <int FMT>
+static int launch_down_nt(const PrefillArgs& a, const Operands& o, cudaStream_t s) {
+    if (o.lo) {
+        if (a.H % 256u) return launch_one<FMT, 1, 128, true>(a, o.hi, o.lo, o.rows_cap, o.a0, o.a1, o.rowscale, nullptr, o.wmaps, s);
+        if (a.ntile <= 16u) return launch_one<FMT, 2, 32, true>(a, o.hi, o.lo, o.rows_cap, o.a0, o.a1, o.rowscale, nullptr, o.wmaps, s);
+        if (a.ntile <= 32u) return launch_one<FMT, 2, 64, true>(a, o.hi, o.lo, o.rows_cap, o.a0, o.a1, o.rowscale, nullptr, o.wmaps, s);
+        return launch_one<FMT, 2, 128, true>(a, o.hi, o.lo, o.rows_cap, o.a0, o.a1, o.rowscale, nullptr, o.wmaps, s);
+    }
+    if (a.H % 256u) return launch_one<FMT, 1, 128, false>(a, o.hi, nullptr, o.rows_cap, o.a0, o.a1, o.rowscale, nullptr, o.wmaps, s);
+    if (a.ntile <= 32u) return launch_one<FMT, 2, 32, false>(a, o.hi, nullptr, o.rows_cap, o.a0, o.a1, o.rowscale, nullptr, o.wmaps, s);
+    if (a.ntile <= 64u) return launch_one<FMT, 2, 64, false>(a, o.hi, nullptr, o.rows_cap, o.a0, o.a1, o.rowscale, nullptr, o.wmaps, s);
+    if (a.ntile <= 128u) return launch_one<FMT, 2, 128, false>(a, o.hi, nullptr, o.rows_cap, o.a0, o.a1, o.rowscale, nullptr, o.wmaps, s);
+    if (a.ntile <= 160u) return launch_one<FMT, 2, 160, false>(a, o.hi, nullptr, o.rows_cap, o.a0, o.a1, o.rowscale, nullptr, o.wmaps, s);
+    return launch_one<FMT, 2, 192, false>(a, o.hi, nullptr, o.rows_cap, o.a0, o.a1, o.rowscale, nullptr, o.wmaps, s);
+}
+static int gate_up_any(const PrefillArgs& a, const Operands& o, cudaStream_t s) {
     switch (a.fmt) {
-        case STRATA_MOE_FMT_MXFP4:
-            return wide ? launch_down_fmt<STRATA_MOE_FMT_MXFP4, 192>(a, act16, act_rowscale, pairs_cap, wmaps, s)
-                        : launch_down_fmt<STRATA_MOE_FMT_MXFP4, 128>(a, act16, act_rowscale, pairs_cap, wmaps, s);
-        case STRATA_MOE_FMT_NVFP4:
-            return wide ? launch_down_fmt<STRATA_MOE_FMT_NVFP4, 192>(a, act16, act_rowscale, pairs_cap, wmaps, s)
-                        : launch_down_fmt<STRATA_MOE_FMT_NVFP4, 128>(a, act16, act_rowscale, pairs_cap, wmaps, s);
+        case STRATA_MOE_FMT_MXFP4: return launch_gate_up_nt<STRATA_MOE_FMT_MXFP4>(a, o, s);
+        case STRATA_MOE_FMT_NVFP4: return launch_gate_up_nt<STRATA_MOE_FMT_NVFP4>(a, o, s);
+        case STRATA_MOE_FMT_INT4G128: return launch_gate_up_nt<STRATA_MOE_FMT_INT4G128>(a, o, s);
+        case kFmtBf16W: return launch_gate_up_nt<kFmtBf16W>(a, o, s);
         default: return -1;
     }
 }
-
-int launch_prefill(const PrefillArgs& a, const void* x16, const float* x_rowscale, void* act16,
-                   uint32_t pairs_cap, const void* wmaps, cudaStream_t s, cudaEvent_t mid) {
-    const bool wide = a.ntile != 128u;
-#define STRATA_PREFILL_CASE(F)                                                                              \
-    case F:                                                                                                 \
-        if (a.ntile == 160u) return launch_fmt<F, 160>(a, x16, x_rowscale, act16, pairs_cap, wmaps, s, mid); \
-        return wide ? launch_fmt<F, 192>(a, x16, x_rowscale, act16, pairs_cap, wmaps, s, mid)               \
-                    : launch_fmt<F, 128>(a, x16, x_rowscale, act16, pairs_cap, wmaps, s, mid);
+static int down_any(const PrefillArgs& a, const Operands& o, cudaStream_t s) {
     switch (a.fmt) {
-        STRATA_PREFILL_CASE(STRATA_MOE_FMT_MXFP4)
-        STRATA_PREFILL_CASE(STRATA_MOE_FMT_NVFP4)
-        STRATA_PREFILL_CASE(STRATA_MOE_FMT_INT4G128)
+        case STRATA_MOE_FMT_MXFP4: return launch_down_nt<STRATA_MOE_FMT_MXFP4>(a, o, s);
+        case STRATA_MOE_FMT_NVFP4: return launch_down_nt<STRATA_MOE_FMT_NVFP4>(a, o, s);
+        case STRATA_MOE_FMT_INT4G128: return launch_down_nt<STRATA_MOE_FMT_INT4G128>(a, o, s);
+        case kFmtBf16W: return launch_down_nt<kFmtBf16W>(a, o, s);
         default: return -1;
     }
-#undef STRATA_PREFILL_CASE
+}
+// Tiles of shapes whose down projection takes single weight tiles (H % 256 == 128) hold at most 128 rows, or 64 pairs.
+static PrefillArgs with_tile(PrefillArgs a, bool split) {
+    const uint32_t most = split ? 64u : (a.H % 256u ? 128u : 192u);
+    if (a.ntile == 0u || a.ntile > most) a.ntile = most;
+    return a;
+}
+
+int launch_prefill_gate_up(const PrefillArgs& args, const void* x16, const float* x_rowscale, void* act16,
+                           uint32_t pairs_cap, const void* wmaps, cudaStream_t s) {
+    const PrefillArgs a = with_tile(args, args.act_lo != nullptr);
+    launch_tiles(a, s);
+    return gate_up_any(a, Operands{x16, nullptr, pairs_cap, nullptr, nullptr, x_rowscale, act16, wmaps}, s);
+}
+
+int launch_prefill_down(const PrefillArgs& args, const void* act16, const float* act_rowscale, uint32_t pairs_cap,
+                        const void* wmaps, cudaStream_t s) {
+    const PrefillArgs a = with_tile(args, args.act_lo != nullptr);
+    if (!a.reuse_tiles) launch_tiles(a, s);
+    return down_any(a, Operands{act16, a.act_lo, pairs_cap, nullptr, nullptr, act_rowscale, nullptr, wmaps}, s);
+}
+
+int launch_prefill(const PrefillArgs& args, const void* x16, const float* x_rowscale, void* act16,
+                   uint32_t pairs_cap, const void* wmaps, cudaStream_t s, cudaEvent_t mid) {
+    PrefillArgs a = args;
+    const int rc = launch_prefill_gate_up(a, x16, x_rowscale, act16, pairs_cap, wmaps, s);
+    if (rc) return rc;
+    if (mid) cudaEventRecord(mid, s);
+    a.reuse_tiles = 1;
+    return launch_prefill_down(a, act16, nullptr, pairs_cap, wmaps, s);
 }
 
 // BF16 expert (the shared expert) over `rows` token rows in natural order: x [rows, H] BF16,
 // gate/up [I, H], down [H, I] BF16, act [rows_cap, I] BF16 scratch, y [rows, H] fp32.
-// a.offsets must hold {0, rows}; a.n_groups = 1.
-template <int NT>
-static int launch_bf16_nt(const PrefillArgs& a, const void* x, uint32_t rows, const void* w_gate, const void* w_up,
-                          const void* w_down, void* act, uint32_t rows_cap, cudaStream_t s) {
-    BMaps map_x, map_act;
+// args.offsets must hold {0, rows}; args.n_groups = 1.
+int launch_prefill_bf16(const PrefillArgs& args, const void* x, uint32_t rows, const void* w_gate, const void* w_up,
+                        const void* w_down, void* act, uint32_t rows_cap, cudaStream_t s) {
+    const PrefillArgs a = with_tile(args, args.act_lo != nullptr);
     CUtensorMap map_g, map_u, map_d;
-    if (!make_bmaps(&map_x, x, rows, a.H) || !make_bmaps(&map_act, act, rows_cap, a.I) ||
-        !make_map(&map_g, w_gate, a.I, a.H, kMTile) || !make_map(&map_u, w_up, a.I, a.H, kMTile) ||
+    if (!make_map(&map_g, w_gate, a.I, a.H, kMTile) || !make_map(&map_u, w_up, a.I, a.H, kMTile) ||
         !make_map(&map_d, w_down, a.H, a.I, kMTile))
         return -1;
-    const size_t smem = sizeof(PrefillSmem<NT>) + 1024;
-    if (set_smem_attr<kFmtBf16W, NT>(smem)) return -2;
-    prefill_tiles_kernel<<<1, 1024, 0, s>>>(a.offsets, a.n_groups, a.tile_table, a.min_rows, NT);
-    prefill_ffn_kernel<kFmtBf16W, 0, NT><<<kNumSMs, kThreads, smem, s>>>(map_x, map_g, map_u, a, nullptr, act, nullptr);
-    if (a.H % 256u == 0u)
-        prefill_ffn_kernel<kFmtBf16W, 2, NT><<<kNumSMs, kThreads, smem, s>>>(map_act, map_d, map_d, a, nullptr, nullptr,
-                                                                         nullptr);
-    else
-        prefill_ffn_kernel<kFmtBf16W, 1, NT><<<kNumSMs, kThreads, smem, s>>>(map_act, map_d, map_d, a, nullptr, nullptr,
-                                                                         nullptr);
-    g_kernel_launches += 3;
-    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+    launch_tiles(a, s);
+    const int rc = launch_gate_up_nt<kFmtBf16W>(a, Operands{x, nullptr, rows, &map_g, &map_u, nullptr, act, nullptr}, s);
+    if (rc) return rc;
+    return launch_down_nt<kFmtBf16W>(a, Operands{act, a.act_lo, rows_cap, &map_d, &map_d, nullptr, nullptr, nullptr}, s);
 }
 
 // Router projection on the tensor cores: logits[t, e] = sum_h x[t, h] * wg[e, h] for BF16 operands,
@@ -955,50 +1010,31 @@ static int launch_bf16_nt(const PrefillArgs& a, const void* x, uint32_t rows, co
 // N tiles of the single-GEMM modes (one group holding all T rows), so the output lands as [T, E] fp32.
 // The summation order differs from the canonical lane-strided order: these logits feed the fast
 // router, which re-derives everything that reaches the caller in the canonical order.
-// a.offsets must hold {0, T}.  Needs E % 128 == 0 and H % 64 == 0.
-template <int NT>
-static int launch_router_tc_nt(PrefillArgs a, const void* x, uint32_t T, const void* wg, uint32_t E, uint32_t H,
-                               cudaStream_t s) {
-    BMaps map_x;
+// offsets2 must hold {0, T}.  Needs E % 128 == 0 and H % 128 == 0.
+int launch_router_tc(const void* x, uint32_t T, const void* wg, uint32_t E, uint32_t H, float* logits,
+                     uint32_t* tile_table, const uint32_t* offsets2, uint32_t* status, cudaStream_t s) {
+    if (E % 128u || H % 128u || T == 0u) return -1;
     CUtensorMap map_w;
-    if (!make_bmaps(&map_x, x, T, H) || !make_map(&map_w, wg, E, H, kMTile)) return -1;
-    const size_t smem = sizeof(PrefillSmem<NT>) + 1024;
-    if (set_smem_attr<kFmtBf16W, NT>(smem)) return -2;
+    if (!make_map(&map_w, wg, E, H, kMTile)) return -1;
+    PrefillArgs a{};
     a.fmt = kFmtBf16W;
     a.H = E;     // features of the single-GEMM modes
     a.I = H;     // their K
     a.n_groups = 1;
     a.pairs = T;
-    a.min_rows = 0;
-    prefill_tiles_kernel<<<1, 1024, 0, s>>>(a.offsets, 1, a.tile_table, 0, NT);
-    // 256 experts per job while that still gives every other SM a job; with few tokens (a rank's share of an
-    // expert-parallel step) 128 per job: twice the jobs, each half as long (2048 tokens: 16 jobs otherwise)
-    const uint64_t jobs256 = (uint64_t)((T + NT - 1) / NT) * (E / 256u);
-    if (E % 256u == 0u && jobs256 * 2u >= (uint64_t)kNumSMs)
-        prefill_ffn_kernel<kFmtBf16W, 2, NT><<<kNumSMs, kThreads, smem, s>>>(map_x, map_w, map_w, a, nullptr, nullptr, nullptr);
-    else
-        prefill_ffn_kernel<kFmtBf16W, 1, NT><<<kNumSMs, kThreads, smem, s>>>(map_x, map_w, map_w, a, nullptr, nullptr, nullptr);
-    g_kernel_launches += 2;
-    return cudaGetLastError() == cudaSuccess ? 0 : -3;
-}
-
-int launch_router_tc(const void* x, uint32_t T, const void* wg, uint32_t E, uint32_t H, float* logits,
-                     uint32_t* tile_table, const uint32_t* offsets2, uint32_t* status, cudaStream_t s) {
-    if (E % 128u || H % 64u || T == 0u) return -1;
-    PrefillArgs a{};
     a.offsets = offsets2;
     a.y = logits;
     a.tile_table = tile_table;
     a.status = status;
     a.glu = GluParams{STRATA_MOE_ACT_SWIGLU, 1.0f, 1.0f};
-    // 128-token tiles: more tiles than the 192-token geometry gives, and a tile is short (E features x H)
-    return launch_router_tc_nt<128>(a, x, T, wg, E, H, s);
-}
-
-int launch_prefill_bf16(const PrefillArgs& a, const void* x, uint32_t rows, const void* w_gate, const void* w_up,
-                        const void* w_down, void* act, uint32_t rows_cap, cudaStream_t s) {
-    return a.ntile != 128u ? launch_bf16_nt<192>(a, x, rows, w_gate, w_up, w_down, act, rows_cap, s)
-                           : launch_bf16_nt<128>(a, x, rows, w_gate, w_up, w_down, act, rows_cap, s);
+    a.ntile = 128u;   // more tiles than the 192-token geometry gives, and a tile is short (E features x H)
+    launch_tiles(a, s);
+    // 256 experts per job while that still gives every other SM a job; with few tokens (a rank's share of an
+    // expert-parallel step) 128 per job: twice the jobs, each half as long (2048 tokens: 16 jobs otherwise)
+    const uint64_t jobs256 = (uint64_t)((T + 127u) / 128u) * (E / 256u);
+    if (E % 256u == 0u && jobs256 * 2u >= (uint64_t)kNumSMs)
+        return launch_one<kFmtBf16W, 2, 128, false>(a, x, nullptr, T, &map_w, &map_w, nullptr, nullptr, nullptr, s);
+    return launch_one<kFmtBf16W, 1, 128, false>(a, x, nullptr, T, &map_w, &map_w, nullptr, nullptr, nullptr, s);
 }
 
 }  // namespace smoe

@@ -30,11 +30,18 @@ __device__ __forceinline__ uint4 scale8_bf16_to_f16(const uint4& v, float sc) {
     return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
+// eight f16 columns -> columns i and i + 4 side by side
+__device__ __forceinline__ uint4 int4_column_order(const uint4& v) {
+    return make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632), __byte_perm(v.y, v.w, 0x5410),
+                      __byte_perm(v.y, v.w, 0x7632));
+}
+
 // Rows of up to 4096 columns are read ONCE: the lane keeps its sixteen 16-byte pieces in registers between the
 // maximum and the conversion, and all sixteen loads are in flight together (a warp that converts several rows in
 // turn is otherwise bound by one memory round trip per piece).  Longer rows take two passes in batches of eight loads.
 __device__ __forceinline__ void warp_row_to_f16_bf16(const __nv_bfloat16* __restrict__ src, uint32_t C,
-                                                     __half* __restrict__ hi, float* __restrict__ rowscale) {
+                                                     __half* __restrict__ hi, float* __restrict__ rowscale,
+                                                     bool int4_order = false) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint4* p = reinterpret_cast<const uint4*>(src);
     uint4* out = reinterpret_cast<uint4*>(hi);
@@ -73,7 +80,10 @@ __device__ __forceinline__ void warp_row_to_f16_bf16(const __nv_bfloat16* __rest
 #pragma unroll
         for (uint32_t q = 0; q < 16u; ++q) {
             const uint32_t i = lane + 32u * q;
-            if (i < n) out[i] = scale8_bf16_to_f16(keep[q], sc);
+            if (i < n) {
+                const uint4 h = scale8_bf16_to_f16(keep[q], sc);
+                out[i] = int4_order ? int4_column_order(h) : h;
+            }
         }
     } else {
         for (uint32_t base = 0; base < n; base += 256u) {
@@ -86,7 +96,10 @@ __device__ __forceinline__ void warp_row_to_f16_bf16(const __nv_bfloat16* __rest
 #pragma unroll
             for (uint32_t q = 0; q < 8u; ++q) {
                 const uint32_t i = base + lane + 32u * q;
-                if (i < n) out[i] = scale8_bf16_to_f16(v[q], sc);
+                if (i < n) {
+                    const uint4 h = scale8_bf16_to_f16(v[q], sc);
+                    out[i] = int4_order ? int4_column_order(h) : h;
+                }
             }
         }
     }
@@ -97,7 +110,7 @@ __device__ __forceinline__ void warp_row_to_f16_bf16(const __nv_bfloat16* __rest
 // (0xFFFFFFFF = none); hi / rowscale are the bases of the destination arrays.
 __device__ __forceinline__ void warp_row_to_f16_bf16_spread(const __nv_bfloat16* __restrict__ src, uint32_t C,
                                                             __half* __restrict__ hi, float* __restrict__ rowscale,
-                                                            uint32_t mydst, uint32_t k) {
+                                                            uint32_t mydst, uint32_t k, bool int4_order) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint4* p = reinterpret_cast<const uint4*>(src);
     const uint32_t n = C / 8u;
@@ -125,6 +138,7 @@ __device__ __forceinline__ void warp_row_to_f16_bf16_spread(const __nv_bfloat16*
         for (uint32_t q = 0; q < 8u; ++q) {
             const uint32_t i = base + lane + 32u * q;
             v[q] = i < n ? scale8_bf16_to_f16(__ldg(p + i), sc) : make_uint4(0, 0, 0, 0);
+            if (int4_order) v[q] = int4_column_order(v[q]);
         }
         for (uint32_t j = 0; j < k; ++j) {
             const uint32_t d = __shfl_sync(0xFFFFFFFFu, mydst, j);
