@@ -117,16 +117,10 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
         : "memory");
 }
 
-// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024 B apart.
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);       // start address
-    d |= (uint64_t)1 << 16;                         // leading byte offset: unused for swizzled K-major
-    d |= (uint64_t)(1024u >> 4) << 32;              // stride byte offset between 8-row groups
-    d |= (uint64_t)1 << 46;                         // descriptor version of this architecture
-    d |= (uint64_t)2 << 61;                         // 128-byte swizzle
-    return d;
-}
+// Low word of a shared-memory matrix descriptor: start address / 16, leading byte offset unused (1).  K-major operand,
+// 128-byte swizzle, 8-row groups 1024 B apart; the high word (kDescHi) holds the stride between the groups / 16, the
+// descriptor version of this architecture (bit 46) and the swizzle (2 at bit 61).
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (1u << 16); }
 // Instruction descriptor, kind::f16: F16 x F16 (or BF16 x BF16) -> F32, both operands K-major, M = 128.
 __device__ __forceinline__ uint32_t umma_idesc_f16(uint32_t n, uint32_t ab_format /* 0 = F16, 1 = BF16 */) {
     uint32_t d = 0;
@@ -137,40 +131,52 @@ __device__ __forceinline__ uint32_t umma_idesc_f16(uint32_t n, uint32_t ab_forma
     d |= (kMTile >> 4) << 24;   // M
     return d;
 }
-// The four K = 16 MMAs of one 64-column stage, A from tensor memory (lane = row, 32-bit column = two K values, 8
-// columns per MMA).  `never` is a value the compiler cannot see through that is never 0: the branches on it are not
-// taken and only end the basic blocks.  MMAs that follow one another in straight-line code run one after the
-// other without overlap (measured on 512 MMAs of 128 x N x 16, clocks per MMA: A in tensor memory 74 / 106 at
-// N = 128 / 192, A in shared memory 107 / 139); with a branch between them they pipeline (64 / 96 in both forms,
-// the tensor pipe's rate, and 21 at N = 16).
-__device__ __forceinline__ void umma4_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+// The four K = 16 MMAs of one 64-column slab, A from tensor memory (lane = row, 32-bit column = two K values, 8 columns
+// per MMA) or from shared memory; the low words of the shared-memory descriptors come in, the high word is constant.
+//
+// Two things decide what an MMA costs the issuing warp.  (1) Its operands live in uniform registers: the warp runs its
+// loop converged, with values the compiler can prove uniform, and only the MMA itself is left to one elected lane.  With
+// one lane in a divergent branch and operands in ordinary registers an issue took 80 to 140 clocks, so that the issuers
+// were busy for 75 % of the kernel's time and set its pace.  (2) MMAs that follow one another in straight-line code ran
+// without overlap (512 MMAs of 128 x N x 16, clocks per MMA: A in tensor memory 74 / 106 at N = 128 / 192, A in shared
+// memory 107 / 139); with a branch between them they pipeline (64 / 96, the tensor pipe's rate).  `never` is a value the
+// compiler cannot see through that is never 0: the branches on it are not taken and only end the basic blocks.
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);   // see umma_desc_lo
+__device__ __forceinline__ void umma4_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc,
                                              uint32_t accumulate, uint32_t never) {
     asm volatile(
-        "{\n .reg .pred p, t, q;\n .reg .b64 b1, b2, b3;\n .reg .b32 a1, a2, a3;\n"
+        "{\n .reg .pred p, t, q;\n .reg .b64 b0, b1, b2, b3;\n .reg .b32 a1, a2, a3, l1, l2, l3;\n"
         " setp.ne.b32 p, %4, 0;\n setp.eq.b32 t, 0, 0;\n setp.eq.b32 q, %5, 0;\n"
-        " add.u64 b1, %2, 2;\n add.u64 b2, %2, 4;\n add.u64 b3, %2, 6;\n"
+        " add.u32 l1, %2, 2;\n add.u32 l2, %2, 4;\n add.u32 l3, %2, 6;\n"
+        " mov.b64 b0, {%2, %6};\n mov.b64 b1, {l1, %6};\n mov.b64 b2, {l2, %6};\n mov.b64 b3, {l3, %6};\n"
         " add.u32 a1, %1, 8;\n add.u32 a2, %1, 16;\n add.u32 a3, %1, 24;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n @q bra DONE;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b0, %3, p;\n @q bra DONE;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n @q bra DONE;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, t;\n @q bra DONE;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, t;\n DONE:\n}" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(never)
+        "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(never), "n"(kDescHi)
         : "memory");
 }
-// The same four MMAs with both operands in shared memory (128-byte swizzled K-major tiles).
-__device__ __forceinline__ void umma4_f16_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+__device__ __forceinline__ void umma4_f16_ss(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
                                              uint32_t accumulate, uint32_t never) {
     asm volatile(
-        "{\n .reg .pred p, t, q;\n .reg .b64 a1, a2, a3, b1, b2, b3;\n"
+        "{\n .reg .pred p, t, q;\n .reg .b64 a0, a1, a2, a3, b0, b1, b2, b3;\n .reg .b32 k1, k2, k3, l1, l2, l3;\n"
         " setp.ne.b32 p, %4, 0;\n setp.eq.b32 t, 0, 0;\n setp.eq.b32 q, %5, 0;\n"
-        " add.u64 b1, %2, 2;\n add.u64 b2, %2, 4;\n add.u64 b3, %2, 6;\n"
-        " add.u64 a1, %1, 2;\n add.u64 a2, %1, 4;\n add.u64 a3, %1, 6;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n @q bra DONE;\n"
+        " add.u32 l1, %2, 2;\n add.u32 l2, %2, 4;\n add.u32 l3, %2, 6;\n"
+        " add.u32 k1, %1, 2;\n add.u32 k2, %1, 4;\n add.u32 k3, %1, 6;\n"
+        " mov.b64 b0, {%2, %6};\n mov.b64 b1, {l1, %6};\n mov.b64 b2, {l2, %6};\n mov.b64 b3, {l3, %6};\n"
+        " mov.b64 a0, {%1, %6};\n mov.b64 a1, {k1, %6};\n mov.b64 a2, {k2, %6};\n mov.b64 a3, {k3, %6};\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], a0, b0, %3, p;\n @q bra DONE;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, t;\n @q bra DONE;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, t;\n @q bra DONE;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, t;\n DONE:\n}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(never)
+        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(never), "n"(kDescHi)
         : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(e));
+    return e != 0u;
 }
 // This thread's 32 words -> 32 consecutive columns of its tensor-memory lane.
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t v[32]) {
@@ -433,48 +439,55 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
         }
     } else if (warp == 1 || warp == 3) {
         // ---------------------------------------------------------------- MMA issuers
-        const uint32_t mi = warp == 3 ? 1u : 0u;   // which weight tile of the stage this thread feeds
-        if (lane == 0 && (DUAL || mi == 0u)) {
+        const uint32_t mi = warp == 3 ? 1u : 0u;   // which weight tile of the stage this warp feeds
+        if (DUAL || mi == 0u) {
+            // the whole warp walks the loop (see umma4_f16_ts): every loop condition is a vote or comes from lane 0
+            auto uni = [](uint32_t v) { return __shfl_sync(0xFFFFFFFFu, v, 0); };
+            auto all = [](bool b) { return __all_sync(0xFFFFFFFFu, b); };
+            const bool el = elect_one();
+            const uint32_t tm = uni(tmem_base), tiles = uni(total);
             Ring<kAStages> ra;
             Ring<kBStages> rb;
             Ring<kAccBufs> rc;
-            const uint64_t bdesc0 = umma_desc_sw128(smem_u32(b_base));
-            const uint64_t adesc0 = umma_desc_sw128(smem_u32(arena) + mi * kBfATile);
+            const uint32_t b_lo0 = umma_desc_lo(smem_u32(b_base));
+            const uint32_t a_lo0 = umma_desc_lo(smem_u32(arena) + mi * kBfATile);
             bool ok = true;
             TileInfo t, tn;
-            bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat);
-            for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
-                const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
-                if (!mbar_wait(&S.acc_empty[rc.i], rc.ph ^ 1u, abort_flag)) { ok = false; break; }
+            tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat);
+            for (uint32_t tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
+                tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
+                const uint32_t rows = uni(t.n);
+                if (!all(mbar_wait(&S.acc_empty[rc.i], rc.ph ^ 1u, abort_flag))) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t n = SPLIT ? 32u << box_of(t.n) : (t.n + 15u) & ~15u;
+                const uint32_t n = SPLIT ? 32u << box_of(rows) : (rows + 15u) & ~15u;
                 const uint32_t idesc = umma_idesc_f16(n, BF ? 1u : 0u);
-                const uint32_t d = tmem_base + rc.i * (2u * NT) + mi * NT;
+                const uint32_t d = tm + rc.i * (2u * NT) + mi * NT;
                 for (uint32_t ks = 0; ks < k_stages; ++ks) {
-                    if (!mbar_wait(&S.full_a[ra.i], ra.ph, abort_flag) || !mbar_wait(&S.full_b[rb.i], rb.ph, abort_flag)) {
-                        ok = false;
-                        break;
-                    }
+                    const bool got = mbar_wait(&S.full_a[ra.i], ra.ph, abort_flag) && mbar_wait(&S.full_b[rb.i], rb.ph, abort_flag);
+                    if (!all(got)) { ok = false; break; }
                     tc_fence_after();
-                    const uint64_t bdesc = bdesc0 + rb.i * (G::kBTile >> 4);
-                    const uint64_t adesc = adesc0 + ra.i * (kBfAStage >> 4);
-                    const uint32_t ta = tmem_base + kAccCols + ra.i * G::kAStageCols + mi * (kKst / 2u);
+                    const uint32_t b_lo = b_lo0 + rb.i * (G::kBTile >> 4);
+                    const uint32_t a_lo = a_lo0 + ra.i * (kBfAStage >> 4);
+                    const uint32_t ta = tm + kAccCols + ra.i * G::kAStageCols + mi * (kKst / 2u);
+                    if (el) {
 #pragma unroll
-                    for (uint32_t h = 0; h < kSlabs; ++h) {
-                        if (BF) umma4_f16_ss(d, adesc + h * (kATile >> 4), bdesc + h * (NT * 128u >> 4), idesc, h ? 1u : ks, a.H);
-                        else umma4_f16_ts(d, ta + h * (kBK / 2u), bdesc + h * (NT * 128u >> 4), idesc, h ? 1u : ks, a.H);
+                        for (uint32_t h = 0; h < kSlabs; ++h) {
+                            if (BF) umma4_f16_ss(d, a_lo + h * (kATile >> 4), b_lo + h * (NT * 128u >> 4), idesc, h ? 1u : ks, a.H);
+                            else umma4_f16_ts(d, ta + h * (kBK / 2u), b_lo + h * (NT * 128u >> 4), idesc, h ? 1u : ks, a.H);
+                        }
+                        umma_commit(&S.empty_a[ra.i]);  // a stage is free once both issuers' MMAs have read it
+                        umma_commit(&S.empty_b[rb.i]);
                     }
-                    umma_commit(&S.empty_a[ra.i]);  // a stage is free once both issuers' MMAs have read it
-                    umma_commit(&S.empty_b[rb.i]);
+                    __syncwarp();
                     ra.next();
                     rb.next();
                 }
-                if (ok) umma_commit(&S.acc_full[rc.i]);
+                if (ok && el) umma_commit(&S.acc_full[rc.i]);
+                __syncwarp();
                 rc.next();
                 t = tn;
-                have = hn;
             }
-            if (!ok) { *abort_flag = 1; atomicOr(a.status, kStatusWaitTimeout); }
+            if (!ok && lane == 0) { *abort_flag = 1; atomicOr(a.status, kStatusWaitTimeout); }
         }
     } else if (warp == 2) {
         // ---------------------------------------------------------------- TMA producer: weights
