@@ -1,5 +1,6 @@
 // Host side of the C ABI declared in include/strata_moe.h: contexts, resident weights,
 // workspaces and the launch sequence of one MoE layer.
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -32,6 +33,7 @@ struct strata_moe_ctx {
     bool pev_valid = false;
     unsigned long long launches_at_create = 0;
     unsigned long long* d_router_rechecks = nullptr;   // tokens the fast router handed to the canonical kernels
+    uint32_t* d_dsv4_tiny = nullptr;   // sticky: the exact mode saw activations below 2^-120 (see dsv4_exact.cu)
     uint64_t router_fast_tokens = 0;                    // tokens routed through the fast path
     // handle-based commands (strata_moe_command_*): an internal layer whose expert slots borrow the
     // uploaded weights named by the command in flight
@@ -325,7 +327,7 @@ int sync_tables(strata_moe_layer* L) {
     }
     // tensor maps of the packed weights for the tensor-core path's TMA producer
     L->wmaps_ok = false;
-    if (L->d.format != STRATA_MOE_FMT_BF16 && tensor_path_ok(L, L->d.format, L->d.intermediate)) {
+    if (tensor_path_ok(L, L->d.format, L->d.intermediate)) {
         struct alignas(64) Blob { unsigned char b[128]; };
         std::vector<Blob> maps((size_t)3 * n);
         bool ok = true;
@@ -334,7 +336,9 @@ int sync_tables(strata_moe_layer* L) {
             const uint32_t cols = r == STRATA_MOE_ROLE_DOWN ? L->d.intermediate : L->d.hidden;
             for (uint32_t e = 0; e < n && ok; ++e)
                 ok = L->tab[r].packed[e] && ((uintptr_t)L->tab[r].packed[e] & 15u) == 0 &&
-                     prefill_encode_weight_map(&maps[(size_t)r * n + e], L->tab[r].packed[e], rows, cols) == 0;
+                     (L->d.format == STRATA_MOE_FMT_BF16
+                          ? prefill_encode_weight_map_bf16(&maps[(size_t)r * n + e], L->tab[r].packed[e], rows, cols)
+                          : prefill_encode_weight_map(&maps[(size_t)r * n + e], L->tab[r].packed[e], rows, cols)) == 0;
         }
         if (ok) {
             CK(cudaMemcpy(L->d_wmaps, maps.data(), maps.size() * sizeof(Blob), cudaMemcpyHostToDevice));
@@ -378,7 +382,7 @@ bool all_registered(const strata_moe_layer* L, std::string* why) {
 
 // rows-per-expert threshold between the weight-streaming path and the tensor-core tile path
 bool use_prefill(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups) {
-    if (!tensor_path_ok(L, L->d.format, L->d.intermediate)) return false;
+    if (!tensor_path_ok(L, L->d.format, L->d.intermediate) || L->d.format == STRATA_MOE_FMT_BF16) return false;
     if (L->d.format == STRATA_MOE_FMT_MXFP4 && !L->f16_ok) return false;  // needs the f16 weight window
     if (!L->wmaps_ok) return false;
     // average rows per expert from which the tensor-core path wins (measured: FP4 formats cross over
@@ -386,6 +390,16 @@ bool use_prefill(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups) {
     const int thr = L->knobs.prefill_min_rows >= 0 ? L->knobs.prefill_min_rows
                                                    : (L->d.format == STRATA_MOE_FMT_INT4G128 ? 8 : 12);
     return (uint64_t)pairs >= (uint64_t)n_groups * (uint64_t)thr;
+}
+
+// BF16 experts on the tensor-core kernel, the activation between the projections as a BF16 hi + lo pair.  A tile is 128
+// weight rows over all of K, so the calls that fill the GPU with tiles three times over take it; with fewer the last
+// round of tiles would leave most SMs idle and the weight-streaming kernel, which splits finer, is faster.
+bool use_bf16_tiles(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups) {
+    if (L->d.format != STRATA_MOE_FMT_BF16 || !L->wmaps_ok || !tensor_path_ok(L, L->d.format, L->d.intermediate)) return false;
+    if (L->knobs.prefill_min_rows >= 0) return pairs >= n_groups * (uint64_t)L->knobs.prefill_min_rows;
+    const double active = n_groups * (1.0 - pow(1.0 - 1.0 / n_groups, (double)pairs));   // groups with rows under even routing
+    return active * (L->d.intermediate / 128u) >= 3.0 * kNumSMs;
 }
 
 bool use_prefill_down(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups) {
@@ -512,6 +526,29 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         if (launch_prefill(p, L->xg, L->x_rowscale, L->act_hi, L->max_pairs, L->d_wmaps, s,
                            ctx->timing ? ctx->pev[5] : nullptr) != 0)
             return fail(ctx, STRATA_MOE_E_CUDA, "prefill launch failed");
+        mark(ctx, 6);
+        CK(cudaGetLastError());
+        return 0;
+    }
+    if (use_bf16_tiles(L, pairs, n_groups)) {
+        launch_gather_rows_plain(x_src, perm, k_div, bound, L->d.hidden, L->xg, s);
+        mark(ctx, 4);
+        PrefillArgs p{};
+        p.fmt = L->d.format;
+        p.H = L->d.hidden;
+        p.I = L->d.intermediate;
+        p.n_groups = n_groups;
+        p.pairs = pairs;
+        p.offsets = offsets;
+        p.y = y;
+        p.tile_table = static_cast<uint32_t*>(L->prefill_scratch);
+        p.status = ctx->d_status;
+        p.glu = GluParams{L->d.activation, L->d.gate_beta, L->d.linear_beta};
+        p.ntile = pairs <= 8u * n_groups ? 16u : (pairs <= 20u * n_groups ? 32u : 64u);
+        p.act_lo = L->act_lo;
+        if (launch_prefill(p, L->xg, nullptr, L->act_hi, L->max_pairs, L->d_wmaps, s, ctx->timing ? ctx->pev[5] : nullptr) != 0)
+            return fail(ctx, STRATA_MOE_E_CUDA, "BF16 expert launch failed");
+        if (y_half) *y_half = false;
         mark(ctx, 6);
         CK(cudaGetLastError());
         return 0;
@@ -761,6 +798,11 @@ int strata_moe_create(int device, void* stream, strata_moe_ctx** out) {
         strata_moe_destroy(ctx);
         return STRATA_MOE_E_CUDA;
     }
+    if (cudaMalloc(&ctx->d_dsv4_tiny, sizeof(uint32_t)) != cudaSuccess ||
+        cudaMemset(ctx->d_dsv4_tiny, 0, sizeof(uint32_t)) != cudaSuccess) {
+        strata_moe_destroy(ctx);
+        return STRATA_MOE_E_CUDA;
+    }
     ctx->launches_at_create = g_kernel_launches;
     *out = ctx;
     return 0;
@@ -789,6 +831,7 @@ void strata_moe_destroy(strata_moe_ctx* ctx) {
         p = nullptr;
     }
     if (ctx->d_status) cudaFree(ctx->d_status);
+    if (ctx->d_dsv4_tiny) cudaFree(ctx->d_dsv4_tiny);
     if (ctx->d_router_rechecks) cudaFree(ctx->d_router_rechecks);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
@@ -1677,11 +1720,12 @@ static int dsv4_grouped_core(strata_moe_layer* L, const float* rows_f32, const u
     const uint32_t H = L->d.hidden, I = L->d.intermediate, n = L->d.expert_count;
     float* xq = L->y;            // [pairs, H] scratch: the E4M3-quantised input rows
     float* act = L->act_f32;     // [pairs, I]
-    launch_dsv4_quantize(rows_f32, row_index, 1, pairs, H, xq, s);
+    uint32_t* tiny = ctx->d_dsv4_tiny;
+    launch_dsv4_quantize(rows_f32, row_index, 1, pairs, H, xq, s, tiny);
     launch_dsv4_gate_up(n, offsets, H, I, wt(L->tab[0]), wt(L->tab[1]), xq, coefficients, swiglu_limit, act,
-                        ctx->d_status, s);
-    launch_dsv4_quantize(act, nullptr, 1, pairs, I, act, s);
-    launch_dsv4_down(n, offsets, H, I, wt(L->tab[2]), act, y, ctx->d_status, s);
+                        ctx->d_status, s, tiny);
+    launch_dsv4_quantize(act, nullptr, 1, pairs, I, act, s, tiny);
+    launch_dsv4_down(n, offsets, H, I, wt(L->tab[2]), act, y, ctx->d_status, s, tiny);
     CK(cudaGetLastError());
     return 0;
 }
@@ -2207,10 +2251,10 @@ int strata_moe_command_enqueue_rows_dsv4(strata_moe_ctx* ctx, const float* hidde
         const uint32_t* off2 = d_off + n_slots + 1;
         WeightTable g{d_sp + 0, d_sp + 1, nullptr, nullptr, nullptr}, u{d_sp + 2, d_sp + 3, nullptr, nullptr, nullptr},
             dn{d_sp + 4, d_sp + 5, nullptr, nullptr, nullptr};
-        launch_dsv4_quantize(d_hidden, d_rows + pairs, 1, n_shared_rows, H, d_sx, s);
-        launch_dsv4_gate_up(1, off2, H, I, g, u, d_sx, nullptr, swiglu_limit, d_sact, ctx->d_status, s, true);
-        launch_dsv4_quantize(d_sact, nullptr, 1, n_shared_rows, I, d_sact, s);
-        launch_dsv4_down(1, off2, H, I, dn, d_sact, d_sy, ctx->d_status, s, true);
+        launch_dsv4_quantize(d_hidden, d_rows + pairs, 1, n_shared_rows, H, d_sx, s, ctx->d_dsv4_tiny);
+        launch_dsv4_gate_up(1, off2, H, I, g, u, d_sx, nullptr, swiglu_limit, d_sact, ctx->d_status, s, ctx->d_dsv4_tiny, true);
+        launch_dsv4_quantize(d_sact, nullptr, 1, n_shared_rows, I, d_sact, s, ctx->d_dsv4_tiny);
+        launch_dsv4_down(1, off2, H, I, dn, d_sact, d_sy, ctx->d_status, s, ctx->d_dsv4_tiny, true);
         CK(cudaGetLastError());
     }
     ctx->cmd_kind = 2;

@@ -271,14 +271,14 @@ void launch_ep_combine(const EpWindows& w, const EpPlan& pl, const float* shared
 
 // dsv4_exact.cu : bit-exact DeepSeek-V4 numerical mode (CUDA-core kernels, reference summation order)
 void launch_dsv4_quantize(const float* src, const uint32_t* perm, uint32_t k_div, uint32_t rows, uint32_t cols,
-                          float* dst, cudaStream_t s);
+                          float* dst, cudaStream_t s, uint32_t* tiny = nullptr);
 void launch_dsv4_gate_up(uint32_t n_groups, const uint32_t* offsets, uint32_t H, uint32_t I, const WeightTable& gate,
                          const WeightTable& up, const float* xq, const float* coef, float limit, float* act,
-                         uint32_t* status, cudaStream_t s, bool fp8 = false);
+                         uint32_t* status, cudaStream_t s, const uint32_t* tiny, bool fp8 = false);
 void launch_dsv4_join(const float* y, const uint32_t* inv, const float* shared, uint32_t T, uint32_t k, uint32_t H,
                       float* out, uint32_t* status, cudaStream_t s);
 void launch_dsv4_down(uint32_t n_groups, const uint32_t* offsets, uint32_t H, uint32_t I, const WeightTable& down,
-                      const float* actq, float* y, uint32_t* status, cudaStream_t s, bool fp8 = false);
+                      const float* actq, float* y, uint32_t* status, cudaStream_t s, const uint32_t* tiny, bool fp8 = false);
 
 // Launch counter (every wrapper above bumps it once per kernel launch; host threads of several
 // contexts share it).

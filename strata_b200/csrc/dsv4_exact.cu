@@ -13,10 +13,12 @@
 // partial sums in a fixed tree (five shuffle rounds per warp, then the eight warp sums).  The
 // result depends on that association, so this kernel keeps it and only changes who computes it:
 // ONE warp owns an output row; lane l plays the reference's threads 8l .. 8l+7 (eight
-// accumulators per token), which makes every weight load a contiguous 128 bytes per warp, and
-// up to four token rows of the expert share one pass over the weights.  The reduction tree is
-// evaluated in the same order with two shuffle rounds, three in-register rounds and the final
-// three rounds over the eight "warp" sums.
+// accumulators per token), which makes every weight load a contiguous 128 bytes per warp; a warp
+// works on four weight rows at once (an activation load serves all of them) and two token rows of
+// the expert share one pass over the weights.  The reduction tree is evaluated in the same order
+// with two shuffle rounds, three in-register rounds and the final three rounds over the eight
+// "warp" sums.  Bound by FP32 and conversion instructions: about 3 + T per weight and lane for T
+// token rows.
 #include "common.cuh"
 #include "libm_exact.cuh"
 
@@ -112,15 +114,14 @@ __device__ __forceinline__ float block_tree(float v[8], uint32_t lane) {
     return w;
 }
 
-constexpr int kRT = 4;   // token rows that share one pass over a weight row
-
 }  // namespace
 
 // ------------------------------------------------------------------------------ quantise
 // One warp per (row, 128-column block).  dst row pos <- src row (perm ? perm[pos] / k_div : pos).
 __global__ void __launch_bounds__(256) dsv4_quantize_kernel(const float* __restrict__ src,
                                                             const uint32_t* __restrict__ perm, uint32_t k_div,
-                                                            uint32_t rows, uint32_t cols, float* __restrict__ dst) {
+                                                            uint32_t rows, uint32_t cols, float* __restrict__ dst,
+                                                            uint32_t* tiny) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t blocks = (cols + 127u) / 128u;
     const size_t task = (size_t)blockIdx.x * 8u + (threadIdx.x >> 5);
@@ -140,6 +141,7 @@ __global__ void __launch_bounds__(256) dsv4_quantize_kernel(const float* __restr
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, off));
     const float scale = block_scale_dev(mx);
+    if (tiny != nullptr && lane == 0 && mx > 0.0f && scale < 7.5e-37f) *tiny = 1u;   // 2^-120: see dsv4_rows
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const uint32_t c = lane + 32u * i;
@@ -157,89 +159,179 @@ struct Dsv4Args {
     float limit;
     float* out;                // [pairs, R]
     uint32_t* status;
+    const uint32_t* tiny;      // nonzero: activations so small were seen that x * w may round (or nullptr: assume so)
 };
+
+constexpr uint32_t kDsv4Warps = 4, kDsv4Ctas = 3;   // warps per CTA, CTAs per SM (170 registers a thread: no spills)
+constexpr uint32_t kDsv4MaxGroups = 1024;
+
+// One warp, RW weight rows (DUAL: RW / 2 gate rows and the same up rows), NTOK token rows at `pos0` (only `cnt` of them
+// exist; the others repeat the last one and are dropped).
+//
+// The reference's step is sum = fma(x * w, scale, sum).  x has four significant bits, w two (FP4) or four (FP8) and
+// scale is a power of two, so x * w and w * scale are both exact and fma(x, w * scale, sum) rounds the same exact
+// number: one multiply per weight instead of one per weight and token.  That needs w * scale finite (scale byte below
+// 250) and x * w not below the subnormal grid; both are checked and the chunk takes the reference's two steps otherwise.
+template <bool DUAL, bool FP8, int RW, int NTOK>
+__device__ __forceinline__ void dsv4_rows(const Dsv4Args& a, uint32_t g, uint32_t row, size_t pos0, uint32_t cnt,
+                                          bool two_step, uint32_t lane, bool& bad) {
+    const uint32_t K = a.K;
+    constexpr int HALF = DUAL ? RW / 2 : RW;
+    const uint8_t *p[RW], *s[RW];
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+        const uint32_t rr = row + (uint32_t)(r % HALF);
+        const WeightTable& w = DUAL && r >= HALF ? a.w1 : a.w0;
+        p[r] = w.packed[g] + (FP8 ? (size_t)rr * K : (size_t)rr * (K / 2u)) + lane * (FP8 ? 8u : 4u);
+        s[r] = w.scales[g] + (FP8 ? (size_t)(rr / 128u) * ((K + 127u) / 128u) : (size_t)rr * (K / 32u));
+    }
+    const float* xr[NTOK];
+#pragma unroll
+    for (int k = 0; k < NTOK; ++k) xr[k] = a.x + (pos0 + min((uint32_t)k, cnt - 1u)) * K + lane * 8u;
+    float acc[RW][NTOK][8];
+#pragma unroll
+    for (int r = 0; r < RW; ++r)
+#pragma unroll
+        for (int k = 0; k < NTOK; ++k)
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc[r][k][q] = 0.0f;
+    // weights and scales of the next 256 columns are requested before the current ones are used
+    uint2 wq[RW];
+    uint32_t sq[RW];
+    auto load = [&](uint32_t c) {
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+            if (FP8) {
+                wq[r] = __ldg(reinterpret_cast<const uint2*>(p[r] + c));
+                sq[r] = __ldg(s[r] + (c + lane * 8u) / 128u);
+            } else {
+                wq[r].x = __ldg(reinterpret_cast<const uint32_t*>(p[r] + c / 2u));
+                sq[r] = __ldg(s[r] + (c + lane * 8u) / 32u);
+            }
+        }
+    };
+    const uint32_t end = K > lane * 8u ? K - lane * 8u : 0u;   // this lane's columns start below K
+    if (end) load(0);
+    for (uint32_t c = 0; c < end; c += 256u) {
+        float xv[NTOK][8];
+#pragma unroll
+        for (int k = 0; k < NTOK; ++k) {
+            const float4 xa = __ldg(reinterpret_cast<const float4*>(xr[k] + c));
+            const float4 xb = __ldg(reinterpret_cast<const float4*>(xr[k] + c) + 1);
+            xv[k][0] = xa.x; xv[k][1] = xa.y; xv[k][2] = xa.z; xv[k][3] = xa.w;
+            xv[k][4] = xb.x; xv[k][5] = xb.y; xv[k][6] = xb.z; xv[k][7] = xb.w;
+        }
+        uint2 w[RW];
+        uint32_t sb[RW];
+#pragma unroll
+        for (int r = 0; r < RW; ++r) { w[r] = wq[r]; sb[r] = sq[r]; }
+        if (c + 256u < end) load(c + 256u);
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+            float wv[8];
+            if (FP8) e4m3x8_f32(w[r], wv);
+            else e2m1x8_f32(w[r].x, wv);
+            const float sc = e8m0_dsv4(sb[r]);
+            if (two_step || sb[r] >= 250u) {
+#pragma unroll
+                for (int k = 0; k < NTOK; ++k)
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        acc[r][k][q] = __fmaf_rn(__fmul_rn(xv[k][q], wv[q]), sc, acc[r][k][q]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) wv[q] = __fmul_rn(wv[q], sc);
+#pragma unroll
+                for (int k = 0; k < NTOK; ++k)
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) acc[r][k][q] = __fmaf_rn(xv[k][q], wv[q], acc[r][k][q]);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NTOK; ++k) {
+        if ((uint32_t)k >= cnt) break;      // uniform across the warp
+        const size_t pos = pos0 + k;
+#pragma unroll
+        for (int r = 0; r < HALF; ++r) {
+            const float t0 = block_tree(acc[r][k], lane);
+            if (DUAL) {
+                const float t1 = block_tree(acc[r + (DUAL ? HALF : 0)][k], lane);
+                if (lane == 0) {
+                    const float g_r = bf16_round_dev(t0), u_r = bf16_round_dev(t1);
+                    if (!(fabsf(g_r) <= 3.0e38f) || !(fabsf(u_r) <= 3.0e38f)) bad = true;
+                    const float lg = fminf(g_r, a.limit);
+                    const float lu = fmaxf(-a.limit, fminf(u_r, a.limit));
+                    const float gt = __uint_as_float(__float_as_uint(lg) & 0xFFFF0000u);  // table index = top 16 bits
+                    const float silu = (fabsf(gt) <= 3.0e38f) ? __fmul_rn(gt, sigmoid_two_branch(gt)) : gt;
+                    float act = __fmul_rn(silu, lu);
+                    act = __fmul_rn(act, a.coef ? a.coef[pos] : 1.0f);
+                    a.out[pos * a.R + row + r] = bf16_round_dev(act);
+                }
+            } else if (lane == 0) {
+                a.out[pos * a.R + row + r] = bf16_round_dev(t0);
+            }
+        }
+    }
+}
 
 // FP8 = false: E2M1 nibbles + one E8M0 scale per 32 columns of a row.
 // FP8 = true : E4M3 bytes + one E8M0 scale per 128 x 128 block (scales [ceil(R / 128), ceil(K / 128)]).
+//
+// A warp takes four output rows of one expert with rows (gate/up: two of each).  Every CTA first compacts the list of
+// experts that have rows: walking all of them cost a chain of offset loads per empty expert and left most warps of a
+// small step with nothing else (4 tokens of 4096 x 2048 x 256 experts, 22 with rows: 0.86 ms per step before).
 template <bool DUAL, bool FP8>
-__global__ void __launch_bounds__(128) dsv4_rows_kernel(Dsv4Args a) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const size_t total = (size_t)a.n_groups * a.R;
-    const uint32_t K = a.K;
+__global__ void __launch_bounds__(kDsv4Warps * 32, kDsv4Ctas) dsv4_rows_kernel(Dsv4Args a) {
+    __shared__ uint16_t list[kDsv4MaxGroups];
+    __shared__ uint32_t warp_base[kDsv4Warps + 1];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const bool two_step = a.tiny == nullptr || *a.tiny != 0u;
     bool bad = false;
-    for (size_t task = (size_t)blockIdx.x * 4u + (threadIdx.x >> 5); task < total; task += (size_t)gridDim.x * 4u) {
-        const uint32_t g = (uint32_t)(task / a.R), row = (uint32_t)(task % a.R);
-        const uint32_t row0 = a.offsets[g], cnt = a.offsets[g + 1] - row0;
-        if (cnt == 0u) continue;
-        const size_t prow = FP8 ? (size_t)row * K : (size_t)row * (K / 2u);
-        const size_t srow = FP8 ? (size_t)(row / 128u) * ((K + 127u) / 128u) : (size_t)row * (K / 32u);
-        const uint8_t* p0 = a.w0.packed[g] + prow;
-        const uint8_t* s0 = a.w0.scales[g] + srow;
-        const uint8_t* p1 = DUAL ? a.w1.packed[g] + prow : nullptr;
-        const uint8_t* s1 = DUAL ? a.w1.scales[g] + srow : nullptr;
-        for (uint32_t tb = 0; tb < cnt; tb += kRT) {
-            float acc0[kRT][8], acc1[DUAL ? kRT : 1][8];
-#pragma unroll
-            for (int r = 0; r < kRT; ++r)
-#pragma unroll
-                for (int s = 0; s < 8; ++s) {
-                    acc0[r][s] = 0.0f;
-                    if (DUAL) acc1[r][s] = 0.0f;
-                }
-            for (uint32_t c0 = lane * 8u; c0 < K; c0 += 256u) {
-                float w0v[8], w1v[8];
-                float sc0, sc1 = 0.0f;
-                if (FP8) {
-                    e4m3x8_f32(__ldg(reinterpret_cast<const uint2*>(p0 + c0)), w0v);
-                    sc0 = e8m0_dsv4(__ldg(s0 + c0 / 128u));
-                    if (DUAL) {
-                        e4m3x8_f32(__ldg(reinterpret_cast<const uint2*>(p1 + c0)), w1v);
-                        sc1 = e8m0_dsv4(__ldg(s1 + c0 / 128u));
-                    }
+    for (uint32_t g0 = 0; g0 < a.n_groups; g0 += kDsv4MaxGroups) {
+        const uint32_t ng = min(kDsv4MaxGroups, a.n_groups - g0);
+        // ordered compaction: warp w scans groups [w * span, (w + 1) * span)
+        const uint32_t span = (ng + kDsv4Warps - 1u) / kDsv4Warps;
+        uint32_t mine = 0;
+        for (uint32_t q = 0; q < span; q += 32u) {
+            const uint32_t g = warp * span + q + lane;
+            const bool has = q + lane < span && g < ng && a.offsets[g0 + g + 1] != a.offsets[g0 + g];
+            mine += __popc(__ballot_sync(0xFFFFFFFFu, has));
+        }
+        if (lane == 0) warp_base[warp + 1u] = mine;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            warp_base[0] = 0;
+            for (uint32_t w = 0; w < kDsv4Warps; ++w) warp_base[w + 1u] += warp_base[w];
+        }
+        __syncthreads();
+        uint32_t at = warp_base[warp];
+        for (uint32_t q = 0; q < span; q += 32u) {
+            const uint32_t g = warp * span + q + lane;
+            const bool has = q + lane < span && g < ng && a.offsets[g0 + g + 1] != a.offsets[g0 + g];
+            const uint32_t b = __ballot_sync(0xFFFFFFFFu, has);
+            if (has) list[at + __popc(b & ((1u << lane) - 1u))] = (uint16_t)g;
+            at += __popc(b);
+        }
+        __syncthreads();
+        constexpr uint32_t RB = DUAL ? 2u : 4u;      // output rows per task (R is a multiple of 128)
+        const uint32_t per = a.R / RB, total = warp_base[kDsv4Warps] * per;
+        for (uint32_t task = blockIdx.x * kDsv4Warps + warp; task < total; task += gridDim.x * kDsv4Warps) {
+            const uint32_t slot = task / per, row = (task - slot * per) * RB;
+            const uint32_t g = g0 + list[slot];
+            const uint32_t row0 = a.offsets[g], cnt = a.offsets[g + 1] - row0;
+            for (uint32_t tb = 0; tb < cnt;) {
+                const uint32_t left = cnt - tb;
+                if (left == 1u) {
+                    dsv4_rows<DUAL, FP8, 4, 1>(a, g, row, (size_t)row0 + tb, 1u, two_step, lane, bad);
+                    tb += 1u;
                 } else {
-                    e2m1x8_f32(__ldg(reinterpret_cast<const uint32_t*>(p0 + c0 / 2u)), w0v);
-                    sc0 = e8m0_dsv4(__ldg(s0 + c0 / 32u));
-                    if (DUAL) {
-                        e2m1x8_f32(__ldg(reinterpret_cast<const uint32_t*>(p1 + c0 / 2u)), w1v);
-                        sc1 = e8m0_dsv4(__ldg(s1 + c0 / 32u));
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < kRT; ++r) {
-                    if (tb + r >= cnt) break;
-                    const float4* xp = reinterpret_cast<const float4*>(a.x + (size_t)(row0 + tb + r) * K + c0);
-                    const float4 xa = __ldg(xp), xb = __ldg(xp + 1);
-                    const float xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-#pragma unroll
-                    for (int s = 0; s < 8; ++s) {
-                        acc0[r][s] = __fmaf_rn(__fmul_rn(xv[s], w0v[s]), sc0, acc0[r][s]);
-                        if (DUAL) acc1[r][s] = __fmaf_rn(__fmul_rn(xv[s], w1v[s]), sc1, acc1[r][s]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < kRT; ++r) {
-                if (tb + r >= cnt) break;       // uniform across the warp
-                const size_t pos = (size_t)row0 + tb + r;
-                const float t0 = block_tree(acc0[r], lane);
-                if (DUAL) {
-                    const float t1 = block_tree(acc1[r], lane);
-                    if (lane == 0) {
-                        const float g_r = bf16_round_dev(t0), u_r = bf16_round_dev(t1);
-                        if (!(fabsf(g_r) <= 3.0e38f) || !(fabsf(u_r) <= 3.0e38f)) bad = true;
-                        const float lg = fminf(g_r, a.limit);
-                        const float lu = fmaxf(-a.limit, fminf(u_r, a.limit));
-                        const float gt = __uint_as_float(__float_as_uint(lg) & 0xFFFF0000u);  // table index = top 16 bits
-                        const float silu = (fabsf(gt) <= 3.0e38f) ? __fmul_rn(gt, sigmoid_two_branch(gt)) : gt;
-                        float act = __fmul_rn(silu, lu);
-                        act = __fmul_rn(act, a.coef ? a.coef[pos] : 1.0f);
-                        a.out[pos * a.R + row] = bf16_round_dev(act);
-                    }
-                } else if (lane == 0) {
-                    a.out[pos * a.R + row] = bf16_round_dev(t0);
+                    dsv4_rows<DUAL, FP8, 4, 2>(a, g, row, (size_t)row0 + tb, min(2u, left), two_step, lane, bad);
+                    tb += 2u;
                 }
             }
         }
+        __syncthreads();     // the list is rebuilt for the next block of groups
     }
     if (bad) atomicOr(a.status, kStatusNonFiniteOutput);
 }
@@ -281,31 +373,35 @@ void launch_dsv4_join(const float* y, const uint32_t* inv, const float* shared, 
 
 // ------------------------------------------------------------------------------ launchers
 void launch_dsv4_quantize(const float* src, const uint32_t* perm, uint32_t k_div, uint32_t rows, uint32_t cols,
-                          float* dst, cudaStream_t s) {
+                          float* dst, cudaStream_t s, uint32_t* tiny) {
     if (rows == 0 || cols == 0) return;
     const size_t tasks = (size_t)rows * ((cols + 127u) / 128u);
-    dsv4_quantize_kernel<<<(unsigned)((tasks + 7) / 8), 256, 0, s>>>(src, perm, k_div, rows, cols, dst);
+    dsv4_quantize_kernel<<<(unsigned)((tasks + 7) / 8), 256, 0, s>>>(src, perm, k_div, rows, cols, dst, tiny);
     ++g_kernel_launches;
+}
+
+// a full house of resident CTAs walks the tasks; fewer CTAs when even a full house of groups has fewer tasks
+static unsigned dsv4_grid(size_t tasks) {
+    const size_t ctas = (tasks + kDsv4Warps - 1) / kDsv4Warps;
+    return (unsigned)(ctas < (size_t)kNumSMs * kDsv4Ctas ? ctas : (size_t)kNumSMs * kDsv4Ctas);
 }
 
 void launch_dsv4_gate_up(uint32_t n_groups, const uint32_t* offsets, uint32_t H, uint32_t I, const WeightTable& gate,
                          const WeightTable& up, const float* xq, const float* coef, float limit, float* act,
-                         uint32_t* status, cudaStream_t s, bool fp8) {
-    Dsv4Args a{n_groups, H, I, offsets, gate, up, xq, coef, limit, act, status};
-    const size_t warps = (size_t)n_groups * I;
-    const unsigned grid = (unsigned)((warps + 3) / 4 < (size_t)kNumSMs * 16u ? (warps + 3) / 4 : (size_t)kNumSMs * 16u);
-    if (fp8) dsv4_rows_kernel<true, true><<<grid, 128, 0, s>>>(a);
-    else dsv4_rows_kernel<true, false><<<grid, 128, 0, s>>>(a);
+                         uint32_t* status, cudaStream_t s, const uint32_t* tiny, bool fp8) {
+    Dsv4Args a{n_groups, H, I, offsets, gate, up, xq, coef, limit, act, status, tiny};
+    const unsigned grid = dsv4_grid((size_t)n_groups * (I / 2u));
+    if (fp8) dsv4_rows_kernel<true, true><<<grid, kDsv4Warps * 32, 0, s>>>(a);
+    else dsv4_rows_kernel<true, false><<<grid, kDsv4Warps * 32, 0, s>>>(a);
     ++g_kernel_launches;
 }
 
 void launch_dsv4_down(uint32_t n_groups, const uint32_t* offsets, uint32_t H, uint32_t I, const WeightTable& down,
-                      const float* actq, float* y, uint32_t* status, cudaStream_t s, bool fp8) {
-    Dsv4Args a{n_groups, I, H, offsets, down, down, actq, nullptr, 0.0f, y, status};
-    const size_t warps = (size_t)n_groups * H;
-    const unsigned grid = (unsigned)((warps + 3) / 4 < (size_t)kNumSMs * 16u ? (warps + 3) / 4 : (size_t)kNumSMs * 16u);
-    if (fp8) dsv4_rows_kernel<false, true><<<grid, 128, 0, s>>>(a);
-    else dsv4_rows_kernel<false, false><<<grid, 128, 0, s>>>(a);
+                      const float* actq, float* y, uint32_t* status, cudaStream_t s, const uint32_t* tiny, bool fp8) {
+    Dsv4Args a{n_groups, I, H, offsets, down, down, actq, nullptr, 0.0f, y, status, tiny};
+    const unsigned grid = dsv4_grid((size_t)n_groups * (H / 4u));
+    if (fp8) dsv4_rows_kernel<false, true><<<grid, kDsv4Warps * 32, 0, s>>>(a);
+    else dsv4_rows_kernel<false, false><<<grid, kDsv4Warps * 32, 0, s>>>(a);
     ++g_kernel_launches;
 }
 
