@@ -1348,7 +1348,8 @@ int strata_moe_forward(strata_moe_layer* L, const void* x, uint32_t T, float* ou
         launch_router_logits(xb, L->router, T, d.hidden, d.experts, lg, s, ctx->d_status);
         mark(ctx, 1);
         front_done = launch_front_small(rp, lg, L->bias, T, ids, w, counts, offsets, perm, L->inv, L->active, L->n_active,
-                                        xb, d.hidden, convert ? L->xg : nullptr, L->x_rowscale, ctx->d_status, s);
+                                        xb, d.hidden, convert ? L->xg : nullptr, L->x_rowscale, d.format == STRATA_MOE_FMT_INT4G128,
+                                        ctx->d_status, s);
         if (front_done) {
             x_ready = convert;
             mark(ctx, 2);

@@ -930,7 +930,7 @@ __global__ void __launch_bounds__(kFrontWarps * 32) front_small_kernel(
     uint32_t* __restrict__ ids, float* __restrict__ weights, uint32_t* __restrict__ counts,
     uint32_t* __restrict__ offsets, uint32_t* __restrict__ perm, uint32_t* __restrict__ inv,
     uint32_t* __restrict__ active_list, uint32_t* __restrict__ n_active, const __nv_bfloat16* __restrict__ x, uint32_t H,
-    __half* __restrict__ xg, float* __restrict__ x_rowscale, uint32_t* status) {
+    __half* __restrict__ xg, float* __restrict__ x_rowscale, bool int4_order, uint32_t* status) {
     extern __shared__ float fsm2[];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t E = p.experts, k = p.top_k, P = T * k;
@@ -1005,14 +1005,14 @@ __global__ void __launch_bounds__(kFrontWarps * 32) front_small_kernel(
     __syncthreads();
     if (xg != nullptr)
         for (uint32_t pos = warp; pos < P; pos += kFrontWarps)
-            warp_row_to_f16_bf16(x + (size_t)(perm_s[pos] / k) * H, H, xg + (size_t)pos * H, x_rowscale + pos);
+            warp_row_to_f16_bf16(x + (size_t)(perm_s[pos] / k) * H, H, xg + (size_t)pos * H, x_rowscale + pos, int4_order);
 }
 
 // false: the shape is outside the kernel's limits and nothing was launched
 bool launch_front_small(const RouterParams& p, const float* logits, const float* bias, uint32_t T, uint32_t* ids,
                         float* weights, uint32_t* counts, uint32_t* offsets, uint32_t* perm, uint32_t* inv,
                         uint32_t* active_list, uint32_t* n_active, const __nv_bfloat16* x, uint32_t H, void* xg,
-                        float* x_rowscale, uint32_t* status, cudaStream_t s) {
+                        float* x_rowscale, bool int4_order, uint32_t* status, cudaStream_t s) {
     if (T == 0 || T > kFrontWarps || T * p.top_k > kFrontMaxPairs || p.experts > kFrontMaxExperts || p.top_k > 32u)
         return false;
     if (xg != nullptr && (H % 8u || (((uintptr_t)x | (uintptr_t)xg) & 15u))) return false;
@@ -1029,7 +1029,7 @@ bool launch_front_small(const RouterParams& p, const float* logits, const float*
     }
     front_small_kernel<<<1, kFrontWarps * 32, smem, s>>>(p, logits, bias, T, ids, weights, counts, offsets, perm, inv,
                                                          active_list, n_active, x, H, static_cast<__half*>(xg),
-                                                         x_rowscale, status);
+                                                         x_rowscale, int4_order, status);
     ++g_kernel_launches;
     return true;
 }

@@ -1,0 +1,61 @@
+"""Tile geometries of the tensor-core expert kernel at their edges, against the CPU oracle (needs a B200)."""
+import numpy as np
+import pytest
+
+from strata_b200 import MoeContext, MoeLayer, synth
+from tests import helpers as Hh
+
+pytestmark = pytest.mark.gpu
+
+# One f16 rounding per SwiGLU output and, for the formats with a block scale, one per decoded weight (2^-12 each, a sum
+# of independent errors): 1e-3 holds all of it.  BF16 experts carry the SwiGLU output as a BF16 pair (2^-17): what is
+# left is FP32 summation order.
+TOL_F16, TOL_PAIR = 1e-3, 1e-4
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    return MoeContext(0)
+
+
+def check(ctx, cfg, tol):
+    layer = synth.build_layer(cfg, "cuda")
+    ml = MoeLayer(ctx, cfg)
+    ml.load_synth(layer)
+    out, aux = ml.forward(layer.x, want_aux=True)
+    ctx.synchronize()
+    ref = Hh.run_oracle(cfg, layer.x.cpu())
+    assert np.array_equal(aux["perm"].cpu().numpy().astype(np.uint32), ref["perm"])
+    rel, mx = Hh.error_metrics(out.cpu().numpy(), ref["out"])
+    assert rel <= tol and mx <= 2.0 ** -6, (rel, mx)
+    return aux["counts"].cpu().numpy()
+
+
+def config(fmt, T, E, k, H=512, I=256):
+    return synth.MoeConfig(f"tiles{fmt}_{T}", H=H, I=I, E=E, k=k, fmt=fmt, T=T, seed=11)
+
+
+@pytest.mark.parametrize("T,E,k", [(8, 8, 8), (16, 16, 8), (5, 4, 3)])
+def test_int4_decode_batch_on_tensor_tiles(ctx, T, E, k, monkeypatch):
+    # at most 16 tokens: the fused front end converts the rows, and the tiles read INT4 columns in their own order
+    monkeypatch.setenv("STRATA_MOE_PREFILL_MIN_ROWS", "1")
+    check(ctx, config(synth.FMT_INT4, T, E, k), TOL_F16)
+
+
+@pytest.mark.parametrize("H", [512, 384])       # 384: single weight tiles in the down projection, half a block at the end
+@pytest.mark.parametrize("fmt", [synth.FMT_MXFP4, synth.FMT_NVFP4, synth.FMT_INT4])
+@pytest.mark.parametrize("ntile,T", [(32, 33), (64, 65), (128, 129), (160, 161), (192, 193)])
+def test_one_row_beyond_a_tile(ctx, fmt, ntile, T, H, monkeypatch):
+    # every token visits both experts: a full tile and a tile of one row each
+    monkeypatch.setenv("STRATA_MOE_PREFILL_MIN_ROWS", "1")
+    monkeypatch.setenv("STRATA_MOE_PREFILL_NTILE", str(ntile))
+    counts = check(ctx, config(fmt, T, 2, 2, H=H), TOL_F16)
+    assert counts.tolist() == [T, T]
+
+
+@pytest.mark.parametrize("H", [512, 384])
+@pytest.mark.parametrize("T,E,k", [(3, 16, 2), (17, 2, 2), (33, 8, 4), (65, 2, 2), (130, 2, 2)])
+def test_bf16_expert_tiles(ctx, T, E, k, H, monkeypatch):
+    # tiles of 16, 32 and 64 token rows (hi + lo pairs), one row beyond them, empty groups
+    monkeypatch.setenv("STRATA_MOE_PREFILL_MIN_ROWS", "0")
+    check(ctx, config(synth.FMT_BF16, T, E, k, H=H), TOL_PAIR)
