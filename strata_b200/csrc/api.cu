@@ -33,7 +33,7 @@ struct strata_moe_ctx {
     bool pev_valid = false;
     unsigned long long launches_at_create = 0;
     unsigned long long* d_router_rechecks = nullptr;   // tokens the fast router handed to the canonical kernels
-    uint32_t* d_dsv4_tiny = nullptr;   // sticky: the exact mode saw activations below 2^-120 (see dsv4_exact.cu)
+    uint32_t* d_dsv4_tiny = nullptr;   // sticky: the exact mode saw activations outside 2^-120 .. 2^109 (see dsv4_exact.cu)
     uint64_t router_fast_tokens = 0;                    // tokens routed through the fast path
     // handle-based commands (strata_moe_command_*): an internal layer whose expert slots borrow the
     // uploaded weights named by the command in flight

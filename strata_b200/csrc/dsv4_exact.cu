@@ -141,7 +141,8 @@ __global__ void __launch_bounds__(256) dsv4_quantize_kernel(const float* __restr
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, off));
     const float scale = block_scale_dev(mx);
-    if (tiny != nullptr && lane == 0 && mx > 0.0f && scale < 7.5e-37f) *tiny = 1u;   // 2^-120: see dsv4_rows
+    // below 2^-120 or above 2^109: see dsv4_rows
+    if (tiny != nullptr && lane == 0 && mx > 0.0f && !(scale >= 7.5e-37f && scale <= 6.4e32f)) *tiny = 1u;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const uint32_t c = lane + 32u * i;
@@ -159,7 +160,7 @@ struct Dsv4Args {
     float limit;
     float* out;                // [pairs, R]
     uint32_t* status;
-    const uint32_t* tiny;      // nonzero: activations so small were seen that x * w may round (or nullptr: assume so)
+    const uint32_t* tiny;      // nonzero: activations so small or large were seen that x * w may round or overflow (or nullptr: assume so)
 };
 
 constexpr uint32_t kDsv4Warps = 4, kDsv4Ctas = 3;   // warps per CTA, CTAs per SM (170 registers a thread: no spills)
@@ -170,8 +171,10 @@ constexpr uint32_t kDsv4MaxGroups = 1024;
 //
 // The reference's step is sum = fma(x * w, scale, sum).  x has four significant bits, w two (FP4) or four (FP8) and
 // scale is a power of two, so x * w and w * scale are both exact and fma(x, w * scale, sum) rounds the same exact
-// number: one multiply per weight instead of one per weight and token.  That needs w * scale finite (scale byte below
-// 250) and x * w not below the subnormal grid; both are checked and the chunk takes the reference's two steps otherwise.
+// number: one multiply per weight instead of one per weight and token.  That needs w * scale finite (6 * 2^(byte - 127)
+// for FP4, 448 * 2^(byte - 127) for FP8: bytes below 250 / 247) and x * w neither below the subnormal grid nor beyond the
+// largest float (x is at most 448 block scales and w at most 448: scales up to 2^109); all are checked and the chunk
+// takes the reference's two steps otherwise.
 template <bool DUAL, bool FP8, int RW, int NTOK>
 __device__ __forceinline__ void dsv4_rows(const Dsv4Args& a, uint32_t g, uint32_t row, size_t pos0, uint32_t cnt,
                                           bool two_step, uint32_t lane, bool& bad) {
@@ -232,7 +235,7 @@ __device__ __forceinline__ void dsv4_rows(const Dsv4Args& a, uint32_t g, uint32_
             if (FP8) e4m3x8_f32(w[r], wv);
             else e2m1x8_f32(w[r].x, wv);
             const float sc = e8m0_dsv4(sb[r]);
-            if (two_step || sb[r] >= 250u) {
+            if (two_step || sb[r] >= (FP8 ? 247u : 250u)) {
 #pragma unroll
                 for (int k = 0; k < NTOK; ++k)
 #pragma unroll

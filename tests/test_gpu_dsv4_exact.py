@@ -72,6 +72,52 @@ def test_grouped_experts_bit_exact(ctx, H, I, E, counts):
     assert np.abs(got).max() > 0
 
 
+@pytest.mark.parametrize("magnitude,shift", [(3e-38, 100), (1e-30, 75), (1e25, -80)])
+def test_grouped_experts_bit_exact_at_extreme_magnitudes(magnitude, shift):
+    """Gate and up scales moved by 2^shift bring the result back.  Activations whose products with the weights are subnormal or huge, rows spread over few of many experts."""
+    ctx = MoeContext(0)      # the range flag is sticky: keep it out of the other tests
+    H, I, E = 256, 128, 70
+    cfg = synth.MoeConfig("dsv4rng", H=H, I=I, E=E, k=2, fmt=synth.FMT_MXFP4, T=8, seed=29)
+    layer = synth.build_layer(cfg, "cuda")
+    for r in ("gate", "up"):
+        layer.scales[r] = (layer.scales[r].int() + shift).to(torch.uint8)
+    ml = MoeLayer(ctx, cfg, max_tokens=16)
+    ml.load_synth(layer)
+    counts = np.zeros(E, np.int32)
+    counts[[0, 17, 18, 35, 69]] = [1, 2, 1, 3, 1]
+    offsets = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    x = (np.random.default_rng(3).standard_normal((int(counts.sum()), H)) * magnitude).astype(np.float32)
+    y = ml.experts_grouped_dsv4(torch.from_numpy(x).cuda(), torch.from_numpy(offsets).cuda(), None, swiglu_limit=10.0)
+    ctx.synchronize()
+    got, port, scratch, pos = y.cpu().numpy(), O.port(), np.empty(I, np.float32), 0
+    for e in np.flatnonzero(counts):
+        args = [a for r in ("gate", "up", "down") for a in (layer.packed[r][e], layer.scales[r][e])]
+        args = [a.cpu().numpy().reshape(-1) for a in args]
+        for _ in range(counts[e]):
+            want = np.empty(H, np.float32)
+            assert port.orc_dsv4_expert(_p(want, f32p), _p(x[pos], f32p), *[_p(a, u8p) for a in args], H, I, 1.0, 10.0,
+                                        _p(scratch, f32p)) == 0
+            assert np.array_equal(got[pos].view(np.uint32), want.view(np.uint32)), (e, pos)
+            pos += 1
+    assert np.abs(got).max() > 0
+
+
+def test_overflowing_product_is_reported():
+    """The reference multiplies activation and weight first: 1e38 x 6 overflows although the block scale would bring the
+    product back into range, and the call reports a non-finite value."""
+    from strata_b200 import StrataMoeError
+    ctx = MoeContext(0)
+    cfg = synth.MoeConfig("dsv4inf", H=256, I=128, E=2, k=1, fmt=synth.FMT_MXFP4, T=2, seed=31)
+    layer = synth.build_layer(cfg, "cuda")
+    ml = MoeLayer(ctx, cfg, max_tokens=4)
+    ml.load_synth(layer)
+    x = torch.zeros(1, 256, device="cuda")
+    x[0, 0] = 1e38
+    with pytest.raises(StrataMoeError):
+        ml.experts_grouped_dsv4(x, torch.tensor([0, 1, 1], dtype=torch.int32, device="cuda"))
+        ctx.synchronize()
+
+
 def test_rejects_other_formats(ctx):
     from strata_b200 import StrataMoeError
     cfg = synth.MoeConfig("dsv4x_nv", H=256, I=128, E=2, k=1, fmt=synth.FMT_NVFP4, T=2, seed=1)
