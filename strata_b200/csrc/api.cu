@@ -72,13 +72,12 @@ struct LayerKnobs {
     bool no_f16_path = false;       // STRATA_MOE_NO_F16_PATH: FP4 formats use the general BF16 decoders
     bool no_prefill_path = false;   // STRATA_MOE_NO_PREFILL_PATH: never use the tensor-core tile path
     bool no_stream_ring = false;    // STRATA_MOE_NO_STREAM_RING: small batches use the register-streaming kernels
+    bool no_pair_tiles = false;     // STRATA_MOE_NO_PAIR_TILES: small groups never take the tensor-core tiles
     bool no_half_y = false;         // STRATA_MOE_NO_HALF_Y: the tensor-core down kernel always stores fp32 expert rows
     bool no_small_front = false;    // STRATA_MOE_NO_SMALL_FRONT: decode batches keep the separate route / group / convert kernels
     int prefill_min_rows = -1;      // STRATA_MOE_PREFILL_MIN_ROWS: average rows per expert for the tensor-core path
-    int prefill_down_min_rows = -1; // STRATA_MOE_PREFILL_DOWN_MIN_ROWS
-    int prefill_ntile = 0;          // STRATA_MOE_PREFILL_NTILE: 128, 160 or 192
-    int mixed_min_rows = -1;        // STRATA_MOE_MIXED_MIN_ROWS
-    int mixed_min_tokens = -1;      // STRATA_MOE_MIXED_MIN_TOKENS
+    int prefill_ntile = 0;          // STRATA_MOE_PREFILL_NTILE: 32, 64, 128, 160 or 192
+    int pair_ntile = 0;             // STRATA_MOE_PAIR_NTILE: token rows per tile (16, 32 or 64) of the paired-activation tiles
     int fast_router_min_tokens = 0; // STRATA_MOE_FAST_ROUTER_MIN_TOKENS: 0 = default (512), negative = never
     int no_spread = 0;              // STRATA_MOE_NO_SPREAD=1: operand conversion per grouped row instead of per source row
     int host_chunks = 0;            // STRATA_MOE_HOST_CHUNKS: token chunks of a host-buffer call (0 = chosen from the rows per expert)
@@ -95,11 +94,10 @@ static LayerKnobs read_knobs() {
     k.no_prefill_path = getenv("STRATA_MOE_NO_PREFILL_PATH") != nullptr;
     k.no_stream_ring = getenv("STRATA_MOE_NO_STREAM_RING") != nullptr;
     k.prefill_min_rows = num("STRATA_MOE_PREFILL_MIN_ROWS", -1);
-    k.prefill_down_min_rows = num("STRATA_MOE_PREFILL_DOWN_MIN_ROWS", -1);
     k.prefill_ntile = num("STRATA_MOE_PREFILL_NTILE", 0);
-    k.mixed_min_rows = num("STRATA_MOE_MIXED_MIN_ROWS", -1);
-    k.mixed_min_tokens = num("STRATA_MOE_MIXED_MIN_TOKENS", -1);
+    k.pair_ntile = num("STRATA_MOE_PAIR_NTILE", 0);
     k.no_small_front = getenv("STRATA_MOE_NO_SMALL_FRONT") != nullptr;
+    k.no_pair_tiles = getenv("STRATA_MOE_NO_PAIR_TILES") != nullptr;
     k.no_half_y = getenv("STRATA_MOE_NO_HALF_Y") != nullptr;
     k.fast_router_min_tokens = num("STRATA_MOE_FAST_ROUTER_MIN_TOKENS", 0);
     k.stream_ring_max_rows = num("STRATA_MOE_STREAM_RING_MAX_ROWS", 8);
@@ -144,6 +142,7 @@ struct strata_moe_layer {
     bool wmaps_ok = false;
     // f16 decode path for the FP4 formats
     bool f16_ok = false;
+    bool int4_f16_ok = false;   // every INT4 weight q * scale is exact in f16
     bool stream_ok = false;   // shapes and alignments allow the TMA ring kernels
     uint8_t* arena_cur = nullptr;   // weight arena: next free byte of the newest chunk (chunks are in `owned`)
     size_t arena_left = 0, arena_next = 4u << 20;
@@ -307,6 +306,24 @@ int sync_tables(strata_moe_layer* L) {
         }
     }
     if (L->knobs.no_f16_path) L->f16_ok = false;
+    L->int4_f16_ok = false;
+    if (L->d.format == STRATA_MOE_FMT_INT4G128) {
+        bool complete = true;
+        for (int r = 0; r < 3; ++r)
+            for (uint32_t e = 0; e < n; ++e) complete &= L->tab[r].scales[e] != nullptr;
+        if (complete) {
+            CK(cudaMemsetAsync(L->d_not_ok, 0, sizeof(uint32_t), ctx->stream));
+            for (int r = 0; r < 3; ++r) {
+                const uint32_t rows = r == STRATA_MOE_ROLE_DOWN ? L->d.hidden : L->d.intermediate;
+                const uint32_t cols = r == STRATA_MOE_ROLE_DOWN ? L->d.intermediate : L->d.hidden;
+                launch_int4_scale_range(L->tab[r].d_scales, n, scale_bytes(L->d.format, rows, cols) / 2u, L->d_not_ok, ctx->stream);
+            }
+            uint32_t not_ok = 1;
+            CK(cudaMemcpyAsync(&not_ok, L->d_not_ok, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+            CK(cudaStreamSynchronize(ctx->stream));
+            L->int4_f16_ok = not_ok == 0;
+        }
+    }
     // the bulk-copy ring needs 16-byte aligned packed rows and scale rows
     L->stream_ok = L->f16_ok && !L->knobs.no_stream_ring &&
                    decode_stream_supported(L->d.format, L->d.hidden, L->d.intermediate);
@@ -402,34 +419,48 @@ bool use_bf16_tiles(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups
     return active * (L->d.intermediate / 128u) >= 3.0 * kNumSMs;
 }
 
-bool use_prefill_down(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups) {
-    if (!tensor_path_ok(L, L->d.format, L->d.intermediate) || !L->f16_ok || !L->wmaps_ok) return false;
-    const int thr = L->knobs.prefill_down_min_rows >= 0 ? L->knobs.prefill_down_min_rows : 8;
-    return (uint64_t)pairs >= (uint64_t)n_groups * (uint64_t)thr;
+// Ring kernels for decode-sized calls whose typical group fits an 8-row token tile (measured: 8 tokens of c0 99 us against
+// 114 us for the register-streaming kernels).  At most 32 rows per call can reach one expert (an expert gets at most one
+// row per token): with more tokens a skewed router makes groups of many rows, whose weights the 8-row ring tile would
+// stream again for every 8 rows.
+bool use_ring(const strata_moe_layer* L, uint32_t typical_rows, uint32_t max_rows) {
+    const uint32_t ring_rows = (uint32_t)L->knobs.stream_ring_max_rows;
+    return L->stream_ok && typical_rows <= ring_rows && max_rows <= 4u * ring_rows;
 }
 
-// Token tile of the tensor-core path: 192 when groups are large (an expert with up to 192 rows is decoded
-// once), 128 with its deeper weight ring when they are small, 160 (three weight stages) for groups of about 128
-// rows, nearly all of which still fit one tile (c2, 128 rows per expert on average: 2.99 -> 2.96 ms per step).
-uint32_t prefill_ntile(const strata_moe_layer* L, uint64_t pairs, uint64_t n_groups) {
+// Calls below the rows-per-expert line of use_prefill on the tensor-core tiles, the activation between the projections as
+// an f16 hi + lo pair of pre-scaled rows (22 bits, what the weight-streaming kernels carry).  The weights must be exact in
+// f16: FP4 formats inside the exponent window, INT4 with scales of at least 2^-14 (three bits times eight fit eleven).
+// INT4 always takes the tiles (gate/up + down, 6144 x 2048 x 256 experts: 4 tokens 344 -> 223 us, 128 tokens 2874 -> 1339
+// with the general BF16 decoders before); the FP4 formats when the ring kernels do not (4096 x 2048 x 256: 32 tokens 389 us
+// with the ring, 441 with tiles; 64 tokens 731 with the register-streaming kernels, 649 with tiles; 256 tokens 1189 -> 791).
+bool use_pair_tiles(const strata_moe_layer* L, bool ring) {
+    if (!tensor_path_ok(L, L->d.format, L->d.intermediate) || !L->wmaps_ok || L->knobs.no_pair_tiles) return false;
+    if (L->d.format == STRATA_MOE_FMT_INT4G128) return L->int4_f16_ok;
+    return L->f16_ok && !ring;
+}
+
+// Token tile of the tensor-core path: 192 when groups are large (an expert with up to 192 rows is decoded once), 160
+// (three weight stages) for groups of about 128 rows, nearly all of which still fit one tile (c2, 128 rows per expert on
+// average: 2.99 -> 2.96 ms per step), 128 and 64 with their deeper weight rings for smaller ones.  Not 32: it gains
+// nothing on even loads (6144 x 2048 INT4, 8 rows per expert: 1346 us for both GEMMs, 1272 with 64) and a skewed router's
+// hot experts would take twice the passes.  For the same reason not 64 once an expert can get more than 512 rows: 7168 x
+// 1024 x 896 under Zipf, 1024 tokens, 886 us with 64 and 725 with 128 (3072 x 1024 x 256, even, 1024 tokens: 357 / 387).
+uint32_t prefill_ntile(const strata_moe_layer* L, uint64_t pairs, uint64_t n_groups, uint32_t max_rows) {
     if (L->knobs.prefill_ntile == 64 || L->knobs.prefill_ntile == 32) return (uint32_t)L->knobs.prefill_ntile;
     if (L->knobs.prefill_ntile) return L->knobs.prefill_ntile == 128 ? 128u : (L->knobs.prefill_ntile == 160 ? 160u : 192u);
-    if (pairs <= 18u * n_groups) return 32u;
-    if (pairs <= 44u * n_groups) return 64u;
+    if (pairs <= 44u * n_groups) return max_rows > 512u ? 128u : 64u;
     if (pairs <= 96u * n_groups) return 128u;
     return pairs <= 140u * n_groups ? 160u : 192u;
 }
 
-// Row count from which a single group is handed to the tensor-core path inside an otherwise
-// weight-streaming step; 0 = mixed dispatch off.
-uint32_t mixed_min_rows(const strata_moe_layer* L, uint32_t max_rows_per_group) {
-    if (!tensor_path_ok(L, L->d.format, L->d.intermediate) || !L->f16_ok || !L->wmaps_ok) return 0;
-    const int thr = L->knobs.mixed_min_rows >= 0 ? L->knobs.mixed_min_rows : 24;   // above what one or two passes of the streaming kernel cover
-    if (thr <= 0) return 0;
-    // The two extra launches cost about 10 us even when no group qualifies: worth it only for steps
-    // long enough that a hot expert's repeated passes would dominate.
-    const uint32_t min_tokens = L->knobs.mixed_min_tokens >= 0 ? (uint32_t)L->knobs.mixed_min_tokens : 128u;
-    return max_rows_per_group >= (uint32_t)thr && max_rows_per_group >= min_tokens ? (uint32_t)thr : 0u;
+// Token rows per tile of the paired-activation tiles (a row takes two columns of the down MMA).  An expert gets at most
+// one row per token, so max_rows bounds a group.  Larger tiles cost even loads little (6144 x 2048 x 256 INT4 experts, 128
+// tokens, gate/up + down: 1339 us with 16 rows, 1325 with 32, 1377 with 64) and save a skewed router's hot experts their
+// repeated passes (7168 x 1024 x 896 under Zipf, 256 tokens: 801 / 525 / 395 us).
+uint32_t pair_ntile(const strata_moe_layer* L, uint32_t max_rows) {
+    if (L->knobs.pair_ntile) return (uint32_t)L->knobs.pair_ntile;
+    return max_rows <= 16u ? 16u : (max_rows <= 64u ? 32u : 64u);
 }
 
 __global__ void set_pair_kernel(uint32_t* p, uint32_t a, uint32_t b) {
@@ -492,16 +523,18 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
     if (pairs == 0) return 0;
     const uint32_t bound = pairs;
     if (pairs_dev && expected_pairs) pairs = expected_pairs < bound ? expected_pairs : bound;
+    const bool int4 = L->d.format == STRATA_MOE_FMT_INT4G128;
     // x_ready: the caller's front-end kernel already left the f16 rows and their factors in the workspace
+    auto rows_for_tiles = [&]() {
+        if (x_ready) return;
+        if (spread && !L->knobs.no_spread)
+            launch_rows_to_f16_spread(x_src, spread->dest, spread->k, spread->rows, spread->rows_dev, bound,
+                                      L->d.hidden, L->xg, L->x_rowscale, s, int4);
+        else
+            launch_rows_to_f16_bf16(x_src, perm, k_div, bound, L->d.hidden, L->xg, L->x_rowscale, s, pairs_dev, int4);
+    };
     if (use_prefill(L, pairs, n_groups)) {
-        if (!x_ready) {
-            if (spread && !L->knobs.no_spread)
-                launch_rows_to_f16_spread(x_src, spread->dest, spread->k, spread->rows, spread->rows_dev, bound,
-                                          L->d.hidden, L->xg, L->x_rowscale, s, L->d.format == STRATA_MOE_FMT_INT4G128);
-            else
-                launch_rows_to_f16_bf16(x_src, perm, k_div, bound, L->d.hidden, L->xg, L->x_rowscale, s, pairs_dev,
-                                        L->d.format == STRATA_MOE_FMT_INT4G128);
-        }
+        rows_for_tiles();
         mark(ctx, 4);
         PrefillArgs p{};
         p.fmt = L->d.format;
@@ -517,7 +550,7 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         p.tile_table = static_cast<uint32_t*>(L->prefill_scratch);
         p.status = ctx->d_status;
         p.glu = GluParams{L->d.activation, L->d.gate_beta, L->d.linear_beta};
-        p.ntile = prefill_ntile(L, pairs, n_groups);
+        p.ntile = prefill_ntile(L, pairs, n_groups, max_rows);
         // the caller combines right away and can take the expert rows as f16: half the bytes written here and read
         // by the combine pass, which is bound by exactly those bytes
         p.y_half = (y_half && *y_half && !L->knobs.no_half_y) ? 1u : 0u;
@@ -557,6 +590,42 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
     // predicted that path with the same test
     if (y_half && *y_half && y != L->y) return fail(ctx, STRATA_MOE_E_INVALID, "f16 output buffer offered to a path that writes fp32");
     if (y_half) *y_half = false;
+    // rows of a typical group (1.5 x the average rows per expert): the token tile of the streaming kernels is sized for
+    // it, not for the worst case -- a larger group just takes another pass over its weights
+    const uint64_t avg15 = ((uint64_t)pairs * 3u) / ((uint64_t)n_groups * 2u);
+    const uint32_t typical = (uint32_t)(avg15 < 1u ? 1u : (avg15 < max_rows ? avg15 : max_rows));
+    const bool ring = use_ring(L, typical, max_rows);
+    if (use_pair_tiles(L, ring)) {
+        rows_for_tiles();
+        mark(ctx, 4);
+        PrefillArgs p{};
+        p.fmt = L->d.format;
+        p.H = L->d.hidden;
+        p.I = L->d.intermediate;
+        p.n_groups = n_groups;
+        p.pairs = pairs;
+        p.offsets = offsets;
+        p.gate = wt(L->tab[0]);
+        p.up = wt(L->tab[1]);
+        p.down = wt(L->tab[2]);
+        p.y = y;
+        p.tile_table = static_cast<uint32_t*>(L->prefill_scratch);
+        p.status = ctx->d_status;
+        p.glu = GluParams{L->d.activation, L->d.gate_beta, L->d.linear_beta};
+        p.ntile = pair_ntile(L, max_rows);
+        p.act_f32 = L->act_f32;
+        p.act_lo = L->act_lo;
+        if (launch_prefill_gate_up(p, L->xg, L->x_rowscale, L->act_hi, L->max_pairs, L->d_wmaps, s) != 0)
+            return fail(ctx, STRATA_MOE_E_CUDA, "gate/up tile launch failed");
+        mark(ctx, 5);
+        launch_rows_to_f16_f32(L->act_f32, 0, bound, L->d.intermediate, L->act_hi, L->act_lo, L->act_rowscale, s, pairs_dev, int4);
+        p.reuse_tiles = 1;
+        if (launch_prefill_down(p, L->act_hi, L->act_rowscale, L->max_pairs, L->d_wmaps, s) != 0)
+            return fail(ctx, STRATA_MOE_E_CUDA, "down tile launch failed");
+        mark(ctx, 6);
+        CK(cudaGetLastError());
+        return 0;
+    }
     DecodeArgs a{};
     a.fmt = L->d.format;
     a.H = L->d.hidden;
@@ -565,13 +634,7 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
     a.offsets = offsets;
     a.active_list = active;
     a.n_active = n_active;
-    // token tile of the streaming kernels: sized for the typical group (1.5 x the average rows per
-    // expert), not the worst case -- a larger group just takes another pass over its weights
-    {
-        const uint64_t avg15 = ((uint64_t)pairs * 3u) / ((uint64_t)n_groups * 2u);
-        uint32_t hint = (uint32_t)(avg15 < 1u ? 1u : avg15);
-        a.max_rows_per_group = hint < max_rows ? hint : max_rows;
-    }
+    a.max_rows_per_group = typical;
     a.gate = wt(L->tab[0]);
     a.up = wt(L->tab[1]);
     a.down = wt(L->tab[2]);
@@ -588,80 +651,24 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         a.act_f32 = L->act_f32;
         a.act_rowscale = L->act_rowscale;
         a.x_rows = (uint32_t)L->max_pairs;
-        // Mixed dispatch for uneven loads: groups with many rows (a hot expert under a skewed router) go
-        // to the tensor-core path, the rest stay on the weight-streaming kernels.  An expert receives at
-        // most one row per token, so nothing qualifies while max_rows is below the threshold.
-        const uint32_t big = mixed_min_rows(L, max_rows);
-        const bool down_all_tensor = use_prefill_down(L, pairs, n_groups);
-        PrefillArgs p{};
-        p.fmt = L->d.format;
-        p.H = L->d.hidden;
-        p.I = L->d.intermediate;
-        p.n_groups = n_groups;
-        p.pairs = pairs;
-        p.offsets = offsets;
-        p.gate = wt(L->tab[0]);
-        p.up = wt(L->tab[1]);
-        p.down = wt(L->tab[2]);
-        p.y = y;
-        p.tile_table = static_cast<uint32_t*>(L->prefill_scratch);
-        p.status = ctx->d_status;
-        p.glu = GluParams{L->d.activation, L->d.gate_beta, L->d.linear_beta};
-        p.ntile = 128;   // hybrid down: few rows per expert
-        a.skip_from = big;
         if (!x_ready) launch_rows_to_f16_bf16(x_src, perm, k_div, bound, L->d.hidden, L->xg, L->x_rowscale, s, pairs_dev);
         mark(ctx, 4);
-        // the ring kernels win while a group fits one 8-row token tile (measured: 8 tokens of c0 99 us against 114 us;
-        // 256 tokens of c1, 16-row tiles and several passes per group: 419 us against 339 us)
-        // ... and only for decode-sized calls (at most 32 rows per call can reach one expert: an expert gets at most one
-        // row per token).  With more tokens a skewed router makes groups of many rows, whose weights the 8-row ring tile
-        // would stream again for every 8 rows: measured at the c4 shape (896 experts, Zipf, 256 tokens) 1.13 ms per step
-        // with the ring kernels for the small groups against 0.96 ms with the register-streaming kernels for all; at 64
-        // uniformly routed tokens of c1 the two are equal (0.405 / 0.408 ms).
-        const uint32_t ring_rows = (uint32_t)L->knobs.stream_ring_max_rows;
-        const bool ring = L->stream_ok && a.max_rows_per_group <= ring_rows && max_rows <= 4u * ring_rows;
-        // ring kernels, no group on the tensor-core path: the gate/up epilogue writes the down kernel's f16 operand itself
-        // and the separate conversion pass is skipped
-        const bool act_direct = ring && !big && !down_all_tensor;
-        a.act_direct = act_direct ? 1u : 0u;
+        // ring kernels: the gate/up epilogue writes the down kernel's f16 operand itself
+        a.act_direct = ring ? 1u : 0u;
         a.act_rowscale_out = L->act_rowscale;
         if (ring) {
             if (launch_decode_stream_gate_up(a, L->d_smaps, s) != 0) return fail(ctx, STRATA_MOE_E_CUDA, "stream gate/up launch failed");
         } else {
             launch_decode_fp4_gate_up(a, s);
         }
-        if (!big) mark(ctx, 5);     // the gate/up phase is the kernel alone; the f16 split below belongs to the down phase
-        if (!act_direct)
+        mark(ctx, 5);     // the gate/up phase is the kernel alone; the f16 split below belongs to the down phase
+        if (!ring)
             launch_rows_to_f16_f32(L->act_f32, 0, bound, L->d.intermediate, L->act_hi, L->act_lo,
                                    L->act_rowscale, s, pairs_dev);
-        if (big) {   // after the conversion above: these rows' f16 activations and unit row factors overwrite it
-            p.min_rows = big;
-            p.ntile = 128;   // measured at the c4 shape: 407 us with 128-token tiles, 439 us with 192
-            p.act_rowscale_out = L->act_rowscale;
-            if (launch_prefill_gate_up(p, L->xg, L->x_rowscale, L->act_hi, L->max_pairs, L->d_wmaps, s) != 0)
-                return fail(ctx, STRATA_MOE_E_CUDA, "prefill gate/up launch failed");
-            mark(ctx, 5);
-        }
-        // Medium batches: the down projection (short K, many output tiles) is faster on the tensor-core
-        // path from about 8 rows per expert, the gate/up projection only from about 12.
-        p.act_rowscale_out = nullptr;
-        if (down_all_tensor) {
-            p.min_rows = 0;
-            p.ntile = 128;
-            if (launch_prefill_down(p, L->act_hi, L->act_rowscale, L->max_pairs, L->d_wmaps, s) != 0)
-                return fail(ctx, STRATA_MOE_E_CUDA, "prefill down launch failed");
+        if (ring) {
+            if (launch_decode_stream_down(a, L->d_smaps, s) != 0) return fail(ctx, STRATA_MOE_E_CUDA, "stream down launch failed");
         } else {
-            if (ring) {
-                if (launch_decode_stream_down(a, L->d_smaps, s) != 0) return fail(ctx, STRATA_MOE_E_CUDA, "stream down launch failed");
-            } else {
-                launch_decode_fp4_down(a, s);
-            }
-            if (big) {
-                p.min_rows = big;
-                p.reuse_tiles = 1;   // same groups as the gate/up launch above
-                if (launch_prefill_down(p, L->act_hi, L->act_rowscale, L->max_pairs, L->d_wmaps, s) != 0)
-                    return fail(ctx, STRATA_MOE_E_CUDA, "prefill down launch failed");
-            }
+            launch_decode_fp4_down(a, s);
         }
         mark(ctx, 6);
         CK(cudaGetLastError());
@@ -694,7 +701,7 @@ int run_shared(strata_moe_layer* L, const __nv_bfloat16* x, const __nv_bfloat16*
         p.I = L->d.shared_intermediate;
         p.n_groups = 1;
         p.pairs = T;
-        p.ntile = prefill_ntile(L, T, 1);
+        p.ntile = prefill_ntile(L, T, 1, T);
         p.offsets = offsets2;
         p.y = L->sh_y;
         p.tile_table = L->shared_tiles;
@@ -1343,7 +1350,7 @@ int strata_moe_forward(strata_moe_layer* L, const void* x, uint32_t T, float* ou
     bool x_ready = false, front_done = false;
     if (T <= 16 && !L->knobs.no_small_front) {
         float* lg = (aux && aux->logits) ? aux->logits : L->logits;
-        const bool convert = use_prefill(L, P, d.experts) || L->f16_ok;
+        const bool convert = use_prefill(L, P, d.experts) || L->f16_ok || use_pair_tiles(L, false);
         RouterParams rp{d.experts, d.top_k, d.score_kind, d.normalize, d.norm_init, d.weight_scale, d.softcap};
         launch_router_logits(xb, L->router, T, d.hidden, d.experts, lg, s, ctx->d_status);
         mark(ctx, 1);

@@ -92,7 +92,6 @@ struct DecodeArgs {
     uint32_t max_rows_per_group;   // upper bound used to pick the token tile
     uint32_t ksplit;               // decode.cu: 1 = the four warps of a CTA split K of one tile (few tiles)
     GluParams glu;                 // activation between gate/up and down
-    uint32_t skip_from;            // groups with at least this many rows are left to another kernel (0 = none)
     WeightTable gate, up, down;
     const __nv_bfloat16* x_hi;     // [pairs, H] K-permuted (or natural for BF16 weights)
     const __nv_bfloat16* x_lo;     // optional low part (fp32 inputs), nullptr otherwise
@@ -119,7 +118,8 @@ void launch_rows_to_f16_spread(const __nv_bfloat16* x, const uint32_t* dest, uin
                                const uint32_t* rows_dev, uint32_t dst_bound, uint32_t C, void* hi, float* rowscale,
                                cudaStream_t s, bool int4_order = false);
 void launch_rows_to_f16_f32(const float* x, uint32_t src_rows, uint32_t rows, uint32_t C, void* hi, void* lo,
-                            float* rowscale, cudaStream_t s, const uint32_t* rows_dev = nullptr);
+                            float* rowscale, cudaStream_t s, const uint32_t* rows_dev = nullptr, bool int4_order = false);
+void launch_int4_scale_range(const uint8_t* const* scales, uint32_t n, size_t count, uint32_t* not_ok, cudaStream_t s);
 void launch_mx_scale_range(const uint8_t* const* scales, uint32_t n, size_t bytes, uint32_t* emin,
                            float* post_scale, uint32_t* not_ok, cudaStream_t s);
 void launch_dequant_export_f16(int fmt, const uint8_t* packed, const uint8_t* scales, uint32_t emin,
@@ -148,7 +148,7 @@ struct PrefillArgs {
     uint32_t min_rows;             // only groups with at least this many rows get tiles (0 = all)
     uint32_t reuse_tiles;          // down-only launch: the tile list of the preceding gate/up launch is still valid
     void* act_lo;                  // [pairs_cap, I] or nullptr: the activation travels as a 16-bit hi + lo pair (gate/up writes, down reads both)
-    float* act_rowscale_out;       // gate/up: receives 1.0 for every row written (the activation is not pre-scaled), or nullptr
+    float* act_f32;                // gate/up: the activation leaves as fp32 rows [pairs, I] (the caller converts), or nullptr
 };
 bool prefill_supported(int fmt, uint32_t H, uint32_t I);
 size_t prefill_scratch_bytes(uint32_t n_groups, uint32_t pairs);

@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(128, NT == 1 ? 4 : (NT == 2 ? 3 : 2)) decode_f
         const uint32_t g = a.active_list ? a.active_list[slot] : slot;
         const uint32_t rt = tile - slot * tiles_per_group;
         const uint32_t row0 = a.offsets[g], cnt = a.offsets[g + 1] - row0;
-        if (cnt == 0u || (a.skip_from != 0u && cnt >= a.skip_from)) continue;   // big groups: tensor-core path
+        if (cnt == 0u) continue;
         const uint32_t row = (DUAL ? rt * 16u : rt * 32u) + gid;
 
         Fp4Stream p0, p1;
@@ -402,6 +402,15 @@ __global__ void __launch_bounds__(256) rows_to_f16_kernel(const void* __restrict
                 h[q] = __float2half_rn(f[q]);
                 l[q] = __float2half_rn(f[q] - __half2float(h[q]));
             }
+            if (int4_order) {   // columns i and i + 4 of every eight side by side (C is a multiple of 8)
+                const size_t at = (size_t)pos * C + (i >> 1) * 8u + (i & 1u);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    hi[at + 2 * q] = h[q];
+                    if (lo != nullptr) lo[at + 2 * q] = l[q];
+                }
+                continue;
+            }
             *reinterpret_cast<uint2*>(hi + (size_t)pos * C + i * 4u) =
                 make_uint2((uint32_t)__half_as_ushort(h[0]) | ((uint32_t)__half_as_ushort(h[1]) << 16),
                            (uint32_t)__half_as_ushort(h[2]) | ((uint32_t)__half_as_ushort(h[3]) << 16));
@@ -449,11 +458,11 @@ void launch_rows_to_f16_spread(const __nv_bfloat16* x, const uint32_t* dest, uin
 }
 
 void launch_rows_to_f16_f32(const float* x, uint32_t src_rows, uint32_t rows, uint32_t C, void* hi, void* lo,
-                            float* rowscale, cudaStream_t s, const uint32_t* rows_dev) {
+                            float* rowscale, cudaStream_t s, const uint32_t* rows_dev, bool int4_order) {
     if (rows == 0) return;
     rows_to_f16_kernel<true><<<(rows + 7) / 8, 256, 0, s>>>(x, nullptr, 1, src_rows, rows, C,
                                                            static_cast<__half*>(hi), static_cast<__half*>(lo),
-                                                           rowscale, rows_dev, false);
+                                                           rowscale, rows_dev, int4_order);
     ++g_kernel_launches;
 }
 
@@ -500,6 +509,19 @@ __global__ void __launch_bounds__(256) mx_scale_range_kernel(const uint8_t* cons
     }
 }
 
+// INT4: raises *not_ok unless every group scale (BF16) is zero or has a magnitude in [2^-14, 2^12): then q * scale, q of
+// at most three significant bits and the scale of eight, is an f16 number.
+__global__ void __launch_bounds__(256) int4_scale_range_kernel(const uint8_t* const* __restrict__ scales, size_t count,
+                                                               uint32_t* __restrict__ not_ok) {
+    const unsigned short* p = reinterpret_cast<const unsigned short*>(scales[blockIdx.x]);
+    bool bad = false;
+    for (size_t i = (size_t)blockIdx.y * 256u + threadIdx.x; i < count; i += (size_t)gridDim.y * 256u) {
+        const uint32_t m = __ldg(p + i) & 0x7FFFu, e = m >> 7;
+        bad |= m != 0u && (e < 127u - 14u || e >= 127u + 12u);
+    }
+    if (__any_sync(0xFFFFFFFFu, bad) && (threadIdx.x & 31u) == 0u) atomicOr(not_ok, 1u);
+}
+
 // Dequantised weights through the f16 decoders above (the values the f16 MMA path consumes),
 // widened to fp32 and multiplied by the accumulator-side factor.
 __global__ void dequant_export_f16_kernel(int fmt, const uint8_t* __restrict__ packed,
@@ -536,6 +558,12 @@ __global__ void dequant_export_f16_kernel(int fmt, const uint8_t* __restrict__ p
 void launch_dequant_export_f16(int fmt, const uint8_t* packed, const uint8_t* scales, uint32_t emin,
                                float post_scale, uint32_t rows, uint32_t cols, float* out, cudaStream_t s) {
     dequant_export_f16_kernel<<<148 * 4, 256, 0, s>>>(fmt, packed, scales, emin, post_scale, rows, cols, out);
+    ++g_kernel_launches;
+}
+
+void launch_int4_scale_range(const uint8_t* const* scales, uint32_t n, size_t count, uint32_t* not_ok, cudaStream_t s) {
+    if (n == 0) return;
+    int4_scale_range_kernel<<<dim3(n, 16), 256, 0, s>>>(scales, count, not_ok);
     ++g_kernel_launches;
 }
 

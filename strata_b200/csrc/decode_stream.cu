@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kSThreads, 1) decode_stream_kernel(DecodeArgs 
             j.row0 = a.offsets[j.g];
             j.cnt = a.offsets[j.g + 1] - j.row0;
             j.tb = 0;
-            if (j.cnt == 0u || (a.skip_from != 0u && j.cnt >= a.skip_from)) {   // empty, or left to the tensor-core path
+            if (j.cnt == 0u) {
                 u = (slot + 1u) * upe;
                 continue;
             }

@@ -729,7 +729,6 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
                     const size_t pos = (size_t)t.row0 + c0 + j;
                     const float rs = rowscale ? rowscale[pos] : 1.0f;   // undoes the pre-scale of the activation row
                     if (GU) {
-                        if (a.act_rowscale_out != nullptr && feat == 0u) a.act_rowscale_out[pos] = 1.0f;
                         const float gv = __uint_as_float(g[j]) * s0 * rs, uv = __uint_as_float(u[j]) * s1 * rs;
                         float v;
                         if (a.glu.kind == STRATA_MOE_ACT_SWIGLU) {
@@ -739,15 +738,16 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
                         } else {
                             v = glu_other(gv, uv, a.glu);
                         }
-                        if (!(fabsf(v) <= (BF ? 3.0e38f : 65504.0f))) bad = true;
-                        if (BF) {
+                        if (!(fabsf(v) <= (BF || a.act_f32 ? 3.0e38f : 65504.0f))) bad = true;
+                        if (!BF && a.act_f32) {
+                            a.act_f32[pos * R + feat] = v;
+                        } else if (BF) {
                             const __nv_bfloat16 h = __float2bfloat16_rn(v);
                             static_cast<__nv_bfloat16*>(act_out_v)[pos * R + act_col] = h;
                             if (a.act_lo) static_cast<__nv_bfloat16*>(a.act_lo)[pos * R + act_col] = __float2bfloat16_rn(v - __bfloat162float(h));
                         } else {
                             const __half h = __float2half_rn(v);
                             static_cast<__half*>(act_out_v)[pos * R + act_col] = h;
-                            if (a.act_lo) static_cast<__half*>(a.act_lo)[pos * R + act_col] = __float2half_rn(v - __half2float(h));
                         }
                     } else {
                         const float v = __uint_as_float(g[j]) * s0 * rs;

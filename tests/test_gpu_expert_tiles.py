@@ -1,6 +1,7 @@
 """Tile geometries of the tensor-core expert kernel at their edges, against the CPU oracle (needs a B200)."""
 import numpy as np
 import pytest
+import torch
 
 from strata_b200 import MoeContext, MoeLayer, synth
 from tests import helpers as Hh
@@ -59,3 +60,30 @@ def test_bf16_expert_tiles(ctx, T, E, k, H, monkeypatch):
     # tiles of 16, 32 and 64 token rows (hi + lo pairs), one row beyond them, empty groups
     monkeypatch.setenv("STRATA_MOE_PREFILL_MIN_ROWS", "0")
     check(ctx, config(synth.FMT_BF16, T, E, k, H=H), TOL_PAIR)
+
+
+@pytest.mark.parametrize("H", [512, 384])
+@pytest.mark.parametrize("fmt", [synth.FMT_MXFP4, synth.FMT_NVFP4, synth.FMT_INT4])
+@pytest.mark.parametrize("rows,T,E,k", [(16, 3, 16, 2), (16, 17, 4, 2), (32, 33, 8, 2), (64, 65, 16, 2), (64, 130, 32, 2)])
+def test_paired_activation_tiles(ctx, fmt, rows, T, E, k, H, monkeypatch):
+    # fewer than eight rows per expert on average (raised by the switch for the small shapes), a row beyond a tile
+    monkeypatch.setenv("STRATA_MOE_PREFILL_MIN_ROWS", "1000")
+    monkeypatch.setenv("STRATA_MOE_NO_STREAM_RING", "1")
+    monkeypatch.setenv("STRATA_MOE_PAIR_NTILE", str(rows))
+    check(ctx, config(fmt, T, E, k, H=H), TOL_PAIR)
+
+
+def test_int4_scales_outside_f16_keep_the_general_decoders(ctx, monkeypatch):
+    # q * scale would not be exact in f16: the call must take the same path as with the tiles switched off
+    cfg = config(synth.FMT_INT4, 9, 16, 2)
+    layer = synth.build_layer(cfg, "cuda")
+    layer.scales["down"] = (layer.scales["down"].view(torch.bfloat16) * 2.0 ** -12).view(torch.uint8)
+    outs = []
+    for off in (False, True):
+        if off:
+            monkeypatch.setenv("STRATA_MOE_NO_PAIR_TILES", "1")
+        ml = MoeLayer(ctx, cfg)
+        ml.load_synth(layer)
+        outs.append(ml.forward(layer.x))
+        ctx.synchronize()
+    assert torch.equal(*outs) and bool((outs[0] != 0).any())
