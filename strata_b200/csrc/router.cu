@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kBigWarps * 32, 1) router_logits_big_kernel(
 void launch_router_logits(const __nv_bfloat16* x, const __nv_bfloat16* wg, uint32_t T, uint32_t H,
                           uint32_t E, float* logits, cudaStream_t s, uint32_t* status) {
     if (T == 0) return;
-    // decode batches: whole rows by bulk copy, one warp per token (25 -> about 6 us for 8 tokens at E = 256, H = 4096)
+    // decode batches: whole rows by bulk copy, one warp per token (25 -> about 6 us for 8 tokens at E = 256, H = 4096), and up to a few hundred tokens
     if (status != nullptr && launch_router_logits_small(x, wg, T, H, E, logits, status, s)) return;
     // few tokens: one expert row per warp, two warps per CTA, so the rows spread over many SMs;
     // many tokens: register-blocked kernel (4 rows per warp, 32 rows per CTA)
@@ -336,6 +336,36 @@ void launch_router_logits(const __nv_bfloat16* x, const __nv_bfloat16* wg, uint3
     ++g_kernel_launches;
 }
 
+// The largest remaining entry of a warp's row by (value desc, index asc), one cached maximum per lane over the entries
+// lane, lane + 32, ...: a round is two warp reductions and a rescan by the one lane whose entry was taken, where every
+// lane used to rescan its entries and (value, index) pairs were folded by ten shuffles.
+struct LaneBest {
+    float v;
+    uint32_t i;
+    __device__ __forceinline__ void scan(const float* choice, uint32_t E, uint32_t lane) {
+        v = -INFINITY;
+        i = 0xFFFFFFFFu;
+        for (uint32_t e = lane; e < E; e += 32u) {
+            const float c = choice[e];
+            if (c > v || i == 0xFFFFFFFFu) { v = c; i = e; }
+        }
+    }
+    // the winning index, agreed by the warp
+    __device__ __forceinline__ uint32_t winner() const {
+        const uint32_t b = __float_as_uint(v + 0.0f);                       // -0 orders with +0
+        const uint32_t key = (b & 0x80000000u) ? ~b : b | 0x80000000u;      // unsigned order = float order
+        const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, i == 0xFFFFFFFFu ? 0u : key);
+        return __reduce_min_sync(0xFFFFFFFFu, key == top ? i : 0xFFFFFFFFu);
+    }
+    // marks entry w as taken; only its lane reads or writes it
+    __device__ __forceinline__ void take(uint32_t w, float* choice, uint32_t E, uint32_t lane) {
+        if (i == w && w != 0xFFFFFFFFu) {
+            choice[w] = -INFINITY;
+            scan(choice, E, lane);
+        }
+    }
+};
+
 // Scores, top-k and routing weights of ONE token by one warp.  score / choice: [E] floats of shared memory each.
 // Scores and selection values of the experts first, first + step, ... of one token (every rule but softmax, whose
 // normaliser needs the whole row).  Returns true when a logit or bias is not finite.
@@ -361,11 +391,12 @@ __device__ __forceinline__ bool route_scores_part(const RouterParams& p, const f
 }
 
 // scores_ready: score / choice were filled by route_scores_part (bad_in = its verdict); else they are computed here.
+// ids_local: a second home of the ids; store = false leaves ids and weights alone.
 __device__ __forceinline__ void route_token(const RouterParams& p, const float* __restrict__ logits,
                                             const float* __restrict__ bias, uint32_t tok, float* score, float* choice,
                                             uint32_t* __restrict__ ids, float* __restrict__ weights, uint32_t* status,
                                             const uint32_t* __restrict__ forced_ids, bool scores_ready = false,
-                                            bool bad_in = false) {
+                                            bool bad_in = false, uint32_t* ids_local = nullptr, bool store = true) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t E = p.experts, k = p.top_k;
     const float* lg = logits + (size_t)tok * E;
@@ -409,24 +440,15 @@ __device__ __forceinline__ void route_token(const RouterParams& p, const float* 
         if (bi >= E) { bad = true; bi = 0; }
         if (lane == r) { my_id = bi; my_w = score[bi]; }
     }
-    for (uint32_t r = 0; forced_ids == nullptr && r < k; ++r) {
-        float bv = -INFINITY;
-        uint32_t bi = 0xFFFFFFFFu;
-        for (uint32_t e = lane; e < E; e += 32u) {
-            const float v = choice[e];
-            if (v > bv || bi == 0xFFFFFFFFu) {
-                if (v > bv || bi == 0xFFFFFFFFu) { bv = v; bi = e; }
-            }
+    if (forced_ids == nullptr) {
+        LaneBest best;
+        best.scan(choice, E, lane);
+        for (uint32_t r = 0; r < k; ++r) {
+            uint32_t bi = best.winner();
+            best.take(bi, choice, E, lane);
+            if (bi >= E) { bad = true; bi = 0; }
+            if (lane == r) { my_id = bi; my_w = score[bi]; }
         }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float ov = __shfl_xor_sync(0xFFFFFFFFu, bv, off);
-            const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, bi, off);
-            if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-        }
-        if (bi >= E) { bad = true; bi = 0; }
-        if (lane == r) { my_id = bi; my_w = score[bi]; }
-        if (lane == 0) choice[bi] = -INFINITY;
         __syncwarp();
     }
     // weights: sum in rank order, divide, scale (lane r holds rank r; k <= 32)
@@ -443,7 +465,8 @@ __device__ __forceinline__ void route_token(const RouterParams& p, const float* 
     } else {
         w = __fmul_rn(my_w, p.weight_scale);
     }
-    if (lane < k) {
+    if (lane < k && ids_local != nullptr) ids_local[lane] = my_id;
+    if (lane < k && store) {
         ids[(size_t)tok * k + lane] = my_id;
         weights[(size_t)tok * k + lane] = w;
     }
@@ -466,6 +489,20 @@ __global__ void __launch_bounds__(kRouteWarps * 32) route_kernel(
     if (list) T = *count;     // tokens list[0 .. *count), the grid strides over them
     for (uint32_t slot = blockIdx.x * kRouteWarps + warp; slot < T; slot += gridDim.x * kRouteWarps)
         route_token(p, logits, bias, list ? list[slot] : slot, score, choice, ids, weights, status, forced_ids);
+}
+
+// Few tokens: one CTA per token, whose four warps share the scores (the exact exp / log1p replicas are the long part of a
+// token) before warp 0 selects.  Not for the softmax rule.
+__global__ void __launch_bounds__(kRouteWarps * 32) route_token_kernel(
+    RouterParams p, const float* __restrict__ logits, const float* __restrict__ bias, uint32_t* __restrict__ ids,
+    float* __restrict__ weights, uint32_t* status, const uint32_t* __restrict__ forced_ids) {
+    extern __shared__ float smem[];
+    float* score = smem;
+    float* choice = score + p.experts;
+    const uint32_t tok = blockIdx.x;
+    const bool bad = route_scores_part(p, logits + (size_t)tok * p.experts, bias, score, choice, threadIdx.x, kRouteWarps * 32u);
+    const bool any_bad = __syncthreads_or(bad) != 0;
+    if (threadIdx.x < 32u) route_token(p, logits, bias, tok, score, choice, ids, weights, status, forced_ids, true, any_bad);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -591,24 +628,16 @@ __global__ void __launch_bounds__(kFastWarps * 32) route_fast_kernel(
         __syncwarp();
         // step 2: the k largest approximate values; lane r keeps the lower bound of the r-th
         float my_low = INFINITY;
+        LaneBest best;
+        best.scan(choice, E, lane);
         for (uint32_t r = 0; r < k; ++r) {
-            float bv = -INFINITY;
-            uint32_t bi = 0xFFFFFFFFu;
-            for (uint32_t e = lane; e < E; e += 32u) {
-                const float v = choice[e];
-                if (v > bv || bi == 0xFFFFFFFFu) { bv = v; bi = e; }
-            }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const float ov = __shfl_xor_sync(0xFFFFFFFFu, bv, off);
-                const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, bi, off);
-                if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-            }
+            uint32_t bi = best.winner();
+            const float bv = __shfl_sync(0xFFFFFFFFu, best.v, bi & 31u);
+            best.take(bi, choice, E, lane);
             if (bi >= E) { bad = true; bi = 0; }
             if (lane == r) { cand[r] = bi; my_low = bv - eps[bi]; }
-            if (lane == 0) choice[bi] = -INFINITY;
-            __syncwarp();
         }
+        __syncwarp();
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) my_low = fminf(my_low, __shfl_xor_sync(0xFFFFFFFFu, my_low, off));
         // step 3: every other expert whose value could reach the weakest of those lower bounds joins the candidates
@@ -737,7 +766,7 @@ __global__ void __launch_bounds__(kFastWarps * 32) route_fast_kernel(
 }
 
 // ---------------------------------------------------------------------------------------
-// Canonical logits for a handful of tokens (decode batches), latency-oriented.
+// Canonical logits for decode batches (a handful to a few hundred tokens), latency-oriented.
 //
 // The staged kernel above walks a row in 256-column chunks with two block barriers per chunk; for eight tokens that
 // chain of load -> barrier -> arithmetic -> barrier takes 25 us at H = 4096 although the router is only 2 MB.  Here a
@@ -852,7 +881,7 @@ __global__ void __launch_bounds__(kSmallMaxTokens * 32) router_logits_small_kern
 
 bool launch_router_logits_small(const __nv_bfloat16* x, const __nv_bfloat16* wg, uint32_t T, uint32_t H, uint32_t E,
                                 float* logits, uint32_t* status, cudaStream_t s) {
-    if (T == 0 || T > kSmallMaxTokens || H % 128u || status == nullptr) return false;
+    if (T == 0 || H % 128u || status == nullptr) return false;
     if ((((uintptr_t)x | (uintptr_t)wg) & 15u) != 0) return false;
     const size_t smem = 128u + (size_t)kSmallRows * (H * 2u + kSmallPad) + (size_t)kSmallMaxTokens * 64u * 16u;
     if (smem > 200u * 1024u) return false;
@@ -866,11 +895,17 @@ bool launch_router_logits_small(const __nv_bfloat16* x, const __nv_bfloat16* wg,
             return false;
         attr[dev] = true;
     }
-    // two tokens per CTA while that keeps the grid within two CTAs per SM: more SMs stream and decode (a CTA whose
-    // rows another CTA already fetched reads them from L2)
+    // two tokens per CTA while the whole grid is resident at once (eight rows of 7168 columns leave room for one CTA per
+    // SM, of 4096 columns for two): more SMs stream and decode (a CTA whose rows another CTA already fetched reads them
+    // from L2)
     const uint32_t row_groups = (E + kSmallRows - 1) / kSmallRows;
+    const uint32_t resident = (smem > 112u * 1024u ? 1u : 2u) * (uint32_t)kNumSMs;
     uint32_t tpc = 2u;
-    while (tpc < T && row_groups * ((T + tpc - 1u) / tpc) > 2u * (uint32_t)kNumSMs) tpc *= 2u;
+    while (tpc < T && tpc < kSmallMaxTokens && row_groups * ((T + tpc - 1u) / tpc) > resident) tpc *= 2u;
+    // More tokens in further CTAs of the same rows, up to two CTAs per SM (measured against the staged kernels below: 32
+    // tokens x 896 experts x 7168 columns 64 against 187 us, 32 x 256 x 4096 19 / 39, 128 x 256 x 7168 64 / 87, 128 x 256 x
+    // 3072 29 / 41; beyond, 256 x 256 x 4096, 62 / 43).
+    if (T > kSmallMaxTokens && row_groups * ((T + tpc - 1u) / tpc) > 2u * (uint32_t)kNumSMs) return false;
     if (tpc > T) tpc = T;
     const uint32_t warps = tpc < 4u ? 4u : tpc;      // warp 0 also issues the copies
     dim3 grid(row_groups, (T + tpc - 1u) / tpc);
@@ -919,7 +954,10 @@ void launch_route_fast(const RouterParams& p, float* logits, const float* bias, 
 // ---------------------------------------------------------------------------------------
 // Decode front end in ONE launch: scores / top-k / weights, grouping and the gather + f16 conversion of the routed
 // rows, for at most 16 tokens.  As separate kernels (route, group, convert) these cost 14 + 12 + 8 us for 8 tokens,
-// mostly launch latency and single-CTA barrier chains.  One CTA of 16 warps: warp w routes token w; the pairs
+// mostly launch latency and single-CTA barrier chains.  Every CTA of 16 warps does the same routing and grouping (a
+// chain of barriers, nothing to gain by splitting it), the first one stores it, and the conversion of the rows, which is
+// throughput, is divided among the CTAs: with one CTA it took most of the kernel's 150 us for 16 tokens, top-16 of 896
+// experts, 7168 columns, and of its 22 us for 8 tokens, top-6 of 256, 4096 columns.  Warp w routes token w; the pairs
 // (<= 512) are counted per expert in shared memory, offsets come from a two-level warp scan (two experts per thread,
 // so up to 1024 experts), every pair finds its stable position by counting the earlier pairs of its expert; then the
 // warps convert the routed rows.  Outputs are those of route_kernel, the grouping kernels and rows_to_f16_kernel.
@@ -934,6 +972,7 @@ __global__ void __launch_bounds__(kFrontWarps * 32) front_small_kernel(
     extern __shared__ float fsm2[];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t E = p.experts, k = p.top_k, P = T * k;
+    const bool first = blockIdx.x == 0u;
     uint32_t* cnt = reinterpret_cast<uint32_t*>(fsm2 + (size_t)kFrontWarps * 2u * E);   // [E]
     uint32_t* off = cnt + E;                                                            // [E]
     uint32_t* ids_s = off + E;                                                          // [P]
@@ -955,8 +994,8 @@ __global__ void __launch_bounds__(kFrontWarps * 32) front_small_kernel(
     __syncthreads();
     if (warp < T) {
         float* score = fsm2 + (size_t)warp * 2u * E;
-        route_token(p, logits, bias, warp, score, score + E, ids, weights, status, nullptr, coop, bad_s[warp] != 0u);
-        if (lane < k) ids_s[warp * k + lane] = ids[(size_t)warp * k + lane];    // this lane's own store
+        route_token(p, logits, bias, warp, score, score + E, ids, weights, status, nullptr, coop, bad_s[warp] != 0u,
+                    ids_s + warp * k, first);
     }
     __syncthreads();
     if (tid < P) atomicAdd(&cnt[ids_s[tid]], 1u);
@@ -976,19 +1015,19 @@ __global__ void __launch_bounds__(kFrontWarps * 32) front_small_kernel(
     uint32_t base = 0, basea = 0;
     for (uint32_t w = 0; w < warp; ++w) { base += wtot[w]; basea += wact[w]; }
     const uint32_t oa = base + inc - run, ra = basea + inca - act;      // exclusive prefixes at expert 2t
-    if (ea < E) {
+    if (ea < E) off[ea] = oa;
+    if (eb < E) off[eb] = oa + ca;
+    if (first && ea < E) {
         counts[ea] = ca;
         offsets[ea] = oa;
-        off[ea] = oa;
         if (ca) active_list[ra] = ea;
     }
-    if (eb < E) {
+    if (first && eb < E) {
         counts[eb] = cb;
         offsets[eb] = oa + ca;
-        off[eb] = oa + ca;
         if (cb) active_list[ra + (ca != 0u)] = eb;
     }
-    if (tid == blockDim.x - 1u) {
+    if (first && tid == blockDim.x - 1u) {
         offsets[E] = base + inc;
         *n_active = basea + inca;
     }
@@ -998,13 +1037,15 @@ __global__ void __launch_bounds__(kFrontWarps * 32) front_small_kernel(
         uint32_t r = 0;
         for (uint32_t j = 0; j < tid; ++j) r += ids_s[j] == e ? 1u : 0u;
         const uint32_t pos = off[e] + r;
-        perm[pos] = tid;
-        inv[tid] = pos;
+        if (first) {
+            perm[pos] = tid;
+            inv[tid] = pos;
+        }
         perm_s[pos] = tid;
     }
     __syncthreads();
     if (xg != nullptr)
-        for (uint32_t pos = warp; pos < P; pos += kFrontWarps)
+        for (uint32_t pos = blockIdx.x + warp * gridDim.x; pos < P; pos += kFrontWarps * gridDim.x)
             warp_row_to_f16_bf16(x + (size_t)(perm_s[pos] / k) * H, H, xg + (size_t)pos * H, x_rowscale + pos, int4_order);
 }
 
@@ -1027,7 +1068,8 @@ bool launch_front_small(const RouterParams& p, const float* logits, const float*
             return false;
         attr[dev] = true;
     }
-    front_small_kernel<<<1, kFrontWarps * 32, smem, s>>>(p, logits, bias, T, ids, weights, counts, offsets, perm, inv,
+    const uint32_t grid = xg == nullptr ? 1u : (T * p.top_k + 3u) / 4u;   // four rows per CTA
+    front_small_kernel<<<grid, kFrontWarps * 32, smem, s>>>(p, logits, bias, T, ids, weights, counts, offsets, perm, inv,
                                                          active_list, n_active, x, H, static_cast<__half*>(xg),
                                                          x_rowscale, int4_order, status);
     ++g_kernel_launches;
@@ -1117,8 +1159,13 @@ void launch_route(const RouterParams& p, const float* logits, const float* bias,
                   uint32_t* ids, float* weights, uint32_t* status, cudaStream_t s, const uint32_t* forced_ids) {
     if (T == 0) return;
     const size_t smem = (size_t)kRouteWarps * 2u * p.experts * sizeof(float);
-    route_kernel<<<(T + kRouteWarps - 1) / kRouteWarps, kRouteWarps * 32, smem, s>>>(
-        p, logits, bias, T, ids, weights, status, forced_ids, nullptr, nullptr);
+    // up to four resident CTAs per SM a token per CTA finishes sooner; beyond that only throughput counts
+    if (T <= 4u * (uint32_t)kNumSMs && p.score_kind != STRATA_MOE_SCORE_SOFTMAX)
+        route_token_kernel<<<T, kRouteWarps * 32, 2u * p.experts * sizeof(float), s>>>(p, logits, bias, ids, weights, status,
+                                                                                       forced_ids);
+    else
+        route_kernel<<<(T + kRouteWarps - 1) / kRouteWarps, kRouteWarps * 32, smem, s>>>(
+            p, logits, bias, T, ids, weights, status, forced_ids, nullptr, nullptr);
     ++g_kernel_launches;
 }
 
