@@ -515,10 +515,20 @@ __global__ void __launch_bounds__(256) int4_scale_range_kernel(const uint8_t* co
                                                                uint32_t* __restrict__ not_ok) {
     const unsigned short* p = reinterpret_cast<const unsigned short*>(scales[blockIdx.x]);
     bool bad = false;
-    for (size_t i = (size_t)blockIdx.y * 256u + threadIdx.x; i < count; i += (size_t)gridDim.y * 256u) {
-        const uint32_t m = __ldg(p + i) & 0x7FFFu, e = m >> 7;
-        bad |= m != 0u && (e < 127u - 14u || e >= 127u + 12u);
+    auto check = [&](uint32_t m) {
+        m &= 0x7FFFu;
+        bad |= m != 0u && (m < (127u - 14u) << 7 || m >= (127u + 12u) << 7);
+    };
+    const size_t first = (size_t)blockIdx.y * 256u + threadIdx.x, step = (size_t)gridDim.y * 256u;
+    const size_t whole = (reinterpret_cast<uintptr_t>(p) & 15u) == 0u ? count / 8u : 0u;      // 16-byte pieces
+    for (size_t i = first; i < whole; i += step) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(p) + i);
+        for (uint32_t w : {v.x, v.y, v.z, v.w}) {
+            check(w);
+            check(w >> 16);
+        }
     }
+    for (size_t i = whole * 8u + first; i < count; i += step) check(__ldg(p + i));
     if (__any_sync(0xFFFFFFFFu, bad) && (threadIdx.x & 31u) == 0u) atomicOr(not_ok, 1u);
 }
 
@@ -563,7 +573,7 @@ void launch_dequant_export_f16(int fmt, const uint8_t* packed, const uint8_t* sc
 
 void launch_int4_scale_range(const uint8_t* const* scales, uint32_t n, size_t count, uint32_t* not_ok, cudaStream_t s) {
     if (n == 0) return;
-    int4_scale_range_kernel<<<dim3(n, 16), 256, 0, s>>>(scales, count, not_ok);
+    int4_scale_range_kernel<<<dim3(n, 8), 256, 0, s>>>(scales, count, not_ok);
     ++g_kernel_launches;
 }
 
