@@ -223,7 +223,7 @@ cudaError_t ws_reserve(strata_moe_ctx* ctx, int slot, size_t bytes) {
     ctx->ws_bytes[slot] = bytes;
     e = cudaMemset(raw, kCanary, kGuard);
     if (e == cudaSuccess) e = cudaMemset(raw + kGuard + body, kCanary, kGuard);
-    // rows the tensor-core path owns are still swept by the f32 -> f16 conversion pass: keep them finite
+    // rows of no group are swept by the f32 -> f16 conversion pass as well: keep them finite
     if (e == cudaSuccess && slot == kWsActF32) e = cudaMemset(ctx->ws[slot], 0, bytes);
     return e;
 }

@@ -1,28 +1,28 @@
 // Large-batch ("prefill") expert FFN: grouped GEMMs on the 5th-generation tensor cores.
 //
 // Orientation: the WEIGHTS are the M operand (128 output features per tile) and the expert's
-// token rows are the N operand (up to 128 per tile, any multiple of 16), so ragged expert
+// token rows are the N operand (up to 192 per tile, any multiple of 16), so ragged expert
 // groups cost at most 15 padded rows instead of a padded 128-row tile.  D (FP32) lives in
 // tensor memory: lane = output feature, column = token.
 //
 //   warp 0        TMA producer: activation tiles [N x 64] f16 -> shared memory (128-byte swizzle)
-//   warps 1, 3    MMA issuers: one thread each issues tcgen05.mma (kind::f16, M=128, K=16) per k-slice,
-//                 warp 1 for the first weight tile of a stage, warp 3 for the second.  An issuing
-//                 thread is serial (barrier polls, descriptor arithmetic, commits) and the tensor
-//                 pipe drains whenever it is not issuing; two issuers cover each other's gaps
-//   warp 2        TMA producer for the packed 4-bit weights: [128 rows x 128 B] blocks (256 columns,
-//                 four pipeline stages) land in a double-buffered, 128-byte-swizzled staging area
-//   warps 4..19   decoders: each lane owns one weight row (= one tensor-memory lane) and reads 16
-//                 packed bytes (32 columns) of it per stage from the staging area, decodes exactly
+//   warps 1, 3    MMA issuers: the warp walks its loop converged and one elected lane issues tcgen05.mma
+//                 (kind::f16, M=128, K=16), warp 1 for the first weight tile of a stage, warp 3 for the second.
+//                 An issuer is serial (barrier polls, commits) and the tensor pipe drains whenever it is not
+//                 issuing; two issuers cover each other's gaps
+//   warp 2        TMA producer for the packed 4-bit weights: [128 rows x 128 B] blocks (256 columns)
+//                 land in a 128-byte-swizzled staging ring
+//   warps 4..19   decoders: each lane owns one weight row (= one tensor-memory lane), reads 32 packed
+//                 bytes (64 columns) of it per turn from the staging area, decodes exactly
 //                 to f16 (hardware E2M1 conversion / INT4 magic-number trick), applies the block
-//                 scale and writes the 16 f16x2 words straight into TENSOR MEMORY (tcgen05.st):
+//                 scale and writes the 32 f16x2 words straight into TENSOR MEMORY (tcgen05.st):
 //                 the decoded weights are the A operand of a tensor-memory-sourced MMA and never
 //                 touch shared memory, which halves the shared-memory traffic per MMA
 //   warps 20..27  epilogue: tcgen05.ld the accumulators, fuse SwiGLU (gate/up) or the output
 //                 scale (down), store
-// Tensor memory (512 columns): accumulators in columns 0..255 (two tiles x up to 128 tokens),
-// a four-stage ring of decoded weight slices in columns 256..511 (2 tiles x 32 columns per
-// stage).  BF16 weights (the shared expert) need no decode and keep the shared-memory A operand.
+// Tensor memory (512 columns): the accumulators (two tiles x NT tokens, two sets of them for small tiles), behind them
+// the ring of decoded weight slices (see Geo).  BF16 weights (the shared expert, BF16 experts) need no decode and keep
+// the shared-memory A operand.
 // CTAs are persistent (one per SM) and walk a tile list built on the device from the
 // per-expert offsets.
 //
