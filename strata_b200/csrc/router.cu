@@ -585,6 +585,11 @@ __device__ __forceinline__ void chain_fma8(float (&c)[8], const uint4& xv, const
 constexpr uint32_t kMaxCand = 32;     // candidates per token: one lane each
 constexpr uint32_t kFastStageFloats = (512u + 64u) * 4u;   // per warp: two weight buffers of 256 vectors, two activation buffers of 32
 
+// COOP: a CTA per token, for calls whose tokens are all resident at once.  A token's time is a chain of memory round trips
+// (28 batches of the canonical dot products at 7168 columns, once per eight candidates), so its four warps take eight
+// candidates each and share the scores; warp 0 selects (256 tokens, top-16 of 896: 608 -> 578 us per step).  Otherwise a
+// warp per token.
+template <bool COOP>
 __global__ void __launch_bounds__(kFastWarps * 32) route_fast_kernel(
     RouterParams p, const float* __restrict__ logits, const float* __restrict__ bias,
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wg, uint32_t T, uint32_t H,
@@ -598,14 +603,17 @@ __global__ void __launch_bounds__(kFastWarps * 32) route_fast_kernel(
     const size_t per_warp = kFastStageFloats + 2u * (size_t)E + 4u * kMaxCand;
     uint4* wbuf = reinterpret_cast<uint4*>(fsm + warp * per_warp);
     uint4* xbuf = wbuf + 512;
-    float* choice = fsm + warp * per_warp + kFastStageFloats;
+    const bool lead = !COOP || warp == 0u;      // this warp selects
+    __shared__ uint32_t cand_count, cand_safe;
+    float* choice = fsm + (COOP ? 0u : warp) * per_warp + kFastStageFloats;
     float* eps = choice + E;
     uint32_t* cand = reinterpret_cast<uint32_t*>(eps + E);
     float* canon = reinterpret_cast<float*>(cand + kMaxCand);
     uint32_t* sel_id = reinterpret_cast<uint32_t*>(canon + kMaxCand);
     float* sel_sc = reinterpret_cast<float*>(sel_id + kMaxCand);
     float worst = 0.0f;        // largest |canonical - approximate| / delta this warp has seen
-    for (uint32_t tok = blockIdx.x * kFastWarps + warp; tok < T; tok += gridDim.x * kFastWarps) {
+    for (uint32_t tok = COOP ? blockIdx.x : blockIdx.x * kFastWarps + warp; tok < T;
+         tok += COOP ? gridDim.x : gridDim.x * kFastWarps) {
         const float* lg = logits + (size_t)tok * E;
         bool bad = false;
         float mx = 0.0f;
@@ -617,7 +625,7 @@ __global__ void __launch_bounds__(kFastWarps * 32) route_fast_kernel(
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, off));
         const float delta = 1.220703125e-4f * fmaxf(2.0f, mx);
-        for (uint32_t e = lane; e < E; e += 32u) {
+        for (uint32_t e = COOP ? threadIdx.x : lane; e < E; e += COOP ? kFastWarps * 32u : 32u) {
             float slope;
             const float sc = score_and_slope(p, lg[e], slope);
             const float b = bias ? bias[e] : 0.0f;
@@ -625,42 +633,55 @@ __global__ void __launch_bounds__(kFastWarps * 32) route_fast_kernel(
             choice[e] = __fadd_rn(sc, b);
             eps[e] = 1.25f * slope * delta + 4.8e-7f * (fabsf(sc) + fabsf(b)) + 1e-30f;
         }
-        __syncwarp();
-        // step 2: the k largest approximate values; lane r keeps the lower bound of the r-th
-        float my_low = INFINITY;
-        LaneBest best;
-        best.scan(choice, E, lane);
-        for (uint32_t r = 0; r < k; ++r) {
-            uint32_t bi = best.winner();
-            const float bv = __shfl_sync(0xFFFFFFFFu, best.v, bi & 31u);
-            best.take(bi, choice, E, lane);
-            if (bi >= E) { bad = true; bi = 0; }
-            if (lane == r) { cand[r] = bi; my_low = bv - eps[bi]; }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) my_low = fminf(my_low, __shfl_xor_sync(0xFFFFFFFFu, my_low, off));
-        // step 3: every other expert whose value could reach the weakest of those lower bounds joins the candidates
+        if (COOP) bad = __syncthreads_or(bad) != 0;
+        else __syncwarp();
         uint32_t n = k;
-        for (uint32_t base = 0; base < E; base += 32u) {
-            const uint32_t e = base + lane;
-            const bool in = e < E && (choice[e] + eps[e] >= my_low);      // the k found above hold -inf
-            const uint32_t m = __ballot_sync(0xFFFFFFFFu, in);
-            if (in) {
-                const uint32_t pos = n + __popc(m & ((1u << lane) - 1u));
-                if (pos < kMaxCand) cand[pos] = e;
+        bool safe = true;
+        if (lead) {
+            // step 2: the k largest approximate values; lane r keeps the lower bound of the r-th
+            float my_low = INFINITY;
+            LaneBest best;
+            best.scan(choice, E, lane);
+            for (uint32_t r = 0; r < k; ++r) {
+                uint32_t bi = best.winner();
+                const float bv = __shfl_sync(0xFFFFFFFFu, best.v, bi & 31u);
+                best.take(bi, choice, E, lane);
+                if (bi >= E) { bad = true; bi = 0; }
+                if (lane == r) { cand[r] = bi; my_low = bv - eps[bi]; }
             }
-            n += __popc(m);
+            __syncwarp();
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) my_low = fminf(my_low, __shfl_xor_sync(0xFFFFFFFFu, my_low, off));
+            // step 3: every other expert whose value could reach the weakest of those lower bounds joins the candidates
+            for (uint32_t base = 0; base < E; base += 32u) {
+                const uint32_t e = base + lane;
+                const bool in = e < E && (choice[e] + eps[e] >= my_low);      // the k found above hold -inf
+                const uint32_t m = __ballot_sync(0xFFFFFFFFu, in);
+                if (in) {
+                    const uint32_t pos = n + __popc(m & ((1u << lane) - 1u));
+                    if (pos < kMaxCand) cand[pos] = e;
+                }
+                n += __popc(m);
+            }
+            safe = !__any_sync(0xFFFFFFFFu, bad) && n <= kMaxCand;
+            __syncwarp();
         }
-        bool safe = !__any_sync(0xFFFFFFFFu, bad) && n <= kMaxCand;
-        __syncwarp();
+        if (COOP) {
+            if (threadIdx.x == 0u) {
+                cand_count = n;
+                cand_safe = safe ? 1u : 0u;
+            }
+            __syncthreads();
+            n = cand_count;
+            safe = cand_safe != 0u;
+        }
         // step 4: canonical-order logits of the candidates, eight per pass.  The canonical dot product gives lane v the
         // columns v, v + 32, ... (one multiply-add chain per lane, increasing column order) and folds the 32 chains by
         // five shuffle-down rounds.  Here four lanes serve one expert and each owns EIGHT of those chains (columns
         // 8*sub .. 8*sub+7 of every 32): one 16-byte load feeds eight chains, the chains keep their order, and the
         // fold below pairs the same chains in the same rounds, so the sum is bit-identical.
         const uint32_t grp = lane >> 2, sub = lane & 3u, per_lane = H / 32u;
-        for (uint32_t r0 = 0; r0 < n && safe; r0 += 8u) {
+        for (uint32_t r0 = COOP ? warp * 8u : 0u; r0 < n && safe; r0 += COOP ? kFastWarps * 8u : 8u) {
             const uint32_t r = r0 + grp;
             const uint32_t e = cand[r < n ? r : n - 1u];
             const uint4* wrow = reinterpret_cast<const uint4*>(wg + (size_t)e * H) + sub;
@@ -706,7 +727,12 @@ __global__ void __launch_bounds__(kFastWarps * 32) route_fast_kernel(
             c[0] = __fadd_rn(c[0], c[1]);
             if (sub == 0u && r < n) canon[r] = c[0];
         }
-        __syncwarp();
+        if (COOP) {
+            __syncthreads();
+            if (!lead) continue;       // the barrier behind the next token's scores follows warp 0's last use of the arrays
+        } else {
+            __syncwarp();
+        }
         // step 5: exact values of the candidates; the premise of the bounds is checked on each of them
         const bool mine = safe && lane < n;
         uint32_t my_e = 0xFFFFFFFFu;
@@ -934,14 +960,20 @@ void launch_route_fast(const RouterParams& p, float* logits, const float* bias, 
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr[dev]) {
-        cudaFuncSetAttribute(route_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(route_fast_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(route_fast_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         attr[dev] = true;
     }
     cudaMemsetAsync(count, 0, sizeof(uint32_t), s);
     uint32_t grid = (T + kFastWarps - 1) / kFastWarps;
     if (grid > (uint32_t)kNumSMs * 8u) grid = (uint32_t)kNumSMs * 8u;
-    route_fast_kernel<<<grid, kFastWarps * 32, smem, s>>>(p, logits, bias, x, wg, T, H, ids, weights, list, count,
-                                                          recheck_total, status);
+    // a CTA per token while all are resident at once (three CTAs of 68 KB per SM at 896 experts)
+    if (T <= 3u * (uint32_t)kNumSMs)
+        route_fast_kernel<true><<<T, kFastWarps * 32, smem, s>>>(p, logits, bias, x, wg, T, H, ids, weights, list, count,
+                                                                 recheck_total, status);
+    else
+        route_fast_kernel<false><<<grid, kFastWarps * 32, smem, s>>>(p, logits, bias, x, wg, T, H, ids, weights, list, count,
+                                                                     recheck_total, status);
     // the tokens on the list, completely in the canonical order (few: the grids stride over the list)
     const uint32_t E = p.experts;
     dim3 g2((E + 7) / 8, 32);
