@@ -229,6 +229,8 @@ def test_inkling_sink_router_matches_reference():
     """orc_route_sigmoid_sink against the compiled inkling_route_sigmoid_sink (src/models/inkling/inkling_ops.cpp:184-275):
     ids and weights bit for bit, with ties and strongly negative logits (the log-sigmoid branch that must not underflow)."""
     ref = O.ref()
+    if ref is None:
+        pytest.skip("compiled reference not built")
     rng = np.random.default_rng(7)
     E, S, k = 256, 2, 6
     for trial in range(200):
@@ -255,6 +257,8 @@ def test_stable_bf16_hash_matches_reference():
     """orc_stable_bf16_hash against the compiled stable_bf16_hash (src/platform/diagnostics.cpp:84-88), ties, subnormals,
     infinities and NaNs (which the reference truncates instead of rounding) included."""
     ref = O.ref()
+    if ref is None:
+        pytest.skip("compiled reference not built")
     ref.ref_stable_bf16_hash.restype = C.c_uint64
     ref.ref_stable_bf16_hash.argtypes = [C.POINTER(C.c_float), C.c_size_t]
     rng = np.random.default_rng(3)
