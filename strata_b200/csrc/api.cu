@@ -478,8 +478,8 @@ int run_router(strata_moe_layer* L, const __nv_bfloat16* x, uint32_t T, float* l
     cudaStream_t s = ctx->stream;
     const strata_moe_layer_desc& d = L->d;
     RouterParams rp{d.experts, d.top_k, d.score_kind, d.normalize, d.norm_init, d.weight_scale, d.softcap};
-    // the tensor-core projection and its exact recheck cost 75 to 150 us for any few hundred tokens, the canonical projection
-    // about 1 us per 7 million products (256 tokens x 896 experts x 7168: 285 us with its selection, the fast path 146)
+    // the tensor-core projection and its exact recheck cost 75 to 120 us for any few hundred tokens, the canonical projection
+    // about 1 us per 7 million products (256 tokens x 896 experts x 7168: 285 us with its selection, the fast path about 115)
     const int thr = L->knobs.fast_router_min_tokens;
     const bool many = thr == 0 ? T >= 512u || (uint64_t)T * d.experts * d.hidden >= 700000000ull : thr > 0 && T >= (uint32_t)thr;
     const bool fast = logits_out == nullptr && many && route_fast_supported(rp, d.hidden) &&
