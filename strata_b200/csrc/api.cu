@@ -342,7 +342,8 @@ int sync_tables(strata_moe_layer* L) {
         }
         if (L->stream_ok) CK(cudaMemcpy(L->d_smaps, maps.data(), maps.size() * sizeof(Blob3), cudaMemcpyHostToDevice));
     }
-    // tensor maps of the packed weights for the tensor-core path's TMA producer
+    // tensor maps of the packed weights for the tensor-core path's TMA producer.  Its decoders read the scales in pieces
+    // of up to 16 bytes; borrowed scales that lie on a smaller boundary leave the layer on the streaming kernels
     L->wmaps_ok = false;
     if (tensor_path_ok(L, L->d.format, L->d.intermediate)) {
         struct alignas(64) Blob { unsigned char b[128]; };
@@ -353,6 +354,7 @@ int sync_tables(strata_moe_layer* L) {
             const uint32_t cols = r == STRATA_MOE_ROLE_DOWN ? L->d.intermediate : L->d.hidden;
             for (uint32_t e = 0; e < n && ok; ++e)
                 ok = L->tab[r].packed[e] && ((uintptr_t)L->tab[r].packed[e] & 15u) == 0 &&
+                     (uintptr_t)L->tab[r].scales[e] % prefill_scale_align(L->d.format, cols) == 0 &&
                      (L->d.format == STRATA_MOE_FMT_BF16
                           ? prefill_encode_weight_map_bf16(&maps[(size_t)r * n + e], L->tab[r].packed[e], rows, cols)
                           : prefill_encode_weight_map(&maps[(size_t)r * n + e], L->tab[r].packed[e], rows, cols)) == 0;
@@ -1101,6 +1103,9 @@ int strata_moe_set_expert(strata_moe_layer* L, uint32_t expert, int role, const 
         return fail(ctx, STRATA_MOE_E_INVALID, "NVFP4 global scale must be finite and positive");
     if (((uintptr_t)packed & 15u) && source == STRATA_MOE_SRC_DEVICE_BORROW)
         return fail(ctx, STRATA_MOE_E_INVALID, "borrowed weights must be 16-byte aligned");
+    if ((L->d.format == STRATA_MOE_FMT_NVFP4 || L->d.format == STRATA_MOE_FMT_INT4G128) && ((uintptr_t)scales & 1u) &&
+        source == STRATA_MOE_SRC_DEVICE_BORROW)
+        return fail(ctx, STRATA_MOE_E_INVALID, "borrowed NVFP4 and INT4 scales must be 2-byte aligned");
     CK(cudaSetDevice(ctx->device));
     const uint32_t rows = role == STRATA_MOE_ROLE_DOWN ? L->d.hidden : L->d.intermediate;
     const uint32_t cols = role == STRATA_MOE_ROLE_DOWN ? L->d.intermediate : L->d.hidden;

@@ -165,6 +165,7 @@ int launch_prefill_gate_up(const PrefillArgs& a, const void* x16, const float* x
                            uint32_t pairs_cap, const void* wmaps, cudaStream_t s);
 int launch_prefill_down(const PrefillArgs& a, const void* act16, const float* act_rowscale, uint32_t pairs_cap,
                         const void* wmaps, cudaStream_t s);
+uint32_t prefill_scale_align(int fmt, uint32_t K);   // boundary the tile decoders' scale loads need
 int prefill_encode_weight_map_bf16(void* out128, const void* w, uint32_t rows, uint32_t K);
 int prefill_encode_weight_map(void* out128, const void* packed, uint32_t rows, uint32_t K);
 int launch_prefill_bf16(const PrefillArgs& a, const void* x, uint32_t rows, const void* w_gate, const void* w_up,

@@ -477,7 +477,13 @@ __global__ void __launch_bounds__(256) mx_scale_range_kernel(const uint8_t* cons
     __shared__ uint32_t smin[8], smax[8];
     const uint8_t* p = scales[blockIdx.x];
     uint32_t lo = 255u, hi = 0u;
-    for (size_t i = (size_t)threadIdx.x * 16u; i < bytes; i += 256u * 16u) {
+    const size_t whole = (reinterpret_cast<uintptr_t>(p) & 15u) == 0u ? bytes & ~(size_t)15u : 0u;      // 16-byte pieces
+    for (size_t i = whole + threadIdx.x; i < bytes; i += 256u) {
+        const uint32_t e = __ldg(p + i);
+        lo = min(lo, e);
+        hi = max(hi, e);
+    }
+    for (size_t i = (size_t)threadIdx.x * 16u; i < whole; i += 256u * 16u) {
         const uint4 v = __ldg(reinterpret_cast<const uint4*>(p + i));
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll

@@ -876,6 +876,18 @@ int prefill_encode_weight_map(void* out, const void* packed, uint32_t rows, uint
                : -1;
 }
 
+// Alignment of a projection's scales that load_scales relies on: one load per 256-column block of a row when rows are
+// whole blocks, the narrower loads otherwise.
+uint32_t prefill_scale_align(int fmt, uint32_t K) {
+    const bool whole_blocks = K % kPkCols == 0u;
+    switch (fmt) {
+        case STRATA_MOE_FMT_MXFP4: return whole_blocks ? 8u : 4u;
+        case STRATA_MOE_FMT_NVFP4: return whole_blocks ? 16u : 8u;
+        case STRATA_MOE_FMT_INT4G128: return whole_blocks ? 4u : 2u;
+        default: return 1u;
+    }
+}
+
 // Tensor map over one projection's BF16 rows ([rows, K]): boxes of 64 columns x 128 rows.
 int prefill_encode_weight_map_bf16(void* out, const void* w, uint32_t rows, uint32_t K) {
     return make_map(static_cast<CUtensorMap*>(out), w, rows, K, kMTile) ? 0 : -1;
