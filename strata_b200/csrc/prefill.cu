@@ -105,6 +105,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
     }
     return false;
 }
+// Barrier 1 over the epilogue warps; true on every thread when `failed` is true on any.
+__device__ __forceinline__ bool epilogue_vote(bool failed) {
+    uint32_t any;
+    __syncwarp();      // the lanes of the polling warp may come out of their wait one by one
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, 1, %2, p;\n selp.u32 %0, 1, 0, q;\n}"
+        : "=r"(any)
+        : "r"((uint32_t)failed), "n"(kEpilogueWarps * 32u)
+        : "memory");
+    return any != 0u;
+}
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -696,10 +707,10 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
             } else {
                 s0 = s1 = kNoPost ? 1.0f : a.down.post_scale[t.g];
             }
-            // one warp polls, the others sleep on a hardware barrier
-            if (ew == 0u && !mbar_wait(&S.acc_full[rc.i], rc.ph, abort_flag)) *abort_flag = 1;
-            asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueWarps * 32u) : "memory");
-            if (*abort_flag) { ok = false; break; }
+            // One warp polls, the others sleep on a hardware barrier that also carries its verdict: all warps leave after the
+            // same tile.  (The abort flag is no verdict: another role may raise it between two warps' reads, and those that
+            // missed it would meet the next barrier alone.)
+            if (epilogue_vote(ew == 0u && !mbar_wait(&S.acc_full[rc.i], rc.ph, abort_flag))) { ok = false; break; }
             tc_fence_after();
             const uint32_t feat = t.m0 + lane_base + lane;
             const uint32_t act_col = FMT == STRATA_MOE_FMT_INT4G128 ? int4_slot(feat) : feat;   // the down tiles' column order
