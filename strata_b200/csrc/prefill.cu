@@ -91,17 +91,30 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
 // or the hint expires.  A polling warp takes issue slots from the decode warps of its scheduler, so tighter polling
 // is slower (measured on a 333-token INT4 step: gate/up 1.45 ms as here, 1.69 ms with a four-instruction poll loop).
 constexpr uint32_t kWaitHintNs = 4096;
+__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done)
+        : "r"(addr), "r"(parity), "r"(kWaitHintNs)
+        : "memory");
+    return done != 0u;
+}
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const volatile uint32_t* abort_flag) {
     const uint32_t addr = smem_u32(bar);
     for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(done)
-            : "r"(addr), "r"(parity), "r"(kWaitHintNs)
-            : "memory");
-        if (done) return true;
+        if (mbar_try(addr, parity)) return true;
         if ((spin & 63u) == 63u && *abort_flag) return false;
+    }
+    return false;
+}
+// The same for a warp that goes on to warp-wide instructions: lanes may see completion, the time-out or the abort flag at
+// different polls, so the loop itself runs on votes and the warp leaves it as one.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const volatile uint32_t* abort_flag) {
+    const uint32_t addr = smem_u32(bar);
+    for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
+        if (__all_sync(0xFFFFFFFFu, mbar_try(addr, parity))) return true;
+        if ((spin & 63u) == 63u && __any_sync(0xFFFFFFFFu, *abort_flag != 0u)) return false;
     }
     return false;
 }
@@ -624,7 +637,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
                 const uint4 sc = sc_next;
                 if (q + 1u < blocks) sc_next = load_scales(srow, q + 1u);
                 else if (hn && blocks > 1u) sc_next = load_scales(srow, 0);     // the next tile's row by now
-                if (!mbar_wait(&S.pk_full[rp.i], rp.ph, abort_flag)) { ok = false; break; }
+                if (!mbar_wait_warp(&S.pk_full[rp.i], rp.ph, abort_flag)) { ok = false; break; }
                 const uint8_t* pk_row = arena + (rp.i * 2u + which) * kPkTile + arow * 128u;
                 const uint32_t sel[2] = {FMT == STRATA_MOE_FMT_NVFP4 ? (sub ? sc.y : sc.x) : sc.x,
                                          FMT == STRATA_MOE_FMT_NVFP4 ? (sub ? sc.w : sc.z)
@@ -664,7 +677,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&S.pk_empty[rp.i]);  // this warp is done reading the block
                     }
-                    if (!mbar_wait(&S.empty_a[ra.i], ra.ph ^ 1u, abort_flag)) { ok = false; break; }
+                    if (!mbar_wait_warp(&S.empty_a[ra.i], ra.ph ^ 1u, abort_flag)) { ok = false; break; }
                     tc_fence_after();   // the MMAs that read this stage have completed
                     tmem_st32(a_lane + ra.i * G::kAStageCols, v);
                     tmem_st_wait();

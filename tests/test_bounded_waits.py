@@ -20,3 +20,10 @@ def test_epilogue_warps_share_one_verdict():
     assert "*abort_flag)" not in body           # nobody decides on a flag that another role may raise meanwhile
     assert body.count("mbar_wait(") == 1 and re.search(r"if \(epilogue_vote\(ew == 0u && !mbar_wait\(", body)
     assert re.search(r"epilogue_vote\(.*\)\) \{ ok = false; break; \}", body)
+
+
+def test_lanes_of_decoders_and_issuers_leave_together():
+    body = role("weight decoders")
+    assert body.count("mbar_wait_warp(") == 2 and "mbar_wait(" not in body
+    body = role("MMA issuers")
+    assert len(re.findall(r"if \(!all\((got|mbar_wait\(.*\))\)\) \{ ok = false; break; \}", body)) == 2
