@@ -95,7 +95,8 @@ static LayerKnobs read_knobs() {
     k.no_stream_ring = getenv("STRATA_MOE_NO_STREAM_RING") != nullptr;
     k.prefill_min_rows = num("STRATA_MOE_PREFILL_MIN_ROWS", -1);
     k.prefill_ntile = num("STRATA_MOE_PREFILL_NTILE", 0);
-    k.pair_ntile = num("STRATA_MOE_PAIR_NTILE", 0);
+    const int pair_rows = num("STRATA_MOE_PAIR_NTILE", 0);     // the tile sizes there are: the tile list has room for no smaller ones
+    k.pair_ntile = pair_rows <= 0 ? 0 : (pair_rows <= 16 ? 16 : (pair_rows <= 32 ? 32 : 64));
     k.no_small_front = getenv("STRATA_MOE_NO_SMALL_FRONT") != nullptr;
     k.no_pair_tiles = getenv("STRATA_MOE_NO_PAIR_TILES") != nullptr;
     k.no_half_y = getenv("STRATA_MOE_NO_HALF_Y") != nullptr;

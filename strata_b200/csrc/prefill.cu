@@ -70,6 +70,7 @@ constexpr uint32_t kPkCols = 256;                       // columns per packed st
 constexpr uint32_t kPkTile = kMTile * (kPkCols / 2);    // 16 KiB of 4-bit weights: 128 rows x 128 B
 constexpr uint32_t kFirstDecodeWarp = 4, kFirstEpilogueWarp = kFirstDecodeWarp + kDecodeWarps;
 constexpr uint32_t kSpinLimit = 1u << 19;   // x up to kWaitHintNs each: about two seconds
+constexpr uint32_t kMinTileRows = 16;   // token rows of the smallest tile: bounds the tile list
 constexpr int kFmtBf16W = 3;  // plain BF16 weights (shared expert): tiles arrive by TMA, no decode
 
 // ------------------------------------------------------------------------------ PTX helpers
@@ -874,7 +875,7 @@ bool prefill_supported(int fmt, uint32_t H, uint32_t I) {
 }
 
 size_t prefill_scratch_bytes(uint32_t n_groups, uint32_t pairs) {
-    return (4 + 3 * ((size_t)pairs / 16u + n_groups + 1)) * sizeof(uint32_t);   // the smallest tile size bounds it
+    return (4 + 3 * ((size_t)pairs / kMinTileRows + n_groups + 1)) * sizeof(uint32_t);
 }
 
 static bool make_bmaps(BMaps* b, const void* base, uint64_t rows, uint64_t cols) {
@@ -1007,9 +1008,11 @@ static int down_any(const PrefillArgs& a, const Operands& o, cudaStream_t s) {
         default: return -1;
     }
 }
-// Tiles of shapes whose down projection takes single weight tiles (H % 256 == 128) hold at most 128 rows, or 64 pairs.
+// Tiles of shapes whose down projection takes single weight tiles (H % 256 == 128) hold at most 128 rows, or 64 pairs; none
+// is smaller than the tile list has room for.
 static PrefillArgs with_tile(PrefillArgs a, bool split) {
     const uint32_t most = split ? 64u : (a.H % 256u ? 128u : 192u);
+    if (a.ntile != 0u && a.ntile < kMinTileRows) a.ntile = kMinTileRows;
     if (a.ntile == 0u || a.ntile > most) a.ntile = most;
     return a;
 }

@@ -73,6 +73,22 @@ def test_paired_activation_tiles(ctx, fmt, rows, T, E, k, H, monkeypatch):
     check(ctx, config(fmt, T, E, k, H=H), TOL_PAIR)
 
 
+@pytest.mark.parametrize("asked,used", [(1, 16), (15, 16), (17, 32), (1000, 64)])
+def test_paired_tile_switch_takes_existing_sizes_only(ctx, asked, used, monkeypatch):
+    # the tile list is sized for 16-row tiles: other numbers select the next size there is
+    cfg = config(synth.FMT_INT4, 40, 8, 8)
+    monkeypatch.setenv("STRATA_MOE_PREFILL_MIN_ROWS", "1000")
+    layer, outs = synth.build_layer(cfg, "cuda"), []
+    for rows in (asked, used):
+        monkeypatch.setenv("STRATA_MOE_PAIR_NTILE", str(rows))
+        ml = MoeLayer(ctx, cfg)
+        ml.load_synth(layer)
+        outs.append(ml.forward(layer.x))
+        ctx.synchronize()
+    ctx.check_canaries()
+    assert torch.equal(*outs) and bool((outs[0] != 0).any())
+
+
 def test_int4_scales_outside_f16_keep_the_general_decoders(ctx, monkeypatch):
     # q * scale would not be exact in f16: the call must take the same path as with the tiles switched off
     cfg = config(synth.FMT_INT4, 9, 16, 2)
