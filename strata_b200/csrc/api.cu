@@ -412,14 +412,18 @@ bool use_prefill(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups) {
     return (uint64_t)pairs >= (uint64_t)n_groups * (uint64_t)thr;
 }
 
+// Groups with rows under even routing.
+double expected_groups(uint32_t pairs, uint32_t n_groups) {
+    return n_groups * (1.0 - pow(1.0 - 1.0 / n_groups, (double)pairs));
+}
+
 // BF16 experts on the tensor-core kernel, the activation between the projections as a BF16 hi + lo pair.  A tile is 128
 // weight rows over all of K, so the calls that fill the GPU with tiles three times over take it; with fewer the last
 // round of tiles would leave most SMs idle and the weight-streaming kernel, which splits finer, is faster.
 bool use_bf16_tiles(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups) {
     if (L->d.format != STRATA_MOE_FMT_BF16 || !L->wmaps_ok || !tensor_path_ok(L, L->d.format, L->d.intermediate)) return false;
     if (L->knobs.prefill_min_rows >= 0) return pairs >= n_groups * (uint64_t)L->knobs.prefill_min_rows;
-    const double active = n_groups * (1.0 - pow(1.0 - 1.0 / n_groups, (double)pairs));   // groups with rows under even routing
-    return active * (L->d.intermediate / 128u) >= 3.0 * kNumSMs;
+    return expected_groups(pairs, n_groups) * (L->d.intermediate / 128u) >= 3.0 * kNumSMs;
 }
 
 // Ring kernels for decode-sized calls whose typical group fits an 8-row token tile (measured: 8 tokens of c0 99 us against
@@ -431,16 +435,69 @@ bool use_ring(const strata_moe_layer* L, uint32_t typical_rows, uint32_t max_row
     return L->stream_ok && typical_rows <= ring_rows && max_rows <= 4u * ring_rows;
 }
 
+// Calls whose tiles (128 weight rows over all of K) the weight-streaming kernels, which split finer, beat: a round of tiles
+// that leaves most SMs idle, or few columns, over which a tile's set-up does not pay.  All times are whole layers, tiles /
+// streaming.
+//   FP4 (register-streaming kernels): up to 16 tokens below three rounds (H x I, experts, top-k: 7168 x 1408, 128, 8: 1
+//     token 121 / 102 us, 4 tokens 213 / 199, 8 tokens and 3.8 rounds 277 / 301; 2048 x 768, 128, 8: 4 tokens 86 / 72),
+//     and up to 64 tokens below 1536 columns (1152 x 640, 256, 8: 33 tokens 135 / 117, 96 tokens 172 / 166; 1536 x 768,
+//     128, 8: 33 tokens 131 / 129, 64 tokens 141 / 145).
+//   INT4 (general decoders, which issue more instructions per weight): up to 16 tokens and 38 million gate weights (2048 x
+//     768, 128, 8: 3 tokens 80 / 74, 6 tokens 96 / 100), a second round that is nearly empty (6144 x 2816, 16, 4: 3 tokens,
+//     190 tiles, 164 / 145; 4 tokens 166 / 212), or fewer than 1536 columns below three rounds (1152 x 640, 256, 8: 12
+//     tokens 100 / 93, 16 tokens 115 / 127) and, in one round, up to 64 tokens (1024 x 512, 32, 4: 48 tokens 76 / 61).
+//   Without the list of groups the streaming kernels walk all of them, which only pays while those are few (experts_grouped,
+//     1024 x 384, 32 experts: 8 pairs 39 / 31; 1152 x 640, 256 experts: 43 / 47; 4096 x 2048, 256: 48 pairs 180 / 277).
+bool too_small_for_tiles(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups, uint32_t max_rows, bool active_list) {
+    const uint32_t per_group = L->d.intermediate / 128u;
+    const bool short_k = L->d.hidden < 1536u;
+    if (!active_list) return short_k && n_groups * per_group <= (uint32_t)kNumSMs;
+    const double rounds = expected_groups(pairs, n_groups) * per_group / kNumSMs;
+    if (L->d.format != STRATA_MOE_FMT_INT4G128) return (max_rows <= 16u && rounds < 3.0) || (max_rows <= 64u && short_k);
+    if (short_k && ((max_rows <= 16u && rounds < 3.0) || (max_rows <= 64u && rounds <= 1.0))) return true;
+    const double gate_weights = rounds * kNumSMs * 128.0 * L->d.hidden;
+    return max_rows <= 16u && (gate_weights < 38e6 || (rounds > 1.05 && rounds < 1.35));
+}
+
 // Calls below the rows-per-expert line of use_prefill on the tensor-core tiles, the activation between the projections as
 // an f16 hi + lo pair of pre-scaled rows (22 bits, what the weight-streaming kernels carry).  The weights must be exact in
 // f16: FP4 formats inside the exponent window, INT4 with scales of at least 2^-14 (three bits times eight fit eleven).
-// INT4 always takes the tiles (gate/up + down, 6144 x 2048 x 256 experts: 4 tokens 344 -> 223 us, 128 tokens 2874 -> 1339
-// with the general BF16 decoders before); the FP4 formats when the ring kernels do not (4096 x 2048 x 256: 32 tokens 389 us
-// with the ring, 441 with tiles; 64 tokens 731 with the register-streaming kernels, 649 with tiles; 256 tokens 1189 -> 791).
-bool use_pair_tiles(const strata_moe_layer* L, bool ring) {
+// INT4 gains at every size above the smallest calls (gate/up + down, 6144 x 2048 x 256 experts: 4 tokens 344 -> 223 us, 128
+// tokens 2874 -> 1339 with the general BF16 decoders before); the FP4 formats when the ring kernels do not serve the call
+// (4096 x 2048 x 256: 32 tokens 389 us with the ring, 441 with tiles; 64 tokens 731 with the register-streaming kernels,
+// 649 with tiles; 256 tokens 1189 -> 791).
+bool use_pair_tiles(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups, uint32_t max_rows, bool active_list) {
     if (!tensor_path_ok(L, L->d.format, L->d.intermediate) || !L->wmaps_ok || L->knobs.no_pair_tiles) return false;
-    if (L->d.format == STRATA_MOE_FMT_INT4G128) return L->int4_f16_ok;
-    return L->f16_ok && !ring;
+    if (!(L->d.format == STRATA_MOE_FMT_INT4G128 ? L->int4_f16_ok : L->f16_ok)) return false;
+    return L->knobs.pair_ntile != 0 || !too_small_for_tiles(L, pairs, n_groups, max_rows, active_list);
+}
+
+// The kernels that a call's experts run on.
+enum class ExpertPath {
+    kTiles,        // tensor-core tiles, the activation between the projections as one f16
+    kBf16Tiles,    // the same kernel on BF16 weights, the activation as a BF16 hi + lo pair
+    kRing,         // FP4: weight streaming through the bulk-copy ring
+    kPairTiles,    // tensor-core tiles, the activation as an f16 hi + lo pair
+    kFp4Stream,    // FP4: weight streaming through registers
+    kGeneral       // weight streaming with the general decoders on BF16 rows
+};
+// All but the last and the BF16 tiles read f16 rows with a factor each.
+bool reads_f16_rows(ExpertPath p) { return p != ExpertPath::kGeneral && p != ExpertPath::kBf16Tiles; }
+
+// Rows of a typical group (1.5 x the average rows per expert): the token tile of the streaming kernels is sized for it, not
+// for the worst case -- a larger group just takes another pass over its weights.
+uint32_t typical_rows(uint32_t pairs, uint32_t n_groups, uint32_t max_rows) {
+    const uint64_t avg15 = ((uint64_t)pairs * 3u) / ((uint64_t)n_groups * 2u);
+    return (uint32_t)(avg15 < 1u ? 1u : (avg15 < max_rows ? avg15 : max_rows));
+}
+
+// max_rows: most rows a group can have; active_list: the caller has the list of groups with rows.
+ExpertPath expert_path(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups, uint32_t max_rows, bool active_list) {
+    if (use_prefill(L, pairs, n_groups)) return ExpertPath::kTiles;
+    if (use_bf16_tiles(L, pairs, n_groups)) return ExpertPath::kBf16Tiles;
+    if (use_ring(L, typical_rows(pairs, n_groups, max_rows), max_rows)) return ExpertPath::kRing;
+    if (use_pair_tiles(L, pairs, n_groups, max_rows, active_list)) return ExpertPath::kPairTiles;
+    return L->f16_ok ? ExpertPath::kFp4Stream : ExpertPath::kGeneral;
 }
 
 // Token tile of the tensor-core path: 192 when groups are large (an expert with up to 192 rows is decoded once), 160
@@ -539,7 +596,8 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         else
             launch_rows_to_f16_bf16(x_src, perm, k_div, bound, L->d.hidden, L->xg, L->x_rowscale, s, pairs_dev, int4);
     };
-    if (use_prefill(L, pairs, n_groups)) {
+    const ExpertPath path = expert_path(L, pairs, n_groups, max_rows, active != nullptr);
+    if (path == ExpertPath::kTiles) {
         rows_for_tiles();
         mark(ctx, 4);
         PrefillArgs p{};
@@ -569,7 +627,11 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         CK(cudaGetLastError());
         return 0;
     }
-    if (use_bf16_tiles(L, pairs, n_groups)) {
+    // only the path above stores f16 rows; a caller that pointed y at an f16-sized buffer must have predicted it with the
+    // same test
+    if (y_half && *y_half && y != L->y) return fail(ctx, STRATA_MOE_E_INVALID, "f16 output buffer offered to a path that writes fp32");
+    if (y_half) *y_half = false;
+    if (path == ExpertPath::kBf16Tiles) {
         launch_gather_rows_plain(x_src, perm, k_div, bound, L->d.hidden, L->xg, s);
         mark(ctx, 4);
         PrefillArgs p{};
@@ -587,21 +649,11 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         p.act_lo = L->act_lo;
         if (launch_prefill(p, L->xg, nullptr, L->act_hi, L->max_pairs, L->d_wmaps, s, ctx->timing ? ctx->pev[5] : nullptr) != 0)
             return fail(ctx, STRATA_MOE_E_CUDA, "BF16 expert launch failed");
-        if (y_half) *y_half = false;
         mark(ctx, 6);
         CK(cudaGetLastError());
         return 0;
     }
-    // only the all-tensor-core path above stores f16 rows; a caller that pointed y at an f16-sized buffer must have
-    // predicted that path with the same test
-    if (y_half && *y_half && y != L->y) return fail(ctx, STRATA_MOE_E_INVALID, "f16 output buffer offered to a path that writes fp32");
-    if (y_half) *y_half = false;
-    // rows of a typical group (1.5 x the average rows per expert): the token tile of the streaming kernels is sized for
-    // it, not for the worst case -- a larger group just takes another pass over its weights
-    const uint64_t avg15 = ((uint64_t)pairs * 3u) / ((uint64_t)n_groups * 2u);
-    const uint32_t typical = (uint32_t)(avg15 < 1u ? 1u : (avg15 < max_rows ? avg15 : max_rows));
-    const bool ring = use_ring(L, typical, max_rows);
-    if (use_pair_tiles(L, ring)) {
+    if (path == ExpertPath::kPairTiles) {
         rows_for_tiles();
         mark(ctx, 4);
         PrefillArgs p{};
@@ -640,7 +692,7 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
     a.offsets = offsets;
     a.active_list = active;
     a.n_active = n_active;
-    a.max_rows_per_group = typical;
+    a.max_rows_per_group = typical_rows(pairs, n_groups, max_rows);
     a.gate = wt(L->tab[0]);
     a.up = wt(L->tab[1]);
     a.down = wt(L->tab[2]);
@@ -652,7 +704,8 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
     a.y = y;
     a.status = ctx->d_status;
     a.glu = GluParams{L->d.activation, L->d.gate_beta, L->d.linear_beta};
-    if (L->f16_ok) {
+    if (path == ExpertPath::kRing || path == ExpertPath::kFp4Stream) {
+        const bool ring = path == ExpertPath::kRing;
         a.x_rowscale = L->x_rowscale;
         a.act_f32 = L->act_f32;
         a.act_rowscale = L->act_rowscale;
@@ -1359,7 +1412,7 @@ int strata_moe_forward(strata_moe_layer* L, const void* x, uint32_t T, float* ou
     bool x_ready = false, front_done = false;
     if (T <= 16 && !L->knobs.no_small_front) {
         float* lg = (aux && aux->logits) ? aux->logits : L->logits;
-        const bool convert = use_prefill(L, P, d.experts) || L->f16_ok || use_pair_tiles(L, false);
+        const bool convert = reads_f16_rows(expert_path(L, P, d.experts, T, true));
         RouterParams rp{d.experts, d.top_k, d.score_kind, d.normalize, d.norm_init, d.weight_scale, d.softcap};
         launch_router_logits(xb, L->router, T, d.hidden, d.experts, lg, s, ctx->d_status);
         mark(ctx, 1);

@@ -91,6 +91,7 @@ def test_paired_tile_switch_takes_existing_sizes_only(ctx, asked, used, monkeypa
 
 def test_int4_scales_outside_f16_keep_the_general_decoders(ctx, monkeypatch):
     # q * scale would not be exact in f16: the call must take the same path as with the tiles switched off
+    monkeypatch.setenv("STRATA_MOE_PAIR_NTILE", "16")      # the tiles whatever the size of the call
     cfg = config(synth.FMT_INT4, 9, 16, 2)
     layer = synth.build_layer(cfg, "cuda")
     layer.scales["down"] = (layer.scales["down"].view(torch.bfloat16) * 2.0 ** -12).view(torch.uint8)
