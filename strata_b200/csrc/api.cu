@@ -33,7 +33,7 @@ struct strata_moe_ctx {
     bool pev_valid = false;
     unsigned long long launches_at_create = 0;
     unsigned long long* d_router_rechecks = nullptr;   // tokens the fast router handed to the canonical kernels
-    uint32_t* d_dsv4_tiny = nullptr;   // sticky: the exact mode saw activations outside 2^-120 .. 2^109 (see dsv4_exact.cu)
+    uint32_t* d_dsv4_tiny = nullptr;   // the exact call in flight saw activations outside 2^-120 .. 2^109 (see dsv4_exact.cu)
     uint64_t router_fast_tokens = 0;                    // tokens routed through the fast path
     // handle-based commands (strata_moe_command_*): an internal layer whose expert slots borrow the
     // uploaded weights named by the command in flight
@@ -864,8 +864,7 @@ int strata_moe_create(int device, void* stream, strata_moe_ctx** out) {
         strata_moe_destroy(ctx);
         return STRATA_MOE_E_CUDA;
     }
-    if (cudaMalloc(&ctx->d_dsv4_tiny, sizeof(uint32_t)) != cudaSuccess ||
-        cudaMemset(ctx->d_dsv4_tiny, 0, sizeof(uint32_t)) != cudaSuccess) {
+    if (cudaMalloc(&ctx->d_dsv4_tiny, sizeof(uint32_t)) != cudaSuccess) {
         strata_moe_destroy(ctx);
         return STRATA_MOE_E_CUDA;
     }
@@ -1791,6 +1790,7 @@ static int dsv4_grouped_core(strata_moe_layer* L, const float* rows_f32, const u
     float* xq = L->y;            // [pairs, H] scratch: the E4M3-quantised input rows
     float* act = L->act_f32;     // [pairs, I]
     uint32_t* tiny = ctx->d_dsv4_tiny;
+    CK(cudaMemsetAsync(tiny, 0, sizeof(uint32_t), s));
     launch_dsv4_quantize(rows_f32, row_index, 1, pairs, H, xq, s, tiny);
     launch_dsv4_gate_up(n, offsets, H, I, wt(L->tab[0]), wt(L->tab[1]), xq, coefficients, swiglu_limit, act,
                         ctx->d_status, s, tiny);
@@ -2321,6 +2321,7 @@ int strata_moe_command_enqueue_rows_dsv4(strata_moe_ctx* ctx, const float* hidde
         const uint32_t* off2 = d_off + n_slots + 1;
         WeightTable g{d_sp + 0, d_sp + 1, nullptr, nullptr, nullptr}, u{d_sp + 2, d_sp + 3, nullptr, nullptr, nullptr},
             dn{d_sp + 4, d_sp + 5, nullptr, nullptr, nullptr};
+        CK(cudaMemsetAsync(ctx->d_dsv4_tiny, 0, sizeof(uint32_t), s));
         launch_dsv4_quantize(d_hidden, d_rows + pairs, 1, n_shared_rows, H, d_sx, s, ctx->d_dsv4_tiny);
         launch_dsv4_gate_up(1, off2, H, I, g, u, d_sx, nullptr, swiglu_limit, d_sact, ctx->d_status, s, ctx->d_dsv4_tiny, true);
         launch_dsv4_quantize(d_sact, nullptr, 1, n_shared_rows, I, d_sact, s, ctx->d_dsv4_tiny);
