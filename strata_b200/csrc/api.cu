@@ -64,6 +64,7 @@ struct DeviceTable {
     float* d_global = nullptr;
     uint32_t* d_emin = nullptr;   // f16 path tables
     float* d_post = nullptr;
+    std::vector<uint8_t> rescan, inexact;   // INT4: registered since its scales were last looked at; the verdict (q * scale off f16)
 };
 
 // Tuning and test switches, read from the environment ONCE when a layer is created (never on the
@@ -140,6 +141,10 @@ struct strata_moe_layer {
     uint32_t* recheck_count = nullptr;
     float* one_global = nullptr;  // device float 1.0 for the shared expert table
     void* d_wmaps = nullptr;      // [3][n_local] tensor-map descriptors of the packed weights
+    struct alignas(64) TensorMap { unsigned char b[128]; };
+    std::vector<TensorMap> wmaps;            // host copy of d_wmaps and the address each entry was made for
+    std::vector<const uint8_t*> wmaps_of;
+    bool wmaps_changed = false;              // the host copy is ahead of d_wmaps
     bool wmaps_ok = false;
     // f16 decode path for the FP4 formats
     bool f16_ok = false;
@@ -309,20 +314,39 @@ int sync_tables(strata_moe_layer* L) {
     if (L->knobs.no_f16_path) L->f16_ok = false;
     L->int4_f16_ok = false;
     if (L->d.format == STRATA_MOE_FMT_INT4G128) {
-        bool complete = true;
+        bool complete = true, any = false;
         for (int r = 0; r < 3; ++r)
             for (uint32_t e = 0; e < n; ++e) complete &= L->tab[r].scales[e] != nullptr;
-        if (complete) {
-            CK(cudaMemsetAsync(L->d_not_ok, 0, sizeof(uint32_t), ctx->stream));
+        if (complete) {   // only what was registered since the last look: a scan of all is the layer's scales read once (6144 x 2048, 256 experts: 151 MB)
+            CK(cudaMemsetAsync(L->d_not_ok, 0, (size_t)3 * n * sizeof(uint32_t), ctx->stream));
             for (int r = 0; r < 3; ++r) {
                 const uint32_t rows = r == STRATA_MOE_ROLE_DOWN ? L->d.hidden : L->d.intermediate;
                 const uint32_t cols = r == STRATA_MOE_ROLE_DOWN ? L->d.intermediate : L->d.hidden;
-                launch_int4_scale_range(L->tab[r].d_scales, n, scale_bytes(L->d.format, rows, cols) / 2u, L->d_not_ok, ctx->stream);
+                for (uint32_t e = 0; e < n;) {
+                    uint32_t last = e;
+                    while (last < n && L->tab[r].rescan[last]) ++last;
+                    if (last > e) {
+                        launch_int4_scale_range(L->tab[r].d_scales + e, last - e, scale_bytes(L->d.format, rows, cols) / 2u,
+                                                L->d_not_ok + (size_t)r * n + e, ctx->stream);
+                        any = true;
+                    }
+                    e = last + 1u;
+                }
             }
-            uint32_t not_ok = 1;
-            CK(cudaMemcpyAsync(&not_ok, L->d_not_ok, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
-            CK(cudaStreamSynchronize(ctx->stream));
-            L->int4_f16_ok = not_ok == 0;
+            if (any) {
+                std::vector<uint32_t> bad((size_t)3 * n);
+                CK(cudaMemcpyAsync(bad.data(), L->d_not_ok, bad.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+                CK(cudaStreamSynchronize(ctx->stream));
+                for (int r = 0; r < 3; ++r)
+                    for (uint32_t e = 0; e < n; ++e)
+                        if (L->tab[r].rescan[e]) {
+                            L->tab[r].inexact[e] = bad[(size_t)r * n + e] != 0u;
+                            L->tab[r].rescan[e] = 0;
+                        }
+            }
+            L->int4_f16_ok = true;
+            for (int r = 0; r < 3; ++r)
+                for (uint32_t e = 0; e < n; ++e) L->int4_f16_ok &= L->tab[r].inexact[e] == 0;
         }
     }
     // the bulk-copy ring needs 16-byte aligned packed rows and scale rows
@@ -347,23 +371,27 @@ int sync_tables(strata_moe_layer* L) {
     // of up to 16 bytes; borrowed scales that lie on a smaller boundary leave the layer on the streaming kernels
     L->wmaps_ok = false;
     if (tensor_path_ok(L, L->d.format, L->d.intermediate)) {
-        struct alignas(64) Blob { unsigned char b[128]; };
-        std::vector<Blob> maps((size_t)3 * n);
         bool ok = true;
         for (int r = 0; r < 3 && ok; ++r) {
             const uint32_t rows = r == STRATA_MOE_ROLE_DOWN ? L->d.hidden : L->d.intermediate;
             const uint32_t cols = r == STRATA_MOE_ROLE_DOWN ? L->d.intermediate : L->d.hidden;
-            for (uint32_t e = 0; e < n && ok; ++e)
-                ok = L->tab[r].packed[e] && ((uintptr_t)L->tab[r].packed[e] & 15u) == 0 &&
-                     (uintptr_t)L->tab[r].scales[e] % prefill_scale_align(L->d.format, cols) == 0 &&
-                     (L->d.format == STRATA_MOE_FMT_BF16
-                          ? prefill_encode_weight_map_bf16(&maps[(size_t)r * n + e], L->tab[r].packed[e], rows, cols)
-                          : prefill_encode_weight_map(&maps[(size_t)r * n + e], L->tab[r].packed[e], rows, cols)) == 0;
+            for (uint32_t e = 0; e < n && ok; ++e) {
+                const uint8_t* packed = L->tab[r].packed[e];
+                const size_t at = (size_t)r * n + e;
+                ok = packed && ((uintptr_t)packed & 15u) == 0 &&
+                     (uintptr_t)L->tab[r].scales[e] % prefill_scale_align(L->d.format, cols) == 0;
+                if (!ok || L->wmaps_of[at] == packed) continue;      // a map holds the address and the shape, nothing else
+                ok = (L->d.format == STRATA_MOE_FMT_BF16 ? prefill_encode_weight_map_bf16(&L->wmaps[at], packed, rows, cols)
+                                                         : prefill_encode_weight_map(&L->wmaps[at], packed, rows, cols)) == 0;
+                L->wmaps_of[at] = ok ? packed : nullptr;
+                L->wmaps_changed = true;
+            }
         }
-        if (ok) {
-            CK(cudaMemcpy(L->d_wmaps, maps.data(), maps.size() * sizeof(Blob), cudaMemcpyHostToDevice));
-            L->wmaps_ok = true;
+        if (ok && L->wmaps_changed) {
+            CK(cudaMemcpy(L->d_wmaps, L->wmaps.data(), L->wmaps.size() * sizeof(L->wmaps[0]), cudaMemcpyHostToDevice));
+            L->wmaps_changed = false;
         }
+        L->wmaps_ok = ok;
     }
     L->tables_dirty = false;
     return 0;
@@ -1007,6 +1035,8 @@ int strata_moe_layer_create(strata_moe_ctx* ctx, const strata_moe_layer_desc* de
         t.packed.assign(n, nullptr);
         t.scales.assign(n, nullptr);
         t.global.assign(n, 1.0f);
+        t.rescan.assign(n, 1);
+        t.inexact.assign(n, 0);
         A(dalloc(L, &t.d_packed, n));
         A(dalloc(L, &t.d_scales, n));
         A(dalloc(L, &t.d_global, n));
@@ -1040,12 +1070,14 @@ int strata_moe_layer_create(strata_moe_ctx* ctx, const strata_moe_layer_desc* de
     A(ws_reserve(ctx, kWsActLo, (size_t)P * I * 2));
     A(ws_reserve(ctx, kWsY, (size_t)P * H * 4));
     A(dalloc(L, &L->one_global, 1));
-    A(dalloc(L, &L->d_not_ok, 1));
+    A(dalloc(L, &L->d_not_ok, (size_t)3 * n));
     {
         void* wm = nullptr;
         A(cudaMalloc(&wm, (size_t)3 * n * 128 + 128));
         if (wm) L->owned.push_back(wm);
         L->d_wmaps = wm;
+        L->wmaps.resize((size_t)3 * n);
+        L->wmaps_of.assign((size_t)3 * n, nullptr);
         void* sm = nullptr;
         A(cudaMalloc(&sm, (size_t)9 * n * 128 + 128));
         if (sm) L->owned.push_back(sm);
@@ -1175,6 +1207,7 @@ int strata_moe_set_expert(strata_moe_layer* L, uint32_t expert, int role, const 
     L->tab[role].packed[le] = (const uint8_t*)pp;
     L->tab[role].scales[le] = (const uint8_t*)ps;
     L->tab[role].global[le] = L->d.format == STRATA_MOE_FMT_NVFP4 ? global_scale : 1.0f;
+    L->tab[role].rescan[le] = 1;
     L->tables_dirty = true;
     return 0;
 }

@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(256) mx_scale_range_kernel(const uint8_t* cons
     }
 }
 
-// INT4: raises *not_ok unless every group scale (BF16) is zero or has a magnitude in [2^-14, 2^12): then q * scale, q of
+// INT4: raises a matrix's not_ok word unless every group scale (BF16) of it is zero or has a magnitude in [2^-14, 2^12): then q * scale, q of
 // at most three significant bits and the scale of eight, is an f16 number.
 __global__ void __launch_bounds__(256) int4_scale_range_kernel(const uint8_t* const* __restrict__ scales, size_t count,
                                                                uint32_t* __restrict__ not_ok) {
@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(256) int4_scale_range_kernel(const uint8_t* co
         }
     }
     for (size_t i = whole * 8u + first; i < count; i += step) check(__ldg(p + i));
-    if (__any_sync(0xFFFFFFFFu, bad) && (threadIdx.x & 31u) == 0u) atomicOr(not_ok, 1u);
+    if (__any_sync(0xFFFFFFFFu, bad) && (threadIdx.x & 31u) == 0u) atomicOr(not_ok + blockIdx.x, 1u);
 }
 
 // Dequantised weights through the f16 decoders above (the values the f16 MMA path consumes),

@@ -104,3 +104,55 @@ def test_int4_scales_outside_f16_keep_the_general_decoders(ctx, monkeypatch):
         outs.append(ml.forward(layer.x))
         ctx.synchronize()
     assert torch.equal(*outs) and bool((outs[0] != 0).any())
+
+
+def test_registering_an_int4_expert_again_decides_anew(ctx, monkeypatch):
+    # scales off f16 registered over one expert of a layer in use, rewritten in place and registered, and taken back
+    monkeypatch.setenv("STRATA_MOE_PAIR_NTILE", "16")
+    cfg = config(synth.FMT_INT4, 9, 16, 2)
+    layer = synth.build_layer(cfg, "cuda")
+
+    def fresh():
+        ml = MoeLayer(ctx, cfg)
+        ml.load_synth(layer)
+        out = ml.forward(layer.x)
+        ctx.synchronize()
+        return out
+
+    def streamed():
+        with monkeypatch.context() as m:
+            m.setenv("STRATA_MOE_NO_PAIR_TILES", "1")
+            return fresh()
+
+    ml, on_tiles = MoeLayer(ctx, cfg), fresh()
+    ml.load_synth(layer)
+    assert torch.equal(ml.forward(layer.x), on_tiles) and not torch.equal(on_tiles, streamed())
+    good, rows = layer.scales["down"].clone(), layer.scales["down"]
+    rows[3] = (good[3].view(torch.bfloat16) * 2.0 ** -12).view(torch.uint8)
+    ml.set_expert(3, 2, layer.packed["down"][3], rows[3])
+    assert torch.equal(ml.forward(layer.x), streamed())
+    rows.copy_(good)
+    ml.set_expert(3, 2, layer.packed["down"][3], rows[3])
+    assert torch.equal(ml.forward(layer.x), on_tiles)
+    ctx.synchronize()
+
+
+@pytest.mark.parametrize("fmt", [synth.FMT_BF16, synth.FMT_NVFP4])
+def test_weights_registered_at_another_address_are_used(ctx, fmt, monkeypatch):
+    monkeypatch.setenv("STRATA_MOE_PREFILL_MIN_ROWS", "0")
+    cfg = config(fmt, 33, 8, 4)
+    layer = synth.build_layer(cfg, "cuda")
+    ml = MoeLayer(ctx, cfg)
+    ml.load_synth(layer)
+    before = ml.forward(layer.x).clone()
+    other = {role: layer.packed[role].flip(0).contiguous() for role in synth.ROLES}      # the experts in reverse order
+    layer.packed = {role: torch.cat([other[role][:4], layer.packed[role][4:]]) for role in synth.ROLES}
+    for r, role in enumerate(synth.ROLES):
+        for e in range(4):
+            ml.set_expert(e, r, layer.packed[role][e], layer.scales[role][e], layer.global_scale(role))
+    after = ml.forward(layer.x).clone()
+    ml2 = MoeLayer(ctx, cfg)
+    ml2.load_synth(layer)
+    want = ml2.forward(layer.x)
+    ctx.synchronize()
+    assert torch.equal(after, want) and not torch.equal(after, before)
