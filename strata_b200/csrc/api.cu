@@ -139,6 +139,7 @@ struct strata_moe_layer {
     uint32_t* router_off2 = nullptr;   // {0, T} for it
     uint32_t* recheck_list = nullptr;  // [max_tokens] tokens the fast router hands to the canonical kernels
     uint32_t* recheck_count = nullptr;
+    float* router_norms = nullptr;     // [kFastNormTokens + experts] 2-norms of the fast router's operands
     float* one_global = nullptr;  // device float 1.0 for the shared expert table
     void* d_wmaps = nullptr;      // [3][n_local] tensor-map descriptors of the packed weights
     struct alignas(64) TensorMap { unsigned char b[128]; };
@@ -580,7 +581,7 @@ int run_router(strata_moe_layer* L, const __nv_bfloat16* x, uint32_t T, float* l
             return fail(ctx, STRATA_MOE_E_CUDA, "tensor-core router projection launch failed");
         mark(ctx, 1);
         launch_route_fast(rp, L->logits, L->bias, x, L->router, T, d.hidden, ids, w, L->recheck_list, L->recheck_count,
-                          ctx->d_router_rechecks, ctx->d_status, s);
+                          ctx->d_router_rechecks, L->router_norms, ctx->d_status, s);
         ctx->router_fast_tokens += T;
         return 0;
     }
@@ -1096,6 +1097,7 @@ int strata_moe_layer_create(strata_moe_ctx* ctx, const strata_moe_layer_desc* de
     A(dalloc(L, &L->router_off2, 2));
     A(dalloc(L, &L->recheck_list, (size_t)T));
     A(dalloc(L, &L->recheck_count, 1));
+    A(dalloc(L, &L->router_norms, (size_t)kFastNormTokens + E));
     A(ws_reserve(ctx, kWsXStage, (size_t)T * H * 2));
     A(ws_reserve(ctx, kWsOutStage, (size_t)T * H * 4));
     bind_ws(L);

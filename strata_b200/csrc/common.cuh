@@ -65,8 +65,9 @@ void launch_route_sink(const float* logits, const float* bias, uint32_t T, uint3
 bool route_fast_supported(const RouterParams& p, uint32_t H);
 void launch_route_fast(const RouterParams& p, float* logits, const float* bias, const __nv_bfloat16* x,
                        const __nv_bfloat16* wg, uint32_t T, uint32_t H, uint32_t* ids, float* weights,
-                       uint32_t* list, uint32_t* count, unsigned long long* recheck_total, uint32_t* status,
+                       uint32_t* list, uint32_t* count, unsigned long long* recheck_total, float* norms, uint32_t* status,
                        cudaStream_t s);
+constexpr uint32_t kFastNormTokens = 512;   // below it the fast router bounds its projection error by the norms of its operands
 // group.cu
 size_t group_scratch_bytes(uint32_t pairs, uint32_t n_experts);
 void launch_group(const uint32_t* ids, uint32_t pairs, uint32_t expert_begin, uint32_t n_experts,

@@ -530,11 +530,17 @@ __global__ void __launch_bounds__(kRouteWarps * 32) route_token_kernel(
 //      delta, is kept in recheck_total[1] (float bits) for the statistics;
 //   6. a token with non-finite logits, more than 32 candidates or a failed check goes on a list; the
 //      canonical kernels recompute those completely.
-// delta = 2^-13 * max(2, max_e |logit|): both summation orders round at most a few hundred partial
+// From 512 tokens on delta = 2^-13 * max(2, max_e |logit|): both summation orders round at most a few hundred partial
 // sums of magnitude <= that maximum (relative 2^-24 each; the tensor cores may truncate, 2^-23), so
-// the true distance is orders of magnitude below delta; step 3 verifies that on the selected logits of every
-// token.  For the experts that were NOT selected delta is an assumption, not a proof: a projection error
-// above delta on one of them alone could hide an expert that belongs in the selection.
+// the true distance is orders of magnitude below delta; step 5 verifies that on the candidates of every
+// token.  For the experts that are no candidates this delta is an assumption, not a proof: products that cancel make
+// partial sums larger than any logit, and a projection error above delta on such an expert alone could hide it.
+// Below 512 tokens (calls that the canonical kernels would serve in a few hundred microseconds) delta is a bound for every
+// expert: a partial sum is at most sum |x_i w_i| <= N = |x| |w_e| (2-norms), so the canonical order is within
+// (H / 32 + 5) 2^-24 N of the exact sum, and the tensor cores, which add 16 products to the sum at a time and cut each of
+// the 17 terms off below 2^-25 of the largest, within (H / 16) 17 2^-25 N.  The two norms come from row_norms_kernel, and
+// the four warps of a token take the few candidates more in the same pass.  The slopes stand for their surroundings up to
+// delta = 0.2; a token beyond that goes on the list.
 // The softmax rule normalises over all experts and is not served by this path.
 __device__ __forceinline__ float score_and_slope(const RouterParams& p, float l, float& slope) {
     float cap = 1.0f;
@@ -585,13 +591,35 @@ __device__ __forceinline__ void chain_fma8(float (&c)[8], const uint4& xv, const
 constexpr uint32_t kMaxCand = 32;     // candidates per token: one lane each
 constexpr uint32_t kFastStageFloats = (512u + 64u) * 4u;   // per warp: two weight buffers of 256 vectors, two activation buffers of 32
 
-// COOP: a CTA per token, for calls whose tokens are all resident at once.  A token's time is a chain of memory round trips
+// 2-norms of T rows of x, then of E rows of wg (both [., H] BF16, H a multiple of 8); a warp per row.
+__global__ void __launch_bounds__(256) row_norms_kernel(const __nv_bfloat16* __restrict__ x, uint32_t T,
+                                                        const __nv_bfloat16* __restrict__ wg, uint32_t E, uint32_t H,
+                                                        float* __restrict__ norms) {
+    const uint32_t lane = threadIdx.x & 31u, row = blockIdx.x * 8u + (threadIdx.x >> 5);
+    if (row >= T + E) return;
+    const uint4* p = reinterpret_cast<const uint4*>(row < T ? x + (size_t)row * H : wg + (size_t)(row - T) * H);
+    float sum = 0.0f;
+#pragma unroll 8
+    for (uint32_t i = lane; i < H / 8u; i += 32u) {
+        const uint4 v = __ldg(p + i);
+        for (uint32_t w : {v.x, v.y, v.z, v.w}) {
+            const float a = __uint_as_float(w << 16), b = __uint_as_float(w & 0xFFFF0000u);
+            sum = fmaf(a, a, sum);
+            sum = fmaf(b, b, sum);
+        }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, off);
+    if (lane == 0) norms[row] = sqrtf(sum);
+}
+
+// COOP: a CTA per token, for calls of fewer than 512 tokens.  A token's time is a chain of memory round trips
 // (28 batches of the canonical dot products at 7168 columns, once per eight candidates), so its four warps take eight
 // candidates each and share the scores; warp 0 selects (256 tokens, top-16 of 896: 608 -> 578 us per step).  Otherwise a
 // warp per token.
 template <bool COOP>
 __global__ void __launch_bounds__(kFastWarps * 32) route_fast_kernel(
-    RouterParams p, const float* __restrict__ logits, const float* __restrict__ bias,
+    RouterParams p, const float* __restrict__ logits, const float* __restrict__ norms, const float* __restrict__ bias,
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wg, uint32_t T, uint32_t H,
     uint32_t* __restrict__ ids, float* __restrict__ weights, uint32_t* __restrict__ list,
     uint32_t* __restrict__ count, unsigned long long* __restrict__ recheck_total, uint32_t* status) {
@@ -624,12 +652,16 @@ __global__ void __launch_bounds__(kFastWarps * 32) route_fast_kernel(
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, off));
-        const float delta = 1.220703125e-4f * fmaxf(2.0f, mx);
+        // COOP: per expert, see above (norms: T tokens, then E experts; 1.01 covers their own rounding)
+        const float unit = COOP ? 1.01f * ((float)(H / 16u) * 5.06639481e-7f + (float)(H / 32u + 5u) * 5.96046448e-8f) * norms[tok]
+                                : 1.220703125e-4f * fmaxf(2.0f, mx);
+        auto delta_of = [&](uint32_t e) { return COOP ? unit * norms[T + e] : unit; };
         for (uint32_t e = COOP ? threadIdx.x : lane; e < E; e += COOP ? kFastWarps * 32u : 32u) {
             float slope;
             const float sc = score_and_slope(p, lg[e], slope);
             const float b = bias ? bias[e] : 0.0f;
-            bad |= !isfinite(b);
+            const float delta = delta_of(e);
+            bad |= !isfinite(b) || !(delta <= 0.2f);
             choice[e] = __fadd_rn(sc, b);
             eps[e] = 1.25f * slope * delta + 4.8e-7f * (fabsf(sc) + fabsf(b)) + 1e-30f;
         }
@@ -740,7 +772,7 @@ __global__ void __launch_bounds__(kFastWarps * 32) route_fast_kernel(
         if (mine) {
             my_e = cand[lane];
             const float cl = canon[lane];
-            const float d = fabsf(cl - lg[my_e]);
+            const float d = fabsf(cl - lg[my_e]), delta = delta_of(my_e);
             worst = fmaxf(worst, d / delta);
             if (!(d <= 0.5f * delta)) safe = false;
             float slope_unused;
@@ -947,12 +979,13 @@ bool route_fast_supported(const RouterParams& p, uint32_t H) {
            (size_t)kFastWarps * ((kFastStageFloats + 2u * (size_t)p.experts + 4u * kMaxCand) * sizeof(float)) <= 200u * 1024u;
 }
 
-// logits: approximate [T, E] (tensor-core projection); list [T], count, recheck_total: device scratch.
+// logits: approximate [T, E] (tensor-core projection); list [T], count, recheck_total, norms [kFastNormTokens + E]: device
+// scratch.
 // On return (stream order) ids / weights hold the canonical routing of every token and the canonical
 // logits of the rechecked tokens have replaced their approximate rows.
 void launch_route_fast(const RouterParams& p, float* logits, const float* bias, const __nv_bfloat16* x,
                        const __nv_bfloat16* wg, uint32_t T, uint32_t H, uint32_t* ids, float* weights,
-                       uint32_t* list, uint32_t* count, unsigned long long* recheck_total, uint32_t* status,
+                       uint32_t* list, uint32_t* count, unsigned long long* recheck_total, float* norms, uint32_t* status,
                        cudaStream_t s) {
     if (T == 0) return;
     const size_t smem = (size_t)kFastWarps * ((kFastStageFloats + 2u * (size_t)p.experts + 4u * kMaxCand) * sizeof(float));
@@ -967,13 +1000,15 @@ void launch_route_fast(const RouterParams& p, float* logits, const float* bias, 
     cudaMemsetAsync(count, 0, sizeof(uint32_t), s);
     uint32_t grid = (T + kFastWarps - 1) / kFastWarps;
     if (grid > (uint32_t)kNumSMs * 8u) grid = (uint32_t)kNumSMs * 8u;
-    // a CTA per token while all are resident at once (three CTAs of 68 KB per SM at 896 experts)
-    if (T <= 3u * (uint32_t)kNumSMs)
-        route_fast_kernel<true><<<T, kFastWarps * 32, smem, s>>>(p, logits, bias, x, wg, T, H, ids, weights, list, count,
+    if (T < kFastNormTokens) {
+        row_norms_kernel<<<(T + p.experts + 7u) / 8u, 256, 0, s>>>(x, T, wg, p.experts, H, norms);
+        ++g_kernel_launches;
+        route_fast_kernel<true><<<T, kFastWarps * 32, smem, s>>>(p, logits, norms, bias, x, wg, T, H, ids, weights, list, count,
                                                                  recheck_total, status);
-    else
-        route_fast_kernel<false><<<grid, kFastWarps * 32, smem, s>>>(p, logits, bias, x, wg, T, H, ids, weights, list, count,
-                                                                     recheck_total, status);
+    } else {
+        route_fast_kernel<false><<<grid, kFastWarps * 32, smem, s>>>(p, logits, nullptr, bias, x, wg, T, H, ids, weights, list,
+                                                                     count, recheck_total, status);
+    }
     // the tokens on the list, completely in the canonical order (few: the grids stride over the list)
     const uint32_t E = p.experts;
     dim3 g2((E + 7) / 8, 32);

@@ -32,3 +32,26 @@ def test_router_paths_agree(ctx, T, E, k, H, kind, monkeypatch):
     for ids, weights in results[1:]:
         assert torch.equal(ids, results[0][0])
         assert torch.equal(weights, results[0][1])
+
+
+@pytest.mark.parametrize("magnitude", [2.0 ** 13, 2.0 ** 16, 2.0 ** 19])
+@pytest.mark.parametrize("T", [200, 511])
+def test_cancelling_products_below_512_tokens(ctx, T, magnitude, monkeypatch):
+    """Two large products of opposite sign in one expert's logit: its tensor-core sum is off by far more than its final size
+    suggests, while the logits of the experts that are selected instead are as good as ever."""
+    cfg = synth.MoeConfig(f"cancel{T}", H=512, I=128, E=128, k=8, fmt=synth.FMT_MXFP4, T=T, seed=6)
+    layer = synth.build_layer(cfg, "cuda")
+    layer.x[:, 0] = layer.x[:, 256] = magnitude
+    layer.router_w[:, 0] = layer.router_w[:, 256] = 0.0
+    layer.router_w[77, 0], layer.router_w[77, 256] = 1.0, -1.0
+    results = []
+    for threshold in ("-1", "1"):
+        with monkeypatch.context() as m:
+            m.setenv("STRATA_MOE_FAST_ROUTER_MIN_TOKENS", threshold)
+            ml = MoeLayer(ctx, cfg)
+        ml.load_synth(layer)
+        results.append(ml.route(layer.x))
+        ctx.synchronize()
+    differ = int((results[0][0] != results[1][0]).any(dim=1).sum())
+    assert differ == 0, differ
+    assert torch.equal(results[0][1], results[1][1])
