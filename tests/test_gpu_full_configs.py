@@ -7,11 +7,11 @@ L2 <= 1e-2 and max-abs <= 2^-6 x RMS of the oracle's FP32-accumulate result.  Th
 the reference's own full-shape command test (tests/test_cuda_backend.cpp:1509-1574: the GLM INT4
 command at hidden 6144 / intermediate 2048).
 
-  c1 / c1_sigmoid at 64 and 256 tokens   hybrid route: weight-streaming gate/up + tensor-core down
-  c2 at 4096 tokens                      INT4-g128 on the tcgen05 path, 128 rows per expert, 128-token tiles
+  c1 / c1_sigmoid at 64 and 256 tokens   NVFP4 on paired tcgen05 tiles (the SwiGLU output as an f16 hi + lo pair)
+  c2 at 4096 tokens                      INT4-g128 on the tcgen05 path, 128 rows per expert, 160-token tiles
   c3 at 16384 tokens                     MXFP4 on the tcgen05 path, 512 rows per expert, 192-token tiles
   c3, one rank's share of an 8-GPU run   32 resident experts, the rows they receive (grouped stage call)
-  c4 at 256 tokens                       896 experts, top-16, Zipf-biased router, mixed dispatch
+  c4 at 256 tokens                       896 experts, top-16, Zipf-biased router, paired tiles
 """
 import gc
 

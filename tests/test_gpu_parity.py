@@ -275,6 +275,7 @@ def test_ring_and_register_streaming_kernels_agree(ctx, fmt, monkeypatch):
     cfg = small(fmt, H=1024, I=512, T=9, E=8, k=3, name=f"ring_vs_reg{fmt}")
     layer, ml, out_ring, _ = run_layer(ctx, cfg)
     monkeypatch.setenv("STRATA_MOE_NO_STREAM_RING", "1")   # switches are read when a layer is created
+    monkeypatch.setenv("STRATA_MOE_NO_PAIR_TILES", "1")
     ml2 = MoeLayer(ctx, cfg, max_tokens=layer.x.shape[0])
     ml2.load_synth(layer)
     out_reg = ml2.forward(layer.x)
@@ -336,19 +337,20 @@ def test_prefill_path_odd_hidden_size(ctx):
     assert rel <= PREFILL_TIGHT and mx <= MAX_ABS, (rel, mx)
 
 
-def test_mixed_dispatch_under_a_skewed_router(ctx, monkeypatch):
-    """A Zipf-biased router gives a few experts many rows and most experts few: inside one step the
-    hot experts run on the tensor-core path and the rest on the weight-streaming kernels."""
-    monkeypatch.setenv("STRATA_MOE_MIXED_MIN_TOKENS", "1")   # the default only switches it on from 128 tokens
+@pytest.mark.parametrize("tile", ["16", "32", "64"])
+def test_paired_tiles_under_a_skewed_router(ctx, tile, monkeypatch):
+    """A Zipf-biased router gives a few experts many rows (several tiles) and most experts few; the SwiGLU output travels as
+    a hi + lo pair, so the error is that of FP32 sums and not of a single f16."""
+    monkeypatch.setenv("STRATA_MOE_PAIR_NTILE", tile)
     cfg = small(synth.FMT_MXFP4, T=64, E=64, k=6, zipf_s=1.3, name="skewed")
     layer, ml, out, aux = run_layer(ctx, cfg)
     counts = aux["counts"].cpu().numpy()
     assert counts.max() >= 24 and ((counts > 0) & (counts < 24)).any(), counts
-    assert counts.sum() * 1.0 / cfg.E < 8           # the step as a whole is in the streaming regime
+    assert counts.sum() * 1.0 / cfg.E < 8           # the step as a whole is below the single-f16 tiles' line
     ref = Hh.run_oracle(cfg, layer.x.cpu())
     assert np.array_equal(aux["ids"].cpu().numpy().astype(np.uint32), ref["ids"])
     rel, mx = Hh.error_metrics(out.cpu().numpy(), ref["out"])
-    assert rel <= TENSOR_REL_L2 and mx <= MAX_ABS, (rel, mx)
+    assert rel <= TIGHT_REL_L2 and mx <= MAX_ABS, (rel, mx)
 
 
 @pytest.mark.parametrize("kind,zipf,dup", [(synth.SCORE_SIGMOID, 0.0, False), (synth.SCORE_SIGMOID_PLAIN, 1.1, False),
@@ -390,7 +392,7 @@ def test_workspace_guard_zones_stay_intact():
     for cfg in (small(synth.FMT_MXFP4, T=13, E=8, k=3, H=1024, I=512, name="guard_ring"),
                 small(synth.FMT_NVFP4, T=37, E=8, k=2, H=768, I=256, name="guard_stream"),
                 small(synth.FMT_INT4, T=333, E=8, k=2, H=512, I=256, norm_init=1e-20, name="guard_prefill"),
-                small(synth.FMT_MXFP4, T=64, E=64, k=6, zipf_s=1.3, name="guard_mixed"),
+                small(synth.FMT_MXFP4, T=64, E=64, k=6, zipf_s=1.3, name="guard_skewed"),
                 small(synth.FMT_NVFP4, T=200, I_shared=256, name="guard_shared")):
         layer = synth.build_layer(cfg, "cuda")
         ml = MoeLayer(c, cfg, max_tokens=layer.x.shape[0])
