@@ -72,7 +72,7 @@ struct DeviceTable {
 struct LayerKnobs {
     bool no_f16_path = false;       // STRATA_MOE_NO_F16_PATH: FP4 formats use the general BF16 decoders
     bool no_prefill_path = false;   // STRATA_MOE_NO_PREFILL_PATH: never use the tensor-core tile path
-    bool no_stream_ring = false;    // STRATA_MOE_NO_STREAM_RING: small batches use the register-streaming kernels
+    bool no_stream_ring = false;    // STRATA_MOE_NO_STREAM_RING: FP4 decode batches take the tiles or the register-streaming kernels
     bool no_pair_tiles = false;     // STRATA_MOE_NO_PAIR_TILES: small groups never take the tensor-core tiles
     bool no_half_y = false;         // STRATA_MOE_NO_HALF_Y: the tensor-core down kernel always stores fp32 expert rows
     bool no_small_front = false;    // STRATA_MOE_NO_SMALL_FRONT: decode batches keep the separate route / group / convert kernels

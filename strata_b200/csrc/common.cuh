@@ -146,7 +146,6 @@ struct PrefillArgs {
     uint32_t* status;
     GluParams glu;                 // activation of the gate/up epilogue
     uint32_t ntile;                // tokens per tile (16 .. 192); the launch takes the next geometry that holds it
-    uint32_t min_rows;             // only groups with at least this many rows get tiles (0 = all)
     uint32_t reuse_tiles;          // down-only launch: the tile list of the preceding gate/up launch is still valid
     void* act_lo;                  // [pairs_cap, I] or nullptr: the activation travels as a 16-bit hi + lo pair (gate/up writes, down reads both)
     float* act_f32;                // gate/up: the activation leaves as fp32 rows [pairs, I] (the caller converts), or nullptr

@@ -63,10 +63,10 @@ constexpr uint32_t kMaxStages = 8;   // barriers per ring
 constexpr uint32_t kMTile = 128;    // output features per tile
 constexpr uint32_t kBK = 64;        // columns of one 128-byte swizzled row: the unit of TMA boxes and of a decode turn
 constexpr uint32_t kATile = kMTile * kBK * 2;  // 16 KiB: 128 weight rows x 64 columns of 16 bits
-constexpr uint32_t kDecodeWarps = 16;  // each lane decodes 32 columns of one row per stage
+constexpr uint32_t kDecodeWarps = 16;  // a lane decodes 64 columns of one row per turn
 constexpr uint32_t kEpilogueWarps = 8;   // two per tensor-memory lane quarter: even / odd 16-token chunks
 constexpr uint32_t kThreads = (4 + kDecodeWarps + kEpilogueWarps) * 32;
-constexpr uint32_t kPkCols = 256;                       // columns per packed staging block (4 stages)
+constexpr uint32_t kPkCols = 256;                       // columns per packed staging block (four 64-column slabs)
 constexpr uint32_t kPkTile = kMTile * (kPkCols / 2);    // 16 KiB of 4-bit weights: 128 rows x 128 B
 constexpr uint32_t kFirstDecodeWarp = 4, kFirstEpilogueWarp = kFirstDecodeWarp + kDecodeWarps;
 constexpr uint32_t kSpinLimit = 1u << 19;   // x up to kWaitHintNs each: about two seconds
@@ -393,7 +393,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
     const uint32_t k_stages = K / kKst;
     volatile uint32_t* abort_flag = &S.abort_flag;
     const uint32_t total = a.tile_table[0] * m_tiles;
-    if (total == 0u) return;   // nothing listed (mixed dispatch with no large group): leave before any set-up
+    if (total == 0u) return;   // no rows (a rank that received none): leave before any set-up
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < kMaxStages; ++s) {
@@ -812,8 +812,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
 // ------------------------------------------------------------------------------ tile list
 // table[0] = number of n-tiles, then (expert, first row, rows) per n-tile, experts ascending.
 __global__ void __launch_bounds__(1024) prefill_tiles_kernel(const uint32_t* __restrict__ offsets, uint32_t n_groups,
-                                                             uint32_t* __restrict__ table, uint32_t min_rows,
-                                                             uint32_t kNTile) {
+                                                             uint32_t* __restrict__ table, uint32_t kNTile) {
     __shared__ uint32_t scan[1024];
     const uint32_t tid = threadIdx.x;
     uint32_t cnt = 0, r0 = 0;
@@ -821,7 +820,7 @@ __global__ void __launch_bounds__(1024) prefill_tiles_kernel(const uint32_t* __r
         r0 = offsets[tid];
         cnt = offsets[tid + 1] - r0;
     }
-    const uint32_t mine = cnt >= min_rows ? (cnt + kNTile - 1) / kNTile : 0u;   // small groups: weight-streaming path
+    const uint32_t mine = (cnt + kNTile - 1) / kNTile;
     scan[tid] = mine;
     __syncthreads();
     for (uint32_t off = 1; off < 1024u; off <<= 1) {
@@ -952,7 +951,7 @@ static int launch_one(const PrefillArgs& a, const void* b_hi, const void* b_lo, 
 }
 
 static void launch_tiles(const PrefillArgs& a, cudaStream_t s) {
-    prefill_tiles_kernel<<<1, 1024, 0, s>>>(a.offsets, a.n_groups, a.tile_table, a.min_rows, a.ntile);
+    prefill_tiles_kernel<<<1, 1024, 0, s>>>(a.offsets, a.n_groups, a.tile_table, a.ntile);
     ++g_kernel_launches;
 }
 
@@ -1046,7 +1045,7 @@ int launch_prefill(const PrefillArgs& args, const void* x16, const float* x_rows
 // args.offsets must hold {0, rows}; args.n_groups = 1.
 int launch_prefill_bf16(const PrefillArgs& args, const void* x, uint32_t rows, const void* w_gate, const void* w_up,
                         const void* w_down, void* act, uint32_t rows_cap, cudaStream_t s) {
-    const PrefillArgs a = with_tile(args, args.act_lo != nullptr);
+    const PrefillArgs a = with_tile(args, false);
     CUtensorMap map_g, map_u, map_d;
     if (!make_map(&map_g, w_gate, a.I, a.H, kMTile) || !make_map(&map_u, w_up, a.I, a.H, kMTile) ||
         !make_map(&map_d, w_down, a.H, a.I, kMTile))
@@ -1054,7 +1053,7 @@ int launch_prefill_bf16(const PrefillArgs& args, const void* x, uint32_t rows, c
     launch_tiles(a, s);
     const int rc = launch_gate_up_nt<kFmtBf16W>(a, Operands{x, nullptr, rows, &map_g, &map_u, nullptr, act, nullptr}, s);
     if (rc) return rc;
-    return launch_down_nt<kFmtBf16W>(a, Operands{act, a.act_lo, rows_cap, &map_d, &map_d, nullptr, nullptr, nullptr}, s);
+    return launch_down_nt<kFmtBf16W>(a, Operands{act, nullptr, rows_cap, &map_d, &map_d, nullptr, nullptr, nullptr}, s);
 }
 
 // Router projection on the tensor cores: logits[t, e] = sum_h x[t, h] * wg[e, h] for BF16 operands,
