@@ -476,7 +476,7 @@ bool use_ring(const strata_moe_layer* L, uint32_t typical_rows, uint32_t max_row
 //     190 tiles, 164 / 145; 4 tokens 166 / 212), or fewer than 1536 columns below three rounds (1152 x 640, 256, 8: 12
 //     tokens 100 / 93, 16 tokens 115 / 127) and, in one round, up to 64 tokens (1024 x 512, 32, 4: 48 tokens 76 / 61).
 //   Without the list of groups the streaming kernels walk all of them, which only pays while those are few (experts_grouped,
-//     1024 x 384, 32 experts: 8 pairs 39 / 31; 1152 x 640, 256 experts: 43 / 47; 4096 x 2048, 256: 48 pairs 180 / 277).
+//     1024 x 384, 32 experts: 4 pairs 39 / 31; 1152 x 640, 256 experts: 16 pairs 43 / 47; 4096 x 2048, 256: 48 pairs 180 / 277).
 bool too_small_for_tiles(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups, uint32_t max_rows, bool active_list) {
     const uint32_t per_group = L->d.intermediate / 128u;
     const bool short_k = L->d.hidden < 1536u;
