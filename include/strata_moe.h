@@ -161,9 +161,9 @@ int strata_moe_set_router(strata_moe_layer* layer, const void* gate_bf16, const 
  * gate/up are [I, H], down is [H, I]; packed and scales as the format defines.  Borrowed packed
  * weights must lie on 16 bytes, borrowed NVFP4 and INT4 scales on 2 (scales on 16 bytes serve every
  * kernel, others leave the layer on the weight-streaming ones).  The first call after a registration
- * looks at the values of MXFP4 and INT4 scales and picks kernels that represent them exactly: after
- * rewriting borrowed scales in place, register the projection again (only what was registered since
- * is looked at). */
+ * looks at the values of the scales (NVFP4: whether any is negative or NaN) and picks kernels that
+ * represent them exactly: after rewriting borrowed scales in place, register the projection again
+ * (of INT4 and NVFP4 only what was registered since is looked at). */
 int strata_moe_set_expert(strata_moe_layer* layer, uint32_t expert, int role, const void* packed,
                           const void* scales, float global_scale, int source);
 /* BF16 shared expert projection: gate/up [Is, H], down [H, Is]. */

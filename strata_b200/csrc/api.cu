@@ -54,7 +54,7 @@ struct strata_moe_ctx {
 };
 
 enum WsSlot { kWsXg, kWsXgLo, kWsActHi, kWsActLo, kWsY, kWsActF32, kWsXRow, kWsActRow, kWsShActHi, kWsShActLo, kWsShY,
-              kWsXStage, kWsOutStage, kWsCount };
+              kWsXStage, kWsOutStage, kWsActPlanes, kWsCount };
 
 struct DeviceTable {
     std::vector<const uint8_t*> packed, scales;
@@ -64,8 +64,10 @@ struct DeviceTable {
     float* d_global = nullptr;
     uint32_t* d_emin = nullptr;   // f16 path tables
     float* d_post = nullptr;
-    std::vector<uint8_t> rescan, inexact;   // INT4: registered since its scales were last looked at; the verdict (q * scale off f16)
+    std::vector<uint8_t> rescan, inexact;   // INT4, NVFP4: registered since its scales were last looked at; the verdict (INT4: q * scale off f16; NVFP4: a negative or NaN scale)
 };
+
+constexpr uint32_t kMaxPlaneRows = 64;   // average rows per expert that the activation's digit planes have room for
 
 // Tuning and test switches, read from the environment ONCE when a layer is created (never on the
 // per-call path).  -1 / 0 = built-in default.
@@ -73,6 +75,8 @@ struct LayerKnobs {
     bool no_f16_path = false;       // STRATA_MOE_NO_F16_PATH: FP4 formats use the general BF16 decoders
     bool no_prefill_path = false;   // STRATA_MOE_NO_PREFILL_PATH: never use the tensor-core tile path
     bool no_stream_ring = false;    // STRATA_MOE_NO_STREAM_RING: FP4 decode batches take the tiles or the register-streaming kernels
+    int planes_max_rows = -1;       // STRATA_MOE_PLANES_MAX_ROWS: average rows per expert up to which FP4 calls take the digit planes (0 = never)
+    int planes_tile = 0;            // STRATA_MOE_PLANES_TILE: token rows per tile (16 or 24) of the digit planes
     bool no_pair_tiles = false;     // STRATA_MOE_NO_PAIR_TILES: small groups never take the tensor-core tiles
     bool no_half_y = false;         // STRATA_MOE_NO_HALF_Y: the tensor-core down kernel always stores fp32 expert rows
     bool no_small_front = false;    // STRATA_MOE_NO_SMALL_FRONT: decode batches keep the separate route / group / convert kernels
@@ -94,6 +98,12 @@ static LayerKnobs read_knobs() {
     k.no_f16_path = getenv("STRATA_MOE_NO_F16_PATH") != nullptr;
     k.no_prefill_path = getenv("STRATA_MOE_NO_PREFILL_PATH") != nullptr;
     k.no_stream_ring = getenv("STRATA_MOE_NO_STREAM_RING") != nullptr;
+    k.planes_max_rows = num("STRATA_MOE_PLANES_MAX_ROWS", -1);
+    k.planes_tile = num("STRATA_MOE_PLANES_TILE", 0);
+    // a switch that chooses among the other expert kernels asks for them
+    for (const char* name : {"STRATA_MOE_NO_F16_PATH", "STRATA_MOE_NO_PREFILL_PATH", "STRATA_MOE_NO_STREAM_RING", "STRATA_MOE_STREAM_RING_MAX_ROWS",
+                             "STRATA_MOE_PREFILL_MIN_ROWS", "STRATA_MOE_PREFILL_NTILE", "STRATA_MOE_PAIR_NTILE", "STRATA_MOE_NO_PAIR_TILES"})
+        if (k.planes_max_rows < 0 && getenv(name)) k.planes_max_rows = 0;
     k.prefill_min_rows = num("STRATA_MOE_PREFILL_MIN_ROWS", -1);
     k.prefill_ntile = num("STRATA_MOE_PREFILL_NTILE", 0);
     const int pair_rows = num("STRATA_MOE_PAIR_NTILE", 0);     // the tile sizes there are: the tile list has room for no smaller ones
@@ -150,6 +160,10 @@ struct strata_moe_layer {
     // f16 decode path for the FP4 formats
     bool f16_ok = false;
     bool int4_f16_ok = false;   // every INT4 weight q * scale is exact in f16
+    bool planes_ok = false;     // the FP4 layer's shapes, alignments and scales suit the block-scaled tensor-core kernels
+    uint32_t plane_rows = 0;    // rows that the workspace of the activation's planes holds
+    uint8_t* act_planes = nullptr;
+    void* d_sfmaps = nullptr;   // [3][n_local] tensor maps of the block scales for them
     bool stream_ok = false;   // shapes and alignments allow the TMA ring kernels
     uint8_t* arena_cur = nullptr;   // weight arena: next free byte of the newest chunk (chunks are in `owned`)
     size_t arena_left = 0, arena_next = 4u << 20;
@@ -251,6 +265,7 @@ void bind_ws(strata_moe_layer* L) {
     L->sh_y = static_cast<float*>(c->ws[kWsShY]);
     L->x_stage = static_cast<__nv_bfloat16*>(c->ws[kWsXStage]);
     L->out_stage = static_cast<float*>(c->ws[kWsOutStage]);
+    L->act_planes = static_cast<uint8_t*>(c->ws[kWsActPlanes]);
 }
 
 size_t packed_bytes(int fmt, uint32_t rows, uint32_t cols) {
@@ -314,7 +329,9 @@ int sync_tables(strata_moe_layer* L) {
     }
     if (L->knobs.no_f16_path) L->f16_ok = false;
     L->int4_f16_ok = false;
-    if (L->d.format == STRATA_MOE_FMT_INT4G128) {
+    bool scales_ok = L->f16_ok;      // FP4: what the block-scaled instructions take
+    if (L->d.format == STRATA_MOE_FMT_INT4G128 || L->d.format == STRATA_MOE_FMT_NVFP4) {
+        const bool nv = L->d.format == STRATA_MOE_FMT_NVFP4;
         bool complete = true, any = false;
         for (int r = 0; r < 3; ++r)
             for (uint32_t e = 0; e < n; ++e) complete &= L->tab[r].scales[e] != nullptr;
@@ -327,8 +344,12 @@ int sync_tables(strata_moe_layer* L) {
                     uint32_t last = e;
                     while (last < n && L->tab[r].rescan[last]) ++last;
                     if (last > e) {
-                        launch_int4_scale_range(L->tab[r].d_scales + e, last - e, scale_bytes(L->d.format, rows, cols) / 2u,
-                                                L->d_not_ok + (size_t)r * n + e, ctx->stream);
+                        if (nv)
+                            launch_nv_scale_range(L->tab[r].d_scales + e, last - e, scale_bytes(L->d.format, rows, cols),
+                                                  L->d_not_ok + (size_t)r * n + e, ctx->stream);
+                        else
+                            launch_int4_scale_range(L->tab[r].d_scales + e, last - e, scale_bytes(L->d.format, rows, cols) / 2u,
+                                                    L->d_not_ok + (size_t)r * n + e, ctx->stream);
                         any = true;
                     }
                     e = last + 1u;
@@ -345,28 +366,14 @@ int sync_tables(strata_moe_layer* L) {
                             L->tab[r].rescan[e] = 0;
                         }
             }
-            L->int4_f16_ok = true;
+            bool exact = true;
             for (int r = 0; r < 3; ++r)
-                for (uint32_t e = 0; e < n; ++e) L->int4_f16_ok &= L->tab[r].inexact[e] == 0;
+                for (uint32_t e = 0; e < n; ++e) exact &= L->tab[r].inexact[e] == 0;
+            if (nv) scales_ok &= exact;
+            else L->int4_f16_ok = exact;
+        } else {
+            scales_ok = false;
         }
-    }
-    // the bulk-copy ring needs 16-byte aligned packed rows and scale rows
-    L->stream_ok = L->f16_ok && !L->knobs.no_stream_ring &&
-                   decode_stream_supported(L->d.format, L->d.hidden, L->d.intermediate);
-    for (int r = 0; r < 3 && L->stream_ok; ++r)
-        for (uint32_t e = 0; e < n && L->stream_ok; ++e)
-            L->stream_ok = (((uintptr_t)L->tab[r].packed[e] | (uintptr_t)L->tab[r].scales[e]) & 15u) == 0;
-    if (L->stream_ok) {
-        struct alignas(64) Blob3 { unsigned char b[3 * 128]; };
-        std::vector<Blob3> maps((size_t)3 * n);
-        for (int r = 0; r < 3 && L->stream_ok; ++r) {
-            const uint32_t rows = r == STRATA_MOE_ROLE_DOWN ? L->d.hidden : L->d.intermediate;
-            const uint32_t cols = r == STRATA_MOE_ROLE_DOWN ? L->d.intermediate : L->d.hidden;
-            for (uint32_t e = 0; e < n && L->stream_ok; ++e)
-                L->stream_ok = decode_stream_encode_maps(&maps[(size_t)r * n + e], L->d.format, L->tab[r].packed[e],
-                                                         L->tab[r].scales[e], rows, cols) == 0;
-        }
-        if (L->stream_ok) CK(cudaMemcpy(L->d_smaps, maps.data(), maps.size() * sizeof(Blob3), cudaMemcpyHostToDevice));
     }
     // tensor maps of the packed weights for the tensor-core path's TMA producer.  Its decoders read the scales in pieces
     // of up to 16 bytes; borrowed scales that lie on a smaller boundary leave the layer on the streaming kernels
@@ -393,6 +400,38 @@ int sync_tables(strata_moe_layer* L) {
             L->wmaps_changed = false;
         }
         L->wmaps_ok = ok;
+    }
+    // tensor maps of the block scales for the digit-plane kernels: rows of whole 16-byte pieces, on 16-byte boundaries
+    L->planes_ok = scales_ok && L->wmaps_ok && planes_supported(L->d.format, L->d.hidden, L->d.intermediate);
+    for (int r = 0; r < 3 && L->planes_ok; ++r)
+        for (uint32_t e = 0; e < n && L->planes_ok; ++e) L->planes_ok = ((uintptr_t)L->tab[r].scales[e] & 15u) == 0;
+    if (L->planes_ok) {
+        std::vector<strata_moe_layer::TensorMap> maps((size_t)3 * n);
+        for (int r = 0; r < 3 && L->planes_ok; ++r) {
+            const uint32_t rows = r == STRATA_MOE_ROLE_DOWN ? L->d.hidden : L->d.intermediate;
+            const uint32_t cols = r == STRATA_MOE_ROLE_DOWN ? L->d.intermediate : L->d.hidden;
+            for (uint32_t e = 0; e < n && L->planes_ok; ++e)
+                L->planes_ok = planes_encode_scale_map(&maps[(size_t)r * n + e], L->d.format, L->tab[r].scales[e], rows, cols) == 0;
+        }
+        if (L->planes_ok) CK(cudaMemcpy(L->d_sfmaps, maps.data(), maps.size() * sizeof(maps[0]), cudaMemcpyHostToDevice));
+    }
+    // the bulk-copy ring needs 16-byte aligned packed rows and scale rows; the digit planes take every call that it would serve
+    L->stream_ok = L->f16_ok && !L->knobs.no_stream_ring && !(L->planes_ok && L->knobs.planes_max_rows < 0) &&
+                   decode_stream_supported(L->d.format, L->d.hidden, L->d.intermediate);
+    for (int r = 0; r < 3 && L->stream_ok; ++r)
+        for (uint32_t e = 0; e < n && L->stream_ok; ++e)
+            L->stream_ok = (((uintptr_t)L->tab[r].packed[e] | (uintptr_t)L->tab[r].scales[e]) & 15u) == 0;
+    if (L->stream_ok) {
+        struct alignas(64) Blob3 { unsigned char b[3 * 128]; };
+        std::vector<Blob3> maps((size_t)3 * n);
+        for (int r = 0; r < 3 && L->stream_ok; ++r) {
+            const uint32_t rows = r == STRATA_MOE_ROLE_DOWN ? L->d.hidden : L->d.intermediate;
+            const uint32_t cols = r == STRATA_MOE_ROLE_DOWN ? L->d.intermediate : L->d.hidden;
+            for (uint32_t e = 0; e < n && L->stream_ok; ++e)
+                L->stream_ok = decode_stream_encode_maps(&maps[(size_t)r * n + e], L->d.format, L->tab[r].packed[e],
+                                                         L->tab[r].scales[e], rows, cols) == 0;
+        }
+        if (L->stream_ok) CK(cudaMemcpy(L->d_smaps, maps.data(), maps.size() * sizeof(Blob3), cudaMemcpyHostToDevice));
     }
     L->tables_dirty = false;
     return 0;
@@ -501,8 +540,20 @@ bool use_pair_tiles(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups
     return L->knobs.pair_ntile != 0 || !too_small_for_tiles(L, pairs, n_groups, max_rows, active_list);
 }
 
+// FP4 calls on the digit planes: up to 24 rows per expert on average (one full row tile) and up to 384 tokens, the most that a
+// skewed router can give one expert, whose weights are read again for every 24 rows.  Whole layers, planes / the paths
+// above (L2 flushed): 4096 x 2048 x 256 MXFP4, top-6, 1 token 72 / 78 us, 8 tokens 158 / 186, 64 tokens 475 / 690, 256 tokens 641 /
+// 925; 3072 x 1024 x 256 NVFP4, top-10, 8 tokens 129 / 150, 256 tokens 340 / 430, 384 tokens 387 / 438, 1024 tokens (40 rows) 614 /
+// 504; 7168 x 1024 x 896 MXFP4 under Zipf, top-16, 64 tokens 297 / 385, 256 tokens 561 / 606, 1024 tokens 1577 / 973.
+bool use_planes(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups, uint32_t max_rows) {
+    if (!L->planes_ok || pairs > L->plane_rows) return false;
+    if (L->knobs.planes_max_rows >= 0) return (uint64_t)pairs <= (uint64_t)L->knobs.planes_max_rows * n_groups;
+    return max_rows <= 384u && (uint64_t)pairs <= 24ull * n_groups;
+}
+
 // The kernels that a call's experts run on.
 enum class ExpertPath {
+    kPlanes,       // FP4: block-scaled tensor-core instructions, activations as digit planes
     kTiles,        // tensor-core tiles, the activation between the projections as one f16
     kBf16Tiles,    // the same kernel on BF16 weights, the activation as a BF16 hi + lo pair
     kRing,         // FP4: weight streaming through the bulk-copy ring
@@ -511,7 +562,7 @@ enum class ExpertPath {
     kGeneral       // weight streaming with the general decoders on BF16 rows
 };
 // All but the last and the BF16 tiles read f16 rows with a factor each.
-bool reads_f16_rows(ExpertPath p) { return p != ExpertPath::kGeneral && p != ExpertPath::kBf16Tiles; }
+bool reads_f16_rows(ExpertPath p) { return p != ExpertPath::kGeneral && p != ExpertPath::kBf16Tiles && p != ExpertPath::kPlanes; }
 
 // Rows of a typical group (1.5 x the average rows per expert): the token tile of the streaming kernels is sized for it, not
 // for the worst case -- a larger group just takes another pass over its weights.
@@ -521,7 +572,9 @@ uint32_t typical_rows(uint32_t pairs, uint32_t n_groups, uint32_t max_rows) {
 }
 
 // max_rows: most rows a group can have; active_list: the caller has the list of groups with rows.
-ExpertPath expert_path(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups, uint32_t max_rows, bool active_list) {
+ExpertPath expert_path(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups, uint32_t max_rows, bool active_list,
+                       bool planes = true) {
+    if (planes && use_planes(L, pairs, n_groups, max_rows)) return ExpertPath::kPlanes;
     if (use_prefill(L, pairs, n_groups)) return ExpertPath::kTiles;
     if (use_bf16_tiles(L, pairs, n_groups)) return ExpertPath::kBf16Tiles;
     if (use_ring(L, typical_rows(pairs, n_groups, max_rows), max_rows)) return ExpertPath::kRing;
@@ -606,7 +659,7 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
                 uint32_t pairs, uint32_t n_groups, const uint32_t* offsets, const uint32_t* active,
                 const uint32_t* n_active, uint32_t max_rows, float* y, uint32_t expected_pairs = 0,
                 const uint32_t* pairs_dev = nullptr, bool x_ready = false, bool* y_half = nullptr,
-                float* y_rowscale_out = nullptr, const SpreadRows* spread = nullptr) {
+                float* y_rowscale_out = nullptr, const SpreadRows* spread = nullptr, bool one_row_per_token = false) {
     // `pairs` bounds the row count.  When the exact count exists only on the device (rows received
     // from other ranks) pairs_dev points at it and expected_pairs steers the host-side heuristics.
     Range range("strata_moe.experts");
@@ -625,7 +678,9 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         else
             launch_rows_to_f16_bf16(x_src, perm, k_div, bound, L->d.hidden, L->xg, L->x_rowscale, s, pairs_dev, int4);
     };
-    const ExpertPath path = expert_path(L, pairs, n_groups, max_rows, active != nullptr);
+    ExpertPath path = expert_path(L, pairs, n_groups, max_rows, active != nullptr);
+    if (path == ExpertPath::kPlanes && (bound > L->plane_rows || (perm && !spread)))
+        path = expert_path(L, pairs, n_groups, max_rows, active != nullptr, false);
     if (path == ExpertPath::kTiles) {
         rows_for_tiles();
         mark(ctx, 4);
@@ -678,6 +733,56 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         p.act_lo = L->act_lo;
         if (launch_prefill(p, L->xg, nullptr, L->act_hi, L->max_pairs, L->d_wmaps, s, ctx->timing ? ctx->pev[5] : nullptr) != 0)
             return fail(ctx, STRATA_MOE_E_CUDA, "BF16 expert launch failed");
+        mark(ctx, 6);
+        CK(cudaGetLastError());
+        return 0;
+    }
+    if (path == ExpertPath::kPlanes) {
+        // The planes of the grouped rows take the place of y until the down projection writes it, their scales that of the f16
+        // rows; the activation's have a workspace, their scales go to act_hi.
+        const int fmt = L->d.format;
+        const uint32_t H = L->d.hidden, I = L->d.intermediate;
+        if (perm) launch_rows_to_planes(fmt, x_src, false, spread->rows, spread->rows_dev, H, spread->dest, spread->k, bound, L->y, L->xg, L->x_rowscale, s);
+        else launch_rows_to_planes(fmt, x_src, false, bound, pairs_dev, H, nullptr, 1, bound, L->y, L->xg, L->x_rowscale, s);
+        PlaneArgs p{};
+        p.H = H;
+        p.I = I;
+        p.n_groups = n_groups;
+        p.offsets = offsets;
+        // groups of at most one row per token that fit one tile come from the list of active groups
+        if (active && one_row_per_token && max_rows <= 24u) {
+            p.active_list = active;
+            p.n_active = n_active;
+            p.tile_rows = max_rows <= 8u ? 8u : (max_rows <= 16u ? 16u : 24u);
+        } else {
+            // 24 rows per tile; 16, with a deeper weight ring, where groups of more are rare whatever the router (4096 x 2048 x 256,
+            // 64 tokens: 475 us with 16, 485 with 24; 256 tokens under Zipf, 7168 x 1024 x 896: 598 / 561)
+            p.tile_rows = L->knobs.planes_tile ? (uint32_t)L->knobs.planes_tile : pairs <= 4u * n_groups && max_rows <= 128u ? 16u : 24u;
+            p.tile_table = static_cast<uint32_t*>(L->prefill_scratch);
+            launch_tile_list(offsets, n_groups, static_cast<uint32_t*>(L->prefill_scratch), p.tile_rows, s);
+        }
+        p.planes = reinterpret_cast<const uint8_t*>(L->y);
+        p.x_scales = reinterpret_cast<const uint8_t*>(L->xg);
+        p.plane_rows = bound;
+        const bool nv = fmt == STRATA_MOE_FMT_NVFP4;
+        p.rowscale = nv ? L->x_rowscale : nullptr;
+        p.post0 = nv ? L->tab[0].d_post : nullptr;
+        p.post1 = nv ? L->tab[1].d_post : nullptr;
+        p.out = L->act_f32;
+        p.status = ctx->d_status;
+        p.glu = GluParams{L->d.activation, L->d.gate_beta, L->d.linear_beta};
+        mark(ctx, 4);
+        if (launch_planes_gate_up(fmt, p, L->d_wmaps, L->d_sfmaps, s) != 0)
+            return fail(ctx, STRATA_MOE_E_CUDA, "gate/up plane launch failed");
+        mark(ctx, 5);
+        launch_rows_to_planes(fmt, L->act_f32, true, bound, pairs_dev, I, nullptr, 1, bound, L->act_planes, L->act_hi, L->act_rowscale, s);
+        p.planes = L->act_planes;
+        p.x_scales = reinterpret_cast<const uint8_t*>(L->act_hi);
+        p.rowscale = nv ? L->act_rowscale : nullptr;
+        p.post0 = p.post1 = nv ? L->tab[2].d_post : nullptr;
+        p.out = y;
+        if (launch_planes_down(fmt, p, L->d_wmaps, L->d_sfmaps, s) != 0)
+            return fail(ctx, STRATA_MOE_E_CUDA, "down plane launch failed");
         mark(ctx, 6);
         CK(cudaGetLastError());
         return 0;
@@ -1083,8 +1188,16 @@ int strata_moe_layer_create(strata_moe_ctx* ctx, const strata_moe_layer_desc* de
         A(cudaMalloc(&sm, (size_t)9 * n * 128 + 128));
         if (sm) L->owned.push_back(sm);
         L->d_smaps = sm;
+        void* sf = nullptr;
+        A(cudaMalloc(&sf, (size_t)3 * n * 128 + 128));
+        if (sf) L->owned.push_back(sf);
+        L->d_sfmaps = sf;
     }
     A(ws_reserve(ctx, kWsActF32, (size_t)P * I * 4));
+    if (planes_supported(d.format, H, I)) {     // the digit planes serve small groups only
+        L->plane_rows = (uint32_t)((uint64_t)P < (uint64_t)kMaxPlaneRows * n ? (uint64_t)P : (uint64_t)kMaxPlaneRows * n);
+        A(ws_reserve(ctx, kWsActPlanes, (size_t)L->plane_rows * I * 4));
+    }
     A(ws_reserve(ctx, kWsXRow, (size_t)P * 4));
     A(ws_reserve(ctx, kWsActRow, (size_t)P * 4));
     if (d.shared_intermediate) {
@@ -1474,7 +1587,7 @@ int strata_moe_forward(strata_moe_layer* L, const void* x, uint32_t T, float* ou
     bool y_half = true;
     const SpreadRows spread{L->inv, T, d.top_k, nullptr};
     rc = run_experts(L, xb, perm, d.top_k, P, d.experts, offsets, L->active, L->n_active, T, L->y, 0, nullptr, x_ready,
-                     &y_half, nullptr, d.top_k <= 32u ? &spread : nullptr);
+                     &y_half, nullptr, d.top_k <= 32u ? &spread : nullptr, true);
     if (rc) return rc;
     const float* shared = nullptr;
     if (fork_shared) {
@@ -1505,9 +1618,10 @@ int strata_moe_forward(strata_moe_layer* L, const void* x, uint32_t T, float* ou
     return 0;
 }
 
-// The layer after routing: ids / weights given (device, [T, k], selection-rank order).
-int strata_moe_forward_routed(strata_moe_layer* L, const void* x, uint32_t T, const uint32_t* ids, const float* w,
-                              float* out) {
+// The layer after routing: ids / weights given (device, [T, k], selection-rank order).  distinct: a token's ids are (they
+// come from a router), so that no expert gets more rows than there are tokens.
+static int forward_routed(strata_moe_layer* L, const void* x, uint32_t T, const uint32_t* ids, const float* w, float* out,
+                          bool distinct) {
     if (!L) return STRATA_MOE_E_INVALID;
     strata_moe_ctx* ctx = L->ctx;
     if (!x || !out || !ids || !w) return fail(ctx, STRATA_MOE_E_INVALID, "null pointer");
@@ -1528,12 +1642,19 @@ int strata_moe_forward_routed(strata_moe_layer* L, const void* x, uint32_t T, co
     const strata_moe_layer_desc& d = L->d;
     const uint32_t P = T * d.top_k;
     launch_group(ids, P, 0, d.experts, L->counts, L->offsets, L->perm, L->inv, L->active, L->n_active, L->group_scratch, s);
-    rc = run_experts(L, (const __nv_bfloat16*)x, L->perm, d.top_k, P, d.experts, L->offsets, L->active, L->n_active, T, L->y);
+    const SpreadRows spread{L->inv, T, d.top_k, nullptr};
+    rc = run_experts(L, (const __nv_bfloat16*)x, L->perm, d.top_k, P, d.experts, L->offsets, L->active, L->n_active, T, L->y,
+                     0, nullptr, false, nullptr, nullptr, &spread, distinct);
     if (rc) return rc;
     launch_combine(L->y, L->inv, w, nullptr, T, d.top_k, d.hidden, d.output_scale, out, ctx->d_status, s);
     CK(cudaGetLastError());
     ctx->stats.forward_calls++;
     return 0;
+}
+
+int strata_moe_forward_routed(strata_moe_layer* L, const void* x, uint32_t T, const uint32_t* ids, const float* w,
+                              float* out) {
+    return forward_routed(L, x, T, ids, w, out, false);
 }
 
 int strata_moe_forward_host(strata_moe_layer* L, const void* x_host, uint32_t T, float* out_host) {
@@ -2000,7 +2121,7 @@ int strata_moe_latent_forward(strata_moe_latent* lat, const void* x, uint32_t T,
     if (launch_router_tc(x, T, lat->down, lat->HL, lat->H, lat->latent_f32, lat->tiles, lat->off2, ctx->d_status, s) != 0)
         return fail(ctx, STRATA_MOE_E_CUDA, "latent down projection launch failed");
     launch_f32_to_bf16(lat->latent_f32, (size_t)T * lat->HL, lat->latent_bf16, s);
-    rc = strata_moe_forward_routed(lat->experts, lat->latent_bf16, T, ids, w, lat->mix);
+    rc = forward_routed(lat->experts, lat->latent_bf16, T, ids, w, lat->mix, true);
     if (rc) return rc;
     launch_rmsnorm_bf16(lat->mix, lat->norm, T, lat->HL, lat->eps, lat->mixn, ctx->d_status, s);
     if (launch_router_tc(lat->mixn, T, lat->up, lat->H, lat->HL, out, lat->tiles, lat->off2, ctx->d_status, s) != 0)

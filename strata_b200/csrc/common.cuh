@@ -121,6 +121,7 @@ void launch_rows_to_f16_spread(const __nv_bfloat16* x, const uint32_t* dest, uin
 void launch_rows_to_f16_f32(const float* x, uint32_t src_rows, uint32_t rows, uint32_t C, void* hi, void* lo,
                             float* rowscale, cudaStream_t s, const uint32_t* rows_dev = nullptr, bool int4_order = false);
 void launch_int4_scale_range(const uint8_t* const* scales, uint32_t n, size_t count, uint32_t* not_ok, cudaStream_t s);
+void launch_nv_scale_range(const uint8_t* const* scales, uint32_t n, size_t bytes, uint32_t* not_ok, cudaStream_t s);
 void launch_mx_scale_range(const uint8_t* const* scales, uint32_t n, size_t bytes, uint32_t* emin,
                            float* post_scale, uint32_t* not_ok, cudaStream_t s);
 void launch_dequant_export_f16(int fmt, const uint8_t* packed, const uint8_t* scales, uint32_t emin,
@@ -170,6 +171,33 @@ int prefill_encode_weight_map_bf16(void* out128, const void* w, uint32_t rows, u
 int prefill_encode_weight_map(void* out128, const void* packed, uint32_t rows, uint32_t K);
 int launch_prefill_bf16(const PrefillArgs& a, const void* x, uint32_t rows, const void* w_gate, const void* w_up,
                         const void* w_down, void* act, uint32_t rows_cap, cudaStream_t s);
+// Tile list of a grouped launch: scratch of prefill_scratch_bytes() at `table`, `rows` (16 .. 192) token rows per tile.
+void launch_tile_list(const uint32_t* offsets, uint32_t n_groups, uint32_t* table, uint32_t rows, cudaStream_t s);
+// fp4_planes.cu : FP4 weights on the block-scaled tensor-core instructions, activations as E2M1 digit planes
+struct PlaneArgs {
+    uint32_t H, I, n_groups;
+    const uint32_t* offsets;       // [n_groups + 1]
+    const uint32_t* tile_table;    // tile list of tile_rows rows, or nullptr: every listed group has at most tile_rows rows
+    const uint32_t* active_list;   // [n_active], read when there is no tile list
+    const uint32_t* n_active;
+    uint32_t tile_rows;            // 8, 16 or 24
+    const uint8_t *planes, *x_scales;   // of the grouped rows, as launch_rows_to_planes lays them out
+    uint32_t plane_rows;
+    const float* rowscale;         // factor per row, or nullptr
+    const float *post0, *post1;    // [n_groups] factors of the first and second weight tile, or nullptr
+    float* out;                    // act [rows, I] or y [rows, H]
+    uint32_t* status;
+    GluParams glu;
+};
+bool planes_supported(int fmt, uint32_t H, uint32_t I);
+int planes_encode_scale_map(void* out128, int fmt, const void* scales, uint32_t rows, uint32_t K);
+// rows of `cols` BF16 (or FP32) values -> planes (cols * 4 bytes per plane row), scales (cols / 32 or cols / 16), rowscale (NVFP4);
+// source row r goes to plane rows dest[r * k .. r * k + k - 1], or to plane row r.
+void launch_rows_to_planes(int fmt, const void* src, bool f32, uint32_t rows, const uint32_t* rows_dev, uint32_t cols,
+                           const uint32_t* dest, uint32_t k, uint32_t plane_rows, void* planes, void* scales, float* rowscale,
+                           cudaStream_t s);
+int launch_planes_gate_up(int fmt, const PlaneArgs& a, const void* wmaps, const void* smaps, cudaStream_t s);
+int launch_planes_down(int fmt, const PlaneArgs& a, const void* wmaps, const void* smaps, cudaStream_t s);
 // Router projection on the tensor cores (approximate summation order; see router.cu for its use).
 // tile_table: scratch of prefill_scratch_bytes(1, T); offsets2: device {0, T}.
 int launch_router_tc(const void* x_bf16, uint32_t T, const void* wg_bf16, uint32_t E, uint32_t H, float* logits,

@@ -538,6 +538,21 @@ __global__ void __launch_bounds__(256) int4_scale_range_kernel(const uint8_t* co
     if (__any_sync(0xFFFFFFFFu, bad) && (threadIdx.x & 31u) == 0u) atomicOr(not_ok + blockIdx.x, 1u);
 }
 
+// NVFP4: is any E4M3 scale of a projection negative or NaN?  (The block-scaled tensor-core instructions read them unsigned.)
+__global__ void __launch_bounds__(256) nv_scale_range_kernel(const uint8_t* const* __restrict__ scales, size_t bytes,
+                                                             uint32_t* __restrict__ not_ok) {
+    const uint8_t* p = scales[blockIdx.x];
+    bool bad = false;
+    const size_t first = (size_t)blockIdx.y * 256u + threadIdx.x, step = (size_t)gridDim.y * 256u;
+    const size_t whole = (reinterpret_cast<uintptr_t>(p) & 15u) == 0u ? bytes / 16u : 0u;
+    for (size_t i = first; i < whole; i += step) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(p) + i);
+        for (uint32_t w : {v.x, v.y, v.z, v.w}) bad |= (w & 0x80808080u) != 0u || ((w + 0x01010101u) & 0x80808080u) != 0u;
+    }
+    for (size_t i = whole * 16u + first; i < bytes; i += step) bad |= __ldg(p + i) >= 0x7Fu;
+    if (__any_sync(0xFFFFFFFFu, bad) && (threadIdx.x & 31u) == 0u) atomicOr(not_ok + blockIdx.x, 1u);
+}
+
 // Dequantised weights through the f16 decoders above (the values the f16 MMA path consumes),
 // widened to fp32 and multiplied by the accumulator-side factor.
 __global__ void dequant_export_f16_kernel(int fmt, const uint8_t* __restrict__ packed,
@@ -580,6 +595,12 @@ void launch_dequant_export_f16(int fmt, const uint8_t* packed, const uint8_t* sc
 void launch_int4_scale_range(const uint8_t* const* scales, uint32_t n, size_t count, uint32_t* not_ok, cudaStream_t s) {
     if (n == 0) return;
     int4_scale_range_kernel<<<dim3(n, 8), 256, 0, s>>>(scales, count, not_ok);
+    ++g_kernel_launches;
+}
+
+void launch_nv_scale_range(const uint8_t* const* scales, uint32_t n, size_t bytes, uint32_t* not_ok, cudaStream_t s) {
+    if (n == 0) return;
+    nv_scale_range_kernel<<<dim3(n, 8), 256, 0, s>>>(scales, bytes, not_ok);
     ++g_kernel_launches;
 }
 

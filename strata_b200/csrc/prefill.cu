@@ -38,6 +38,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "tc5.cuh"
 
 namespace smoe {
 
@@ -69,83 +70,11 @@ constexpr uint32_t kThreads = (4 + kDecodeWarps + kEpilogueWarps) * 32;
 constexpr uint32_t kPkCols = 256;                       // columns per packed staging block (four 64-column slabs)
 constexpr uint32_t kPkTile = kMTile * (kPkCols / 2);    // 16 KiB of 4-bit weights: 128 rows x 128 B
 constexpr uint32_t kFirstDecodeWarp = 4, kFirstEpilogueWarp = kFirstDecodeWarp + kDecodeWarps;
-constexpr uint32_t kSpinLimit = 1u << 19;   // x up to kWaitHintNs each: about two seconds
 constexpr uint32_t kMinTileRows = 16;   // token rows of the smallest tile: bounds the tile list
 constexpr int kFmtBf16W = 3;  // plain BF16 weights (shared expert): tiles arrive by TMA, no decode
 
 // ------------------------------------------------------------------------------ PTX helpers
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-// Bounded waits: false when the phase did not complete within the limit (about two seconds) or another role raised
-// the abort flag.  Each try_wait carries a suspend-time hint: the hardware parks the thread until the phase completes
-// or the hint expires.  A polling warp takes issue slots from the decode warps of its scheduler, so tighter polling
-// is slower (measured on a 333-token INT4 step: gate/up 1.45 ms as here, 1.69 ms with a four-instruction poll loop).
-constexpr uint32_t kWaitHintNs = 4096;
-__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity), "r"(kWaitHintNs)
-        : "memory");
-    return done != 0u;
-}
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const volatile uint32_t* abort_flag) {
-    const uint32_t addr = smem_u32(bar);
-    for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
-        if (mbar_try(addr, parity)) return true;
-        if ((spin & 63u) == 63u && *abort_flag) return false;
-    }
-    return false;
-}
-// The same for a warp that goes on to warp-wide instructions: lanes may see completion, the time-out or the abort flag at
-// different polls, so the loop itself runs on votes and the warp leaves it as one.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const volatile uint32_t* abort_flag) {
-    const uint32_t addr = smem_u32(bar);
-    for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
-        if (__all_sync(0xFFFFFFFFu, mbar_try(addr, parity))) return true;
-        if ((spin & 63u) == 63u && __any_sync(0xFFFFFFFFu, *abort_flag != 0u)) return false;
-    }
-    return false;
-}
-// Barrier 1 over the epilogue warps; true on every thread when `failed` is true on any.
-__device__ __forceinline__ bool epilogue_vote(bool failed) {
-    uint32_t any;
-    __syncwarp();      // the lanes of the polling warp may come out of their wait one by one
-    asm volatile(
-        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, 1, %2, p;\n selp.u32 %0, 1, 0, q;\n}"
-        : "=r"(any)
-        : "r"((uint32_t)failed), "n"(kEpilogueWarps * 32u)
-        : "memory");
-    return any != 0u;
-}
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint32_t x, uint32_t y,
-                                            uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// Low word of a shared-memory matrix descriptor: start address / 16, leading byte offset unused (1).  K-major operand,
-// 128-byte swizzle, 8-row groups 1024 B apart; the high word (kDescHi) holds the stride between the groups / 16, the
-// descriptor version of this architecture (bit 46) and the swizzle (2 at bit 61).
-__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (1u << 16); }
+__device__ __forceinline__ bool epilogue_vote(bool failed) { return group_vote<kEpilogueWarps * 32u>(failed); }
 // Instruction descriptor, kind::f16: F16 x F16 (or BF16 x BF16) -> F32, both operands K-major, M = 128.
 __device__ __forceinline__ uint32_t umma_idesc_f16(uint32_t n, uint32_t ab_format /* 0 = F16, 1 = BF16 */) {
     uint32_t d = 0;
@@ -166,7 +95,6 @@ __device__ __forceinline__ uint32_t umma_idesc_f16(uint32_t n, uint32_t ab_forma
 // without overlap (512 MMAs of 128 x N x 16, clocks per MMA: A in tensor memory 74 / 106 at N = 128 / 192, A in shared
 // memory 107 / 139); with a branch between them they pipeline (64 / 96, the tensor pipe's rate).  `never` is a value the
 // compiler cannot see through that is never 0: the branches on it are not taken and only end the basic blocks.
-constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);   // see umma_desc_lo
 __device__ __forceinline__ void umma4_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc,
                                              uint32_t accumulate, uint32_t never) {
     asm volatile(
@@ -198,35 +126,6 @@ __device__ __forceinline__ void umma4_f16_ss(uint32_t tmem_d, uint32_t a_lo, uin
         "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(never), "n"(kDescHi)
         : "memory");
 }
-__device__ __forceinline__ bool elect_one() {
-    uint32_t e;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(e));
-    return e != 0u;
-}
-// This thread's 32 words -> 32 consecutive columns of its tensor-memory lane.
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t v[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
-        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t v[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-
 // ------------------------------------------------------------------------------ decoders (f16)
 __device__ __forceinline__ void p_e2m1x8_f16(uint32_t w, uint32_t r[4]) {
     asm("{\n .reg .b8 b0, b1, b2, b3;\n mov.b32 {b0, b1, b2, b3}, %4;\n"
@@ -318,35 +217,6 @@ __device__ __forceinline__ uint32_t int4_slot(uint32_t c) {
     const uint32_t p = c & 7u;
     return (c & ~7u) | ((p & 3u) << 1) | (p >> 2);
 }
-
-// After a wait on copies that an aborting producer issued but nobody may consume: give each a bounded chance to land.
-__device__ __forceinline__ void drain_copies(uint64_t* full, uint32_t issued, uint32_t stages) {
-    const uint32_t pending = issued < stages ? issued : stages;
-    for (uint32_t q = 0; q < pending; ++q) {
-        const uint32_t j = issued - 1u - q;
-        const uint32_t addr = smem_u32(&full[j % stages]);
-        for (uint32_t spin = 0; spin < (1u << 16); ++spin) {
-            uint32_t done;
-            asm volatile(
-                "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                " selp.u32 %0, 1, 0, p;\n}"
-                : "=r"(done)
-                : "r"(addr), "r"((j / stages) & 1u)
-                : "memory");
-            if (done) break;
-        }
-    }
-}
-
-// A position in a ring of N stages and the parity its barriers have there.
-template <uint32_t N>
-struct Ring {
-    uint32_t i = 0, ph = 0;
-    __device__ __forceinline__ void next(uint32_t step = 1u) {
-        i += step;
-        if (i >= N) { i -= N; ph ^= 1u; }
-    }
-};
 
 // MODE 0: gate + up tiles of the same 128 features, SwiGLU, act (16-bit) out.  K = H, features over I.
 // MODE 1: one down tile (128 features), y (fp32) out.                          K = I, features over H.
@@ -839,25 +709,21 @@ __global__ void __launch_bounds__(1024) prefill_tiles_kernel(const uint32_t* __r
 }
 
 // ------------------------------------------------------------------------------ host side
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
+TensorMapEncodeFn tensor_map_encoder() {
+    static TensorMapEncodeFn fn = nullptr;
     if (!fn) {
         void* p = nullptr;
         cudaDriverEntryPointQueryResult q;
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
             q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
+            fn = reinterpret_cast<TensorMapEncodeFn>(p);
     }
     return fn;
 }
 
 // 16-bit matrix [rows, cols] row-major; box = 64 columns x box_rows rows, 128-byte swizzle.
 static bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-    EncodeTiledFn fn = encode_fn();
+    TensorMapEncodeFn fn = tensor_map_encoder();
     if (!fn) return false;
     const cuuint64_t dims[2] = {cols, rows};
     const cuuint64_t strides[1] = {cols * 2};
@@ -870,7 +736,7 @@ static bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t c
 
 bool prefill_supported(int fmt, uint32_t H, uint32_t I) {
     if (fmt < 0 || fmt > kFmtBf16W) return false;
-    return H % 128u == 0 && I % 128u == 0 && encode_fn() != nullptr;
+    return H % 128u == 0 && I % 128u == 0 && tensor_map_encoder() != nullptr;
 }
 
 size_t prefill_scratch_bytes(uint32_t n_groups, uint32_t pairs) {
@@ -886,7 +752,7 @@ static bool make_bmaps(BMaps* b, const void* base, uint64_t rows, uint64_t cols)
 // Tensor map over one projection's packed 4-bit rows ([rows, K/2] bytes): 128-byte x 128-row
 // boxes, 128-byte swizzle.  `out` receives the 128-byte descriptor (host memory).
 int prefill_encode_weight_map(void* out, const void* packed, uint32_t rows, uint32_t K) {
-    EncodeTiledFn fn = encode_fn();
+    TensorMapEncodeFn fn = tensor_map_encoder();
     if (!fn) return -1;
     const cuuint64_t dims[2] = {K / 2u, rows};
     const cuuint64_t strides[1] = {K / 2u};
@@ -950,10 +816,11 @@ static int launch_one(const PrefillArgs& a, const void* b_hi, const void* b_lo, 
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-static void launch_tiles(const PrefillArgs& a, cudaStream_t s) {
-    prefill_tiles_kernel<<<1, 1024, 0, s>>>(a.offsets, a.n_groups, a.tile_table, a.ntile);
+void launch_tile_list(const uint32_t* offsets, uint32_t n_groups, uint32_t* table, uint32_t rows, cudaStream_t s) {
+    prefill_tiles_kernel<<<1, 1024, 0, s>>>(offsets, n_groups, table, rows);
     ++g_kernel_launches;
 }
+static void launch_tiles(const PrefillArgs& a, cudaStream_t s) { launch_tile_list(a.offsets, a.n_groups, a.tile_table, a.ntile, s); }
 
 // Operands of the gate/up or the down launch beside PrefillArgs.
 struct Operands {
