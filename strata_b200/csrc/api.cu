@@ -64,6 +64,7 @@ struct DeviceTable {
     float* d_global = nullptr;
     uint32_t* d_emin = nullptr;   // f16 path tables
     float* d_post = nullptr;
+    std::vector<uint8_t> top_exp;           // INT4: exponent field of the largest scale when all lie within six octaves, else 0
     std::vector<uint8_t> rescan, inexact;   // INT4, NVFP4: registered since its scales were last looked at; the verdict (INT4: q * scale off f16; NVFP4: a negative or NaN scale)
 };
 
@@ -159,6 +160,7 @@ struct strata_moe_layer {
     bool wmaps_ok = false;
     // f16 decode path for the FP4 formats
     bool f16_ok = false;
+    bool int4_narrow = false;   // ... and the scales of every projection lie within six octaves
     bool int4_f16_ok = false;   // every INT4 weight q * scale is exact in f16
     bool planes_ok = false;     // the FP4 layer's shapes, alignments and scales suit the block-scaled tensor-core kernels
     uint32_t plane_rows = 0;    // rows that the workspace of the activation's planes holds
@@ -336,7 +338,7 @@ int sync_tables(strata_moe_layer* L) {
         for (int r = 0; r < 3; ++r)
             for (uint32_t e = 0; e < n; ++e) complete &= L->tab[r].scales[e] != nullptr;
         if (complete) {   // only what was registered since the last look: a scan of all is the layer's scales read once (6144 x 2048, 256 experts: 151 MB)
-            CK(cudaMemsetAsync(L->d_not_ok, 0, (size_t)3 * n * sizeof(uint32_t), ctx->stream));
+            CK(cudaMemsetAsync(L->d_not_ok, 0, (size_t)6 * n * sizeof(uint32_t), ctx->stream));
             for (int r = 0; r < 3; ++r) {
                 const uint32_t rows = r == STRATA_MOE_ROLE_DOWN ? L->d.hidden : L->d.intermediate;
                 const uint32_t cols = r == STRATA_MOE_ROLE_DOWN ? L->d.intermediate : L->d.hidden;
@@ -346,23 +348,29 @@ int sync_tables(strata_moe_layer* L) {
                     if (last > e) {
                         if (nv)
                             launch_nv_scale_range(L->tab[r].d_scales + e, last - e, scale_bytes(L->d.format, rows, cols),
-                                                  L->d_not_ok + (size_t)r * n + e, ctx->stream);
+                                                  L->d_not_ok + 2u * ((size_t)r * n + e), ctx->stream);
                         else
                             launch_int4_scale_range(L->tab[r].d_scales + e, last - e, scale_bytes(L->d.format, rows, cols) / 2u,
-                                                    L->d_not_ok + (size_t)r * n + e, ctx->stream);
+                                                    L->d_not_ok + 2u * ((size_t)r * n + e), ctx->stream);
                         any = true;
                     }
                     e = last + 1u;
                 }
             }
             if (any) {
-                std::vector<uint32_t> bad((size_t)3 * n);
-                CK(cudaMemcpyAsync(bad.data(), L->d_not_ok, bad.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+                std::vector<uint32_t> seen((size_t)6 * n);
+                CK(cudaMemcpyAsync(seen.data(), L->d_not_ok, seen.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
                 CK(cudaStreamSynchronize(ctx->stream));
                 for (int r = 0; r < 3; ++r)
                     for (uint32_t e = 0; e < n; ++e)
                         if (L->tab[r].rescan[e]) {
-                            L->tab[r].inexact[e] = bad[(size_t)r * n + e] != 0u;
+                            const uint32_t* w = &seen[2u * ((size_t)r * n + e)];
+                            // INT4: q * scale, q of at most three significant bits and the scale of eight, is an f16 number
+                            // while every non-zero scale has a magnitude in [2^-14, 2^12)
+                            const uint32_t least = 0x7FFFu - w[0], most = w[1];
+                            L->tab[r].inexact[e] = nv ? w[0] != 0u : most >= (127u + 12u) << 7 || least < (127u - 14u) << 7;
+                            L->tab[r].top_exp[e] = nv || (most != 0u && (least >> 7) + 5u < (most >> 7)) ? 0u
+                                                   : (uint8_t)(most ? most >> 7 : 127u);
                             L->tab[r].rescan[e] = 0;
                         }
             }
@@ -371,6 +379,21 @@ int sync_tables(strata_moe_layer* L) {
                 for (uint32_t e = 0; e < n; ++e) exact &= L->tab[r].inexact[e] == 0;
             if (nv) scales_ok &= exact;
             else L->int4_f16_ok = exact;
+            if (any && exact && !nv) {
+                // scales of at most six octaves in every projection: the tiles decode with one multiply-add per pair
+                L->int4_narrow = true;
+                for (int r = 0; r < 3; ++r)
+                    for (uint32_t e = 0; e < n; ++e) L->int4_narrow &= L->tab[r].top_exp[e] != 0;
+                for (int r = 0; r < 3 && L->int4_narrow; ++r) {
+                    std::vector<uint32_t> mult(n), post(n);      // floats 2^(15 - top exponent) and 2^(top exponent + 9)
+                    for (uint32_t e = 0; e < n; ++e) {
+                        mult[e] = (269u - L->tab[r].top_exp[e]) << 23;
+                        post[e] = (L->tab[r].top_exp[e] + 9u) << 23;
+                    }
+                    CK(cudaMemcpy(L->tab[r].d_emin, mult.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice));
+                    CK(cudaMemcpy(L->tab[r].d_post, post.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice));
+                }
+            }
         } else {
             scales_ok = false;
         }
@@ -698,6 +721,7 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         p.tile_table = static_cast<uint32_t*>(L->prefill_scratch);
         p.status = ctx->d_status;
         p.glu = GluParams{L->d.activation, L->d.gate_beta, L->d.linear_beta};
+        p.narrow = L->int4_f16_ok && L->int4_narrow ? 1u : 0u;
         p.ntile = prefill_ntile(L, pairs, n_groups, max_rows);
         // the caller combines right away and can take the expert rows as f16: half the bytes written here and read
         // by the combine pass, which is bound by exactly those bytes
@@ -804,6 +828,7 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         p.tile_table = static_cast<uint32_t*>(L->prefill_scratch);
         p.status = ctx->d_status;
         p.glu = GluParams{L->d.activation, L->d.gate_beta, L->d.linear_beta};
+        p.narrow = L->int4_narrow ? 1u : 0u;
         p.ntile = pair_ntile(L, max_rows);
         p.act_f32 = L->act_f32;
         p.act_lo = L->act_lo;
@@ -1143,6 +1168,7 @@ int strata_moe_layer_create(strata_moe_ctx* ctx, const strata_moe_layer_desc* de
         t.global.assign(n, 1.0f);
         t.rescan.assign(n, 1);
         t.inexact.assign(n, 0);
+        t.top_exp.assign(n, 0);
         A(dalloc(L, &t.d_packed, n));
         A(dalloc(L, &t.d_scales, n));
         A(dalloc(L, &t.d_global, n));
@@ -1176,7 +1202,7 @@ int strata_moe_layer_create(strata_moe_ctx* ctx, const strata_moe_layer_desc* de
     A(ws_reserve(ctx, kWsActLo, (size_t)P * I * 2));
     A(ws_reserve(ctx, kWsY, (size_t)P * H * 4));
     A(dalloc(L, &L->one_global, 1));
-    A(dalloc(L, &L->d_not_ok, (size_t)3 * n));
+    A(dalloc(L, &L->d_not_ok, (size_t)6 * n));
     {
         void* wm = nullptr;
         A(cudaMalloc(&wm, (size_t)3 * n * 128 + 128));

@@ -120,7 +120,7 @@ void launch_rows_to_f16_spread(const __nv_bfloat16* x, const uint32_t* dest, uin
                                cudaStream_t s, bool int4_order = false);
 void launch_rows_to_f16_f32(const float* x, uint32_t src_rows, uint32_t rows, uint32_t C, void* hi, void* lo,
                             float* rowscale, cudaStream_t s, const uint32_t* rows_dev = nullptr, bool int4_order = false);
-void launch_int4_scale_range(const uint8_t* const* scales, uint32_t n, size_t count, uint32_t* not_ok, cudaStream_t s);
+void launch_int4_scale_range(const uint8_t* const* scales, uint32_t n, size_t count, uint32_t* range, cudaStream_t s);
 void launch_nv_scale_range(const uint8_t* const* scales, uint32_t n, size_t bytes, uint32_t* not_ok, cudaStream_t s);
 void launch_mx_scale_range(const uint8_t* const* scales, uint32_t n, size_t bytes, uint32_t* emin,
                            float* post_scale, uint32_t* not_ok, cudaStream_t s);
@@ -149,6 +149,7 @@ struct PrefillArgs {
     uint32_t ntile;                // tokens per tile (16 .. 192); the launch takes the next geometry that holds it
     uint32_t reuse_tiles;          // down-only launch: the tile list of the preceding gate/up launch is still valid
     void* act_lo;                  // [pairs_cap, I] or nullptr: the activation travels as a 16-bit hi + lo pair (gate/up writes, down reads both)
+    uint32_t narrow;               // INT4: the scales of every projection span at most six octaves (emin / post_scale are set)
     float* act_f32;                // gate/up: the activation leaves as fp32 rows [pairs, I] (the caller converts), or nullptr
 };
 bool prefill_supported(int fmt, uint32_t H, uint32_t I);

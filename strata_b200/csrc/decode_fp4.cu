@@ -515,30 +515,36 @@ __global__ void __launch_bounds__(256) mx_scale_range_kernel(const uint8_t* cons
     }
 }
 
-// INT4: raises a matrix's not_ok word unless every group scale (BF16) of it is zero or has a magnitude in [2^-14, 2^12): then q * scale, q of
-// at most three significant bits and the scale of eight, is an f16 number.
+// INT4: the largest and the smallest non-zero magnitude of a projection's group scales (BF16), as range[2 i + 1] = the largest bit
+// pattern and range[2 i] = 0x7FFF - the smallest (both 0 to begin with, and when every scale is 0).
 __global__ void __launch_bounds__(256) int4_scale_range_kernel(const uint8_t* const* __restrict__ scales, size_t count,
-                                                               uint32_t* __restrict__ not_ok) {
+                                                               uint32_t* __restrict__ range) {
     const unsigned short* p = reinterpret_cast<const unsigned short*>(scales[blockIdx.x]);
-    bool bad = false;
-    auto check = [&](uint32_t m) {
+    uint32_t small = 0, large = 0;
+    auto look = [&](uint32_t m) {
         m &= 0x7FFFu;
-        bad |= m != 0u && (m < (127u - 14u) << 7 || m >= (127u + 12u) << 7);
+        large = max(large, m);
+        if (m) small = max(small, 0x7FFFu - m);
     };
     const size_t first = (size_t)blockIdx.y * 256u + threadIdx.x, step = (size_t)gridDim.y * 256u;
     const size_t whole = (reinterpret_cast<uintptr_t>(p) & 15u) == 0u ? count / 8u : 0u;      // 16-byte pieces
     for (size_t i = first; i < whole; i += step) {
         const uint4 v = __ldg(reinterpret_cast<const uint4*>(p) + i);
         for (uint32_t w : {v.x, v.y, v.z, v.w}) {
-            check(w);
-            check(w >> 16);
+            look(w);
+            look(w >> 16);
         }
     }
-    for (size_t i = whole * 8u + first; i < count; i += step) check(__ldg(p + i));
-    if (__any_sync(0xFFFFFFFFu, bad) && (threadIdx.x & 31u) == 0u) atomicOr(not_ok + blockIdx.x, 1u);
+    for (size_t i = whole * 8u + first; i < count; i += step) look(__ldg(p + i));
+    small = __reduce_max_sync(0xFFFFFFFFu, small);
+    large = __reduce_max_sync(0xFFFFFFFFu, large);
+    if ((threadIdx.x & 31u) == 0u) {
+        atomicMax(range + 2u * blockIdx.x, small);
+        atomicMax(range + 2u * blockIdx.x + 1u, large);
+    }
 }
 
-// NVFP4: is any E4M3 scale of a projection negative or NaN?  (The block-scaled tensor-core instructions read them unsigned.)
+// NVFP4: not_ok[2 i] = 1 when an E4M3 scale of projection i is negative or NaN.  (The block-scaled tensor-core instructions read them unsigned.)
 __global__ void __launch_bounds__(256) nv_scale_range_kernel(const uint8_t* const* __restrict__ scales, size_t bytes,
                                                              uint32_t* __restrict__ not_ok) {
     const uint8_t* p = scales[blockIdx.x];
@@ -550,7 +556,7 @@ __global__ void __launch_bounds__(256) nv_scale_range_kernel(const uint8_t* cons
         for (uint32_t w : {v.x, v.y, v.z, v.w}) bad |= (w & 0x80808080u) != 0u || ((w + 0x01010101u) & 0x80808080u) != 0u;
     }
     for (size_t i = whole * 16u + first; i < bytes; i += step) bad |= __ldg(p + i) >= 0x7Fu;
-    if (__any_sync(0xFFFFFFFFu, bad) && (threadIdx.x & 31u) == 0u) atomicOr(not_ok + blockIdx.x, 1u);
+    if (__any_sync(0xFFFFFFFFu, bad) && (threadIdx.x & 31u) == 0u) atomicOr(not_ok + 2u * blockIdx.x, 1u);
 }
 
 // Dequantised weights through the f16 decoders above (the values the f16 MMA path consumes),
@@ -592,9 +598,9 @@ void launch_dequant_export_f16(int fmt, const uint8_t* packed, const uint8_t* sc
     ++g_kernel_launches;
 }
 
-void launch_int4_scale_range(const uint8_t* const* scales, uint32_t n, size_t count, uint32_t* not_ok, cudaStream_t s) {
+void launch_int4_scale_range(const uint8_t* const* scales, uint32_t n, size_t count, uint32_t* range, cudaStream_t s) {
     if (n == 0) return;
-    int4_scale_range_kernel<<<dim3(n, 8), 256, 0, s>>>(scales, count, not_ok);
+    int4_scale_range_kernel<<<dim3(n, 8), 256, 0, s>>>(scales, count, range);
     ++g_kernel_launches;
 }
 

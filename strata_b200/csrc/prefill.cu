@@ -71,6 +71,7 @@ constexpr uint32_t kPkCols = 256;                       // columns per packed st
 constexpr uint32_t kPkTile = kMTile * (kPkCols / 2);    // 16 KiB of 4-bit weights: 128 rows x 128 B
 constexpr uint32_t kFirstDecodeWarp = 4, kFirstEpilogueWarp = kFirstDecodeWarp + kDecodeWarps;
 constexpr uint32_t kMinTileRows = 16;   // token rows of the smallest tile: bounds the tile list
+constexpr int kFmtInt4N = 4;    // INT4 whose scales span at most six octaves per projection (see p_int4x8_narrow)
 constexpr int kFmtBf16W = 3;  // plain BF16 weights (shared expert): tiles arrive by TMA, no decode
 
 // ------------------------------------------------------------------------------ PTX helpers
@@ -165,6 +166,21 @@ __device__ __forceinline__ void p_int4x8_f16(uint32_t w, uint32_t r[4]) {
     r[1] = p_fma_f16x2(p_magic(w, 0x00F000F0u), k16th, km72);
     r[2] = p_sub_f16x2(p_magic(w8, 0x000F000Fu), k1032);
     r[3] = p_fma_f16x2(p_magic(w8, 0x00F000F0u), k16th, km72);
+}
+// The same weights times their scale in ONE multiply-add per pair, 9 instructions for 8 weights where the above and the
+// multiplication by the scale take 13.  A nibble that a mask leaves in the low bits of a half is the subnormal f16 number
+// n 2^-24, or n 2^-20 four bits higher; with m24 = 2^24 s, m20 = 2^20 s and c = -8 s the multiply-add is (n - 8) s, exact:
+// its result has at most eleven significant bits.  2^24 s has to stay below 2^16, and s at or above 2^-14 keeps the products
+// normal numbers (of subnormal ones the MMA keeps fewer bits), so the scales of a projection, times a power of two of its own
+// (WeightTable::emin holds 2^24 of it as a float, post_scale undoes it), lie in [2^-14, 2^-8): six octaves, and the bits of the
+// result are those of the decode above.  6144 x 2048 x 256 experts, whole layer: 4 tokens 268 -> 252 us, 333 tokens 1440 -> 1391,
+// 4096 tokens 2608 -> 2565.
+__device__ __forceinline__ void p_int4x8_narrow(uint32_t w, uint32_t m24, uint32_t m20, uint32_t c, uint32_t r[4]) {
+    const uint32_t w8 = w >> 8;
+    r[0] = p_fma_f16x2(w & 0x000F000Fu, m24, c);
+    r[1] = p_fma_f16x2(w & 0x00F000F0u, m20, c);
+    r[2] = p_fma_f16x2(w8 & 0x000F000Fu, m24, c);
+    r[3] = p_fma_f16x2(w8 & 0x00F000F0u, m20, c);
 }
 // Pins 32 computed registers before whatever follows.
 __device__ __forceinline__ void keep32(const uint32_t v[32]) {
@@ -446,6 +462,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
         const uint32_t a_lane = tmem_base + (((warp & 3u) * 32u) << 16) + kAccCols + which * (kKst / 2u) +
                                 (kSlabs == 2u ? sub * (kBK / 2u) : 0u);
         const uint32_t off0 = ((2u * sub) ^ (arow & 7u)) << 4, off1 = off0 ^ 16u;   // this warp's first slab; the other is ^ 64
+        constexpr bool kEmin = FMT == STRATA_MOE_FMT_MXFP4 || FMT == kFmtInt4N;
         const WeightTable& wt = GU ? (which ? a.up : a.gate) : a.down;
         const uint32_t blocks = (K + kPkCols - 1u) / kPkCols, k_slabs = K / kBK;
         const size_t scale_row = FMT == STRATA_MOE_FMT_MXFP4 ? K / 32u : FMT == STRATA_MOE_FMT_NVFP4 ? K / 16u : K / 128u * 2u;
@@ -491,11 +508,11 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
         TileInfo t, tn;
         bool have = (DUAL || wd < kDecodeWarps / 2u) && tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat);
         const uint8_t *srow = nullptr, *sbase = nullptr;
-        uint32_t emin = 0;
+        uint32_t emin = 0;      // MXFP4: smallest scale byte; narrow INT4: the float its scales are multiplied by
         uint4 sc_next = make_uint4(0, 0, 0, 0);
         if (have) {
             srow = wt.scales[t.g] + (t.m0 + arow + which * kSecond) * scale_row;
-            if (FMT == STRATA_MOE_FMT_MXFP4) emin = wt.emin[t.g];
+            if (kEmin) emin = wt.emin[t.g];
             sc_next = load_scales(srow, 0);
         }
         for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
@@ -517,6 +534,15 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
                 for (uint32_t jj = 0; jj < 2u; ++jj) {
                     if (q * 4u + jj * 2u >= k_slabs) break;   // K % 256 == 128: the last block holds two slabs
                     uint32_t v[32];
+                    uint32_t m24 = 0, m20 = 0, mc = 0;
+                    if (FMT == kFmtInt4N) {
+                        // one scale for the slab's 64 columns; powers of two are steps of the exponent field (a zero stays zero)
+                        const float sf = __uint_as_float(sel[jj] << 16) * __uint_as_float(emin);
+                        m24 = (uint32_t)__half_as_ushort(__float2half_rn(sf)) * 0x00010001u;
+                        const bool zero = (m24 & 0x7FFFu) == 0u;
+                        m20 = zero ? 0u : m24 - 4u * 0x04000400u;
+                        mc = zero ? 0u : (m24 - 21u * 0x04000400u) ^ 0x80008000u;
+                    }
 #pragma unroll
                     for (uint32_t c = 0; c < 2u; ++c) {
                         const uint4 p = *reinterpret_cast<const uint4*>(pk_row + ((c ? off1 : off0) ^ (jj * 64u)));
@@ -529,7 +555,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
                             asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(pair) : "h"((unsigned short)(sel[jj] >> (16u * c))));
                             m[0] = __byte_perm(pair, pair, 0x1010);
                             m[1] = __byte_perm(pair, pair, 0x3232);
-                        } else {
+                        } else if (FMT == STRATA_MOE_FMT_INT4G128) {
                             const uint32_t h = __half_as_ushort(__float2half_rn(__uint_as_float(sel[jj] << 16)));
                             m[0] = m[1] = h * 0x00010001u;
                         }
@@ -537,6 +563,10 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
 #pragma unroll
                         for (uint32_t i = 0; i < 4u; ++i) {
                             uint32_t r[4];
+                            if (FMT == kFmtInt4N) {
+                                p_int4x8_narrow(w[i], m24, m20, mc, &v[c * 16u + i * 4u]);
+                                continue;
+                            }
                             if (FMT == STRATA_MOE_FMT_INT4G128) p_int4x8_f16(w[i], r);
                             else p_e2m1x8_f16(w[i], r);
 #pragma unroll
@@ -562,7 +592,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
                 if (hn) {
                     if (q == 0u) {
                         sbase = wt.scales[tn.g];
-                        if (FMT == STRATA_MOE_FMT_MXFP4) emin_n = wt.emin[tn.g];
+                        if (kEmin) emin_n = wt.emin[tn.g];
                     }
                     if (q + 2u == blocks || blocks == 1u) srow = sbase + (tn.m0 + arow + which * kSecond) * scale_row;
                     if (blocks == 1u) sc_next = load_scales(srow, 0);
@@ -597,7 +627,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
             if (epilogue_vote(ew == 0u && !mbar_wait(&S.acc_full[rc.i], rc.ph, abort_flag))) { ok = false; break; }
             tc_fence_after();
             const uint32_t feat = t.m0 + lane_base + lane;
-            const uint32_t act_col = FMT == STRATA_MOE_FMT_INT4G128 ? int4_slot(feat) : feat;   // the down tiles' column order
+            const uint32_t act_col = FMT == STRATA_MOE_FMT_INT4G128 || FMT == kFmtInt4N ? int4_slot(feat) : feat;   // the down tiles' column order
             const uint32_t taddr = tmem_base + rc.i * (2u * NT) + (lane_base << 16);
             const uint32_t lo_at = 16u << box_of(t.n);      // SPLIT: accumulator columns of the lo rows
             for (uint32_t c0 = (ew >> 2) * 16u; c0 < t.n; c0 += 16u * (kEpilogueWarps / 4u)) {
@@ -860,7 +890,8 @@ static int gate_up_any(const PrefillArgs& a, const Operands& o, cudaStream_t s) 
     switch (a.fmt) {
         case STRATA_MOE_FMT_MXFP4: return launch_gate_up_nt<STRATA_MOE_FMT_MXFP4>(a, o, s);
         case STRATA_MOE_FMT_NVFP4: return launch_gate_up_nt<STRATA_MOE_FMT_NVFP4>(a, o, s);
-        case STRATA_MOE_FMT_INT4G128: return launch_gate_up_nt<STRATA_MOE_FMT_INT4G128>(a, o, s);
+        case STRATA_MOE_FMT_INT4G128:
+            return a.narrow ? launch_gate_up_nt<kFmtInt4N>(a, o, s) : launch_gate_up_nt<STRATA_MOE_FMT_INT4G128>(a, o, s);
         case kFmtBf16W: return launch_gate_up_nt<kFmtBf16W>(a, o, s);
         default: return -1;
     }
@@ -869,7 +900,8 @@ static int down_any(const PrefillArgs& a, const Operands& o, cudaStream_t s) {
     switch (a.fmt) {
         case STRATA_MOE_FMT_MXFP4: return launch_down_nt<STRATA_MOE_FMT_MXFP4>(a, o, s);
         case STRATA_MOE_FMT_NVFP4: return launch_down_nt<STRATA_MOE_FMT_NVFP4>(a, o, s);
-        case STRATA_MOE_FMT_INT4G128: return launch_down_nt<STRATA_MOE_FMT_INT4G128>(a, o, s);
+        case STRATA_MOE_FMT_INT4G128:
+            return a.narrow ? launch_down_nt<kFmtInt4N>(a, o, s) : launch_down_nt<STRATA_MOE_FMT_INT4G128>(a, o, s);
         case kFmtBf16W: return launch_down_nt<kFmtBf16W>(a, o, s);
         default: return -1;
     }
