@@ -7,6 +7,7 @@
 
 #include <nvtx3/nvToolsExt.h>
 #include <new>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -676,13 +677,20 @@ struct SpreadRows {
     const uint32_t* rows_dev;   // device-side count of source rows, or null
 };
 
+// A down projection in blocks of output columns: `done` is called, in stream order, behind the kernel of each block.
+struct ColumnBlocks {
+    uint32_t blocks;
+    std::function<int(uint32_t col0, uint32_t cols, bool y_half)> done;
+};
+
 // Expert FFN over grouped rows.  x_nat: rows in natural column order (group order).
 // If x_kperm is non-null it already holds the K-permuted copy.
 int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t* perm, uint32_t k_div,
                 uint32_t pairs, uint32_t n_groups, const uint32_t* offsets, const uint32_t* active,
                 const uint32_t* n_active, uint32_t max_rows, float* y, uint32_t expected_pairs = 0,
                 const uint32_t* pairs_dev = nullptr, bool x_ready = false, bool* y_half = nullptr,
-                float* y_rowscale_out = nullptr, const SpreadRows* spread = nullptr, bool one_row_per_token = false) {
+                float* y_rowscale_out = nullptr, const SpreadRows* spread = nullptr, bool one_row_per_token = false,
+                const ColumnBlocks* columns = nullptr) {
     // `pairs` bounds the row count.  When the exact count exists only on the device (rows received
     // from other ranks) pairs_dev points at it and expected_pairs steers the host-side heuristics.
     Range range("strata_moe.experts");
@@ -728,6 +736,20 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         p.y_half = (y_half && *y_half && !L->knobs.no_half_y) ? 1u : 0u;
         if (y_half) *y_half = p.y_half != 0u;
         p.y_rowscale_out = p.y_half ? y_rowscale_out : nullptr;
+        if (columns) {
+            if (launch_prefill_gate_up(p, L->xg, L->x_rowscale, L->act_hi, L->max_pairs, L->d_wmaps, s) != 0)
+                return fail(ctx, STRATA_MOE_E_CUDA, "prefill launch failed");
+            p.reuse_tiles = 1;
+            p.feats = p.H / columns->blocks;
+            for (uint32_t b = 0; b < columns->blocks; ++b) {
+                p.feat0 = b * p.feats;
+                if (launch_prefill_down(p, L->act_hi, nullptr, L->max_pairs, L->d_wmaps, s) != 0)
+                    return fail(ctx, STRATA_MOE_E_CUDA, "prefill launch failed");
+                const int rc = columns->done(p.feat0, p.feats, p.y_half != 0u);
+                if (rc) return rc;
+            }
+            return 0;
+        }
         if (launch_prefill(p, L->xg, L->x_rowscale, L->act_hi, L->max_pairs, L->d_wmaps, s,
                            ctx->timing ? ctx->pev[5] : nullptr) != 0)
             return fail(ctx, STRATA_MOE_E_CUDA, "prefill launch failed");
@@ -1540,8 +1562,10 @@ int strata_moe_combine(strata_moe_layer* L, const float* y, const uint32_t* inv,
     return 0;
 }
 
-int strata_moe_forward(strata_moe_layer* L, const void* x, uint32_t T, float* out,
-                       const strata_moe_aux* aux) {
+// column_blocks > 1 (only for calls on the large-batch tiles, whose kernels it cuts): the output comes in that many blocks of
+// columns, `block_done` is called behind each.
+static int forward_layer(strata_moe_layer* L, const void* x, uint32_t T, float* out, const strata_moe_aux* aux,
+                         uint32_t column_blocks, const std::function<int(uint32_t col0, uint32_t cols)>& block_done) {
     if (!L) return STRATA_MOE_E_INVALID;
     strata_moe_ctx* ctx = L->ctx;
     if (!x || !out) return fail(ctx, STRATA_MOE_E_INVALID, "null pointer");
@@ -1612,9 +1636,23 @@ int strata_moe_forward(strata_moe_layer* L, const void* x, uint32_t T, float* ou
     }
     bool y_half = true;
     const SpreadRows spread{L->inv, T, d.top_k, nullptr};
+    bool joined = false;
+    const ColumnBlocks columns{column_blocks, [&](uint32_t col0, uint32_t cols, bool half) -> int {
+        if (fork_shared && !joined) CK(cudaStreamWaitEvent(s, ctx->ev_join, 0));
+        joined = true;
+        launch_combine(L->y, L->inv, w, fork_shared ? L->sh_y : nullptr, T, d.top_k, d.hidden, d.output_scale, out, ctx->d_status, s,
+                       half, col0, cols);
+        CK(cudaGetLastError());
+        return block_done(col0, cols);
+    }};
     rc = run_experts(L, xb, perm, d.top_k, P, d.experts, offsets, L->active, L->n_active, T, L->y, 0, nullptr, x_ready,
-                     &y_half, nullptr, d.top_k <= 32u ? &spread : nullptr, true);
+                     &y_half, nullptr, d.top_k <= 32u ? &spread : nullptr, true,
+                     column_blocks > 1u ? &columns : nullptr);
     if (rc) return rc;
+    if (column_blocks > 1u) {
+        ctx->stats.forward_calls++;
+        return 0;
+    }
     const float* shared = nullptr;
     if (fork_shared) {
         CK(cudaStreamWaitEvent(s, ctx->ev_join, 0));
@@ -1642,6 +1680,10 @@ int strata_moe_forward(strata_moe_layer* L, const void* x, uint32_t T, float* ou
     }
     ctx->stats.forward_calls++;
     return 0;
+}
+
+int strata_moe_forward(strata_moe_layer* L, const void* x, uint32_t T, float* out, const strata_moe_aux* aux) {
+    return forward_layer(L, x, T, out, aux, 1u, nullptr);
 }
 
 // The layer after routing: ids / weights given (device, [T, k], selection-rank order).  distinct: a token's ids are (they
@@ -1692,7 +1734,8 @@ int strata_moe_forward_host(strata_moe_layer* L, const void* x_host, uint32_t T,
     CK(cudaSetDevice(ctx->device));
     bind_ws(L);
     const size_t H = L->d.hidden;
-    const size_t in_bytes = (size_t)T * H * 2, out_bytes = (size_t)T * H * 4;
+    const size_t in_bytes = (size_t)T * H * 2, out_bytes = (size_t)T * H * 4, out_row = H * 4;
+    constexpr size_t kColumnBlockBytes = 16u << 20;
     ctx->stats.h2d_bytes += in_bytes;
     ctx->stats.d2h_bytes += out_bytes;
     // Large batches go through in token chunks: the copy of chunk i + 1 into the device and the copy of chunk i - 1
@@ -1720,20 +1763,41 @@ int strata_moe_forward_host(strata_moe_layer* L, const void* x_host, uint32_t T,
     while (parts > 1u && !(use_prefill(L, T * L->d.top_k, L->d.experts) &&
                            use_prefill(L, (T / parts) * L->d.top_k, L->d.experts)))
         --parts;
+    if (parts > 1u || T * out_row >= kColumnBlockBytes) {
+        if (!ctx->copy_in) {
+            CK(cudaStreamCreateWithFlags(&ctx->copy_in, cudaStreamNonBlocking));
+            CK(cudaStreamCreateWithFlags(&ctx->copy_out, cudaStreamNonBlocking));
+            for (int i = 0; i < 4; ++i) {
+                CK(cudaEventCreateWithFlags(&ctx->ev_in[i], cudaEventDisableTiming));
+                CK(cudaEventCreateWithFlags(&ctx->ev_done[i], cudaEventDisableTiming));
+            }
+        }
+    }
     if (parts <= 1u) {
         CK(cudaMemcpyAsync(L->x_stage, x_host, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
-        int rc = strata_moe_forward(L, L->x_stage, T, L->out_stage, nullptr);
-        if (rc) return rc;
-        CK(cudaMemcpyAsync(out_host, L->out_stage, out_bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        return strata_moe_synchronize(ctx);
-    }
-    if (!ctx->copy_in) {
-        CK(cudaStreamCreateWithFlags(&ctx->copy_in, cudaStreamNonBlocking));
-        CK(cudaStreamCreateWithFlags(&ctx->copy_out, cudaStreamNonBlocking));
-        for (int i = 0; i < 4; ++i) {
-            CK(cudaEventCreateWithFlags(&ctx->ev_in[i], cudaEventDisableTiming));
-            CK(cudaEventCreateWithFlags(&ctx->ev_done[i], cudaEventDisableTiming));
+        // A large result goes out in four blocks of columns: a block's copy runs beside the down projection of the next ones.
+        // Columns are independent and keep their tiles, so the bits are those of the one-piece call (4096 tokens of c2: the 100 MB
+        // of the result, 1.9 ms of copy, start 0.6 ms earlier).  Below 16 MB the copy is shorter than what more launches cost.
+        uint32_t blocks = 1u;
+        if (T * out_row >= kColumnBlockBytes && H % 1024u == 0u && !ctx->timing && L->knobs.host_chunks == 0 &&
+            sync_tables(L) == 0 && expert_path(L, T * L->d.top_k, L->d.experts, T, true) == ExpertPath::kTiles)
+            blocks = 4u;
+        uint32_t sent = 0;
+        int rc = forward_layer(L, L->x_stage, T, L->out_stage, nullptr, blocks, [&](uint32_t col0, uint32_t cols) -> int {
+            CK(cudaEventRecord(ctx->ev_done[sent], ctx->stream));
+            CK(cudaStreamWaitEvent(ctx->copy_out, ctx->ev_done[sent], 0));
+            ++sent;
+            CK(cudaMemcpy2DAsync(out_host + col0, out_row, L->out_stage + col0, out_row, (size_t)cols * 4, T, cudaMemcpyDeviceToHost,
+                                 ctx->copy_out));
+            return 0;
+        });
+        if (rc) {
+            if (sent) cudaStreamSynchronize(ctx->copy_out);
+            return rc;
         }
+        if (blocks > 1u) CK(cudaStreamSynchronize(ctx->copy_out));
+        else CK(cudaMemcpyAsync(out_host, L->out_stage, out_bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        return strata_moe_synchronize(ctx);
     }
     // whatever the caller enqueued on the context's stream comes first
     CK(cudaEventRecord(ctx->ev_done[0], ctx->stream));

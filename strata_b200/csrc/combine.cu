@@ -19,13 +19,14 @@ __global__ void __launch_bounds__(256) combine_kernel(const void* __restrict__ y
                                                       const float* __restrict__ weights,
                                                       const float* __restrict__ shared, uint32_t T,
                                                       uint32_t k, uint32_t H, float output_scale,
-                                                      float* __restrict__ out, uint32_t* status) {
+                                                      float* __restrict__ out, uint32_t* status, uint32_t col0,
+                                                      uint32_t cols) {
     constexpr uint32_t V = Y_HALF ? 8u : 4u;     // columns per thread: one 16-byte load of an expert row either way
-    const uint32_t per_row = H / V;
+    const uint32_t per_row = cols / V;
     bool bad = false;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)T * per_row;
          i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t t = (uint32_t)(i / per_row), c = (uint32_t)(i % per_row) * V;
+        const uint32_t t = (uint32_t)(i / per_row), c = col0 + (uint32_t)(i % per_row) * V;
         float o[V];
 #pragma unroll
         for (uint32_t q = 0; q < V; ++q) o[q] = 0.0f;
@@ -96,14 +97,15 @@ __global__ void __launch_bounds__(256) combine_kernel(const void* __restrict__ y
 
 void launch_combine(const void* y, const uint32_t* inv, const float* weights, const float* shared,
                     uint32_t T, uint32_t k, uint32_t H, float output_scale, float* out,
-                    uint32_t* status, cudaStream_t s, bool y_half) {
+                    uint32_t* status, cudaStream_t s, bool y_half, uint32_t col0, uint32_t cols) {
     if (T == 0) return;
-    const size_t n = (size_t)T * (H / (y_half ? 8u : 4u));
+    if (cols == 0) cols = H;
+    const size_t n = (size_t)T * (cols / (y_half ? 8u : 4u));
     const uint32_t grid = (uint32_t)((n + 255) / 256 < 148u * 8u ? (n + 255) / 256 : 148u * 8u);
     if (y_half)
-        combine_kernel<true><<<grid, 256, 0, s>>>(y, inv, weights, shared, T, k, H, output_scale, out, status);
+        combine_kernel<true><<<grid, 256, 0, s>>>(y, inv, weights, shared, T, k, H, output_scale, out, status, col0, cols);
     else
-        combine_kernel<false><<<grid, 256, 0, s>>>(y, inv, weights, shared, T, k, H, output_scale, out, status);
+        combine_kernel<false><<<grid, 256, 0, s>>>(y, inv, weights, shared, T, k, H, output_scale, out, status, col0, cols);
     ++g_kernel_launches;
 }
 

@@ -147,6 +147,7 @@ struct PrefillArgs {
     uint32_t* status;
     GluParams glu;                 // activation of the gate/up epilogue
     uint32_t ntile;                // tokens per tile (16 .. 192); the launch takes the next geometry that holds it
+    uint32_t feat0, feats;         // down: output features feat0 .. feat0 + feats - 1 only (multiples of 256); feats = 0: all of them
     uint32_t reuse_tiles;          // down-only launch: the tile list of the preceding gate/up launch is still valid
     void* act_lo;                  // [pairs_cap, I] or nullptr: the activation travels as a 16-bit hi + lo pair (gate/up writes, down reads both)
     uint32_t narrow;               // INT4: the scales of every projection span at most six octaves (emin / post_scale are set)
@@ -211,7 +212,7 @@ void launch_add_rows(float* out, const float* a, size_t n, cudaStream_t s);
 // combine.cu
 void launch_combine(const void* y, const uint32_t* inv, const float* weights, const float* shared,
                     uint32_t T, uint32_t k, uint32_t H, float output_scale, float* out,
-                    uint32_t* status, cudaStream_t s, bool y_half = false);
+                    uint32_t* status, cudaStream_t s, bool y_half = false, uint32_t col0 = 0, uint32_t cols = 0);
 void launch_dequant_export(int fmt, const uint8_t* packed, const uint8_t* scales, float global_scale,
                            uint32_t rows, uint32_t cols, float* out, cudaStream_t s);
 

@@ -217,13 +217,13 @@ struct __align__(1024) PrefillSmem {
 };
 
 __device__ __forceinline__ bool tile_lookup(const uint32_t* table, uint32_t tile, uint32_t total, uint32_t m_tiles,
-                                            TileInfo& t, uint32_t tile_feat) {
+                                            TileInfo& t, uint32_t tile_feat, uint32_t first_feat) {
     if (tile >= total) return false;
     const uint32_t j = tile / m_tiles;
     t.g = table[4 + 3 * j];
     t.row0 = table[4 + 3 * j + 1];
     t.n = table[4 + 3 * j + 2];
-    t.m0 = (tile - j * m_tiles) * tile_feat;
+    t.m0 = first_feat + (tile - j * m_tiles) * tile_feat;
     return true;
 }
 
@@ -275,7 +275,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
     constexpr uint32_t kSecond = MODE == 2 ? kMTile : 0u;              // row offset of the second weight tile
     const uint32_t K = GU ? a.H : a.I;
     const uint32_t R = GU ? a.I : a.H;
-    const uint32_t m_tiles = R / kTileFeat;
+    const uint32_t m_tiles = (!GU && a.feats ? a.feats : R) / kTileFeat;
     const uint32_t k_stages = K / kKst;
     volatile uint32_t* abort_flag = &S.abort_flag;
     const uint32_t total = a.tile_table[0] * m_tiles;
@@ -321,9 +321,9 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
             Ring<kBStages> rb;
             bool ok = true;
             TileInfo t, tn;
-            bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat);
+            bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat, a.feat0);
             for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
-                const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
+                const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat, a.feat0);
                 const uint32_t bsel = box_of(t.n), rows = 16u << bsel;
                 const bool tail = NT > 128 && t.n > 128u;   // rows from 128 on arrive as a second box: 64 rows (192-token tile) or 32
                 constexpr uint32_t kTailSel = NT == 192 ? 2u : 1u, kTailRows = 16u << kTailSel;
@@ -364,9 +364,9 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
             const uint32_t a_lo0 = umma_desc_lo(smem_u32(arena) + mi * kBfATile);
             bool ok = true;
             TileInfo t, tn;
-            tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat);
+            tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat, a.feat0);
             for (uint32_t tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
-                tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
+                tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat, a.feat0);
                 const uint32_t rows = uni(t.n);
                 if (!all(mbar_wait(&S.acc_empty[rc.i], rc.ph ^ 1u, abort_flag))) { ok = false; break; }
                 tc_fence_after();
@@ -408,9 +408,9 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
             TileInfo t, tn;
             Ring<BF ? kAStages : kPkBufs> rw;
             const uint32_t blocks = BF ? k_stages : (K + kPkCols - 1u) / kPkCols;
-            bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat);
+            bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat, a.feat0);
             for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
-                const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
+                const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat, a.feat0);
                 // BF16: a map per expert when there is a table, else the one matrix pair of the launch
                 const CUtensorMap* m0 = BF && !wmaps ? &map_a0 : wmaps + (GU ? 0u : 2u) * a.n_groups + t.g;
                 const CUtensorMap* m1 = BF && !wmaps ? &map_a1 : wmaps + (GU ? 1u : 2u) * a.n_groups + t.g;
@@ -506,7 +506,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
         Ring<kPkBufs> rp;
         bool ok = true;
         TileInfo t, tn;
-        bool have = (DUAL || wd < kDecodeWarps / 2u) && tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat);
+        bool have = (DUAL || wd < kDecodeWarps / 2u) && tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat, a.feat0);
         const uint8_t *srow = nullptr, *sbase = nullptr;
         uint32_t emin = 0;      // MXFP4: smallest scale byte; narrow INT4: the float its scales are multiplied by
         uint4 sc_next = make_uint4(0, 0, 0, 0);
@@ -518,7 +518,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
         for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
             // the next tile's entry, scale base and first scales are requested one step before they are needed: a chain of
             // dependent loads at every tile start would stop the decoders for about a thousand clocks
-            const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
+            const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat, a.feat0);
             uint32_t emin_n = 0;
             const uint32_t mx_add = (uint32_t)(2 - (int32_t)emin) * 0x04000400u;
             for (uint32_t q = 0; q < blocks; ++q) {
@@ -610,9 +610,9 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
         Ring<kAccBufs> rc;
         bool ok = true, bad = false;
         TileInfo t, tn;
-        bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat);
+        bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat, a.feat0);
         for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
-            const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
+            const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat, a.feat0);
             constexpr bool kNoPost = FMT == STRATA_MOE_FMT_INT4G128 || BF;
             float s0, s1 = 1.0f;
             if (GU) {
