@@ -146,9 +146,6 @@ struct strata_moe_layer {
     __nv_bfloat16* x_stage = nullptr;
     float* out_stage = nullptr;
     void* prefill_scratch = nullptr;
-    uint32_t* shared_tiles = nullptr;  // tile list of the shared expert's grouped GEMM
-    uint32_t* router_tiles = nullptr;  // tile list of the tensor-core router projection
-    uint32_t* router_off2 = nullptr;   // {0, T} for it
     uint32_t* recheck_list = nullptr;  // [max_tokens] tokens the fast router hands to the canonical kernels
     uint32_t* recheck_count = nullptr;
     float* router_norms = nullptr;     // [kFastNormTokens + experts] 2-norms of the fast router's operands
@@ -651,10 +648,7 @@ int run_router(strata_moe_layer* L, const __nv_bfloat16* x, uint32_t T, float* l
     const bool fast = logits_out == nullptr && many && route_fast_supported(rp, d.hidden) &&
                       tensor_path_ok(L, 3, d.intermediate) && (((uintptr_t)x | (uintptr_t)L->router) & 15u) == 0;
     if (fast) {
-        set_pair_kernel<<<1, 1, 0, s>>>(L->router_off2, 0u, T);
-        ++g_kernel_launches;
-        if (launch_router_tc(x, T, L->router, d.experts, d.hidden, L->logits, L->router_tiles, L->router_off2,
-                             ctx->d_status, s) != 0)
+        if (launch_router_tc(x, T, L->router, d.experts, d.hidden, L->logits, ctx->d_status, s) != 0)
             return fail(ctx, STRATA_MOE_E_CUDA, "tensor-core router projection launch failed");
         mark(ctx, 1);
         launch_route_fast(rp, L->logits, L->bias, x, L->router, T, d.hidden, ids, w, L->recheck_list, L->recheck_count,
@@ -927,9 +921,9 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
     return 0;
 }
 
-// shared expert over T rows in natural order; offsets table = {0, T} in L->offsets scratch tail
+// shared expert over T rows in natural order, on the context's stream or on `st`
 int run_shared(strata_moe_layer* L, const __nv_bfloat16* x, const __nv_bfloat16* x_lo, uint32_t T,
-               const uint32_t* offsets2, cudaStream_t st = nullptr) {
+               cudaStream_t st = nullptr) {
     strata_moe_ctx* ctx = L->ctx;
     if (!st) st = ctx->stream;
     // enough rows to fill tensor-core tiles (and BF16 inputs): grouped-GEMM path with one group
@@ -942,9 +936,7 @@ int run_shared(strata_moe_layer* L, const __nv_bfloat16* x, const __nv_bfloat16*
         p.n_groups = 1;
         p.pairs = T;
         p.ntile = prefill_ntile(L, T, 1, T);
-        p.offsets = offsets2;
         p.y = L->sh_y;
-        p.tile_table = L->shared_tiles;
         p.status = ctx->d_status;
         p.glu = GluParams{L->d.activation, L->d.gate_beta, L->d.linear_beta};
         if (launch_prefill_bf16(p, x, T, L->shared_w[0], L->shared_w[1], L->shared_w[2], L->sh_act_hi,
@@ -958,7 +950,10 @@ int run_shared(strata_moe_layer* L, const __nv_bfloat16* x, const __nv_bfloat16*
     a.H = L->d.hidden;
     a.I = L->d.shared_intermediate;
     a.n_groups = 1;
-    a.offsets = offsets2;
+    uint32_t* off2 = L->offsets + L->d.experts + 1 + 2;    // {0, T} in the tail of the offsets; only the shared expert's kernels use it
+    set_pair_kernel<<<1, 1, 0, st>>>(off2, 0u, T);
+    ++g_kernel_launches;
+    a.offsets = off2;
     a.max_rows_per_group = T;
     WeightTable g{L->d_shared_ptr[0], L->d_shared_ptr[0], L->one_global, nullptr, nullptr};
     WeightTable u{L->d_shared_ptr[1], L->d_shared_ptr[1], L->one_global, nullptr, nullptr};
@@ -1249,13 +1244,10 @@ int strata_moe_layer_create(strata_moe_ctx* ctx, const strata_moe_layer_desc* de
     A(ws_reserve(ctx, kWsXRow, (size_t)P * 4));
     A(ws_reserve(ctx, kWsActRow, (size_t)P * 4));
     if (d.shared_intermediate) {
-        A(dalloc(L, &L->shared_tiles, prefill_scratch_bytes(1, T) / sizeof(uint32_t) + 4));
         A(ws_reserve(ctx, kWsShActHi, (size_t)T * d.shared_intermediate * 2));
         A(ws_reserve(ctx, kWsShActLo, (size_t)T * d.shared_intermediate * 2));
         A(ws_reserve(ctx, kWsShY, (size_t)T * H * 4));
     }
-    A(dalloc(L, &L->router_tiles, prefill_scratch_bytes(1, T) / sizeof(uint32_t) + 4));
-    A(dalloc(L, &L->router_off2, 2));
     A(dalloc(L, &L->recheck_list, (size_t)T));
     A(dalloc(L, &L->recheck_count, 1));
     A(dalloc(L, &L->router_norms, (size_t)kFastNormTokens + E));
@@ -1549,10 +1541,7 @@ int strata_moe_combine(strata_moe_layer* L, const float* y, const uint32_t* inv,
     if (x_shared && L->d.shared_intermediate) {
         for (int r = 0; r < 3; ++r)
             if (!L->shared_w[r]) return fail(ctx, STRATA_MOE_E_INVALID, "shared expert weights were never set");
-        uint32_t* off2 = L->offsets + L->d.experts + 1 + 2;
-        set_pair_kernel<<<1, 1, 0, ctx->stream>>>(off2, 0u, T);
-        ++g_kernel_launches;
-        int rc = run_shared(L, static_cast<const __nv_bfloat16*>(x_shared), nullptr, T, off2);
+        int rc = run_shared(L, static_cast<const __nv_bfloat16*>(x_shared), nullptr, T);
         if (rc) return rc;
         shared = L->sh_y;
     }
@@ -1595,12 +1584,9 @@ static int forward_layer(strata_moe_layer* L, const void* x, uint32_t T, float* 
     const uint32_t P = T * d.top_k;
     if (fork_shared) {
         // the shared expert needs only x: it runs on the side stream while the routed path runs here
-        uint32_t* off2 = L->offsets + d.experts + 1 + 2;
-        set_pair_kernel<<<1, 1, 0, s>>>(off2, 0u, T);
-        ++g_kernel_launches;
         CK(cudaEventRecord(ctx->ev_fork, s));
         CK(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
-        rc = run_shared(L, xb, nullptr, T, off2, ctx->side);
+        rc = run_shared(L, xb, nullptr, T, ctx->side);
         if (rc) return rc;
         CK(cudaEventRecord(ctx->ev_join, ctx->side));
     }
@@ -1658,10 +1644,7 @@ static int forward_layer(strata_moe_layer* L, const void* x, uint32_t T, float* 
         CK(cudaStreamWaitEvent(s, ctx->ev_join, 0));
         shared = L->sh_y;
     } else if (d.shared_intermediate) {   // timed run: keep the phases serial so they can be told apart
-        uint32_t* off2 = L->offsets + d.experts + 1 + 2;
-        set_pair_kernel<<<1, 1, 0, s>>>(off2, 0u, T);
-        ++g_kernel_launches;
-        rc = run_shared(L, xb, nullptr, T, off2);
+        rc = run_shared(L, xb, nullptr, T);
         if (rc) return rc;
         shared = L->sh_y;
     }
@@ -1956,14 +1939,12 @@ int strata_moe_enqueue_dense(strata_moe_layer* L, const float* hidden_host, uint
     if (with_shared) {
         for (int r = 0; r < 3; ++r)
             if (!L->shared_w[r]) return fail(ctx, STRATA_MOE_E_INVALID, "shared expert weights were never set");
-        uint32_t* off2 = L->offsets + d.experts + 1 + 2;
-        set_pair_kernel<<<1, 1, 0, s>>>(off2, 0u, rows);
         // natural-layout hi/lo split of the fp32 rows for the BF16 shared expert
         __nv_bfloat16* sh_hi = L->x_stage;
         __nv_bfloat16* sh_lo = reinterpret_cast<__nv_bfloat16*>(L->out_stage);
         split_f32_kernel<<<148, 256, 0, s>>>(L->dense_hidden, (size_t)rows * H, sh_hi, sh_lo);
-        g_kernel_launches += 2;
-        int rc = run_shared(L, sh_hi, sh_lo, rows, off2);
+        ++g_kernel_launches;
+        int rc = run_shared(L, sh_hi, sh_lo, rows);
         if (rc) return rc;
     }
     CK(cudaGetLastError());
@@ -2077,7 +2058,7 @@ struct strata_moe_latent {
     std::vector<void*> owned;
     float *latent_f32 = nullptr, *mix = nullptr, *w = nullptr;
     __nv_bfloat16 *latent_bf16 = nullptr, *mixn = nullptr;
-    uint32_t *tiles = nullptr, *off2 = nullptr, *ids = nullptr;
+    uint32_t* ids = nullptr;
 };
 
 int strata_moe_latent_create(strata_moe_ctx* ctx, const strata_moe_layer_desc* desc, uint32_t model_hidden,
@@ -2117,8 +2098,6 @@ int strata_moe_latent_create(strata_moe_ctx* ctx, const strata_moe_layer_desc* d
     alloc((void**)&lat->mix, T * lat->HL * 4);
     alloc((void**)&lat->latent_bf16, T * lat->HL * 2);
     alloc((void**)&lat->mixn, T * lat->HL * 2);
-    alloc((void**)&lat->tiles, prefill_scratch_bytes(1, (uint32_t)T) + 16);
-    alloc((void**)&lat->off2, 16);
     alloc((void**)&lat->ids, T * desc->top_k * 4);
     alloc((void**)&lat->w, T * desc->top_k * 4);
     if (rc != 0 || e != cudaSuccess) {
@@ -2195,26 +2174,21 @@ int strata_moe_latent_forward(strata_moe_latent* lat, const void* x, uint32_t T,
     if (shared) {   // the shared experts need only x: side stream, joined before the final add
         for (int r = 0; r < 3; ++r)
             if (!R->shared_w[r]) return fail(ctx, STRATA_MOE_E_INVALID, "shared expert weights were never set");
-        uint32_t* off2 = R->offsets + rd.experts + 1 + 2;
-        set_pair_kernel<<<1, 1, 0, s>>>(off2, 0u, T);
-        ++g_kernel_launches;
         CK(cudaEventRecord(ctx->ev_fork, s));
         CK(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
-        int rc = run_shared(R, xb, nullptr, T, off2, ctx->side);
+        int rc = run_shared(R, xb, nullptr, T, ctx->side);
         if (rc) return rc;
         CK(cudaEventRecord(ctx->ev_join, ctx->side));
     }
     int rc = strata_moe_route(R, x, T, nullptr, ids, w);      // routing reads the raw hidden state
     if (rc) return rc;
-    set_pair_kernel<<<1, 1, 0, s>>>(lat->off2, 0u, T);
-    ++g_kernel_launches;
-    if (launch_router_tc(x, T, lat->down, lat->HL, lat->H, lat->latent_f32, lat->tiles, lat->off2, ctx->d_status, s) != 0)
+    if (launch_router_tc(x, T, lat->down, lat->HL, lat->H, lat->latent_f32, ctx->d_status, s) != 0)
         return fail(ctx, STRATA_MOE_E_CUDA, "latent down projection launch failed");
     launch_f32_to_bf16(lat->latent_f32, (size_t)T * lat->HL, lat->latent_bf16, s);
     rc = forward_routed(lat->experts, lat->latent_bf16, T, ids, w, lat->mix, true);
     if (rc) return rc;
     launch_rmsnorm_bf16(lat->mix, lat->norm, T, lat->HL, lat->eps, lat->mixn, ctx->d_status, s);
-    if (launch_router_tc(lat->mixn, T, lat->up, lat->H, lat->HL, out, lat->tiles, lat->off2, ctx->d_status, s) != 0)
+    if (launch_router_tc(lat->mixn, T, lat->up, lat->H, lat->HL, out, ctx->d_status, s) != 0)
         return fail(ctx, STRATA_MOE_E_CUDA, "latent up projection launch failed");
     if (shared) {
         CK(cudaStreamWaitEvent(s, ctx->ev_join, 0));
@@ -2763,12 +2737,9 @@ int strata_moe_ep_begin(strata_moe_ep* ep, const void* x, uint32_t T) {
     ep->T = T;
     ep->forked = false;
     if (d.shared_intermediate && T) {
-        uint32_t* off2 = L->offsets + d.experts + 1 + 2;
-        set_pair_kernel<<<1, 1, 0, s>>>(off2, 0u, T);
-        ++g_kernel_launches;
         CK(cudaEventRecord(ctx->ev_fork, s));
         CK(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
-        rc = run_shared(L, ep->x, nullptr, T, off2, ctx->side);
+        rc = run_shared(L, ep->x, nullptr, T, ctx->side);
         if (rc) return rc;
         CK(cudaEventRecord(ctx->ev_join, ctx->side));
         ep->forked = true;

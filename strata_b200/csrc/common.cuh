@@ -143,7 +143,7 @@ struct PrefillArgs {
     float* y;                      // [pairs, H] fp32
     uint32_t y_half;               // down: store y as f16 [pairs, H] into the same buffer (values beyond the f16 range are reported)
     float* y_rowscale_out;         // down with y_half: receives 1.0 for every row written (rows are not scaled), or nullptr
-    uint32_t* tile_table;          // scratch of prefill_scratch_bytes()
+    uint32_t* tile_table;          // scratch of prefill_scratch_bytes(); nullptr: one group of rows 0 .. pairs - 1, its tiles follow from that
     uint32_t* status;
     GluParams glu;                 // activation of the gate/up epilogue
     uint32_t ntile;                // tokens per tile (16 .. 192); the launch takes the next geometry that holds it
@@ -201,9 +201,8 @@ void launch_rows_to_planes(int fmt, const void* src, bool f32, uint32_t rows, co
 int launch_planes_gate_up(int fmt, const PlaneArgs& a, const void* wmaps, const void* smaps, cudaStream_t s);
 int launch_planes_down(int fmt, const PlaneArgs& a, const void* wmaps, const void* smaps, cudaStream_t s);
 // Router projection on the tensor cores (approximate summation order; see router.cu for its use).
-// tile_table: scratch of prefill_scratch_bytes(1, T); offsets2: device {0, T}.
-int launch_router_tc(const void* x_bf16, uint32_t T, const void* wg_bf16, uint32_t E, uint32_t H, float* logits,
-                     uint32_t* tile_table, const uint32_t* offsets2, uint32_t* status, cudaStream_t s);
+int launch_router_tc(const void* x_bf16, uint32_t T, const void* wg_bf16, uint32_t E, uint32_t H, float* logits, uint32_t* status,
+                     cudaStream_t s);
 // latent.cu : row kernels of the LatentMoE wrapper
 void launch_f32_to_bf16(const float* src, size_t n, __nv_bfloat16* dst, cudaStream_t s);
 void launch_rmsnorm_bf16(const float* x, const float* weight, uint32_t rows, uint32_t cols, float eps,

@@ -216,14 +216,20 @@ struct __align__(1024) PrefillSmem {
     uint32_t abort_flag;
 };
 
-__device__ __forceinline__ bool tile_lookup(const uint32_t* table, uint32_t tile, uint32_t total, uint32_t m_tiles,
-                                            TileInfo& t, uint32_t tile_feat, uint32_t first_feat) {
+__device__ __forceinline__ bool tile_lookup(const PrefillArgs& a, uint32_t tile, uint32_t total, uint32_t m_tiles, TileInfo& t,
+                                            uint32_t tile_feat) {
     if (tile >= total) return false;
     const uint32_t j = tile / m_tiles;
-    t.g = table[4 + 3 * j];
-    t.row0 = table[4 + 3 * j + 1];
-    t.n = table[4 + 3 * j + 2];
-    t.m0 = first_feat + (tile - j * m_tiles) * tile_feat;
+    if (a.tile_table) {
+        t.g = a.tile_table[4 + 3 * j];
+        t.row0 = a.tile_table[4 + 3 * j + 1];
+        t.n = a.tile_table[4 + 3 * j + 2];
+    } else {
+        t.g = 0;
+        t.row0 = j * a.ntile;
+        t.n = min(a.ntile, a.pairs - t.row0);
+    }
+    t.m0 = a.feat0 + (tile - j * m_tiles) * tile_feat;
     return true;
 }
 
@@ -278,7 +284,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
     const uint32_t m_tiles = (!GU && a.feats ? a.feats : R) / kTileFeat;
     const uint32_t k_stages = K / kKst;
     volatile uint32_t* abort_flag = &S.abort_flag;
-    const uint32_t total = a.tile_table[0] * m_tiles;
+    const uint32_t total = (a.tile_table ? a.tile_table[0] : (a.pairs + a.ntile - 1u) / a.ntile) * m_tiles;
     if (total == 0u) return;   // no rows (a rank that received none): leave before any set-up
 
     if (threadIdx.x == 0) {
@@ -321,9 +327,9 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
             Ring<kBStages> rb;
             bool ok = true;
             TileInfo t, tn;
-            bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat, a.feat0);
+            bool have = tile_lookup(a, blockIdx.x, total, m_tiles, t, kTileFeat);
             for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
-                const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat, a.feat0);
+                const bool hn = tile_lookup(a, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
                 const uint32_t bsel = box_of(t.n), rows = 16u << bsel;
                 const bool tail = NT > 128 && t.n > 128u;   // rows from 128 on arrive as a second box: 64 rows (192-token tile) or 32
                 constexpr uint32_t kTailSel = NT == 192 ? 2u : 1u, kTailRows = 16u << kTailSel;
@@ -364,9 +370,9 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
             const uint32_t a_lo0 = umma_desc_lo(smem_u32(arena) + mi * kBfATile);
             bool ok = true;
             TileInfo t, tn;
-            tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat, a.feat0);
+            tile_lookup(a, blockIdx.x, total, m_tiles, t, kTileFeat);
             for (uint32_t tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
-                tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat, a.feat0);
+                tile_lookup(a, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
                 const uint32_t rows = uni(t.n);
                 if (!all(mbar_wait(&S.acc_empty[rc.i], rc.ph ^ 1u, abort_flag))) { ok = false; break; }
                 tc_fence_after();
@@ -408,9 +414,9 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
             TileInfo t, tn;
             Ring<BF ? kAStages : kPkBufs> rw;
             const uint32_t blocks = BF ? k_stages : (K + kPkCols - 1u) / kPkCols;
-            bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat, a.feat0);
+            bool have = tile_lookup(a, blockIdx.x, total, m_tiles, t, kTileFeat);
             for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
-                const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat, a.feat0);
+                const bool hn = tile_lookup(a, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
                 // BF16: a map per expert when there is a table, else the one matrix pair of the launch
                 const CUtensorMap* m0 = BF && !wmaps ? &map_a0 : wmaps + (GU ? 0u : 2u) * a.n_groups + t.g;
                 const CUtensorMap* m1 = BF && !wmaps ? &map_a1 : wmaps + (GU ? 1u : 2u) * a.n_groups + t.g;
@@ -506,7 +512,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
         Ring<kPkBufs> rp;
         bool ok = true;
         TileInfo t, tn;
-        bool have = (DUAL || wd < kDecodeWarps / 2u) && tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat, a.feat0);
+        bool have = (DUAL || wd < kDecodeWarps / 2u) && tile_lookup(a, blockIdx.x, total, m_tiles, t, kTileFeat);
         const uint8_t *srow = nullptr, *sbase = nullptr;
         uint32_t emin = 0;      // MXFP4: smallest scale byte; narrow INT4: the float its scales are multiplied by
         uint4 sc_next = make_uint4(0, 0, 0, 0);
@@ -518,7 +524,7 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
         for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
             // the next tile's entry, scale base and first scales are requested one step before they are needed: a chain of
             // dependent loads at every tile start would stop the decoders for about a thousand clocks
-            const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat, a.feat0);
+            const bool hn = tile_lookup(a, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
             uint32_t emin_n = 0;
             const uint32_t mx_add = (uint32_t)(2 - (int32_t)emin) * 0x04000400u;
             for (uint32_t q = 0; q < blocks; ++q) {
@@ -610,9 +616,9 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
         Ring<kAccBufs> rc;
         bool ok = true, bad = false;
         TileInfo t, tn;
-        bool have = tile_lookup(a.tile_table, blockIdx.x, total, m_tiles, t, kTileFeat, a.feat0);
+        bool have = tile_lookup(a, blockIdx.x, total, m_tiles, t, kTileFeat);
         for (uint32_t tile = blockIdx.x; ok && have; tile += gridDim.x) {
-            const bool hn = tile_lookup(a.tile_table, tile + gridDim.x, total, m_tiles, tn, kTileFeat, a.feat0);
+            const bool hn = tile_lookup(a, tile + gridDim.x, total, m_tiles, tn, kTileFeat);
             constexpr bool kNoPost = FMT == STRATA_MOE_FMT_INT4G128 || BF;
             float s0, s1 = 1.0f;
             if (GU) {
@@ -941,15 +947,15 @@ int launch_prefill(const PrefillArgs& args, const void* x16, const float* x_rows
 
 // BF16 expert (the shared expert) over `rows` token rows in natural order: x [rows, H] BF16,
 // gate/up [I, H], down [H, I] BF16, act [rows_cap, I] BF16 scratch, y [rows, H] fp32.
-// args.offsets must hold {0, rows}; args.n_groups = 1.
 int launch_prefill_bf16(const PrefillArgs& args, const void* x, uint32_t rows, const void* w_gate, const void* w_up,
                         const void* w_down, void* act, uint32_t rows_cap, cudaStream_t s) {
-    const PrefillArgs a = with_tile(args, false);
+    PrefillArgs a = with_tile(args, false);
+    a.tile_table = nullptr;
+    a.pairs = rows;
     CUtensorMap map_g, map_u, map_d;
     if (!make_map(&map_g, w_gate, a.I, a.H, kMTile) || !make_map(&map_u, w_up, a.I, a.H, kMTile) ||
         !make_map(&map_d, w_down, a.H, a.I, kMTile))
         return -1;
-    launch_tiles(a, s);
     const int rc = launch_gate_up_nt<kFmtBf16W>(a, Operands{x, nullptr, rows, &map_g, &map_u, nullptr, act, nullptr}, s);
     if (rc) return rc;
     return launch_down_nt<kFmtBf16W>(a, Operands{act, nullptr, rows_cap, &map_d, &map_d, nullptr, nullptr, nullptr}, s);
@@ -960,9 +966,9 @@ int launch_prefill_bf16(const PrefillArgs& args, const void* x, uint32_t rows, c
 // N tiles of the single-GEMM modes (one group holding all T rows), so the output lands as [T, E] fp32.
 // The summation order differs from the canonical lane-strided order: these logits feed the fast
 // router, which re-derives everything that reaches the caller in the canonical order.
-// offsets2 must hold {0, T}.  Needs E % 128 == 0 and H % 128 == 0.
-int launch_router_tc(const void* x, uint32_t T, const void* wg, uint32_t E, uint32_t H, float* logits,
-                     uint32_t* tile_table, const uint32_t* offsets2, uint32_t* status, cudaStream_t s) {
+// Needs E % 128 == 0 and H % 128 == 0.
+int launch_router_tc(const void* x, uint32_t T, const void* wg, uint32_t E, uint32_t H, float* logits, uint32_t* status,
+                     cudaStream_t s) {
     if (E % 128u || H % 128u || T == 0u) return -1;
     CUtensorMap map_w;
     if (!make_map(&map_w, wg, E, H, kMTile)) return -1;
@@ -972,13 +978,10 @@ int launch_router_tc(const void* x, uint32_t T, const void* wg, uint32_t E, uint
     a.I = H;     // their K
     a.n_groups = 1;
     a.pairs = T;
-    a.offsets = offsets2;
     a.y = logits;
-    a.tile_table = tile_table;
     a.status = status;
     a.glu = GluParams{STRATA_MOE_ACT_SWIGLU, 1.0f, 1.0f};
     a.ntile = 128u;   // more tiles than the 192-token geometry gives, and a tile is short (E features x H)
-    launch_tiles(a, s);
     // 256 experts per job while that still gives every other SM a job; with few tokens (a rank's share of an
     // expert-parallel step) 128 per job: twice the jobs, each half as long (2048 tokens: 16 jobs otherwise)
     const uint64_t jobs256 = (uint64_t)((T + 127u) / 128u) * (E / 256u);
