@@ -13,82 +13,87 @@
 namespace smoe {
 
 constexpr uint32_t kSegPairs = 128;   // pairs per warp segment
-constexpr uint32_t kSmallPairs = 2048; // single-CTA path up to this many pairs (above, the segmented path is faster: 35 vs ~22 us at 2560 pairs)
+constexpr uint32_t kSmallPairs = 8192; // single-CTA path up to this many pairs: eight rounds of 32 per warp
 
 // ---- small path: one CTA does everything ---------------------------------------------------
+// A warp owns a run of consecutive pairs and ranks them against its own earlier ones (a table of counts per warp and
+// expert), one thread per expert turns the warps' counts into bases, a shuffle scan over the experts gives the offsets: eight
+// block barriers whatever the number of pairs.  (Ranking the warps in turn, a barrier each, and scanning through shared
+// memory took 20 us for 1536 pairs of 256 experts; four kernels of the large path take 18 us with the gaps between them.)
 __global__ void __launch_bounds__(1024) group_small_kernel(
     const uint32_t* __restrict__ ids, uint32_t pairs, uint32_t ebeg, uint32_t nexp,
     uint32_t* __restrict__ counts, uint32_t* __restrict__ offsets, uint32_t* __restrict__ perm,
     uint32_t* __restrict__ inv, uint32_t* __restrict__ active_list, uint32_t* __restrict__ n_active) {
     extern __shared__ uint32_t sm[];
-    uint32_t* cnt = sm;             // [nexp]
-    uint32_t* cur = sm + nexp;      // [nexp] running cursor
-    uint32_t* scan = sm + 2 * nexp; // [1024] scratch
+    __shared__ uint32_t tot[32], act[32];
+    uint32_t* first = sm;                                                   // [nexp] first position of an expert
+    uint16_t* base = reinterpret_cast<uint16_t*>(sm + nexp);                // [32][nexp] counts, then bases, per warp
+    uint16_t* rank = base + 32u * nexp;                                     // [pairs] among the warp's pairs of the expert
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    for (uint32_t e = tid; e < nexp; e += blockDim.x) cnt[e] = 0;
+    const uint32_t rounds = (pairs + 1023u) / 1024u;                        // of 32 pairs per warp
+    for (uint32_t i = tid; i < 16u * nexp; i += 1024u) reinterpret_cast<uint32_t*>(base)[i] = 0u;
     __syncthreads();
-    for (uint32_t i = tid; i < pairs; i += blockDim.x) {
-        const uint32_t e = ids[i] - ebeg;
-        if (e < nexp) atomicAdd(&cnt[e], 1u);
-    }
-    __syncthreads();
-    // exclusive scan over experts (nexp <= 1024): one element per thread, Hillis-Steele
-    const uint32_t mine = tid < nexp ? cnt[tid] : 0u;
-    scan[tid] = mine;
-    __syncthreads();
-    for (uint32_t off = 1; off < 1024u; off <<= 1) {
-        const uint32_t v = tid >= off ? scan[tid - off] : 0u;
-        __syncthreads();
-        scan[tid] += v;
-        __syncthreads();
-    }
-    const uint32_t incl = scan[tid];
-    if (tid < nexp) {
-        counts[tid] = mine;
-        offsets[tid] = incl - mine;
-        cur[tid] = incl - mine;
-        if (tid == nexp - 1) offsets[nexp] = incl;
-    }
-    __syncthreads();
-    // active list (ascending): rank = number of non-empty experts before this one
-    scan[tid] = (tid < nexp && mine) ? 1u : 0u;
-    __syncthreads();
-    for (uint32_t off = 1; off < 1024u; off <<= 1) {
-        const uint32_t v = tid >= off ? scan[tid - off] : 0u;
-        __syncthreads();
-        scan[tid] += v;
-        __syncthreads();
-    }
-    if (active_list) {
-        if (tid < nexp && mine) active_list[scan[tid] - 1u] = tid;
-        if (tid == 1023u) *n_active = scan[1023];
-    }
-    __syncthreads();
-    // stable placement: warps take their 32 pairs in turn
-    const uint32_t nwarps = blockDim.x >> 5;
-    for (uint32_t base = 0; base < pairs; base += blockDim.x) {
-        const uint32_t i = base + tid;
+    uint16_t* mine_w = base + (size_t)warp * nexp;
+    for (uint32_t r = 0; r < rounds; ++r) {
+        const uint32_t i = (warp * rounds + r) * 32u + lane;
         const uint32_t e = i < pairs ? ids[i] - ebeg : 0xFFFFFFFFu;
         const bool ok = e < nexp;
-        for (uint32_t w = 0; w < nwarps; ++w) {
-            if (warp == w && base + w * 32u < pairs) {
-                const uint32_t key = ok ? e : 0xFFFFFFFFu;
-                const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
-                if (ok) {
-                    const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-                    const uint32_t pos = cur[e] + rank;
-                    perm[pos] = i;
-                    if (inv) inv[i] = pos;
-                }
-                __syncwarp();
-                if (ok && lane == (uint32_t)(__ffs(peers) - 1)) cur[e] += __popc(peers);
-            }
-            __syncthreads();
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, ok ? e : 0xFFFFFFFFu);
+        const uint32_t before = ok ? mine_w[e] : 0u;
+        __syncwarp();
+        if (ok) {
+            rank[i] = (uint16_t)(before + __popc(peers & ((1u << lane) - 1u)));
+            if (lane == (uint32_t)(__ffs(peers) - 1)) mine_w[e] = (uint16_t)(before + __popc(peers));
         }
+        __syncwarp();
     }
-    for (uint32_t i = tid; i < pairs; i += blockDim.x) {
+    __syncthreads();
+    uint32_t mine = 0;      // pairs of expert tid (nexp <= 1024)
+    if (tid < nexp)
+        for (uint32_t w = 0; w < 32u; ++w) {
+            const uint32_t v = base[w * nexp + tid];
+            base[w * nexp + tid] = (uint16_t)mine;
+            mine += v;
+        }
+    uint32_t incl = mine, incl_a = mine ? 1u : 0u;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, off), va = __shfl_up_sync(0xFFFFFFFFu, incl_a, off);
+        if ((int)lane >= off) { incl += v; incl_a += va; }
+    }
+    if (lane == 31u) { tot[warp] = incl; act[warp] = incl_a; }
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t t = tot[lane], ta = act[lane];
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, t, off), va = __shfl_up_sync(0xFFFFFFFFu, ta, off);
+            if ((int)lane >= off) { t += v; ta += va; }
+        }
+        tot[lane] = t;
+        act[lane] = ta;
+    }
+    __syncthreads();
+    if (warp) { incl += tot[warp - 1u]; incl_a += act[warp - 1u]; }
+    if (tid < nexp) {
+        counts[tid] = mine;
+        offsets[tid] = first[tid] = incl - mine;
+        if (tid == nexp - 1u) offsets[nexp] = incl;
+        if (active_list && mine) active_list[incl_a - 1u] = tid;
+    }
+    if (active_list && tid == 1023u) *n_active = incl_a;
+    __syncthreads();
+    for (uint32_t r = 0; r < rounds; ++r) {
+        const uint32_t i = (warp * rounds + r) * 32u + lane;
+        if (i >= pairs) break;
         const uint32_t e = ids[i] - ebeg;
-        if (!(e < nexp) && inv) inv[i] = 0xFFFFFFFFu;
+        if (e < nexp) {
+            const uint32_t pos = first[e] + mine_w[e] + rank[i];
+            perm[pos] = i;
+            if (inv) inv[i] = pos;
+        } else if (inv) {
+            inv[i] = 0xFFFFFFFFu;
+        }
     }
 }
 
@@ -211,7 +216,14 @@ void launch_group(const uint32_t* ids, uint32_t pairs, uint32_t expert_begin, ui
                   uint32_t* counts, uint32_t* offsets, uint32_t* perm, uint32_t* inv,
                   uint32_t* active_list, uint32_t* n_active, void* scratch, cudaStream_t s) {
     if (pairs <= kSmallPairs) {
-        const size_t smem = (2u * (size_t)n_experts + 1024u) * sizeof(uint32_t);
+        static bool attr[64] = {};   // the shared-memory opt-in is per device
+        const size_t smem = (size_t)n_experts * (4u + 64u) + (size_t)pairs * 2u;
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev >= 0 && dev < 64 && !attr[dev]) {
+            cudaFuncSetAttribute(group_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 * 68 + (int)kSmallPairs * 2);
+            attr[dev] = true;
+        }
         group_small_kernel<<<1, 1024, smem, s>>>(ids, pairs, expert_begin, n_experts, counts, offsets,
                                                 perm, inv, active_list, n_active);
         ++g_kernel_launches;
