@@ -928,14 +928,19 @@ int run_shared(strata_moe_layer* L, const __nv_bfloat16* x, const __nv_bfloat16*
     if (!st) st = ctx->stream;
     // enough rows to fill tensor-core tiles (and BF16 inputs): grouped-GEMM path with one group
     const uint32_t thr = L->knobs.prefill_min_rows >= 0 ? (uint32_t)L->knobs.prefill_min_rows : 24u;
-    if (!x_lo && T >= thr && tensor_path_ok(L, 3, L->d.shared_intermediate)) {
+    // A wide shared expert also for fewer rows, the activation as a BF16 hi + lo pair like that of the streaming kernel: its
+    // tiles stream the weights as fast on a third of the SMs and leave the others to the routed path's small kernels beside it
+    // (Kimi's 6144 columns, 48 tiles; the streaming kernel took every SM and the router beside it 61 us instead of 13).
+    const bool wide = L->d.shared_intermediate >= 40u * 128u && L->knobs.prefill_min_rows < 0;
+    if (!x_lo && (T >= thr || wide) && tensor_path_ok(L, 3, L->d.shared_intermediate)) {
         PrefillArgs p{};
         p.fmt = 3;
         p.H = L->d.hidden;
         p.I = L->d.shared_intermediate;
         p.n_groups = 1;
         p.pairs = T;
-        p.ntile = prefill_ntile(L, T, 1, T);
+        p.ntile = T >= thr ? prefill_ntile(L, T, 1, T) : (T <= 16u ? 16u : 32u);
+        p.act_lo = T >= thr ? nullptr : L->sh_act_lo;
         p.y = L->sh_y;
         p.status = ctx->d_status;
         p.glu = GluParams{L->d.activation, L->d.gate_beta, L->d.linear_beta};

@@ -946,10 +946,10 @@ int launch_prefill(const PrefillArgs& args, const void* x16, const float* x_rows
 }
 
 // BF16 expert (the shared expert) over `rows` token rows in natural order: x [rows, H] BF16,
-// gate/up [I, H], down [H, I] BF16, act [rows_cap, I] BF16 scratch, y [rows, H] fp32.
+// gate/up [I, H], down [H, I] BF16, act (and args.act_lo: a hi + lo pair) [rows_cap, I] BF16 scratch, y [rows, H] fp32.
 int launch_prefill_bf16(const PrefillArgs& args, const void* x, uint32_t rows, const void* w_gate, const void* w_up,
                         const void* w_down, void* act, uint32_t rows_cap, cudaStream_t s) {
-    PrefillArgs a = with_tile(args, false);
+    PrefillArgs a = with_tile(args, args.act_lo != nullptr);
     a.tile_table = nullptr;
     a.pairs = rows;
     CUtensorMap map_g, map_u, map_d;
@@ -958,7 +958,7 @@ int launch_prefill_bf16(const PrefillArgs& args, const void* x, uint32_t rows, c
         return -1;
     const int rc = launch_gate_up_nt<kFmtBf16W>(a, Operands{x, nullptr, rows, &map_g, &map_u, nullptr, act, nullptr}, s);
     if (rc) return rc;
-    return launch_down_nt<kFmtBf16W>(a, Operands{act, nullptr, rows_cap, &map_d, &map_d, nullptr, nullptr, nullptr}, s);
+    return launch_down_nt<kFmtBf16W>(a, Operands{act, a.act_lo, rows_cap, &map_d, &map_d, nullptr, nullptr, nullptr}, s);
 }
 
 // Router projection on the tensor cores: logits[t, e] = sum_h x[t, h] * wg[e, h] for BF16 operands,
