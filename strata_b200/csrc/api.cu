@@ -684,7 +684,7 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
                 const uint32_t* n_active, uint32_t max_rows, float* y, uint32_t expected_pairs = 0,
                 const uint32_t* pairs_dev = nullptr, bool x_ready = false, bool* y_half = nullptr,
                 float* y_rowscale_out = nullptr, const SpreadRows* spread = nullptr, bool one_row_per_token = false,
-                const ColumnBlocks* columns = nullptr) {
+                const ColumnBlocks* columns = nullptr, bool x_settled = false) {
     // `pairs` bounds the row count.  When the exact count exists only on the device (rows received
     // from other ranks) pairs_dev points at it and expected_pairs steers the host-side heuristics.
     Range range("strata_moe.experts");
@@ -782,8 +782,8 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         // rows; the activation's have a workspace, their scales go to act_hi.
         const int fmt = L->d.format;
         const uint32_t H = L->d.hidden, I = L->d.intermediate;
-        if (perm) launch_rows_to_planes(fmt, x_src, false, spread->rows, spread->rows_dev, H, spread->dest, spread->k, bound, L->y, L->xg, L->x_rowscale, s);
-        else launch_rows_to_planes(fmt, x_src, false, bound, pairs_dev, H, nullptr, 1, bound, L->y, L->xg, L->x_rowscale, s);
+        if (perm) launch_rows_to_planes(fmt, x_src, false, spread->rows, spread->rows_dev, H, spread->dest, spread->k, bound, L->y, L->xg, L->x_rowscale, x_settled, s);
+        else launch_rows_to_planes(fmt, x_src, false, bound, pairs_dev, H, nullptr, 1, bound, L->y, L->xg, L->x_rowscale, false, s);
         PlaneArgs p{};
         p.H = H;
         p.I = I;
@@ -815,7 +815,7 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         if (launch_planes_gate_up(fmt, p, L->d_wmaps, L->d_sfmaps, s) != 0)
             return fail(ctx, STRATA_MOE_E_CUDA, "gate/up plane launch failed");
         mark(ctx, 5);
-        launch_rows_to_planes(fmt, L->act_f32, true, bound, pairs_dev, I, nullptr, 1, bound, L->act_planes, L->act_hi, L->act_rowscale, s);
+        launch_rows_to_planes(fmt, L->act_f32, true, bound, pairs_dev, I, nullptr, 1, bound, L->act_planes, L->act_hi, L->act_rowscale, false, s);
         p.planes = L->act_planes;
         p.x_scales = reinterpret_cast<const uint8_t*>(L->act_hi);
         p.rowscale = nv ? L->act_rowscale : nullptr;
@@ -1638,7 +1638,7 @@ static int forward_layer(strata_moe_layer* L, const void* x, uint32_t T, float* 
     }};
     rc = run_experts(L, xb, perm, d.top_k, P, d.experts, offsets, L->active, L->n_active, T, L->y, 0, nullptr, x_ready,
                      &y_half, nullptr, d.top_k <= 32u ? &spread : nullptr, true,
-                     column_blocks > 1u ? &columns : nullptr);
+                     column_blocks > 1u ? &columns : nullptr, front_done);
     if (rc) return rc;
     if (column_blocks > 1u) {
         ctx->stats.forward_calls++;

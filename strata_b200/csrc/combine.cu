@@ -14,13 +14,11 @@ namespace smoe {
 // Y_HALF: the expert rows are f16 (the tensor-core down kernel can store them so: half the bytes of the pass that
 // bounds this kernel); they widen exactly and the arithmetic below is unchanged.
 template <bool Y_HALF>
-__global__ void __launch_bounds__(256) combine_kernel(const void* __restrict__ y_v,
-                                                      const uint32_t* __restrict__ inv,
-                                                      const float* __restrict__ weights,
-                                                      const float* __restrict__ shared, uint32_t T,
-                                                      uint32_t k, uint32_t H, float output_scale,
-                                                      float* __restrict__ out, uint32_t* status, uint32_t col0,
+__global__ void __launch_bounds__(256) combine_kernel(const void* y_v, const uint32_t* inv, const float* weights,
+                                                      const float* shared, uint32_t T, uint32_t k, uint32_t H,
+                                                      float output_scale, float* out, uint32_t* status, uint32_t col0,
                                                       uint32_t cols) {
+    pdl_wait();
     constexpr uint32_t V = Y_HALF ? 8u : 4u;     // columns per thread: one 16-byte load of an expert row either way
     const uint32_t per_row = cols / V;
     bool bad = false;
@@ -47,9 +45,9 @@ __global__ void __launch_bounds__(256) combine_kernel(const void* __restrict__ y
                 raw[q] = make_uint4(0, 0, 0, 0);
                 if (pos[q] != 0xFFFFFFFFu) {
                     if (Y_HALF)
-                        raw[q] = __ldg(reinterpret_cast<const uint4*>(static_cast<const __half*>(y_v) + (size_t)pos[q] * H + c));
+                        raw[q] = *reinterpret_cast<const uint4*>(static_cast<const __half*>(y_v) + (size_t)pos[q] * H + c);
                     else
-                        raw[q] = __ldg(reinterpret_cast<const uint4*>(static_cast<const float*>(y_v) + (size_t)pos[q] * H + c));
+                        raw[q] = *reinterpret_cast<const uint4*>(static_cast<const float*>(y_v) + (size_t)pos[q] * H + c);
                 }
             }
 #pragma unroll
@@ -79,7 +77,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const void* __restrict__ y
         if (shared) {
 #pragma unroll
             for (uint32_t q4 = 0; q4 < V / 4u; ++q4) {
-                const float4 s = __ldg(reinterpret_cast<const float4*>(shared + (size_t)t * H + c) + q4);
+                const float4 s = reinterpret_cast<const float4*>(shared + (size_t)t * H + c)[q4];
                 o[4 * q4] = __fadd_rn(o[4 * q4], s.x);
                 o[4 * q4 + 1] = __fadd_rn(o[4 * q4 + 1], s.y);
                 o[4 * q4 + 2] = __fadd_rn(o[4 * q4 + 2], s.z);
@@ -103,9 +101,9 @@ void launch_combine(const void* y, const uint32_t* inv, const float* weights, co
     const size_t n = (size_t)T * (cols / (y_half ? 8u : 4u));
     const uint32_t grid = (uint32_t)((n + 255) / 256 < 148u * 8u ? (n + 255) / 256 : 148u * 8u);
     if (y_half)
-        combine_kernel<true><<<grid, 256, 0, s>>>(y, inv, weights, shared, T, k, H, output_scale, out, status, col0, cols);
+        launch_behind(combine_kernel<true>, grid, 256, 0, s, y, inv, weights, shared, T, k, H, output_scale, out, status, col0, cols);
     else
-        combine_kernel<false><<<grid, 256, 0, s>>>(y, inv, weights, shared, T, k, H, output_scale, out, status, col0, cols);
+        launch_behind(combine_kernel<false>, grid, 256, 0, s, y, inv, weights, shared, T, k, H, output_scale, out, status, col0, cols);
     ++g_kernel_launches;
 }
 

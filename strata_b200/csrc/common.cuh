@@ -48,6 +48,28 @@ struct WeightTable {
     const float* post_scale;       // [n_local] f16 path: factor applied to the fp32 accumulator
 };
 
+// Kernels launched behind their predecessor in the stream (programmatic dependent launch): the grid may become resident while
+// the predecessor still runs, and pdl_wait() returns when that has completed and its writes are visible.  Before it a kernel
+// touches nothing that the predecessor writes or reads; what it reads afterwards is loaded by ordinary loads (not __ldg or
+// const __restrict__, which promise data that does not change while the kernel exists).  Every kernel of such a chain waits,
+// also one that needs nothing from its predecessor: its own successor relies on it.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---- launch wrappers (definitions in the .cu files) ---------------------------------
 // router.cu
 void launch_router_logits(const __nv_bfloat16* x, const __nv_bfloat16* wg, uint32_t T, uint32_t H,
@@ -194,10 +216,11 @@ struct PlaneArgs {
 bool planes_supported(int fmt, uint32_t H, uint32_t I);
 int planes_encode_scale_map(void* out128, int fmt, const void* scales, uint32_t rows, uint32_t K);
 // rows of `cols` BF16 (or FP32) values -> planes (cols * 4 bytes per plane row), scales (cols / 32 or cols / 16), rowscale (NVFP4);
-// source row r goes to plane rows dest[r * k .. r * k + k - 1], or to plane row r.
+// source row r goes to plane rows dest[r * k .. r * k + k - 1], or to plane row r.  settled: src was written before the kernel that
+// precedes this one in the stream started.
 void launch_rows_to_planes(int fmt, const void* src, bool f32, uint32_t rows, const uint32_t* rows_dev, uint32_t cols,
                            const uint32_t* dest, uint32_t k, uint32_t plane_rows, void* planes, void* scales, float* rowscale,
-                           cudaStream_t s);
+                           bool settled, cudaStream_t s);
 int launch_planes_gate_up(int fmt, const PlaneArgs& a, const void* wmaps, const void* smaps, cudaStream_t s);
 int launch_planes_down(int fmt, const PlaneArgs& a, const void* wmaps, const void* smaps, cudaStream_t s);
 // Router projection on the tensor cores (approximate summation order; see router.cu for its use).

@@ -163,9 +163,8 @@ fp4_planes_kernel(PlaneArgs a, const CUtensorMap* __restrict__ wmaps, const CUte
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t K = GU ? a.H : a.I, rows_out = GU ? a.I : a.H;
     const uint32_t m_tiles = rows_out / kFeat, k_stages = K / kStageK, sf_blocks = k_stages / kPerSf;
-    const uint32_t total = (a.tile_table ? a.tile_table[0] : *a.n_active) * m_tiles;
     volatile uint32_t* abort_flag = &S.abort_flag;
-    if (blockIdx.x >= total) return;
+    pdl_launch_dependents();
 
     if (threadIdx.x == 0) {
         for (uint32_t i = 0; i < G::kStages; ++i) {
@@ -194,6 +193,8 @@ fp4_planes_kernel(PlaneArgs a, const CUtensorMap* __restrict__ wmaps, const CUte
     __syncthreads();
     tc_fence_after();
     const uint32_t tm = S.tmem_base;
+    pdl_wait();      // what the roles read comes from the kernels before
+    const uint32_t total = (a.tile_table ? a.tile_table[0] : *a.n_active) * m_tiles;
 
     bool ok = true;
     if (warp == 0) {
@@ -429,9 +430,11 @@ __device__ __forceinline__ void digit_words(const float x[8], float f1, uint32_t
 template <int FMT, bool F32>
 __global__ void __launch_bounds__(1024) planes_kernel(const void* src, const uint32_t* rows_dev, uint32_t cols, const uint32_t* dest,
                                                       uint32_t k, uint32_t plane_rows, uint8_t* planes, uint8_t* scales,
-                                                      float* rowscale) {
+                                                      float* rowscale, bool settled) {
     __shared__ uint32_t warp_max[32];
     const uint32_t row = blockIdx.x, tid = threadIdx.x, lane = tid & 31u;
+    pdl_launch_dependents();
+    if (!settled) pdl_wait();
     if (rows_dev && row >= *rows_dev) return;
     float x[8];
     if (F32) {
@@ -477,6 +480,7 @@ __global__ void __launch_bounds__(1024) planes_kernel(const void* src, const uin
     }
     uint32_t w[kPlanes];
     digit_words(x, f1, w);
+    if (settled) pdl_wait();     // the digits were made beside the preceding kernel; where they go it decides
     const uint32_t slab = tid >> 5, chunk = lane >> 2, word = lane & 3u, sc = tid / kPerScale;
     for (uint32_t j = blockIdx.y; j < (dest ? k : 1u); j += gridDim.y) {
         const uint32_t pos = dest ? dest[(size_t)row * k + j] : row;
@@ -501,10 +505,10 @@ int launch_planes_one(const PlaneArgs& a, const void* wmaps, const void* smaps, 
             return -2;
         done[dev] = true;
     }
-    fp4_planes_kernel<FMT, GU, R><<<kNumSMs, kPThreads, smem, s>>>(a, static_cast<const CUtensorMap*>(wmaps),
-                                                                   static_cast<const CUtensorMap*>(smaps));
+    const cudaError_t e = launch_behind(fp4_planes_kernel<FMT, GU, R>, kNumSMs, kPThreads, smem, s, a,
+                                        static_cast<const CUtensorMap*>(wmaps), static_cast<const CUtensorMap*>(smaps));
     ++g_kernel_launches;
-    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+    return e == cudaSuccess ? 0 : -3;
 }
 template <int FMT, bool GU>
 int launch_planes_rows(const PlaneArgs& a, const void* wmaps, const void* smaps, cudaStream_t s) {
@@ -515,12 +519,12 @@ int launch_planes_rows(const PlaneArgs& a, const void* wmaps, const void* smaps,
 
 template <int FMT>
 void launch_planes_fmt(const void* src, bool f32, uint32_t rows, const uint32_t* rows_dev, uint32_t cols, const uint32_t* dest,
-                       uint32_t k, uint32_t plane_rows, void* planes, void* scales, float* rowscale, cudaStream_t s) {
+                       uint32_t k, uint32_t plane_rows, void* planes, void* scales, float* rowscale, bool settled, cudaStream_t s) {
     uint8_t *p = static_cast<uint8_t*>(planes), *sc = static_cast<uint8_t*>(scales);
     // the digits of a row are quickly made again: with few rows the copies of a row go to CTAs of their own
     const dim3 grid(rows, dest && rows * k <= 2u * (uint32_t)kNumSMs ? k : 1u);
-    if (f32) planes_kernel<FMT, true><<<grid, cols / 8u, 0, s>>>(src, rows_dev, cols, dest, k, plane_rows, p, sc, rowscale);
-    else planes_kernel<FMT, false><<<grid, cols / 8u, 0, s>>>(src, rows_dev, cols, dest, k, plane_rows, p, sc, rowscale);
+    if (f32) launch_behind(planes_kernel<FMT, true>, grid, cols / 8u, 0, s, src, rows_dev, cols, dest, k, plane_rows, p, sc, rowscale, settled);
+    else launch_behind(planes_kernel<FMT, false>, grid, cols / 8u, 0, s, src, rows_dev, cols, dest, k, plane_rows, p, sc, rowscale, settled);
 }
 
 }  // namespace
@@ -549,12 +553,12 @@ int planes_encode_scale_map(void* out128, int fmt, const void* scales, uint32_t 
 
 void launch_rows_to_planes(int fmt, const void* src, bool f32, uint32_t rows, const uint32_t* rows_dev, uint32_t cols,
                            const uint32_t* dest, uint32_t k, uint32_t plane_rows, void* planes, void* scales, float* rowscale,
-                           cudaStream_t s) {
+                           bool settled, cudaStream_t s) {
     if (rows == 0u) return;
     if (fmt == STRATA_MOE_FMT_MXFP4)
-        launch_planes_fmt<STRATA_MOE_FMT_MXFP4>(src, f32, rows, rows_dev, cols, dest, k, plane_rows, planes, scales, rowscale, s);
+        launch_planes_fmt<STRATA_MOE_FMT_MXFP4>(src, f32, rows, rows_dev, cols, dest, k, plane_rows, planes, scales, rowscale, settled, s);
     else
-        launch_planes_fmt<STRATA_MOE_FMT_NVFP4>(src, f32, rows, rows_dev, cols, dest, k, plane_rows, planes, scales, rowscale, s);
+        launch_planes_fmt<STRATA_MOE_FMT_NVFP4>(src, f32, rows, rows_dev, cols, dest, k, plane_rows, planes, scales, rowscale, settled, s);
     ++g_kernel_launches;
 }
 

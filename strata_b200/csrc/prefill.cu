@@ -717,9 +717,11 @@ prefill_ffn_kernel(const __grid_constant__ BMaps maps_b, const __grid_constant__
 
 // ------------------------------------------------------------------------------ tile list
 // table[0] = number of n-tiles, then (expert, first row, rows) per n-tile, experts ascending.
-__global__ void __launch_bounds__(1024) prefill_tiles_kernel(const uint32_t* __restrict__ offsets, uint32_t n_groups,
-                                                             uint32_t* __restrict__ table, uint32_t kNTile) {
+__global__ void __launch_bounds__(1024) prefill_tiles_kernel(const uint32_t* offsets, uint32_t n_groups, uint32_t* table,
+                                                             uint32_t kNTile) {
     __shared__ uint32_t scan[1024];
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t tid = threadIdx.x;
     uint32_t cnt = 0, r0 = 0;
     if (tid < n_groups) {
@@ -853,7 +855,7 @@ static int launch_one(const PrefillArgs& a, const void* b_hi, const void* b_lo, 
 }
 
 void launch_tile_list(const uint32_t* offsets, uint32_t n_groups, uint32_t* table, uint32_t rows, cudaStream_t s) {
-    prefill_tiles_kernel<<<1, 1024, 0, s>>>(offsets, n_groups, table, rows);
+    launch_behind(prefill_tiles_kernel, 1, 1024, 0, s, offsets, n_groups, table, rows);
     ++g_kernel_launches;
 }
 static void launch_tiles(const PrefillArgs& a, cudaStream_t s) { launch_tile_list(a.offsets, a.n_groups, a.tile_table, a.ntile, s); }

@@ -1037,6 +1037,7 @@ __global__ void __launch_bounds__(kFrontWarps * 32) front_small_kernel(
     uint32_t* __restrict__ active_list, uint32_t* __restrict__ n_active, const __nv_bfloat16* __restrict__ x, uint32_t H,
     __half* __restrict__ xg, float* __restrict__ x_rowscale, bool int4_order, uint32_t* status) {
     extern __shared__ float fsm2[];
+    pdl_launch_dependents();
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t E = p.experts, k = p.top_k, P = T * k;
     const bool first = blockIdx.x == 0u;
