@@ -369,7 +369,7 @@ struct LaneBest {
 // Scores, top-k and routing weights of ONE token by one warp.  score / choice: [E] floats of shared memory each.
 // Scores and selection values of the experts first, first + step, ... of one token (every rule but softmax, whose
 // normaliser needs the whole row).  Returns true when a logit or bias is not finite.
-__device__ __forceinline__ bool route_scores_part(const RouterParams& p, const float* __restrict__ lg,
+__device__ __forceinline__ bool route_scores_part(const RouterParams& p, const float* lg,
                                                   const float* __restrict__ bias, float* score, float* choice,
                                                   uint32_t first, uint32_t step) {
     bool bad = false;
@@ -392,7 +392,7 @@ __device__ __forceinline__ bool route_scores_part(const RouterParams& p, const f
 
 // scores_ready: score / choice were filled by route_scores_part (bad_in = its verdict); else they are computed here.
 // ids_local: a second home of the ids; store = false leaves ids and weights alone.
-__device__ __forceinline__ void route_token(const RouterParams& p, const float* __restrict__ logits,
+__device__ __forceinline__ void route_token(const RouterParams& p, const float* logits,
                                             const float* __restrict__ bias, uint32_t tok, float* score, float* choice,
                                             uint32_t* __restrict__ ids, float* __restrict__ weights, uint32_t* status,
                                             const uint32_t* __restrict__ forced_ids, bool scores_ready = false,
@@ -937,16 +937,100 @@ __global__ void __launch_bounds__(kSmallMaxTokens * 32) router_logits_small_kern
                 if (ring::mbar_test(&bars[q], 0u)) break;
 }
 
+// The fewest tokens: two expert rows per CTA, so that their fetch and their arithmetic spread over the GPU (eight rows per CTA
+// are 32 CTAs of 256 experts, each with one warp per token and a chain of 26 instructions per 32 columns: 13 us for one token
+// of 4096 columns, most of it that chain).  The token rows come whole into shared memory beside the expert rows, in column
+// quarters of one mbarrier each; a warp computes one token, its halves one expert row each, a lane two of the 32 chains (columns
+// 2 l and 2 l + 1 of every 32): the canonical order, and its fold by shuffles of 8, 4, 2 and 1 lanes and a last addition
+// within the lane.
+constexpr uint32_t kPairRows = 2;
+constexpr uint32_t kPairSmem = 100u * 1024u;     // two CTAs per SM
+
+__global__ void __launch_bounds__(kSmallMaxTokens * 32) router_logits_pair_kernel(
+    const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wg, uint32_t T, uint32_t H, uint32_t E,
+    float* __restrict__ logits, uint32_t* status) {
+    extern __shared__ __align__(128) uint8_t small_smem[];
+    uint64_t* bars = reinterpret_cast<uint64_t*>(small_smem);     // [4]
+    uint8_t* rows = small_smem + 128;                             // two expert rows, then the token rows
+    const uint32_t pitch = H * 2u + kSmallPad;                    // the two rows' 64-byte pieces lie in different banks
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t e0 = blockIdx.x * kPairRows, nrows = min(kPairRows, E - e0);
+    const uint32_t steps = H / 32u;                               // 64-byte steps of a row
+    __shared__ uint32_t abort_flag;
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < 4; ++q) ring::mbar_init(&bars[q], 1);
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    pdl_launch_dependents();
+    if (warp == 0) {
+        if (lane == 0)
+            for (uint32_t q = 0; q < 4u; ++q)
+                ring::mbar_arrive_expect_tx(&bars[q], (nrows + T) * (steps * (q + 1u) / 4u - steps * q / 4u) * 64u);
+        __syncwarp();
+        if (lane < nrows + T)
+            for (uint32_t q = 0; q < 4u; ++q) {
+                const uint32_t j0 = steps * q / 4u, j1 = steps * (q + 1u) / 4u;
+                const __nv_bfloat16* src = lane < nrows ? wg + (size_t)(e0 + lane) * H : x + (size_t)(lane - nrows) * H;
+                uint8_t* dst = rows + (size_t)(lane < nrows ? lane : lane - nrows + kPairRows) * pitch;
+                if (j1 > j0)
+                    ring::bulk_g2s(dst + j0 * 64u, reinterpret_cast<const uint8_t*>(src) + j0 * 64u, (j1 - j0) * 64u, &bars[q]);
+            }
+    }
+    const uint32_t half = lane >> 4, row = min(half, nrows - 1u);
+    const uint32_t wat = ring::smem_addr(rows + (size_t)row * pitch) + (lane & 15u) * 4u;
+    const uint32_t xat = ring::smem_addr(rows + (size_t)(kPairRows + warp) * pitch) + (lane & 15u) * 4u;
+    float c0 = 0.0f, c1 = 0.0f;
+    bool ok = true;
+    for (uint32_t q = 0; q < 4u && ok; ++q) {
+        ok = __all_sync(0xFFFFFFFFu, ring::mbar_wait_poll(&bars[q], 0u, &abort_flag));
+        if (!ok) break;
+        const uint32_t j1 = steps * (q + 1u) / 4u;
+#pragma unroll 16
+        for (uint32_t j = steps * q / 4u; j < j1; ++j) {
+            const uint32_t w = ring::lds32(wat + j * 64u), v = ring::lds32(xat + j * 64u);
+            c0 = __fmaf_rn(__uint_as_float(v << 16), __uint_as_float(w << 16), c0);
+            c1 = __fmaf_rn(__uint_as_float(v & 0xFFFF0000u), __uint_as_float(w & 0xFFFF0000u), c1);
+        }
+    }
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) {
+        c0 = __fadd_rn(c0, __shfl_down_sync(0xFFFFFFFFu, c0, off, 16));
+        c1 = __fadd_rn(c1, __shfl_down_sync(0xFFFFFFFFu, c1, off, 16));
+    }
+    if (ok && (lane & 15u) == 0u && half < nrows) logits[(size_t)warp * E + e0 + half] = __fadd_rn(c0, c1);
+    if (!ok && lane == 0) { abort_flag = 1; atomicOr(status, kStatusWaitTimeout); }
+    // the copies target this CTA's shared memory: none may be in flight when the CTA retires
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (uint32_t q = 0; q < 4u; ++q)
+            for (uint32_t spin = 0; spin < (1u << 16); ++spin)
+                if (ring::mbar_test(&bars[q], 0u)) break;
+}
+
 bool launch_router_logits_small(const __nv_bfloat16* x, const __nv_bfloat16* wg, uint32_t T, uint32_t H, uint32_t E,
                                 float* logits, uint32_t* status, cudaStream_t s) {
     if (T == 0 || H % 128u || status == nullptr) return false;
     if ((((uintptr_t)x | (uintptr_t)wg) & 15u) != 0) return false;
     const size_t smem = 128u + (size_t)kSmallRows * (H * 2u + kSmallPad) + (size_t)kSmallMaxTokens * 64u * 16u;
-    if (smem > 200u * 1024u) return false;
     static bool attr[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return false;
+    const size_t smem_pair = 128u + (size_t)(kPairRows + T) * (H * 2u + kSmallPad);
+    if (T <= kSmallMaxTokens && smem_pair <= kPairSmem) {
+        static bool pair_attr[64] = {};
+        if (!pair_attr[dev]) {
+            if (cudaFuncSetAttribute(router_logits_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem) != cudaSuccess)
+                return false;
+            pair_attr[dev] = true;
+        }
+        router_logits_pair_kernel<<<(E + kPairRows - 1u) / kPairRows, T * 32u, smem_pair, s>>>(x, wg, T, H, E, logits, status);
+        ++g_kernel_launches;
+        return true;
+    }
+    if (smem > 200u * 1024u) return false;
     if (!attr[dev]) {
         if (cudaFuncSetAttribute(router_logits_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) !=
             cudaSuccess)
@@ -1031,7 +1115,7 @@ void launch_route_fast(const RouterParams& p, float* logits, const float* bias, 
 constexpr uint32_t kFrontWarps = 16, kFrontMaxPairs = 512, kFrontMaxExperts = 1024;
 
 __global__ void __launch_bounds__(kFrontWarps * 32) front_small_kernel(
-    RouterParams p, const float* __restrict__ logits, const float* __restrict__ bias, uint32_t T,
+    RouterParams p, const float* logits, const float* __restrict__ bias, uint32_t T,
     uint32_t* __restrict__ ids, float* __restrict__ weights, uint32_t* __restrict__ counts,
     uint32_t* __restrict__ offsets, uint32_t* __restrict__ perm, uint32_t* __restrict__ inv,
     uint32_t* __restrict__ active_list, uint32_t* __restrict__ n_active, const __nv_bfloat16* __restrict__ x, uint32_t H,
@@ -1048,6 +1132,7 @@ __global__ void __launch_bounds__(kFrontWarps * 32) front_small_kernel(
     __shared__ uint32_t wtot[kFrontWarps], wact[kFrontWarps], bad_s[kFrontWarps];
     for (uint32_t e = tid; e < E; e += blockDim.x) cnt[e] = 0;
     if (tid < kFrontWarps) bad_s[tid] = 0;
+    pdl_wait();      // the logits
     // scores: the exact exp / log1p replicas are the long part of routing a token, so all 16 warps share them
     // (16 / T warps per token, each a strided subset of the experts); the softmax rule keeps one warp per token
     const bool coop = p.score_kind != STRATA_MOE_SCORE_SOFTMAX;
@@ -1137,9 +1222,8 @@ bool launch_front_small(const RouterParams& p, const float* logits, const float*
         attr[dev] = true;
     }
     const uint32_t grid = xg == nullptr ? 1u : (T * p.top_k + 3u) / 4u;   // four rows per CTA
-    front_small_kernel<<<grid, kFrontWarps * 32, smem, s>>>(p, logits, bias, T, ids, weights, counts, offsets, perm, inv,
-                                                         active_list, n_active, x, H, static_cast<__half*>(xg),
-                                                         x_rowscale, int4_order, status);
+    launch_behind(front_small_kernel, grid, kFrontWarps * 32, smem, s, p, logits, bias, T, ids, weights, counts, offsets, perm, inv,
+                  active_list, n_active, x, H, static_cast<__half*>(xg), x_rowscale, int4_order, status);
     ++g_kernel_launches;
     return true;
 }
