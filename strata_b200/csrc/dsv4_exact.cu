@@ -167,6 +167,7 @@ struct Dsv4Args {
 
 constexpr uint32_t kDsv4Warps = 4, kDsv4Ctas = 3;   // warps per CTA, CTAs per SM (170 registers a thread: no spills)
 constexpr uint32_t kDsv4MaxGroups = 1024;
+constexpr uint32_t kDsv4Ahead = 8;      // steps of 256 columns that the weight copies run ahead
 
 // One warp, RW weight rows (DUAL: RW / 2 gate rows and the same up rows), NTOK token rows at `pos0` (only `cnt` of them
 // exist; the others repeat the last one and are dropped).
@@ -179,7 +180,7 @@ constexpr uint32_t kDsv4MaxGroups = 1024;
 // takes the reference's two steps otherwise.
 template <bool DUAL, bool FP8, int RW, int NTOK>
 __device__ __forceinline__ void dsv4_rows(const Dsv4Args& a, uint32_t g, uint32_t row, size_t pos0, uint32_t cnt,
-                                          bool two_step, uint32_t lane, bool& bad) {
+                                          bool two_step, uint32_t lane, uint32_t* ring, bool& bad) {
     const uint32_t K = a.K;
     constexpr int HALF = DUAL ? RW / 2 : RW;
     const uint8_t *p[RW], *s[RW];
@@ -200,23 +201,32 @@ __device__ __forceinline__ void dsv4_rows(const Dsv4Args& a, uint32_t g, uint32_
         for (int k = 0; k < NTOK; ++k)
 #pragma unroll
             for (int q = 0; q < 8; ++q) acc[r][k][q] = 0.0f;
-    // weights and scales of the next 256 columns are requested before the current ones are used
-    uint2 wq[RW];
+    // Weights come through a ring in shared memory, kDsv4Ahead steps of 256 columns ahead, by asynchronous copies: every lane
+    // fetches and reads its own words, so a wait for its copies is all the synchronisation.  A warp's four rows are 512 bytes a
+    // step; with one step ahead, in registers, an SM had 6 KB in flight and streamed 1.5 TB/s over the GPU (three steps more
+    // in registers spilled and were slower).  A row's scales share one cache line: one step ahead in registers.
+    constexpr uint32_t kWords = FP8 ? 2u : 1u;
     uint32_t sq[RW];
-    auto load = [&](uint32_t c) {
+    auto fetch = [&](uint32_t slot, uint32_t c) {
 #pragma unroll
         for (int r = 0; r < RW; ++r) {
-            if (FP8) {
-                wq[r] = __ldg(reinterpret_cast<const uint2*>(p[r] + c));
-                sq[r] = __ldg(s[r] + (c + lane * 8u) / 128u);
-            } else {
-                wq[r].x = __ldg(reinterpret_cast<const uint32_t*>(p[r] + c / 2u));
-                sq[r] = __ldg(s[r] + (c + lane * 8u) / 32u);
-            }
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(ring + ((slot * RW + r) * 32u + lane) * kWords);
+            if (FP8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(p[r] + c) : "memory");
+            else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(p[r] + c / 2u) : "memory");
         }
     };
+    auto scales = [&](uint32_t c) {
+#pragma unroll
+        for (int r = 0; r < RW; ++r) sq[r] = __ldg(s[r] + (c + lane * 8u) / (FP8 ? 128u : 32u));
+    };
     const uint32_t end = K > lane * 8u ? K - lane * 8u : 0u;   // this lane's columns start below K
-    if (end) load(0);
+#pragma unroll
+    for (uint32_t i = 0; i < kDsv4Ahead; ++i) {
+        if (256u * i < end) fetch(i, 256u * i);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    if (end) scales(0);
+    uint32_t slot = 0;
     for (uint32_t c = 0; c < end; c += 256u) {
         float xv[NTOK][8];
 #pragma unroll
@@ -226,11 +236,20 @@ __device__ __forceinline__ void dsv4_rows(const Dsv4Args& a, uint32_t g, uint32_
             xv[k][0] = xa.x; xv[k][1] = xa.y; xv[k][2] = xa.z; xv[k][3] = xa.w;
             xv[k][4] = xb.x; xv[k][5] = xb.y; xv[k][6] = xb.z; xv[k][7] = xb.w;
         }
+        asm volatile("cp.async.wait_group %0;" ::"n"(kDsv4Ahead - 1u) : "memory");
         uint2 w[RW];
         uint32_t sb[RW];
 #pragma unroll
-        for (int r = 0; r < RW; ++r) { w[r] = wq[r]; sb[r] = sq[r]; }
-        if (c + 256u < end) load(c + 256u);
+        for (int r = 0; r < RW; ++r) {
+            const volatile uint32_t* at = ring + ((slot * RW + r) * 32u + lane) * kWords;
+            w[r].x = at[0];
+            if (FP8) w[r].y = at[1];
+            sb[r] = sq[r];
+        }
+        if (c + 256u * kDsv4Ahead < end) fetch(slot, c + 256u * kDsv4Ahead);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        slot = slot + 1u == kDsv4Ahead ? 0u : slot + 1u;
+        if (c + 256u < end) scales(c + 256u);
 #pragma unroll
         for (int r = 0; r < RW; ++r) {
             float wv[8];
@@ -288,6 +307,7 @@ __device__ __forceinline__ void dsv4_rows(const Dsv4Args& a, uint32_t g, uint32_
 // small step with nothing else (4 tokens of 4096 x 2048 x 256 experts, 22 with rows: 0.86 ms per step before).
 template <bool DUAL, bool FP8>
 __global__ void __launch_bounds__(kDsv4Warps * 32, kDsv4Ctas) dsv4_rows_kernel(Dsv4Args a) {
+    __shared__ __align__(16) uint32_t rings[kDsv4Warps][kDsv4Ahead * 4u * 32u * (FP8 ? 2u : 1u)];   // one per warp
     __shared__ uint16_t list[kDsv4MaxGroups];
     __shared__ uint32_t warp_base[kDsv4Warps + 1];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -328,10 +348,10 @@ __global__ void __launch_bounds__(kDsv4Warps * 32, kDsv4Ctas) dsv4_rows_kernel(D
             for (uint32_t tb = 0; tb < cnt;) {
                 const uint32_t left = cnt - tb;
                 if (left == 1u) {
-                    dsv4_rows<DUAL, FP8, 4, 1>(a, g, row, (size_t)row0 + tb, 1u, two_step, lane, bad);
+                    dsv4_rows<DUAL, FP8, 4, 1>(a, g, row, (size_t)row0 + tb, 1u, two_step, lane, rings[warp], bad);
                     tb += 1u;
                 } else {
-                    dsv4_rows<DUAL, FP8, 4, 2>(a, g, row, (size_t)row0 + tb, min(2u, left), two_step, lane, bad);
+                    dsv4_rows<DUAL, FP8, 4, 2>(a, g, row, (size_t)row0 + tb, min(2u, left), two_step, lane, rings[warp], bad);
                     tb += 2u;
                 }
             }
