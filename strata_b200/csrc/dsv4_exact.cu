@@ -165,7 +165,7 @@ struct Dsv4Args {
     const uint32_t* tiny;      // nonzero: activations so small or large were seen that x * w may round or overflow (or nullptr: assume so)
 };
 
-constexpr uint32_t kDsv4Warps = 4, kDsv4Ctas = 3;   // warps per CTA, CTAs per SM (170 registers a thread: no spills)
+constexpr uint32_t kDsv4Warps = 4, kDsv4Ctas = 4;   // warps per CTA, CTAs per SM (128 registers a thread: a few spills with two token rows, made up for by a third more warps)
 constexpr uint32_t kDsv4MaxGroups = 1024;
 constexpr uint32_t kDsv4Ahead = 8;      // steps of 256 columns that the weight copies run ahead
 
@@ -225,17 +225,28 @@ __device__ __forceinline__ void dsv4_rows(const Dsv4Args& a, uint32_t g, uint32_
         if (256u * i < end) fetch(i, 256u * i);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
+    // the token rows (from L1 and L2) are requested a step ahead as well where registers allow it: one row
+    constexpr bool kNext = NTOK == 1;
+    float4 xa[NTOK], xb[NTOK];
+    auto tokens = [&](uint32_t c) {
+#pragma unroll
+        for (int k = 0; k < NTOK; ++k) {
+            xa[k] = __ldg(reinterpret_cast<const float4*>(xr[k] + c));
+            xb[k] = __ldg(reinterpret_cast<const float4*>(xr[k] + c) + 1);
+        }
+    };
     if (end) scales(0);
+    if (kNext && end) tokens(0);
     uint32_t slot = 0;
     for (uint32_t c = 0; c < end; c += 256u) {
         float xv[NTOK][8];
+        if (!kNext) tokens(c);
 #pragma unroll
         for (int k = 0; k < NTOK; ++k) {
-            const float4 xa = __ldg(reinterpret_cast<const float4*>(xr[k] + c));
-            const float4 xb = __ldg(reinterpret_cast<const float4*>(xr[k] + c) + 1);
-            xv[k][0] = xa.x; xv[k][1] = xa.y; xv[k][2] = xa.z; xv[k][3] = xa.w;
-            xv[k][4] = xb.x; xv[k][5] = xb.y; xv[k][6] = xb.z; xv[k][7] = xb.w;
+            xv[k][0] = xa[k].x; xv[k][1] = xa[k].y; xv[k][2] = xa[k].z; xv[k][3] = xa[k].w;
+            xv[k][4] = xb[k].x; xv[k][5] = xb[k].y; xv[k][6] = xb[k].z; xv[k][7] = xb[k].w;
         }
+        if (kNext && c + 256u < end) tokens(c + 256u);
         asm volatile("cp.async.wait_group %0;" ::"n"(kDsv4Ahead - 1u) : "memory");
         uint2 w[RW];
         uint32_t sb[RW];
