@@ -563,9 +563,10 @@ bool use_pair_tiles(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups
 
 // FP4 calls on the digit planes: up to 24 rows per expert on average (one full row tile) and up to 384 tokens, the most that a
 // skewed router can give one expert, whose weights are read again for every 24 rows.  Whole layers, planes / the paths
-// above (L2 flushed): 4096 x 2048 x 256 MXFP4, top-6, 1 token 72 / 78 us, 8 tokens 158 / 186, 64 tokens 475 / 690, 256 tokens 641 /
-// 925; 3072 x 1024 x 256 NVFP4, top-10, 8 tokens 129 / 150, 256 tokens 340 / 430, 384 tokens 387 / 438, 1024 tokens (40 rows) 614 /
-// 504; 7168 x 1024 x 896 MXFP4 under Zipf, top-16, 64 tokens 297 / 385, 256 tokens 561 / 606, 1024 tokens 1577 / 973.
+// above (L2 flushed): 4096 x 2048 x 256 MXFP4, top-6, 1 token 51 / 78 us, 8 tokens 141 / 186, 64 tokens 481 / 690, 256 tokens 616 /
+// 925; 3072 x 1024 x 256 NVFP4, top-10, 8 tokens 127 / 150, 256 tokens 315 / 430, 384 tokens 358 / 438, 1024 tokens (40 rows) 614 /
+// 504; 7168 x 1024 x 896 MXFP4 under Zipf, top-16, 64 tokens 287 / 385, 256 tokens 535 / 606, 384 tokens 696 / 713, 1024 tokens
+// 1577 / 973.
 bool use_planes(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups, uint32_t max_rows) {
     if (!L->planes_ok || pairs > L->plane_rows) return false;
     if (L->knobs.planes_max_rows >= 0) return (uint64_t)pairs <= (uint64_t)L->knobs.planes_max_rows * n_groups;
@@ -796,7 +797,7 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
             p.tile_rows = max_rows <= 8u ? 8u : (max_rows <= 16u ? 16u : 24u);
         } else {
             // 24 rows per tile; 16, with a deeper weight ring, where groups of more are rare whatever the router (4096 x 2048 x 256,
-            // 64 tokens: 475 us with 16, 485 with 24; 256 tokens under Zipf, 7168 x 1024 x 896: 598 / 561)
+            // 64 tokens: 481 us with 16, 485 with 24; 256 tokens under Zipf, 7168 x 1024 x 896: 571 / 535)
             p.tile_rows = L->knobs.planes_tile ? (uint32_t)L->knobs.planes_tile : pairs <= 4u * n_groups && max_rows <= 128u ? 16u : 24u;
             p.tile_table = static_cast<uint32_t*>(L->prefill_scratch);
             launch_tile_list(offsets, n_groups, static_cast<uint32_t*>(L->prefill_scratch), p.tile_rows, s);

@@ -9,6 +9,9 @@
 // rows of the N operand with one common set of block scales 2^b, and the epilogue adds the eight accumulators with the
 // factors 8^-t.  The products are exact, the sums are the tensor core's FP32 accumulation.
 //
+// Measured (gate/up of 4096 x 2048 x 256 MXFP4 experts, L2 flushed): 256 tokens 360 us, 6.3 TB/s; 8 tokens 77 us, 5.0 TB/s, the
+// last round of tiles and the ramp being the rest.  The kernels that decode: ring 82 us at 8 tokens, tiles 3.5 TB/s.
+//
 // What bounds it: HBM, the packed weights, read once.  An M = 128, N = 8 rows, K = 64 instruction takes N / 2 clocks for
 // 4 KB of weights, which HBM delivers to an SM in 178 clocks: up to 24 rows (N = 192) the tensor pipe keeps up, and a
 // second pass over a larger group's weights still costs less than the decode that the f16 tiles pay.
@@ -47,7 +50,7 @@ constexpr uint32_t kSfTile = kMT * 16u;          // scales of 128 weight rows, 1
 constexpr uint32_t kSfStages = 4;
 constexpr uint32_t kMaxCols = 8192;
 constexpr uint32_t kSfBufs = 2;                  // scale buffers in tensor memory
-constexpr uint32_t kSfWarp0 = 2, kEpiWarp0 = 6, kEpiWarps = 8;
+constexpr uint32_t kEpiWarp0 = 6, kEpiWarps = 8;
 constexpr uint32_t kPThreads = (kEpiWarp0 + kEpiWarps) * 32;
 
 // R: most token rows per tile.
