@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "tile_sizes.h"
 
 using namespace smoe;
 
@@ -101,15 +102,14 @@ static LayerKnobs read_knobs() {
     k.no_prefill_path = getenv("STRATA_MOE_NO_PREFILL_PATH") != nullptr;
     k.no_stream_ring = getenv("STRATA_MOE_NO_STREAM_RING") != nullptr;
     k.planes_max_rows = num("STRATA_MOE_PLANES_MAX_ROWS", -1);
-    k.planes_tile = num("STRATA_MOE_PLANES_TILE", 0);
+    k.planes_tile = existing_tile(num("STRATA_MOE_PLANES_TILE", 0), kPlaneTileSizes);
     // a switch that chooses among the other expert kernels asks for them
     for (const char* name : {"STRATA_MOE_NO_F16_PATH", "STRATA_MOE_NO_PREFILL_PATH", "STRATA_MOE_NO_STREAM_RING", "STRATA_MOE_STREAM_RING_MAX_ROWS",
                              "STRATA_MOE_PREFILL_MIN_ROWS", "STRATA_MOE_PREFILL_NTILE", "STRATA_MOE_PAIR_NTILE", "STRATA_MOE_NO_PAIR_TILES"})
         if (k.planes_max_rows < 0 && getenv(name)) k.planes_max_rows = 0;
     k.prefill_min_rows = num("STRATA_MOE_PREFILL_MIN_ROWS", -1);
     k.prefill_ntile = num("STRATA_MOE_PREFILL_NTILE", 0);
-    const int pair_rows = num("STRATA_MOE_PAIR_NTILE", 0);     // the tile sizes there are: the tile list has room for no smaller ones
-    k.pair_ntile = pair_rows <= 0 ? 0 : (pair_rows <= 16 ? 16 : (pair_rows <= 32 ? 32 : 64));
+    k.pair_ntile = existing_tile(num("STRATA_MOE_PAIR_NTILE", 0), kPairTileSizes);
     k.no_small_front = getenv("STRATA_MOE_NO_SMALL_FRONT") != nullptr;
     k.no_pair_tiles = getenv("STRATA_MOE_NO_PAIR_TILES") != nullptr;
     k.no_half_y = getenv("STRATA_MOE_NO_HALF_Y") != nullptr;
@@ -800,7 +800,8 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
             // 64 tokens: 481 us with 16, 485 with 24; 256 tokens under Zipf, 7168 x 1024 x 896: 571 / 535)
             p.tile_rows = L->knobs.planes_tile ? (uint32_t)L->knobs.planes_tile : pairs <= 4u * n_groups && max_rows <= 128u ? 16u : 24u;
             p.tile_table = static_cast<uint32_t*>(L->prefill_scratch);
-            launch_tile_list(offsets, n_groups, static_cast<uint32_t*>(L->prefill_scratch), p.tile_rows, s);
+            if (launch_tile_list(offsets, n_groups, static_cast<uint32_t*>(L->prefill_scratch), p.tile_rows, s) != 0)
+                return fail(ctx, STRATA_MOE_E_CUDA, "plane tile list launch failed");
         }
         p.planes = reinterpret_cast<const uint8_t*>(L->y);
         p.x_scales = reinterpret_cast<const uint8_t*>(L->xg);

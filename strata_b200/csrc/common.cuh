@@ -196,7 +196,7 @@ int prefill_encode_weight_map(void* out128, const void* packed, uint32_t rows, u
 int launch_prefill_bf16(const PrefillArgs& a, const void* x, uint32_t rows, const void* w_gate, const void* w_up,
                         const void* w_down, void* act, uint32_t rows_cap, cudaStream_t s);
 // Tile list of a grouped launch: scratch of prefill_scratch_bytes() at `table`, `rows` (16 .. 192) token rows per tile.
-void launch_tile_list(const uint32_t* offsets, uint32_t n_groups, uint32_t* table, uint32_t rows, cudaStream_t s);
+int launch_tile_list(const uint32_t* offsets, uint32_t n_groups, uint32_t* table, uint32_t rows, cudaStream_t s);
 // fp4_planes.cu : FP4 weights on the block-scaled tensor-core instructions, activations as E2M1 digit planes
 struct PlaneArgs {
     uint32_t H, I, n_groups;

@@ -515,9 +515,12 @@ int launch_planes_one(const PlaneArgs& a, const void* wmaps, const void* smaps, 
 }
 template <int FMT, bool GU>
 int launch_planes_rows(const PlaneArgs& a, const void* wmaps, const void* smaps, cudaStream_t s) {
-    if (a.tile_rows <= 8u) return launch_planes_one<FMT, GU, 8>(a, wmaps, smaps, s);
-    if (a.tile_rows <= 16u) return launch_planes_one<FMT, GU, 16>(a, wmaps, smaps, s);
-    return launch_planes_one<FMT, GU, 24>(a, wmaps, smaps, s);
+    switch (a.tile_rows) {      // a tile of more rows than the kernel's stages hold would be copied past their end
+        case 8u: return launch_planes_one<FMT, GU, 8>(a, wmaps, smaps, s);
+        case 16u: return launch_planes_one<FMT, GU, 16>(a, wmaps, smaps, s);
+        case 24u: return launch_planes_one<FMT, GU, 24>(a, wmaps, smaps, s);
+        default: return -1;
+    }
 }
 
 template <int FMT>

@@ -854,11 +854,13 @@ static int launch_one(const PrefillArgs& a, const void* b_hi, const void* b_lo, 
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-void launch_tile_list(const uint32_t* offsets, uint32_t n_groups, uint32_t* table, uint32_t rows, cudaStream_t s) {
-    launch_behind(prefill_tiles_kernel, 1, 1024, 0, s, offsets, n_groups, table, rows);
+int launch_tile_list(const uint32_t* offsets, uint32_t n_groups, uint32_t* table, uint32_t rows, cudaStream_t s) {
+    if (rows < kMinTileRows) return -1;      // more tiles than the list has room for
+    const cudaError_t e = launch_behind(prefill_tiles_kernel, 1, 1024, 0, s, offsets, n_groups, table, rows);
     ++g_kernel_launches;
+    return e == cudaSuccess ? 0 : -3;
 }
-static void launch_tiles(const PrefillArgs& a, cudaStream_t s) { launch_tile_list(a.offsets, a.n_groups, a.tile_table, a.ntile, s); }
+static int launch_tiles(const PrefillArgs& a, cudaStream_t s) { return launch_tile_list(a.offsets, a.n_groups, a.tile_table, a.ntile, s); }
 
 // Operands of the gate/up or the down launch beside PrefillArgs.
 struct Operands {
@@ -926,14 +928,15 @@ static PrefillArgs with_tile(PrefillArgs a, bool split) {
 int launch_prefill_gate_up(const PrefillArgs& args, const void* x16, const float* x_rowscale, void* act16,
                            uint32_t pairs_cap, const void* wmaps, cudaStream_t s) {
     const PrefillArgs a = with_tile(args, args.act_lo != nullptr);
-    launch_tiles(a, s);
+    if (const int rc = launch_tiles(a, s)) return rc;
     return gate_up_any(a, Operands{x16, nullptr, pairs_cap, nullptr, nullptr, x_rowscale, act16, wmaps}, s);
 }
 
 int launch_prefill_down(const PrefillArgs& args, const void* act16, const float* act_rowscale, uint32_t pairs_cap,
                         const void* wmaps, cudaStream_t s) {
     const PrefillArgs a = with_tile(args, args.act_lo != nullptr);
-    if (!a.reuse_tiles) launch_tiles(a, s);
+    if (!a.reuse_tiles)
+        if (const int rc = launch_tiles(a, s)) return rc;
     return down_any(a, Operands{act16, a.act_lo, pairs_cap, nullptr, nullptr, act_rowscale, nullptr, wmaps}, s);
 }
 

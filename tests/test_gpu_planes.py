@@ -58,6 +58,18 @@ def test_against_the_oracle(ctx, fmt, H, I, E, k, T):
     ctx.check_canaries()
 
 
+@pytest.mark.parametrize("asked", ["-3", "1", "8", "17", "32", "1000000"])
+def test_tile_switch_takes_existing_sizes_only(ctx, asked, monkeypatch):
+    # a tile list of fewer than 16 rows per tile would outgrow its scratch, one of more than 24 the kernel's stages
+    monkeypatch.setenv("STRATA_MOE_PLANES_TILE", asked)
+    cfg = config(MX, 40, 8, 8)
+    layer = synth.build_layer(cfg, "cuda")
+    ml, out = outputs(ctx, cfg, layer)
+    monkeypatch.delenv("STRATA_MOE_PLANES_TILE")
+    ctx.check_canaries()
+    assert torch.equal(out, outputs(ctx, cfg, layer)[1])
+
+
 @pytest.mark.parametrize("fmt", [MX, NV])
 def test_rows_of_uneven_magnitude(ctx, fmt):
     # a row of zeros, blocks of zeros, one column 2^20 above the rest of its row, a row of the smallest normal numbers, a row
