@@ -175,7 +175,12 @@ int strata_moe_set_shared(strata_moe_layer* layer, int role, const void* weights
  * 1487-1618, src/models/laguna/laguna_runtime.cpp:907-1158, src/models/dsv4/deepseek_runtime.cpp:
  * 6070-6096) including the host-side routing, grouping and combine they wrap around
  * CudaBackend::enqueue_moe.  x_bf16 [T, H] BF16 and out [T, H] fp32 are device pointers.
- * Requires expert_count == experts (single-GPU layer). */
+ * Requires expert_count == experts (single-GPU layer).
+ * Precision: weights as the format defines them, FP32 sums.  FP4 calls of small groups (up to 24 rows per expert on average and
+ * 384 tokens) carry token rows and SwiGLU output to 2^-23 of the largest value of their scale block (32 or 16 columns), rows
+ * with outliers (in a block that is not exact, three quarters of the columns 2^7 or more below its maximum) to 2^-46; other
+ * small calls hold token rows exactly (BF16 down to 2^-32 of the row's maximum) and the SwiGLU output in 22 bits; from 12 (INT4:
+ * 8) rows per expert on the SwiGLU output is one f16. */
 int strata_moe_forward(strata_moe_layer* layer, const void* x_bf16, uint32_t tokens, float* out,
                        const strata_moe_aux* aux);
 /* The same layer AFTER routing: the experts of every token and their routing weights are given

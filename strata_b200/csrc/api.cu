@@ -1,5 +1,6 @@
 // Host side of the C ABI declared in include/strata_moe.h: contexts, resident weights,
 // workspaces and the launch sequence of one MoE layer.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -35,6 +36,8 @@ struct strata_moe_ctx {
     bool pev_valid = false;
     unsigned long long launches_at_create = 0;
     unsigned long long* d_router_rechecks = nullptr;   // tokens the fast router handed to the canonical kernels
+    uint32_t* d_plane_rest = nullptr;  // [2] numbers of the last digit-plane calls whose rows, and whose activation, have remainders
+    uint32_t plane_calls = 0;
     uint32_t* d_dsv4_tiny = nullptr;   // the exact call in flight saw activations outside 2^-120 .. 2^109 (see dsv4_exact.cu)
     uint64_t router_fast_tokens = 0;                    // tokens routed through the fast path
     // handle-based commands (strata_moe_command_*): an internal layer whose expert slots borrow the
@@ -70,7 +73,8 @@ struct DeviceTable {
     std::vector<uint8_t> rescan, inexact;   // INT4, NVFP4: registered since its scales were last looked at; the verdict (INT4: q * scale off f16; NVFP4: a negative or NaN scale)
 };
 
-constexpr uint32_t kMaxPlaneRows = 64;   // average rows per expert that the activation's digit planes have room for
+constexpr uint32_t kMaxPlaneRows = 64;   // average rows per expert that the digit planes have room for
+constexpr uint32_t kPlaneTokens = 384;   // most tokens of a call on the digit planes (see use_planes)
 
 // Tuning and test switches, read from the environment ONCE when a layer is created (never on the
 // per-call path).  -1 / 0 = built-in default.
@@ -570,7 +574,7 @@ bool use_pair_tiles(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups
 bool use_planes(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups, uint32_t max_rows) {
     if (!L->planes_ok || pairs > L->plane_rows) return false;
     if (L->knobs.planes_max_rows >= 0) return (uint64_t)pairs <= (uint64_t)L->knobs.planes_max_rows * n_groups;
-    return max_rows <= 384u && (uint64_t)pairs <= 24ull * n_groups;
+    return max_rows <= kPlaneTokens && (uint64_t)pairs <= 24ull * n_groups;
 }
 
 // The kernels that a call's experts run on.
@@ -779,12 +783,23 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         return 0;
     }
     if (path == ExpertPath::kPlanes) {
-        // The planes of the grouped rows take the place of y until the down projection writes it, their scales that of the f16
-        // rows; the activation's have a workspace, their scales go to act_hi.
+        // The planes of the grouped rows and of their remainders take the place of y until the down projection writes it, their
+        // scales that of the f16 rows.  The activation's planes have a workspace, those of their remainders lie behind y's rows,
+        // their scales go to act_hi.
         const int fmt = L->d.format;
-        const uint32_t H = L->d.hidden, I = L->d.intermediate;
-        if (perm) launch_rows_to_planes(fmt, x_src, false, spread->rows, spread->rows_dev, H, spread->dest, spread->k, bound, L->y, L->xg, L->x_rowscale, x_settled, s);
-        else launch_rows_to_planes(fmt, x_src, false, bound, pairs_dev, H, nullptr, 1, bound, L->y, L->xg, L->x_rowscale, false, s);
+        const bool nv = fmt == STRATA_MOE_FMT_NVFP4;
+        const uint32_t H = L->d.hidden, I = L->d.intermediate, call = ++ctx->plane_calls;
+        auto plane_rows = [&](uint32_t cols, void* planes, void* rest_planes, void* scales, float* factor, uint32_t* any_rest) {
+            uint8_t* at = static_cast<uint8_t*>(scales);      // cols / 16 bytes a row, twice, and a float
+            const size_t bytes = (size_t)bound * (cols / 16u);
+            return PlaneRows{bound, static_cast<uint8_t*>(planes), static_cast<uint8_t*>(rest_planes), at, at + bytes, nv ? factor : nullptr,
+                             reinterpret_cast<float*>(at + 2u * bytes), any_rest, call};
+        };
+        float* behind_y = L->y + (size_t)bound * H;
+        const PlaneRows xr = plane_rows(H, L->y, behind_y, L->xg, L->x_rowscale, ctx->d_plane_rest);
+        const PlaneRows ar = plane_rows(I, L->act_planes, behind_y, L->act_hi, L->act_rowscale, ctx->d_plane_rest + 1);
+        if (perm) launch_rows_to_planes(fmt, x_src, false, spread->rows, spread->rows_dev, H, spread->dest, spread->k, xr, x_settled, s);
+        else launch_rows_to_planes(fmt, x_src, false, bound, pairs_dev, H, nullptr, 1, xr, false, s);
         PlaneArgs p{};
         p.H = H;
         p.I = I;
@@ -803,11 +818,7 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
             if (launch_tile_list(offsets, n_groups, static_cast<uint32_t*>(L->prefill_scratch), p.tile_rows, s) != 0)
                 return fail(ctx, STRATA_MOE_E_CUDA, "plane tile list launch failed");
         }
-        p.planes = reinterpret_cast<const uint8_t*>(L->y);
-        p.x_scales = reinterpret_cast<const uint8_t*>(L->xg);
-        p.plane_rows = bound;
-        const bool nv = fmt == STRATA_MOE_FMT_NVFP4;
-        p.rowscale = nv ? L->x_rowscale : nullptr;
+        p.x = xr;
         p.post0 = nv ? L->tab[0].d_post : nullptr;
         p.post1 = nv ? L->tab[1].d_post : nullptr;
         p.out = L->act_f32;
@@ -817,10 +828,8 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
         if (launch_planes_gate_up(fmt, p, L->d_wmaps, L->d_sfmaps, s) != 0)
             return fail(ctx, STRATA_MOE_E_CUDA, "gate/up plane launch failed");
         mark(ctx, 5);
-        launch_rows_to_planes(fmt, L->act_f32, true, bound, pairs_dev, I, nullptr, 1, bound, L->act_planes, L->act_hi, L->act_rowscale, false, s);
-        p.planes = L->act_planes;
-        p.x_scales = reinterpret_cast<const uint8_t*>(L->act_hi);
-        p.rowscale = nv ? L->act_rowscale : nullptr;
+        launch_rows_to_planes(fmt, L->act_f32, true, bound, pairs_dev, I, nullptr, 1, ar, false, s);
+        p.x = ar;
         p.post0 = p.post1 = nv ? L->tab[2].d_post : nullptr;
         p.out = y;
         if (launch_planes_down(fmt, p, L->d_wmaps, L->d_sfmaps, s) != 0)
@@ -1047,7 +1056,9 @@ int strata_moe_create(int device, void* stream, strata_moe_ctx** out) {
         strata_moe_destroy(ctx);
         return STRATA_MOE_E_CUDA;
     }
-    if (cudaMalloc(&ctx->d_dsv4_tiny, sizeof(uint32_t)) != cudaSuccess) {
+    if (cudaMalloc(&ctx->d_plane_rest, 2 * sizeof(uint32_t)) != cudaSuccess ||
+        cudaMemset(ctx->d_plane_rest, 0, 2 * sizeof(uint32_t)) != cudaSuccess ||
+        cudaMalloc(&ctx->d_dsv4_tiny, sizeof(uint32_t)) != cudaSuccess) {
         strata_moe_destroy(ctx);
         return STRATA_MOE_E_CUDA;
     }
@@ -1079,6 +1090,7 @@ void strata_moe_destroy(strata_moe_ctx* ctx) {
         p = nullptr;
     }
     if (ctx->d_status) cudaFree(ctx->d_status);
+    if (ctx->d_plane_rest) cudaFree(ctx->d_plane_rest);
     if (ctx->d_dsv4_tiny) cudaFree(ctx->d_dsv4_tiny);
     if (ctx->d_router_rechecks) cudaFree(ctx->d_router_rechecks);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
@@ -1245,8 +1257,11 @@ int strata_moe_layer_create(strata_moe_ctx* ctx, const strata_moe_layer_desc* de
     }
     A(ws_reserve(ctx, kWsActF32, (size_t)P * I * 4));
     if (planes_supported(d.format, H, I)) {     // the digit planes serve small groups only
-        L->plane_rows = (uint32_t)((uint64_t)P < (uint64_t)kMaxPlaneRows * n ? (uint64_t)P : (uint64_t)kMaxPlaneRows * n);
+        uint64_t rows = std::min((uint64_t)P, (uint64_t)kMaxPlaneRows * n);
+        if (L->knobs.planes_max_rows < 0) rows = std::min(rows, (uint64_t)kPlaneTokens * d.top_k);
+        L->plane_rows = (uint32_t)rows;
         A(ws_reserve(ctx, kWsActPlanes, (size_t)L->plane_rows * I * 4));
+        A(ws_reserve(ctx, kWsY, (size_t)L->plane_rows * (H + std::max(H, I)) * 4));     // the rows' planes and those of remainders
     }
     A(ws_reserve(ctx, kWsXRow, (size_t)P * 4));
     A(ws_reserve(ctx, kWsActRow, (size_t)P * 4));

@@ -198,6 +198,15 @@ int launch_prefill_bf16(const PrefillArgs& a, const void* x, uint32_t rows, cons
 // Tile list of a grouped launch: scratch of prefill_scratch_bytes() at `table`, `rows` (16 .. 192) token rows per tile.
 int launch_tile_list(const uint32_t* offsets, uint32_t n_groups, uint32_t* table, uint32_t rows, cudaStream_t s);
 // fp4_planes.cu : FP4 weights on the block-scaled tensor-core instructions, activations as E2M1 digit planes
+struct PlaneRows {                 // `rows` plane rows of `cols` columns
+    uint32_t rows;
+    uint8_t *planes, *rest_planes; // cols * 4 bytes a row each; the second of the rows that have a remainder
+    uint8_t *scales, *rest_scales; // cols / 32 (MXFP4) or cols / 16 (NVFP4) bytes a row
+    float* factor;                 // NVFP4: factor of the row; MXFP4: nullptr
+    float* rest_factor;            // factor of the remainder, 0: the row has none
+    uint32_t* any_rest;            // holds `call` when a row has a remainder (a word of an earlier call that is the same by chance
+    uint32_t call;                 // only costs a look at rest_factor)
+};
 struct PlaneArgs {
     uint32_t H, I, n_groups;
     const uint32_t* offsets;       // [n_groups + 1]
@@ -205,9 +214,7 @@ struct PlaneArgs {
     const uint32_t* active_list;   // [n_active], read when there is no tile list
     const uint32_t* n_active;
     uint32_t tile_rows;            // 8, 16 or 24
-    const uint8_t *planes, *x_scales;   // of the grouped rows, as launch_rows_to_planes lays them out
-    uint32_t plane_rows;
-    const float* rowscale;         // factor per row, or nullptr
+    PlaneRows x;                   // of the grouped rows, as launch_rows_to_planes leaves them
     const float *post0, *post1;    // [n_groups] factors of the first and second weight tile, or nullptr
     float* out;                    // act [rows, I] or y [rows, H]
     uint32_t* status;
@@ -215,12 +222,10 @@ struct PlaneArgs {
 };
 bool planes_supported(int fmt, uint32_t H, uint32_t I);
 int planes_encode_scale_map(void* out128, int fmt, const void* scales, uint32_t rows, uint32_t K);
-// rows of `cols` BF16 (or FP32) values -> planes (cols * 4 bytes per plane row), scales (cols / 32 or cols / 16), rowscale (NVFP4);
-// source row r goes to plane rows dest[r * k .. r * k + k - 1], or to plane row r.  settled: src was written before the kernel that
-// precedes this one in the stream started.
+// rows of `cols` BF16 (or FP32) values -> `out`; source row r goes to plane rows dest[r * k .. r * k + k - 1], or to plane row r.
+// settled: src was written before the kernel that precedes this one in the stream started.
 void launch_rows_to_planes(int fmt, const void* src, bool f32, uint32_t rows, const uint32_t* rows_dev, uint32_t cols,
-                           const uint32_t* dest, uint32_t k, uint32_t plane_rows, void* planes, void* scales, float* rowscale,
-                           bool settled, cudaStream_t s);
+                           const uint32_t* dest, uint32_t k, const PlaneRows& out, bool settled, cudaStream_t s);
 int launch_planes_gate_up(int fmt, const PlaneArgs& a, const void* wmaps, const void* smaps, cudaStream_t s);
 int launch_planes_down(int fmt, const PlaneArgs& a, const void* wmaps, const void* smaps, cudaStream_t s);
 // Router projection on the tensor cores (approximate summation order; see router.cu for its use).

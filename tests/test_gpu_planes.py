@@ -91,6 +91,57 @@ def test_rows_of_uneven_magnitude(ctx, fmt):
         assert rel <= TOL, (t, rel)
 
 
+# An outlier whose weight is zero must not be seen in any output: the digits of its block, fixed point against its maximum, hold
+# the rest of the block to 2^-23 of the outlier only, the remainder holds what they leave.  Groups of T rows at the edges of the
+# tiles (8, 16, 24 rows, remainders counted), every row, every third one or one with an outlier; a tile list beyond 24 tokens.
+# Without remainders 4e-6 (2^12) to 4e-3 (2^20) of the output differ; with them the order of FP32 sums is left, about 2e-7.
+EDGES = [(T, step) for T in (1, 4, 5, 8, 12, 13, 18, 24, 25, 49) for step in (1, 3, 100)]
+
+
+def without_column(layer, role, cfg, col):
+    """Zero weights in the byte of column `col` (two columns) of every row of a projection."""
+    rows, cols = cfg.role_shape(role)
+    layer.packed[role].view(cfg.E, rows, cols // 2)[:, :, col // 2] = 0
+
+
+@pytest.mark.parametrize("fmt", [MX, NV])
+@pytest.mark.parametrize("T,step", EDGES)
+def test_token_outlier_of_zero_weight(ctx, fmt, T, step):
+    cfg = config(fmt, T, 2, 2)
+    layer = synth.build_layer(cfg, "cuda")
+    for role in ("gate", "up"):
+        without_column(layer, role, cfg, 76)
+    layer.router_w[:, 76:78] = 0
+    x = layer.x.clone()
+    x[:, 76:78] = 0
+    _, want = outputs(ctx, cfg, layer, x)
+    for t in range(0, T, step):
+        x[t, 77] = 2.0 ** (12, 16, 20)[t // step % 3]
+    _, got = outputs(ctx, cfg, layer, x)
+    for t in range(T):
+        assert float((got[t] - want[t]).norm() / want[t].norm()) <= 1e-6, t
+    ctx.check_canaries()
+
+
+@pytest.mark.parametrize("fmt", [MX, NV])
+@pytest.mark.parametrize("T", [1, 5, 13, 24, 49])
+def test_activation_outlier_of_zero_weight(ctx, fmt, T):
+    # one feature of every expert whose gate and up rows are 2^5 times the others', under a zero column of the down projection
+    cfg = config(fmt, T, 2, 2)
+    layer = synth.build_layer(cfg, "cuda")
+    without_column(layer, "down", cfg, 76)
+    _, want = outputs(ctx, cfg, layer)
+    for role in ("gate", "up"):
+        rows, cols = cfg.role_shape(role)
+        s = layer.scales[role].view(cfg.E, rows, -1)
+        s[:, 77] += 5 if fmt == MX else 5 << 3      # exponent fields
+        assert fmt == MX or int(s[:, 77].max()) < 0x7F
+    _, got = outputs(ctx, cfg, layer)
+    for t in range(T):
+        assert float((got[t] - want[t]).norm() / want[t].norm()) <= 1e-6, t
+    ctx.check_canaries()
+
+
 @pytest.mark.parametrize("fmt", [MX, NV])
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
 def test_rows_that_are_not_finite_are_reported(ctx, fmt, value):
