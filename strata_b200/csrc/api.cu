@@ -1763,11 +1763,17 @@ int strata_moe_forward_host(strata_moe_layer* L, const void* x_host, uint32_t T,
     }
     if (parts > 4u) parts = 4u;
     if (parts > T) parts = T;
-    // only while every chunk stays on the expert path the whole batch would take (the tensor-core path): the paths
-    // round the SwiGLU output differently, and the chunked call must return the one-piece call's bits
-    while (parts > 1u && !(use_prefill(L, T * L->d.top_k, L->d.experts) &&
-                           use_prefill(L, (T / parts) * L->d.top_k, L->d.experts)))
-        --parts;
+    // only while the whole batch and every chunk run on the f16 tiles: the paths round the SwiGLU output differently, and the
+    // chunked call must return the one-piece call's bits (600 tokens of 32 FP4 experts, top-4: 75 rows per expert on the tiles,
+    // a quarter of them on the digit planes)
+    if (parts > 1u) {
+        const int rc = sync_tables(L);
+        if (rc) return rc;
+    }
+    auto on_tiles = [&](uint32_t tokens) {
+        return expert_path(L, tokens * L->d.top_k, L->d.experts, tokens, true) == ExpertPath::kTiles;
+    };
+    while (parts > 1u && !(on_tiles(T) && on_tiles(T / parts) && on_tiles((T + parts - 1u) / parts))) --parts;
     if (parts > 1u || T * out_row >= kColumnBlockBytes) {
         if (!ctx->copy_in) {
             CK(cudaStreamCreateWithFlags(&ctx->copy_in, cudaStreamNonBlocking));
