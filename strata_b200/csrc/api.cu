@@ -1573,6 +1573,19 @@ int strata_moe_combine(strata_moe_layer* L, const float* y, const uint32_t* inv,
     return 0;
 }
 
+// Page-locked from end to end, as far as its first and last bytes tell.
+static bool page_locked(const void* p, size_t bytes) {
+    for (const uint8_t* at : {static_cast<const uint8_t*>(p), static_cast<const uint8_t*>(p) + bytes - 1}) {
+        cudaPointerAttributes attr{};
+        if (cudaPointerGetAttributes(&attr, at) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (attr.type != cudaMemoryTypeHost) return false;
+    }
+    return true;
+}
+
 // column_blocks > 1 (only for calls on the large-batch tiles, whose kernels it cuts): the output comes in that many blocks of
 // columns, `block_done` is called behind each.
 static int forward_layer(strata_moe_layer* L, const void* x, uint32_t T, float* out, const strata_moe_aux* aux,
@@ -1788,10 +1801,12 @@ int strata_moe_forward_host(strata_moe_layer* L, const void* x_host, uint32_t T,
         CK(cudaMemcpyAsync(L->x_stage, x_host, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
         // A large result goes out in four blocks of columns: a block's copy runs beside the down projection of the next ones.
         // Columns are independent and keep their tiles, so the bits are those of the one-piece call (4096 tokens of c2: the 100 MB
-        // of the result, 1.9 ms of copy, start 0.6 ms earlier).  Below 16 MB the copy is shorter than what more launches cost.
+        // of the result, 1.9 ms of copy, start 0.6 ms earlier).  Below 16 MB the copy is shorter than what more launches cost.  Pageable
+        // memory takes the result in one piece: its copies run beside nothing (6144 columns, 1024 tokens: 2.6 - 2.9 ms in one piece,
+        // 2.8 - 3.4 in blocks, from 2048 tokens on the same within the runs' spread; page-locked 1.43 / 1.28).
         uint32_t blocks = 1u;
         if (T * out_row >= kColumnBlockBytes && H % 1024u == 0u && !ctx->timing && L->knobs.host_chunks == 0 &&
-            sync_tables(L) == 0 && expert_path(L, T * L->d.top_k, L->d.experts, T, true) == ExpertPath::kTiles)
+            page_locked(out_host, out_bytes) && sync_tables(L) == 0 && expert_path(L, T * L->d.top_k, L->d.experts, T, true) == ExpertPath::kTiles)
             blocks = 4u;
         uint32_t sent = 0;
         int rc = forward_layer(L, L->x_stage, T, L->out_stage, nullptr, blocks, [&](uint32_t col0, uint32_t cols) -> int {
