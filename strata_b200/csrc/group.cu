@@ -13,11 +13,14 @@
 namespace smoe {
 
 constexpr uint32_t kSegPairs = 128;   // pairs per warp segment
-constexpr uint32_t kSmallPairs = 8192; // single-CTA path up to this many pairs: eight rounds of 32 per warp
+// Single-CTA path up to this many pairs, eight rounds of 32 per warp.  The rounds are serial, the four kernels of the large path cost
+// the same at any of these sizes, most of it the gaps between them (calls in a stream, one CTA / four kernels: 8 experts 8192 pairs
+// 10 / 18 us, 256 experts 5000 pairs 16 / 20, 8192 pairs 22.7 / 21).  Replayed as a graph, with shorter gaps, they meet at 4500.
+constexpr uint32_t kSmallPairs = 8192;
 
 // ---- small path: one CTA does everything ---------------------------------------------------
 // A warp owns a run of consecutive pairs and ranks them against its own earlier ones (a table of counts per warp and
-// expert), one thread per expert turns the warps' counts into bases, a shuffle scan over the experts gives the offsets: eight
+// expert), one thread per expert turns the warps' counts into bases, a shuffle scan over the experts gives the offsets: five
 // block barriers whatever the number of pairs.  (Ranking the warps in turn, a barrier each, and scanning through shared
 // memory took 20 us for 1536 pairs of 256 experts; four kernels of the large path take 18 us with the gaps between them.)
 __global__ void __launch_bounds__(1024) group_small_kernel(
