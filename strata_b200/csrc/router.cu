@@ -1019,7 +1019,11 @@ bool launch_router_logits_small(const __nv_bfloat16* x, const __nv_bfloat16* wg,
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return false;
     const size_t smem_pair = 128u + (size_t)(kPairRows + T) * (H * 2u + kSmallPad);
-    if (T <= kSmallMaxTokens && smem_pair <= kPairSmem) {
+    // The pair kernel's CTAs each fetch all token rows: E / 2 times T rows, where the eight-row CTAs below need a quarter of it.  That
+    // shows where experts and tokens are many and columns, over which a CTA's set-up pays, are few (pair / eight rows: 1024 experts
+    // of 512 columns, 16 tokens 20.2 / 16.0 us, 896 of 1024, 12 tokens 18.0 / 16.6, 512 of 1024, 12 tokens 0.96 of it, 128 of 512, 12
+    // tokens equal, 16 tokens 8.4 / 7.9; 896 of 4096, 10 tokens 0.84 of it, 256 of 4096, 8 tokens half).
+    if (T <= kSmallMaxTokens && smem_pair <= kPairSmem && T * E <= 6u * H && T <= 8u + H / 128u) {
         static bool pair_attr[64] = {};
         if (!pair_attr[dev]) {
             if (cudaFuncSetAttribute(router_logits_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem) != cudaSuccess)
