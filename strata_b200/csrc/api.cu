@@ -683,7 +683,7 @@ struct ColumnBlocks {
 };
 
 // Expert FFN over grouped rows.  x_nat: rows in natural column order (group order).
-// If x_kperm is non-null it already holds the K-permuted copy.
+// perm: grouped row -> source row times k_div, or null (x_src is grouped); with it comes `spread`, the same the other way round.
 int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t* perm, uint32_t k_div,
                 uint32_t pairs, uint32_t n_groups, const uint32_t* offsets, const uint32_t* active,
                 const uint32_t* n_active, uint32_t max_rows, float* y, uint32_t expected_pairs = 0,
@@ -709,8 +709,10 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
             launch_rows_to_f16_bf16(x_src, perm, k_div, bound, L->d.hidden, L->xg, L->x_rowscale, s, pairs_dev, int4);
     };
     ExpertPath path = expert_path(L, pairs, n_groups, max_rows, active != nullptr);
-    if (path == ExpertPath::kPlanes && (bound > L->plane_rows || (perm && !spread)))
+    if (path == ExpertPath::kPlanes && bound > L->plane_rows)
         path = expert_path(L, pairs, n_groups, max_rows, active != nullptr, false);
+    // a caller that leaves the combine to the column blocks must have predicted the path with the same test
+    if (columns && path != ExpertPath::kTiles) return fail(ctx, STRATA_MOE_E_INVALID, "column blocks offered to a path that does not cut them");
     if (path == ExpertPath::kTiles) {
         rows_for_tiles();
         mark(ctx, 4);
@@ -1667,7 +1669,7 @@ static int forward_layer(strata_moe_layer* L, const void* x, uint32_t T, float* 
         return block_done(col0, cols);
     }};
     rc = run_experts(L, xb, perm, d.top_k, P, d.experts, offsets, L->active, L->n_active, T, L->y, 0, nullptr, x_ready,
-                     &y_half, nullptr, d.top_k <= 32u ? &spread : nullptr, true,
+                     &y_half, nullptr, &spread, true,
                      column_blocks > 1u ? &columns : nullptr, front_done);
     if (rc) return rc;
     if (column_blocks > 1u) {
