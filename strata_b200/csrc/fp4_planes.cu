@@ -439,8 +439,12 @@ __device__ __forceinline__ bool plane_roles(const PlaneArgs& a, const CUtensorMa
     return ok;
 }
 
+// Registers: 80 a thread for the smallest tile leave an SM room for a CTA of the shared expert's streaming kernel beside this one
+// and the activation's conversion, which is how a step of few tokens runs.  With the 90 that the remainders' loops ask for (the
+// cap spills 6 bytes there) one of them waited: 1 token of 3072 x 1024 x 256 NVFP4 with the shared expert 63 - 78 us, capped 55, before
+// the remainders 53; 4 tokens 84 - 103, 88, 84.  Larger tiles measured the same with and without.
 template <int FMT, bool GU, int R>
-__global__ void __launch_bounds__(kPThreads, 1)
+__global__ void __maxnreg__(R == 8 ? 80 : 112)
 fp4_planes_kernel(PlaneArgs a, const CUtensorMap* __restrict__ wmaps, const CUtensorMap* __restrict__ smaps /* both [3][n_groups] */) {
     using G = PGeo<R>;
     constexpr uint32_t kFeat = GU ? kMT : 2u * kMT;
