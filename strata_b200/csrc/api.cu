@@ -567,10 +567,12 @@ bool use_pair_tiles(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups
 
 // FP4 calls on the digit planes: up to 24 rows per expert on average (one full row tile) and up to 384 tokens, the most that a
 // skewed router can give one expert, whose weights are read again for every 24 rows.  Whole layers, planes / the paths
-// above (L2 flushed): 4096 x 2048 x 256 MXFP4, top-6, 1 token 51 / 78 us, 8 tokens 141 / 186, 64 tokens 481 / 690, 256 tokens 616 /
-// 925; 3072 x 1024 x 256 NVFP4, top-10, 8 tokens 127 / 150, 256 tokens 315 / 430, 384 tokens 358 / 438, 1024 tokens (40 rows) 614 /
-// 504; 7168 x 1024 x 896 MXFP4 under Zipf, top-16, 64 tokens 287 / 385, 256 tokens 535 / 606, 384 tokens 696 / 713, 1024 tokens
-// 1577 / 973.
+// above (L2 flushed): 4096 x 2048 x 256 MXFP4, top-6, 8 tokens 146 / 180 us, 64 tokens 465 / 701, 256 tokens 629 / 895, 384 tokens
+// 686 / 952, 1024 tokens 926 / 1073; 3072 x 1024 x 256 NVFP4, top-10, 8 tokens 117 / 148, 256 tokens 320 / 422, 384 tokens 365 / 428,
+// 512 tokens 408 / 438, 1024 tokens (40 rows) 670 / 567; 7168 x 1024 x 896 MXFP4 under Zipf, top-16, 64 tokens 291 / 379, 256 tokens
+// 533 / 565, 384 tokens 735 / 731, 512 tokens 997 / 963, 1024 tokens 1634 / 1008.  The host does not know the routing: evenly
+// loaded calls of 385 to about 600 tokens would gain, calls whose tokens all choose the same experts lose from 256 tokens on
+// (the first layer, 128 tokens 172 / 176, 256 tokens 246 / 227, 384 tokens 328 / 287).
 bool use_planes(const strata_moe_layer* L, uint32_t pairs, uint32_t n_groups, uint32_t max_rows) {
     if (!L->planes_ok || pairs > L->plane_rows) return false;
     if (L->knobs.planes_max_rows >= 0) return (uint64_t)pairs <= (uint64_t)L->knobs.planes_max_rows * n_groups;
@@ -813,8 +815,9 @@ int run_experts(strata_moe_layer* L, const __nv_bfloat16* x_src, const uint32_t*
             p.n_active = n_active;
             p.tile_rows = max_rows <= 8u ? 8u : (max_rows <= 16u ? 16u : 24u);
         } else {
-            // 24 rows per tile; 16, with a deeper weight ring, where groups of more are rare whatever the router (4096 x 2048 x 256,
-            // 64 tokens: 481 us with 16, 485 with 24; 256 tokens under Zipf, 7168 x 1024 x 896: 571 / 535)
+            // 24 rows per tile; 16, with a deeper weight ring, where an evenly loaded group has fewer (whole layers, 16 / 24 rows: 4096 x
+            // 2048 x 256, 32 tokens 332 / 338 us, 64 tokens 483 / 494, 128 tokens 576 / 586; 3072 x 1024 x 256 0 - 1 % less; 7168 x 1024 x 896
+            // under Zipf 32 tokens 250 / 256, 64 tokens 293 / 287, 128 tokens 381 / 358, 256 tokens 571 / 535)
             p.tile_rows = L->knobs.planes_tile ? (uint32_t)L->knobs.planes_tile : pairs <= 4u * n_groups && max_rows <= 128u ? 16u : 24u;
             p.tile_table = static_cast<uint32_t*>(L->prefill_scratch);
             if (launch_tile_list(offsets, n_groups, static_cast<uint32_t*>(L->prefill_scratch), p.tile_rows, s) != 0)
@@ -943,7 +946,10 @@ int run_shared(strata_moe_layer* L, const __nv_bfloat16* x, const __nv_bfloat16*
     const uint32_t thr = L->knobs.prefill_min_rows >= 0 ? (uint32_t)L->knobs.prefill_min_rows : 24u;
     // A wide shared expert also for fewer rows, the activation as a BF16 hi + lo pair like that of the streaming kernel: its
     // tiles stream the weights as fast on a third of the SMs and leave the others to the routed path's small kernels beside it
-    // (Kimi's 6144 columns, 48 tiles; the streaming kernel took every SM and the router beside it 61 us instead of 13).
+    // (Kimi's 6144 columns, 48 tiles; the streaming kernel took every SM and the router beside it 61 us instead of 13).  Whole layers of
+    // 32 small experts beside it, tiles / streaming: 1024 columns, 5120 wide, 1 token 55 / 67 us, 23 tokens 62 / 94; 7168, 6144 wide, 100 /
+    // 189 and 150 / 223; beyond one round of tiles too: 148 tiles 207 / 414, 149 tiles 225 / 408, 1024 columns, 32768 wide 195 / 215.  Of
+    // 152 sizes (1024 - 7168 columns, 5120 - 32768 wide, 1 - 23 tokens) none is slower on tiles.
     const bool wide = L->d.shared_intermediate >= 40u * 128u && L->knobs.prefill_min_rows < 0;
     if (!x_lo && (T >= thr || wide) && tensor_path_ok(L, 3, L->d.shared_intermediate)) {
         PrefillArgs p{};

@@ -17,10 +17,11 @@
 // works on four weight rows at once (an activation load serves all of them) and two token rows of
 // the expert share one pass over the weights.  The reduction tree is evaluated in the same order
 // with two shuffle rounds, three in-register rounds and the final three rounds over the eight
-// "warp" sums.  Bound by memory latency (ncu, 4 tokens of 4096 x 2048, 21 experts with rows: gate/up
-// 204 us, down 107 us, DRAM 11 % busy, issue slots 42 %, 2.9 warps per scheduler, nearly half of
-// their time waiting for weight loads): 165 registers leave 12 warps per SM, and each has one
-// 256-column step of four rows, 512 bytes, on the way.
+// "warp" sums.  Bound by instruction issue and latency (ncu, 4 tokens of 4096 x 2048, 21
+// experts with rows: gate/up 156 us, down 83 us, DRAM 15 % busy, issue slots 62 - 64 %, 3.8 warps per
+// scheduler, a fifth of their time waiting for loads of token rows and scales): 128 registers leave 16
+// warps per SM, each with eight 256-column steps of four rows, 4 KB, on the way.  With 165 registers,
+// 12 warps and one step on the way it was 204 us and 107 us, issue slots 42 %.
 #include "common.cuh"
 #include "libm_exact.cuh"
 

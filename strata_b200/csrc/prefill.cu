@@ -173,8 +173,8 @@ __device__ __forceinline__ void p_int4x8_f16(uint32_t w, uint32_t r[4]) {
 // its result has at most eleven significant bits.  2^24 s has to stay below 2^16, and s at or above 2^-14 keeps the products
 // normal numbers (of subnormal ones the MMA keeps fewer bits), so the scales of a projection, times a power of two of its own
 // (WeightTable::emin holds 2^24 of it as a float, post_scale undoes it), lie in [2^-14, 2^-8): six octaves, and the bits of the
-// result are those of the decode above.  6144 x 2048 x 256 experts, whole layer: 4 tokens 268 -> 252 us, 333 tokens 1440 -> 1391,
-// 4096 tokens 2608 -> 2565.
+// result are those of the decode above.  6144 x 2048 x 256 experts, whole layer, in turn: 4 tokens 240 -> 222 us, 333 tokens
+// 1436 -> 1349, 4096 tokens 2559 -> 2514 (2909 -> 2859 once the power cap holds the clock).
 __device__ __forceinline__ void p_int4x8_narrow(uint32_t w, uint32_t m24, uint32_t m20, uint32_t c, uint32_t r[4]) {
     const uint32_t w8 = w >> 8;
     r[0] = p_fma_f16x2(w & 0x000F000Fu, m24, c);
